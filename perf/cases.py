@@ -317,3 +317,89 @@ def tolerance(case):
     if case.get("dtype") == "fp16":
         return {"rel": 2e-3, "max": 0.3}
     return {"rel": 1e-2, "max": 0.5}
+
+
+# ------------------------------------------------------------------------------------------------------------ 64 bits
+MOST_EXACT_FLOPS = 1.2e14      # beyond this the 64-bit computation takes too long
+
+
+def _exact_dense(c, seed):
+    """Softmax attention of the first pass's inputs over every token, and its log2 LSE where the step leaves one."""
+    gen = torch.Generator(device=DEV).manual_seed(seed)
+    qkv = _video_qkv(c, gen, c["branches"])
+    if c["mode"] == "step":
+        for q, k, _ in qkv:                                          # the step before
+            _moved(q, gen), _moved(k, gen)
+    out, lse = [], []
+    for q, k, v in qkv:
+        moved = _moved(q, gen)
+        q = moved if c["mode"] == "step" else q
+        o = torch.empty(q.shape, device=DEV, dtype=torch.float64)
+        l2 = torch.empty(q.shape[1:3], device=DEV, dtype=torch.float64)
+        for h in range(q.shape[2]):
+            kh, vh = k[0, :, h].double(), v[0, :, h].double()
+            for r in range(0, q.shape[1], 4096):
+                s = q[0, r: r + 4096, h].double() @ kh.t() / math.sqrt(128.0)
+                l = torch.logsumexp(s, 1)
+                l2[r: r + 4096, h] = l / math.log(2.0)
+                o[0, r: r + 4096, h] = s.sub_(l[:, None]).exp_() @ vh
+        out.append(o)
+        lse.append(l2)
+    keeps = c["mode"] == "step" and -(-_tokens(c) // 64) >= 64
+    return dict(out=out, lse=lse if keeps else [])
+
+
+def _exact_frozen(c, seed):
+    """Fine attention over the selected blocks plus tanh(gate) (1 without a gate) times the attention of the block means,
+    and the gradients; one (sample, head) and a slab of query blocks at a time."""
+    s = _prepare_vsa(c, seed)
+    q, k, v, gate, cnt, sel = s["q"], s["k"], s["v"], s["gate"], s["cnt"].long(), s["sel"]
+    B, H, L, D = q.shape
+    nb = L // 64
+    ok = (torch.arange(64, device=DEV)[None] < cnt[:, None]).reshape(L).double()
+    leaves = [x for x in (q, k, v, gate) if x is not None]
+    o = torch.zeros(B, H, L, D, device=DEV, dtype=torch.float64)
+    grads = [torch.zeros(x.shape, device=DEV, dtype=torch.float64) for x in leaves]
+    for bh in range(B * H):
+        b, h = divmod(bh, H)
+        x = [t[b, h].detach().double().requires_grad_(c["backward"]) for t in leaves]
+        mean = [(t * ok[:, None]).reshape(nb, 64, D).sum(1) / cnt[:, None] for t in x[:3]]
+        coarse = torch.softmax(mean[0] @ mean[1].t() / math.sqrt(D), 1) @ mean[2]
+        cut = coarse.detach().requires_grad_(c["backward"])
+        ptr = sel.q2k_ptr[b, h].long()
+        mask = torch.zeros(nb, nb, device=DEV, dtype=torch.bool)
+        mask[torch.repeat_interleave(torch.arange(nb, device=DEV), ptr[1:] - ptr[:-1]),
+             sel.q2k_idx[int(ptr[0]): int(ptr[-1])].long()] = True
+        for i in range(0, nb, 32):
+            r = slice(64 * i, min(64 * (i + 32), L))
+            keep = mask[i: i + 32].repeat_interleave(64, 0).repeat_interleave(64, 1) & (ok > 0)[None]
+            some = keep.any(1)
+            a = (x[0][r] @ x[1].t() / math.sqrt(D)).masked_fill(~keep, -math.inf)
+            fine = torch.softmax(a.masked_fill(~some[:, None], 0.0), 1).masked_fill(~some[:, None], 0.0) @ x[2]
+            if gate is None:
+                w = 1.0
+            else:
+                w = torch.tanh(x[3][r])
+                w = w[:, None] if w.dim() == 1 else w
+            y = (fine + w * cut[i: i + 32].repeat_interleave(64, 0)) * ok[r, None]
+            o[b, h, r] = y.detach()
+            if c["backward"]:
+                y.backward(s["dout"][b, h, r].double())
+        if c["backward"]:
+            coarse.backward(cut.grad)
+            for g, t in zip(grads, x):
+                g[b, h] = t.grad
+    return dict(o=o, grads=grads) if c["backward"] else dict(o=o)
+
+
+def exact(case, seed):
+    """What `run` returns on a fresh state, in 64 bits. A step or a routing whose block choice hangs on rounded scores has no
+    such value."""
+    c = case
+    if c["kind"] == "dense" and 4.0 * 128 * _tokens(c) ** 2 * c["heads"] * c["branches"] < MOST_EXACT_FLOPS:
+        return _exact_dense(c, seed)
+    if c["kind"] == "vsa" and c["mode"] == "frozen":
+        L = 64 * _blocks((c["t"], c["h"], c["w"]))
+        if 14.0 * c["dim"] * L ** 2 * c["batch"] * c["heads"] < MOST_EXACT_FLOPS:
+            return _exact_frozen(c, seed)
+    return None
