@@ -66,6 +66,11 @@ int es_sparse_attention(const void* q, const void* k, const void* v, const void*
                         const void* k_rep, const void* v_rep, const float* log_counts, float* mass, int32_t L, int32_t H,
                         float threshold, void* stream);
 
+/* Online-softmax attention over every block, of every tile: out (L, H, 128) bf16 and the log2 LSE, (ceil(L / 128) * 128, H) with
+ * 1e30 in the rows past L. The same attention as es_exact_fallback with every flag set and every block listed, in one sweep
+ * of the keys where that takes two (rounding differs); no lists and no scratch. */
+int es_dense_attention(const void* q, const void* k, const void* v, void* out, float* lse, int32_t L, int32_t H, void* stream);
+
 /* Online-softmax attention over the block list for the tiles whose flag is set; writes out and lse of those tiles.
  * Replaces echosparse/kernels/triton_ops.py:237 `exact_fallback(q, k, v, out, counts, blocks, lse, flags)`.
  * tile_scratch: device scratch of ceil(L / 128) * H + 1 int32, or NULL. With it the flagged tiles are first listed (one

@@ -248,11 +248,6 @@ class _StateTable:
 
 
 # ------------------------------------------------------------------------------------------------------------ dense
-def _dense_into(K, q, k, v, buf, out, lse):
-    """Online-softmax attention over every block: the recomputation kernel with every tile flagged."""
-    K.exact_fallback(q, k, v, out, buf.all_counts, buf.all_blocks, lse, buf.every_tile)
-
-
 def dense_attention(q, k, v, return_lse=False, K=None):
     """Dense softmax attention of [1, L, H, 128] bf16 tensors; with return_lse also the natural-log LSE [1, H, L]."""
     if K is None:
@@ -265,15 +260,9 @@ def dense_attention(q, k, v, return_lse=False, K=None):
         o = torch.nn.functional.scaled_dot_product_attention(q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2))
         return o.transpose(1, 2).contiguous()
     assert B == 1
-    buf = _Buffers.__new__(_Buffers)
-    nq, nb = cdiv(L, BM), cdiv(L, BK)
-    dev = q.device
-    buf.all_counts = torch.full((nq, H), nb, device=dev, dtype=torch.int32)
-    buf.all_blocks = torch.arange(nb, device=dev, dtype=torch.int32).expand(nq, H, nb).contiguous()
-    buf.every_tile = torch.ones(nq, H, device=dev, dtype=torch.int32)
-    lse = torch.empty(nq * BM, H, device=dev)
+    lse = torch.empty(cdiv(L, BM) * BM, H, device=q.device)
     out = torch.empty_like(q[0])
-    _dense_into(K, q[0].contiguous(), k[0].contiguous(), v[0].contiguous(), buf, out, lse)
+    K.dense_attention(q[0].contiguous(), k[0].contiguous(), v[0].contiguous(), out, lse)
     if return_lse:
         return out[None], (lse[:L].t() * LN2)[None]
     return out[None]
@@ -389,10 +378,10 @@ class EchoSparseAttention:
         if cdiv(L, BK) < self.min_blocks:
             return dense_attention(q, k, v, K=self.K)
         if layer in self.dense_layers:
-            # a full-length layer that always runs dense: the workspace already holds the list of all blocks
+            # a full-length layer that always runs dense: nothing reads its LSE
             buf = self._scratch(L, H, D, q.device)
             out = torch.empty_like(q[0])
-            _dense_into(self.K, q[0].contiguous(), k[0].contiguous(), v[0].contiguous(), buf, out, buf.dense_lse)
+            self.K.dense_attention(q[0].contiguous(), k[0].contiguous(), v[0].contiguous(), out, buf.dense_lse)
             return out[None]
         with torch.cuda.device(q.device):
             return self._step(q[0].contiguous(), k[0].contiguous(), v[0].contiguous(), step, branch, layer,
@@ -416,7 +405,8 @@ class EchoSparseAttention:
                 K.exact_fallback(q, k, v, out, buf.all_counts, buf.all_blocks, br.next_offset, buf.flags)
                 br.cur ^= 1
             else:
-                _dense_into(K, q, k, v, buf, out, br.offset)
+                # the first step's LSE decides the block choice of every later one: two sweeps, the LSE of the exact maxima
+                K.exact_fallback(q, k, v, out, buf.all_counts, buf.all_blocks, br.offset, buf.every_tile)
                 br.seeded = True
             return out
         top, refined = self._budget(cdiv(L, BK))

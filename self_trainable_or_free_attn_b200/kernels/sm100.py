@@ -144,6 +144,16 @@ def _tile_list_scratch(flags):
 
 
 @_timed
+def dense_attention(q, k, v, out, lse):
+    """Online-softmax attention over every block."""
+    L, H, hd = q.shape
+    assert hd == D
+    _cuda_bf16(q, k, v, out)
+    N.check(N.load().es_dense_attention(N.ptr(q), N.ptr(k), N.ptr(v), N.ptr(out), N.ptr(lse), L, H, N.stream_ptr()),
+            "dense_attention")
+
+
+@_timed
 def exact_fallback(q, k, v, out, counts, blocks, lse, flags):
     """Online-softmax attention over the block list, for the tiles whose fixed offset was too far off."""
     L, H, hd = q.shape

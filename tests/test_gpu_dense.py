@@ -1,0 +1,41 @@
+"""es_dense_attention: online softmax over every block with offsets from a sample of the columns, against the fp32 oracle at
+ragged lengths, with and without rows for which the sample does not do."""
+import pytest
+import torch
+
+from oracle import echosparse_ref as R
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+# 4: one block; 130: a second, ragged tile; 1000: an odd number of blocks; 4288 and 8256: samples of one and of two iterations
+@pytest.mark.parametrize("L,H,far", [(4, 1, False), (130, 2, False), (1000, 3, True), (4288, 2, True), (8256, 1, False)])
+def test_dense_attention_with_sampled_offsets(L, H, far):
+    """`far`: in head 0 a key outside the sample (the first 128 columns at these lengths) has logits more than 2^60 above the
+    sample's maximum, in head 1 a value of 1e38 meets a P above 4, so that the unnormalised output overflows: both make their
+    tiles start again. Tolerance: P and the output are rounded to bf16 (2^-9 each): 1e-2 of the 2-norm, 3e-2 of a head's
+    largest value in a single one; the LSE is fp32 with logits up to a few hundred: 1e-4 of those."""
+    from self_trainable_or_free_attn_b200 import _native, backends
+    K = backends.kernels(backends.resolve("auto", DEV))
+    g = torch.Generator().manual_seed(L)
+    pos = torch.arange(L, dtype=torch.float32)[:, None, None] / 300.0
+    q, k, v = [(torch.sin(pos * torch.randn(1, H, 128, generator=g) + torch.randn(1, H, 128, generator=g)) * 3.0
+                + 0.05 * torch.randn(L, H, 128, generator=g)).to(torch.bfloat16).to(DEV) for _ in range(3)]
+    if far:
+        k[L - 100, 0] = 90.0 * q[L // 2, 0] / q[L // 2, 0].float().norm()
+        k[L - 90, 1] = 30.0 * q[L // 3, 1] / q[L // 3, 1].float().norm()
+        v[L - 90, 1] = 1e38
+    nq = R.cdiv(L, 128)
+    out, lse = torch.full_like(q, 7.0), torch.zeros(nq * 128, H, device=DEV)
+    K.dense_attention(q, k, v, out, lse)
+    ref, ref_lse = R.dense_attention(q, k, v)
+    if far:
+        sample = (q[:, 0].float() @ k[:128, 0].float().t()).amax(1) * (R.LOG2E / 128 ** 0.5)
+        assert ((ref_lse[:, 0] - sample) > 60).any() and torch.isfinite(ref).all()
+    scale = ref.abs().amax((0, 2), keepdim=True)
+    got, want = out.float() / scale, ref / scale
+    assert (got - want).norm() <= 1e-2 * want.norm() and (got - want).abs().max() <= 3e-2
+    assert (lse[:L] - ref_lse).abs().max() <= 1e-4 * max(1.0, float(ref_lse.abs().max()) / 100)
+    assert (lse[L:] == 1e30).all()
+    assert _native.device_status() == 0
