@@ -1,15 +1,11 @@
-// VSA2 block-sparse attention over CSR block lists: forward (online softmax), backward for dK / dV (one CTA per kv block
-// walking the kv -> q lists) and for dQ (one CTA per query block walking the q -> kv lists). No atomics: every output
-// row has one owner, so results are reproducible bit for bit.
+// VSA2 block-sparse attention over CSR block lists: entry points, and the backward for dK / dV (one CTA per kv block walking
+// the kv -> q lists) and for dQ (one CTA per query block walking the q -> kv lists) on mma.sync. No atomics: every output
+// row has one owner, so results are reproducible bit for bit. The forward is in es_vsa_tc_fwd.cu.
 //
-// Conventions (reference: csrc/vsa/vsa2_kernels.h:1-12 of shaoshitong/self_trainable_or_free_attn):
-//   token tensors [BH, L, D], L = NB * 64, blk_cnt [NB] valid tokens per block (valid tokens first);
-//   CSR: row_ptr [BH * (NB + 1)] absolute offsets into col_idx; lse [BH, L] natural log, -inf for rows without a key
-//   and for padded rows; padded rows output 0 and receive zero gradient.
-// The same kernels serve the coarse branch (block means as a sequence of NBc_pad rows, 64-row tiles with their own counts).
+// Conventions: es_vsa_tc_fwd.cu; padded rows receive zero gradient. The same kernels serve the coarse branch.
 //
-// One CTA = 4 warps x 16 rows of a 64-row block; K / V (or Q / dO) tiles of the walked list are double-buffered in
-// shared memory with cp.async; products on the tensor cores (mma.sync m16n8k16, fp32 accumulation).
+// One CTA = 4 warps x 16 rows of a 64-row block; Q / dO (or K / V) tiles of the walked list are double-buffered in shared
+// memory with cp.async; products on the tensor cores (mma.sync m16n8k16, fp32 accumulation).
 #include <string>
 
 #include "es_api_internal.h"
@@ -17,22 +13,6 @@
 
 namespace es {
 namespace vsa {
-
-struct FwdArgs {
-    const void *q, *k, *v;
-    void* o;
-    float* lse;
-    const int *row_ptr, *col_idx, *blk_cnt;
-    int L, NB;
-    float scale_log2;
-    // Split-KV task mode (es_vsa_split_plan), all null in the plain (block, bh) grid: tasks[t] = {row = bh * NB + block,
-    // first edge, one past the last edge, slot}; slot < 0 writes o / lse, slot >= 0 writes the fp32 normalised partial
-    // part_o[slot] [64, D] and its log2-domain lse part_lse[slot] [64].
-    const int* tasks;
-    const int* task_info;
-    float* part_o;
-    float* part_lse;
-};
 
 // The work item of a CTA: (block, bh) of the grid, or a task of the split plan. False: nothing to do.
 __device__ __forceinline__ bool work_item(const int* tasks, const int* info, const int* row_ptr, int NB, int& blk, int& bh,
@@ -49,142 +29,6 @@ __device__ __forceinline__ bool work_item(const int* tasks, const int* info, con
     return true;
 }
 
-template <typename T, int D>
-__global__ void __launch_bounds__(128) attn_fwd_kernel(const FwdArgs a) {
-    extern __shared__ __align__(128) uint8_t smem[];
-    constexpr uint32_t TILE = TB * D * 2;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    int qb, bh, beg, end, slot;
-    if (!work_item(a.tasks, a.task_info, a.row_ptr, a.NB, qb, bh, beg, end, slot)) return;
-    const uint32_t sQ = smem_addr(smem), sKV = sQ + TILE;           // [stage][K, V]
-    const T* q = static_cast<const T*>(a.q) + ((size_t)bh * a.L + (size_t)qb * TB) * D;
-    const T* kbase = static_cast<const T*>(a.k) + (size_t)bh * a.L * D;
-    const T* vbase = static_cast<const T*>(a.v) + (size_t)bh * a.L * D;
-    const int n = end - beg;
-    const int cnt_q = a.blk_cnt[qb];
-
-    load_tile<T, D>(sQ, q, D, tid);
-    if (n > 0) {
-        const int j = a.col_idx[beg];
-        load_tile<T, D>(sKV, kbase + (size_t)j * TB * D, D, tid);
-        load_tile<T, D>(sKV + TILE, vbase + (size_t)j * TB * D, D, tid);
-    }
-    cp_commit();
-
-    float o[D / 8][4];
-#pragma unroll
-    for (int i = 0; i < D / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
-    uint32_t qa[D / 16][4];
-
-    for (int e = 0; e < n; ++e) {
-        const uint32_t sK = sKV + (uint32_t)(e & 1) * 2 * TILE, sV = sK + TILE;
-        const int kvb = a.col_idx[beg + e];
-        if (e + 1 < n) {
-            const int j = a.col_idx[beg + e + 1];
-            const uint32_t nk = sKV + (uint32_t)((e + 1) & 1) * 2 * TILE;
-            load_tile<T, D>(nk, kbase + (size_t)j * TB * D, D, tid);
-            load_tile<T, D>(nk + TILE, vbase + (size_t)j * TB * D, D, tid);
-        }
-        cp_commit();
-        cp_wait<1>();
-        __syncthreads();
-        if (e == 0) {
-#pragma unroll
-            for (int ks = 0; ks < D / 16; ++ks) load_a<D>(sQ, warp * 16, ks, lane, qa[ks]);
-        }
-        // S = Q K^T (16 rows x 64 keys per warp)
-        float s[8][4];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f;
-#pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks)
-#pragma unroll
-            for (int np = 0; np < 4; ++np) {
-                uint32_t b[4];
-                load_b_nk<D>(sK, np, ks, lane, b);
-                Elt<T>::mma(s[2 * np], qa[ks], b[0], b[1]);
-                Elt<T>::mma(s[2 * np + 1], qa[ks], b[2], b[3]);
-            }
-        // online softmax in the log2 domain; keys past the block's count are masked
-        const int cnt_k = a.blk_cnt[kvb];
-        float mx0 = -INFINITY, mx1 = -INFINITY;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int c = i * 8 + 2 * (lane & 3);
-            s[i][0] = c < cnt_k ? s[i][0] * a.scale_log2 : -INFINITY;
-            s[i][1] = c + 1 < cnt_k ? s[i][1] * a.scale_log2 : -INFINITY;
-            s[i][2] = c < cnt_k ? s[i][2] * a.scale_log2 : -INFINITY;
-            s[i][3] = c + 1 < cnt_k ? s[i][3] * a.scale_log2 : -INFINITY;
-            mx0 = fmaxf(mx0, fmaxf(s[i][0], s[i][1]));
-            mx1 = fmaxf(mx1, fmaxf(s[i][2], s[i][3]));
-        }
-        const float mn0 = fmaxf(m0, quad_max(mx0)), mn1 = fmaxf(m1, quad_max(mx1));
-        const float ms0 = mn0 == -INFINITY ? 0.f : mn0, ms1 = mn1 == -INFINITY ? 0.f : mn1;
-        const float al0 = ex2(m0 - ms0), al1 = ex2(m1 - ms1);
-        m0 = mn0; m1 = mn1;
-        float r0 = 0.f, r1 = 0.f;
-        uint32_t p[8][2];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float p0 = ex2(s[i][0] - ms0), p1 = ex2(s[i][1] - ms0), p2 = ex2(s[i][2] - ms1), p3 = ex2(s[i][3] - ms1);
-            r0 += p0 + p1; r1 += p2 + p3;
-            p[i][0] = Elt<T>::pack(p0, p1);
-            p[i][1] = Elt<T>::pack(p2, p3);
-        }
-        l0 = l0 * al0 + r0; l1 = l1 * al1 + r1;
-#pragma unroll
-        for (int i = 0; i < D / 8; ++i) { o[i][0] *= al0; o[i][1] *= al0; o[i][2] *= al1; o[i][3] *= al1; }
-        // O += P V
-#pragma unroll
-        for (int kt = 0; kt < 4; ++kt) {
-            const uint32_t pa[4] = {p[2 * kt][0], p[2 * kt][1], p[2 * kt + 1][0], p[2 * kt + 1][1]};
-#pragma unroll
-            for (int dp = 0; dp < D / 16; ++dp) {
-                uint32_t b[4];
-                load_b_kn<D>(sV, kt, dp, lane, b);
-                Elt<T>::mma(o[2 * dp], pa, b[0], b[1]);
-                Elt<T>::mma(o[2 * dp + 1], pa, b[2], b[3]);
-            }
-        }
-        __syncthreads();
-    }
-    cp_wait<0>();
-
-    l0 = quad_sum(l0); l1 = quad_sum(l1);
-    const int r0 = warp * 16 + (lane >> 2), r1 = r0 + 8;
-    if (slot >= 0) {
-        // a chunk of a split row: the normalised partial and its log2 lse; the merge masks the padded rows
-        const float i0 = l0 > 0.f ? 1.f / l0 : 0.f, i1 = l1 > 0.f ? 1.f / l1 : 0.f;
-        float* po = a.part_o + (size_t)slot * TB * D;
-#pragma unroll
-        for (int i = 0; i < D / 8; ++i) {
-            const int c = i * 8 + 2 * (lane & 3);
-            *reinterpret_cast<float2*>(po + (size_t)r0 * D + c) = make_float2(o[i][0] * i0, o[i][1] * i0);
-            *reinterpret_cast<float2*>(po + (size_t)r1 * D + c) = make_float2(o[i][2] * i1, o[i][3] * i1);
-        }
-        if ((lane & 3) == 0) {
-            a.part_lse[(size_t)slot * TB + r0] = l0 > 0.f ? m0 + log2f(l0) : -INFINITY;
-            a.part_lse[(size_t)slot * TB + r1] = l1 > 0.f ? m1 + log2f(l1) : -INFINITY;
-        }
-        return;
-    }
-    const bool ok0 = r0 < cnt_q && l0 > 0.f, ok1 = r1 < cnt_q && l1 > 0.f;
-    const float i0 = ok0 ? 1.f / l0 : 0.f, i1 = ok1 ? 1.f / l1 : 0.f;
-    T* out = static_cast<T*>(a.o) + ((size_t)bh * a.L + (size_t)qb * TB) * D;
-#pragma unroll
-    for (int i = 0; i < D / 8; ++i) {
-        const int c = i * 8 + 2 * (lane & 3);
-        *reinterpret_cast<uint32_t*>(out + (size_t)r0 * D + c) = Elt<T>::pack(o[i][0] * i0, o[i][1] * i0);
-        *reinterpret_cast<uint32_t*>(out + (size_t)r1 * D + c) = Elt<T>::pack(o[i][2] * i1, o[i][3] * i1);
-    }
-    if ((lane & 3) == 0) {
-        float* lse = a.lse + (size_t)bh * a.L + (size_t)qb * TB;
-        lse[r0] = ok0 ? (m0 + log2f(l0)) * LN2 : -INFINITY;
-        lse[r1] = ok1 ? (m1 + log2f(l1)) * LN2 : -INFINITY;
-    }
-}
-
 // ---------------------------------------------------------------------------------------------- backward, dK / dV
 struct BwdArgs {
     const void *q, *k, *v, *dout;
@@ -196,7 +40,7 @@ struct BwdArgs {
     const int *row_ptr, *col_idx, *blk_cnt;
     int L, NB;
     float scale, scale_log2;
-    // Split-KV task mode over the walked lists (see FwdArgs): slot >= 0 writes fp32 partial gradients to part0 / part1
+    // Split-KV task mode over the walked lists (es_vsa_tc_fwd.cu): slot >= 0 writes fp32 partial gradients to part0 / part1
     // [slot] [64, D] without the per-block add (the merge adds it once and zeroes the padded rows).
     const int* tasks;
     const int* task_info;
@@ -473,6 +317,10 @@ template <typename K> static int set_smem(K kern, size_t bytes) {
         else { if ((rc__ = set_smem(KERNEL<__half, 64>, SMEM))) return rc__; KERNEL<__half, 64><<<GRID, 128, SMEM, st>>>(ARGS); } \
     } while (0)
 
+// es_vsa_tc_fwd.cu
+int attn_fwd_tc(const void* q, const void* k, const void* v, void* o, float* lse, const int* row_ptr, const int* col_idx,
+                const int* blk_cnt, int BH, int L, int D, int dtype, const int* tasks, const int* task_info, int n_tasks,
+                float* part_o, float* part_lse, cudaStream_t st);
 }  // namespace vsa
 }  // namespace es
 
@@ -484,13 +332,8 @@ extern "C" int es_vsa_attn_fwd(const void* q, const void* k, const void* v, void
                                int32_t dtype, void* stream) {
     if (!q || !k || !v || !o || !lse || !row_ptr || !col_idx || !blk_cnt) return set_error(-1, "es_vsa_attn_fwd: null pointer");
     if (int rc = check_common("es_vsa_attn_fwd", BH, L, D, dtype)) return rc;
-    FwdArgs a{q, k, v, o, lse, row_ptr, col_idx, blk_cnt, L, L / TB, LOG2E / sqrtf((float)D)};
-    cudaStream_t st = (cudaStream_t)stream;
-    const size_t smem = (size_t)5 * TB * D * 2;
-    const dim3 grid(L / TB, BH);
-    VSA_DISPATCH(attn_fwd_kernel, smem, grid, a);
-    ES_CHECK_LAUNCH("attn_fwd_kernel");
-    return 0;
+    return attn_fwd_tc(q, k, v, o, lse, row_ptr, col_idx, blk_cnt, BH, L, D, dtype, nullptr, nullptr, 0, nullptr, nullptr,
+                       (cudaStream_t)stream);
 }
 
 static int fill_bwd(BwdArgs& a, const void* q, const void* k, const void* v, const void* dout, const float* lse,
@@ -559,13 +402,8 @@ extern "C" int es_vsa_attn_fwd_tasks(const void* q, const void* k, const void* v
     if (!q || !k || !v || !o || !lse || !q2k_idx || !blk_cnt) return set_error(-1, "es_vsa_attn_fwd_tasks: null pointer");
     if (int rc = check_common("es_vsa_attn_fwd_tasks", BH, L, D, dtype)) return rc;
     if (int rc = check_tasks("es_vsa_attn_fwd_tasks", tasks, task_info, n_tasks_cap)) return rc;
-    FwdArgs a{q, k, v, o, lse, nullptr, q2k_idx, blk_cnt, L, L / TB, LOG2E / sqrtf((float)D), tasks, task_info, part_o, part_lse};
-    cudaStream_t st = (cudaStream_t)stream;
-    const size_t smem = (size_t)5 * TB * D * 2;
-    const dim3 grid(n_tasks_cap, 1);
-    VSA_DISPATCH(attn_fwd_kernel, smem, grid, a);
-    ES_CHECK_LAUNCH("attn_fwd_kernel");
-    return 0;
+    return attn_fwd_tc(q, k, v, o, lse, nullptr, q2k_idx, blk_cnt, BH, L, D, dtype, tasks, task_info, n_tasks_cap, part_o,
+                       part_lse, (cudaStream_t)stream);
 }
 
 extern "C" int es_vsa_attn_bwd_kv_tasks(const void* q, const void* k, const void* v, const void* dout, const float* lse,

@@ -1,0 +1,427 @@
+// VSA2 fine / coarse forward on the 5th-generation tensor cores: online-softmax attention of one 64-row query block over the
+// 64-token kv blocks of its list, two CTAs per SM.
+//
+// Conventions (reference: csrc/vsa/vsa2_kernels.h:1-12 of shaoshitong/self_trainable_or_free_attn): token tensors [BH, L, D],
+// L = NB * 64, blk_cnt [NB] valid tokens per block (valid tokens first); CSR row_ptr [BH * (NB + 1)] absolute offsets into
+// col_idx; lse [BH, L] natural log, -inf for rows without a key and for padded rows, which output 0. The coarse branch runs
+// here too (block means as a sequence of 64-row tiles with their own counts).
+//
+// An iteration covers two kv blocks (128 keys; one at the end of an odd list):
+//   warps 0-3  softmax: warp w owns rows 16 w .. 16 w + 15 (an M = 64 accumulator sits in 16 lanes of each quarter)
+//   warp 4     issues the MMAs; warp 5 issues the TMA loads
+//   S (64 x 128) = Q K^T as two N = 64 products, one per kv block, and O (64 x D) += P V as four K = 16 steps per block;
+//   Q, K, V and P all come from shared memory, S (columns 0-127) and O (128-255) live in tensor memory.
+// S is read into registers at once and handed back, so QK of iteration i + 1 runs during the softmax of iteration i, and the
+// other CTA of the SM fills what is left. A warp rescales its rows of O (64 registers through tensor memory) only in the
+// iterations in which one of its maxima grew, which after the first few is rare. Waiting until a maximum has grown by a factor
+// 256 is no faster and loses the exact P = 1 of a row's largest term (error against fp64 2.48e-3 instead of 2.40e-3). K and V
+// blocks (16 KB each) go through one ring of five slots.
+//
+// What bounds it: shared memory. Per pair of a query and a kv block an SM fills 32 KB (256 clocks at 128 B/clock), the MMAs
+// read 56 KB (448) and P is written once (64): 0.53 ms for the 196,608 pairs of 32,768 tokens x 12 heads at 32 blocks per list.
+// Measured there, with the coarse branch's launch: 0.73 ms; the mma.sync kernel took 1.35 ms. Wan-1.3B 480p, 64 blocks per
+// list: 1.52 ms, 3.10 ms before. D = 64 at the first shape: 0.51 ms, 0.74 ms before.
+#include "es_vsa_tc.cuh"
+
+namespace es {
+namespace vsa {
+
+namespace {
+constexpr int TB = 64;
+constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
+constexpr int FW_THREADS = 192;
+
+template <int D> struct FwdCfg {
+    static constexpr uint32_t HALF = TB * 128;                   // 64 rows x 64 d: one TMA box
+    static constexpr uint32_t TILE = TB * D * 2;                 // one block: [d half][64 rows][128 B]
+    static constexpr int NSLOT = 5;
+    static constexpr uint32_t Q = 0, P = TILE, RING = P + 2 * HALF, CTL = RING + NSLOT * TILE;
+    static constexpr uint32_t BYTES = CTL + 256;
+};
+struct FwdCtl {
+    uint64_t qfull, full[5], empty[5], sfull, sfree, pfull, pvdone, drain;
+    uint32_t tmem_base;
+    int abort;
+};
+static_assert(sizeof(FwdCtl) <= 256, "control block");
+
+struct FwdTcArgs {
+    void* o;
+    float* lse;
+    const int *row_ptr, *col_idx, *blk_cnt;
+    int L, NB;
+    float scale_log2;
+    // Split-KV task mode (es_vsa_split_plan), all null in the plain (block, bh) grid: tasks[t] = {row = bh * NB + block,
+    // first edge, one past the last edge, slot}; slot < 0 writes o / lse, slot >= 0 writes the fp32 normalised partial
+    // part_o[slot] [64, D] and its log2-domain lse part_lse[slot] [64].
+    const int* tasks;
+    const int* task_info;
+    float *part_o, *part_lse;
+    int* status;
+};
+}  // namespace
+
+template <typename T, int D>
+__global__ void __launch_bounds__(FW_THREADS, 2)
+attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                   const __grid_constant__ CUtensorMap tmV, const FwdTcArgs a) {
+    using C = FwdCfg<D>;
+    extern __shared__ __align__(1024) uint8_t smem[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    int qb, bh, beg, end, slot_out;
+    if (a.tasks) {
+        if ((int)blockIdx.x >= a.task_info[0]) return;
+        const int4 t = reinterpret_cast<const int4*>(a.tasks)[blockIdx.x];
+        bh = t.x / a.NB; qb = t.x - bh * a.NB; beg = t.y; end = t.z; slot_out = t.w;
+    } else {
+        qb = blockIdx.x; bh = blockIdx.y; slot_out = -1;
+        beg = a.row_ptr[(size_t)bh * (a.NB + 1) + qb];
+        end = a.row_ptr[(size_t)bh * (a.NB + 1) + qb + 1];
+    }
+    const int n = end - beg, nt = (n + 1) >> 1;
+    const uint32_t base = smem_u32(smem);
+    FwdCtl* ctl = reinterpret_cast<FwdCtl*>(smem + C::CTL);
+    volatile int* abort_flag = &ctl->abort;
+    if (tid == 0) {
+        mbar_init(smem_u32(&ctl->qfull), 1);
+        for (int i = 0; i < C::NSLOT; ++i) {
+            mbar_init(smem_u32(&ctl->full[i]), 1);
+            mbar_init(smem_u32(&ctl->empty[i]), 1);
+        }
+        mbar_init(smem_u32(&ctl->sfull), 1);
+        mbar_init(smem_u32(&ctl->sfree), 4);
+        mbar_init(smem_u32(&ctl->pfull), 128);
+        mbar_init(smem_u32(&ctl->pvdone), 1);
+        mbar_init(smem_u32(&ctl->drain), 1);
+        ctl->abort = (base & 1023u) ? 1 : 0;                 // the swizzled tiles need a 1024-byte aligned base
+        if (base & 1023u) atomicCAS(a.status, 0, 902);
+        mbar_fence_init();
+        fence_proxy_async_smem();
+    }
+    if (warp == 4) {
+        tmem_alloc(smem_u32(&ctl->tmem_base), 256);
+        tmem_relinquish();
+        tc_fence_before();
+    }
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = ctl->tmem_base;
+    const uint32_t full0 = smem_u32(&ctl->full[0]), empty0 = smem_u32(&ctl->empty[0]);
+    const int row0 = bh * a.L;                               // first row of this (b, h) in the [BH L, D] view
+    uint32_t pseq = 0;                                       // load warp: tiles issued
+
+    if (warp == 5) {
+        // ------------------------------------------------------------ loads: Q, K(0), then K(i + 1), V(i) for every i
+        bool ok = *abort_flag == 0;
+        if (ok && nt > 0) {
+            if (lane == 0) {
+                tma_prefetch_desc(&tmK);
+                tma_prefetch_desc(&tmV);
+                mbar_arrive_expect_tx(smem_u32(&ctl->qfull), C::TILE);
+                for (int d = 0; d < D / 64; ++d)
+                    tma_load_2d(base + C::Q + d * C::HALF, &tmQ, smem_u32(&ctl->qfull), 64 * d, row0 + qb * TB);
+            }
+            int kwin = lane < n ? __ldg(a.col_idx + beg + lane) : 0, kbase = 0;   // a window of 32 list entries per tensor
+            int vwin = kwin, vbase = 0;
+            uint32_t slot = 0, par = 1;
+            auto put = [&](const CUtensorMap* m, int& win, int& wbase, int e) {
+                if (!ok || e >= n) return;
+                if ((e & ~31) != wbase) {
+                    wbase = e & ~31;
+                    win = wbase + lane < n ? __ldg(a.col_idx + beg + wbase + lane) : 0;
+                }
+                const int j = __shfl_sync(0xffffffffu, win, e & 31);
+                if (lane == 0) ok = mbar_wait(empty0 + 8 * slot, par, abort_flag, a.status, 401);
+                ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+                if (!ok) return;
+                if (lane == 0) {
+                    mbar_arrive_expect_tx(full0 + 8 * slot, C::TILE);
+#pragma unroll
+                    for (int d = 0; d < D / 64; ++d)
+                        tma_load_2d(base + C::RING + slot * C::TILE + d * C::HALF, m, full0 + 8 * slot, 64 * d, row0 + j * TB);
+                }
+                __syncwarp();
+                ++pseq;
+                if (++slot == C::NSLOT) { slot = 0; par ^= 1; }
+            };
+            put(&tmK, kwin, kbase, 0);
+            put(&tmK, kwin, kbase, 1);
+            for (int i = 0; i < nt; ++i) {
+                put(&tmK, kwin, kbase, 2 * i + 2);
+                put(&tmK, kwin, kbase, 2 * i + 3);
+                put(&tmV, vwin, vbase, 2 * i);
+                put(&tmV, vwin, vbase, 2 * i + 1);
+            }
+        }
+    } else if (warp == 4) {
+        // ------------------------------------------------------------ MMAs
+        constexpr uint32_t ID_QK = umma_idesc<T>(64, 64, 0, 0), ID_PV = umma_idesc<T>(64, D, 0, 1);
+        const uint64_t dk0 = umma_desc_sw128(0, 16, 1024), dv0 = umma_desc_sw128(0, C::HALF, 1024);
+        const uint32_t k_hi = (uint32_t)(dk0 >> 32), k_lo = (uint32_t)dk0, v_hi = (uint32_t)(dv0 >> 32), v_lo = (uint32_t)dv0;
+        const uint32_t q_lo = k_lo + ((base + C::Q) >> 4), p_lo = k_lo + ((base + C::P) >> 4);
+        uint32_t slot = 0, par = 0;
+        bool ok = *abort_flag == 0;
+        if (nt > 0) ok = ok && mbar_wait_warp(smem_u32(&ctl->qfull), 0, abort_flag, a.status, 402);
+        auto take = [&]() -> uint32_t {
+            const uint32_t s = slot;
+            ok = ok && mbar_wait_warp(full0 + 8 * s, par, abort_flag, a.status, 403);
+            if (++slot == C::NSLOT) { slot = 0; par ^= 1; }
+            return s;
+        };
+        auto issue_qk = [&](int i) {
+#pragma unroll 1
+            for (int b = 0; b < 2; ++b) {
+                if (2 * i + b >= n) break;
+                const uint32_t s = take();
+                if (!ok) return;
+                tc_fence_after();
+                if (elect_one()) {
+                    const uint32_t kb = k_lo + ((base + C::RING + s * C::TILE) >> 4);
+#pragma unroll
+                    for (int ks = 0; ks < D / 16; ++ks) {
+                        const uint32_t off = ((ks >> 2) * C::HALF + (ks & 3) * 32) >> 4;
+                        umma_ss_lohi(tmem + 64 * b, q_lo + off, k_hi, kb + off, k_hi, ID_QK, ks > 0);
+                    }
+                    umma_commit(empty0 + 8 * s);
+                }
+                __syncwarp();
+            }
+            if (elect_one()) umma_commit(smem_u32(&ctl->sfull));
+            __syncwarp();
+        };
+        if (nt > 0 && ok) issue_qk(0);
+        for (int i = 0; i < nt && ok; ++i) {
+            if (i + 1 < nt) {
+                ok = mbar_wait_warp(smem_u32(&ctl->sfree), i & 1, abort_flag, a.status, 404);
+                if (ok) issue_qk(i + 1);
+                if (!ok) break;
+            }
+            ok = mbar_wait_warp(smem_u32(&ctl->pfull), i & 1, abort_flag, a.status, 405);
+            if (!ok) break;
+#pragma unroll 1
+            for (int b = 0; b < 2; ++b) {
+                if (2 * i + b >= n) break;
+                const uint32_t s = take();
+                if (!ok) break;
+                tc_fence_after();
+                if (elect_one()) {
+                    const uint32_t vb = v_lo + ((base + C::RING + s * C::TILE) >> 4), pb = p_lo + ((b * C::HALF) >> 4);
+#pragma unroll
+                    for (int ks = 0; ks < 4; ++ks)
+                        umma_ss_lohi(tmem + 128, pb + ((ks * 32) >> 4), k_hi, vb + ((ks * 2048) >> 4), v_hi, ID_PV,
+                                     (i > 0 || b > 0 || ks > 0) ? 1u : 0u);
+                    umma_commit(empty0 + 8 * s);
+                }
+                __syncwarp();
+            }
+            if (!ok) break;
+            if (elect_one()) umma_commit(smem_u32(&ctl->pvdone));
+            __syncwarp();
+        }
+        // every MMA issued above has finished before tensor memory is freed
+        if (elect_one()) umma_commit(smem_u32(&ctl->drain));
+        __syncwarp();
+        mbar_wait(smem_u32(&ctl->drain), 0, abort_flag, a.status, 406);
+    } else {
+        // ------------------------------------------------------------ softmax and epilogue
+        const uint32_t tw = tmem + ((uint32_t)(32 * warp) << 16);
+        const int cnt_q = a.blk_cnt[qb];
+        float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;      // offsets in use (log2) and row sums relative to them
+        bool ok = *abort_flag == 0;
+        int ca = 0, cb = 0;
+        if (n > 0) ca = __ldg(a.blk_cnt + __ldg(a.col_idx + beg));
+        if (n > 1) cb = __ldg(a.blk_cnt + __ldg(a.col_idx + beg + 1));
+        // stmatrix: lane l gives the address of row (l & 7) of 8 x 8 matrix l >> 3: (rows 0-7, 8-15) x (chunk 2 j, 2 j + 1)
+        const int prow = 16 * warp + (lane & 7) + ((lane >> 3) & 1) * 8;
+        const uint32_t paddr = base + C::P + prow * 128, psw = prow & 7, pch = lane >> 4;
+        for (int i = 0; i < nt && ok; ++i) {
+            const int cnt_a = ca, cnt_b = cb;
+            ca = 2 * i + 2 < n ? __ldg(a.blk_cnt + __ldg(a.col_idx + beg + 2 * i + 2)) : 0;
+            cb = 2 * i + 3 < n ? __ldg(a.blk_cnt + __ldg(a.col_idx + beg + 2 * i + 3)) : 0;
+            ok = mbar_wait_warp(smem_u32(&ctl->sfull), i & 1, abort_flag, a.status, 407);
+            if (!ok) break;
+            tc_fence_after();
+            uint32_t s[64];
+            tmem_ld_16x64(tw, s);
+            tmem_ld_16x64(tw + 64, s + 32);
+            tmem_wait_ld();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&ctl->sfree));
+            if ((cnt_a & cnt_b) != TB) {                     // (counts are 1 .. 64) a short block, or none: mask its keys
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    const int c = (j & 7) * 8 + 2 * (lane & 3), cnt = j < 8 ? cnt_a : cnt_b;
+                    if (c >= cnt) s[4 * j] = s[4 * j + 2] = 0xff800000u;
+                    if (c + 1 >= cnt) s[4 * j + 1] = s[4 * j + 3] = 0xff800000u;
+                }
+            }
+            float x0 = -INFINITY, x1 = -INFINITY;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                x0 = fmaxf(x0, fmaxf(__uint_as_float(s[4 * j]), __uint_as_float(s[4 * j + 1])));
+                x1 = fmaxf(x1, fmaxf(__uint_as_float(s[4 * j + 2]), __uint_as_float(s[4 * j + 3])));
+            }
+            x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, 1));
+            x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, 1));
+            x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, 2)) * a.scale_log2;
+            x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, 2)) * a.scale_log2;
+            float al0 = 1.f, al1 = 1.f;
+            const bool grow = __any_sync(0xffffffffu, x0 > m0 || x1 > m1);
+            if (grow) {
+                const float n0 = fmaxf(m0, x0), n1 = fmaxf(m1, x1);
+                al0 = n0 == -INFINITY ? 0.f : ex2_approx(m0 - n0);
+                al1 = n1 == -INFINITY ? 0.f : ex2_approx(m1 - n1);
+                m0 = n0; m1 = n1;
+            }
+            const float o0 = m0 == -INFINITY ? 0.f : -m0, o1 = m1 == -INFINITY ? 0.f : -m1;
+            const float2 sc = make_float2(a.scale_log2, a.scale_log2);
+            float2 r0 = make_float2(0.f, 0.f), r1 = make_float2(0.f, 0.f);
+            uint32_t p[32];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                const float2 y0 = __ffma2_rn(make_float2(__uint_as_float(s[4 * j]), __uint_as_float(s[4 * j + 1])), sc,
+                                             make_float2(o0, o0));
+                const float2 y1 = __ffma2_rn(make_float2(__uint_as_float(s[4 * j + 2]), __uint_as_float(s[4 * j + 3])), sc,
+                                             make_float2(o1, o1));
+                const float2 p0 = make_float2(ex2_approx(y0.x), ex2_approx(y0.y));
+                const float2 p1 = make_float2(ex2_approx(y1.x), ex2_approx(y1.y));
+                r0 = __fadd2_rn(r0, p0);
+                r1 = __fadd2_rn(r1, p1);
+                p[2 * j] = pack2<T>(p0.x, p0.y);
+                p[2 * j + 1] = pack2<T>(p1.x, p1.y);
+            }
+            l0 = l0 * al0 + (r0.x + r0.y);
+            l1 = l1 * al1 + (r1.x + r1.y);
+            if (i > 0) {
+                // PV(i - 1) has read the previous P and written O
+                ok = mbar_wait_warp(smem_u32(&ctl->pvdone), (i - 1) & 1, abort_flag, a.status, 408);
+                if (!ok) break;
+                if (grow) {
+                    tc_fence_after();
+#pragma unroll
+                    for (int h = 0; h < D / 64; ++h) {
+                        tmem_ld_16x64(tw + 128 + 64 * h, s);
+                        tmem_wait_ld_regs(s);
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            s[4 * j] = __float_as_uint(__uint_as_float(s[4 * j]) * al0);
+                            s[4 * j + 1] = __float_as_uint(__uint_as_float(s[4 * j + 1]) * al0);
+                            s[4 * j + 2] = __float_as_uint(__uint_as_float(s[4 * j + 2]) * al1);
+                            s[4 * j + 3] = __float_as_uint(__uint_as_float(s[4 * j + 3]) * al1);
+                        }
+                        tmem_st_16x64(tw + 128 + 64 * h, s);
+                    }
+                    tmem_wait_st();
+                    tc_fence_before();
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const uint32_t ch = 2 * (j & 3) + pch;
+                stsm4(paddr + (j >> 2) * C::HALF + ((ch ^ psw) << 4), p[4 * j], p[4 * j + 1], p[4 * j + 2], p[4 * j + 3]);
+            }
+            fence_proxy_async_smem();
+            mbar_arrive(smem_u32(&ctl->pfull));
+        }
+        l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
+        l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
+        l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
+        l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+        if (nt > 0) ok = ok && mbar_wait_warp(smem_u32(&ctl->pvdone), (nt - 1) & 1, abort_flag, a.status, 409);
+        if (ok) {
+            tc_fence_after();
+            const int r0 = warp * 16 + (lane >> 2), r1 = r0 + 8;
+            // a chunk of a split row writes every row (the merge masks the padded ones)
+            const bool part = slot_out >= 0;
+            const bool ok0 = (part || r0 < cnt_q) && l0 > 0.f, ok1 = (part || r1 < cnt_q) && l1 > 0.f;
+            const float i0 = ok0 ? 1.f / l0 : 0.f, i1 = ok1 ? 1.f / l1 : 0.f;
+            T* out = static_cast<T*>(a.o) + ((size_t)row0 + (size_t)qb * TB) * D;
+            float* po = part ? a.part_o + (size_t)slot_out * TB * D : nullptr;
+#pragma unroll
+            for (int h = 0; h < D / 64; ++h) {
+                uint32_t o[32];
+#pragma unroll
+                for (int j = 0; j < 32; ++j) o[j] = 0;
+                if (nt > 0) {
+                    tmem_ld_16x64(tw + 128 + 64 * h, o);
+                    tmem_wait_ld_regs(o);
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int c = 64 * h + j * 8 + 2 * (lane & 3);
+                    // a row without a key, or a padded one, is 0 whatever its products hold
+                    const float v0 = ok0 ? __uint_as_float(o[4 * j]) * i0 : 0.f, v1 = ok0 ? __uint_as_float(o[4 * j + 1]) * i0 : 0.f;
+                    const float v2 = ok1 ? __uint_as_float(o[4 * j + 2]) * i1 : 0.f, v3 = ok1 ? __uint_as_float(o[4 * j + 3]) * i1 : 0.f;
+                    if (part) {
+                        *reinterpret_cast<float2*>(po + (size_t)r0 * D + c) = make_float2(v0, v1);
+                        *reinterpret_cast<float2*>(po + (size_t)r1 * D + c) = make_float2(v2, v3);
+                    } else {
+                        *reinterpret_cast<uint32_t*>(out + (size_t)r0 * D + c) = pack2<T>(v0, v1);
+                        *reinterpret_cast<uint32_t*>(out + (size_t)r1 * D + c) = pack2<T>(v2, v3);
+                    }
+                }
+            }
+            if ((lane & 3) == 0) {
+                if (part) {
+                    a.part_lse[(size_t)slot_out * TB + r0] = l0 > 0.f ? m0 + log2f(l0) : -INFINITY;
+                    a.part_lse[(size_t)slot_out * TB + r1] = l1 > 0.f ? m1 + log2f(l1) : -INFINITY;
+                } else {
+                    float* lse = a.lse + (size_t)row0 + (size_t)qb * TB;
+                    lse[r0] = ok0 ? (m0 + log2f(l0)) * kLn2 : -INFINITY;
+                    lse[r1] = ok1 ? (m1 + log2f(l1)) * kLn2 : -INFINITY;
+                }
+            }
+            tc_fence_before();
+        }
+    }
+
+    // ---------------------------------------------------------------- teardown
+    __syncwarp();
+    if (warp == 5 && lane == 0 && *abort_flag) {
+        // a wait gave up: give the loads of this warp a moment (100 us in all) to land before shared memory goes away
+        const uint64_t t_end = global_timer_ns() + 100000ull;
+        for (uint32_t back = 1; back <= (uint32_t)C::NSLOT && back <= pseq; ++back) {
+            const uint32_t sq = pseq - back;
+            while (!mbar_try_wait(full0 + 8 * (sq % C::NSLOT), (sq / C::NSLOT) & 1) && global_timer_ns() < t_end) {}
+        }
+    }
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 4) {
+        tc_fence_after();
+        tmem_dealloc(tmem, 256);
+    }
+}
+
+template <typename T, int D>
+static int launch_fwd(const void* q, const void* k, const void* v, FwdTcArgs a, int BH, dim3 grid, cudaStream_t st) {
+    CUtensorMap tq, tk, tv;
+    int rc;
+    const long long rows = (long long)BH * a.L;
+    if ((rc = make_token_map<T>(&tq, q, D, rows)) || (rc = make_token_map<T>(&tk, k, D, rows)) ||
+        (rc = make_token_map<T>(&tv, v, D, rows)))
+        return rc;
+    auto kern = attn_fwd_tc_kernel<T, D>;
+    if ((rc = opt_in_shared_memory((const void*)kern, (int)FwdCfg<D>::BYTES))) return rc;
+    kern<<<grid, FW_THREADS, FwdCfg<D>::BYTES, st>>>(tq, tk, tv, a);
+    ES_CHECK_LAUNCH("attn_fwd_tc_kernel");
+    return 0;
+}
+
+// The caller has checked the pointers and sizes (D = 64 or 128). tasks == nullptr: one CTA per (query block, bh).
+int attn_fwd_tc(const void* q, const void* k, const void* v, void* o, float* lse, const int* row_ptr, const int* col_idx,
+                const int* blk_cnt, int BH, int L, int D, int dtype, const int* tasks, const int* task_info, int n_tasks,
+                float* part_o, float* part_lse, cudaStream_t st) {
+    int* status = device_status_ptr();
+    if (!status) return set_error(-2, "attn_fwd_tc: the device status word is not available on this device");
+    const FwdTcArgs a{o, lse, row_ptr, col_idx, blk_cnt, L, L / TB, kLog2e / sqrtf((float)D), tasks, task_info, part_o, part_lse, status};
+    const dim3 grid = tasks ? dim3(n_tasks, 1) : dim3(L / TB, BH);
+    if (D == 64)
+        return dtype == 0 ? launch_fwd<__nv_bfloat16, 64>(q, k, v, a, BH, grid, st) : launch_fwd<__half, 64>(q, k, v, a, BH, grid, st);
+    return dtype == 0 ? launch_fwd<__nv_bfloat16, 128>(q, k, v, a, BH, grid, st) : launch_fwd<__half, 128>(q, k, v, a, BH, grid, st);
+}
+
+}  // namespace vsa
+}  // namespace es

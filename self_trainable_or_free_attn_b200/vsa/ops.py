@@ -350,8 +350,9 @@ def split_slots(nnz, chunk, slot_bytes, max_bytes):
     return max(0, min(int(max_bytes) // int(slot_bytes), 2 * (-(-int(nnz) // int(chunk)))))
 
 
-# resident CTAs per SM of the kernels that consume a plan (shared memory: 80 KB forward, 97 KB dK / dV, 96 KB dQ at D = 128)
-_CTAS_PER_SM = {("fwd", 64): 5, ("fwd", 128): 2, ("bwd_kv", 64): 4, ("bwd_kv", 128): 2, ("bwd_q", 64): 4, ("bwd_q", 128): 2}
+# resident CTAs per SM of the kernels that consume a plan (half of tensor memory in the forward; shared memory: 97 KB dK / dV,
+# 96 KB dQ at D = 128)
+_CTAS_PER_SM = {("fwd", 64): 2, ("fwd", 128): 2, ("bwd_kv", 64): 4, ("bwd_kv", 128): 2, ("bwd_q", 64): 4, ("bwd_q", 128): 2}
 
 
 def split_resident(q, kind, policy=None):
