@@ -535,6 +535,15 @@ template <typename K> static int set_smem_t(K kern, size_t bytes) {
 using namespace es;
 using namespace es::vsa;
 
+// es_vsa_attn.cu
+extern "C" int es_vsa_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse, const int32_t* row_ptr,
+                               const int32_t* col_idx, const int32_t* blk_cnt, int32_t BH, int32_t L, int32_t D,
+                               int32_t dtype, void* stream);
+extern "C" int es_vsa_attn_bwd_q(const void* q, const void* k, const void* v, const void* dout, const float* lse,
+                                 const float* delta, void* dq, float* dq_f32, const float* add_dq, int32_t add_nb,
+                                 const int32_t* q2k_ptr, const int32_t* q2k_idx, const int32_t* blk_cnt, int32_t BH,
+                                 int32_t L, int32_t D, int32_t dtype, void* stream);
+
 static void fill_tier(TierArgs& a, int L, int D, int RM, int phases, int mid_stride, int tail_stride) {
     a.L = L; a.NB = L / TB; a.W = (a.NB + 31) / 32; a.RM = RM; a.phases = phases;
     a.mid_stride = mid_stride; a.tail_stride = tail_stride;
@@ -550,6 +559,8 @@ extern "C" int es_vsa_tier_attn_fwd(const void* q, const void* k, const void* v,
     if (!q || !k || !v || !k_mid || !v_mid || !k_tail || !v_tail || !o || !lse || !q2k_ptr || !q2k_idx || !bits_a || !bits_ab || !blk_cnt)
         return set_error(-1, "es_vsa_tier_attn_fwd: null pointer");
     if (int rc = check_tier("es_vsa_tier_attn_fwd", BH, L, D, dtype, mid_reps, phases, mid_stride, tail_stride)) return rc;
+    // tier A alone is the plain fine branch
+    if (phases == PH_A) return es_vsa_attn_fwd(q, k, v, o, lse, q2k_ptr, q2k_idx, blk_cnt, BH, L, D, dtype, stream);
     TierArgs a{};
     a.q = q; a.k = k; a.v = v; a.k_mid = k_mid; a.v_mid = v_mid; a.k_tail = k_tail; a.v_tail = v_tail; a.o = o; a.lse = lse;
     a.row_ptr = q2k_ptr; a.col_idx = q2k_idx; a.bits_a = (const uint32_t*)bits_a; a.bits_ab = (const uint32_t*)bits_ab;
@@ -576,6 +587,9 @@ extern "C" int es_vsa_tier_attn_bwd_q(const void* q, const void* k, const void* 
         return set_error(-1, "es_vsa_tier_attn_bwd_q: null pointer");
     if (int rc = check_tier("es_vsa_tier_attn_bwd_q", BH, L, D, dtype, mid_reps, phases, mid_stride, tail_stride)) return rc;
     if (add_dq && add_nb < L / TB) return set_error(-1, "es_vsa_tier_attn_bwd_q: add_nb smaller than the block count");
+    if (phases == PH_A)
+        return es_vsa_attn_bwd_q(q, k, v, dout, lse, delta, dq, nullptr, add_dq, add_nb, q2k_ptr, q2k_idx, blk_cnt, BH, L, D, dtype,
+                                 stream);
     TierArgs a{};
     a.q = q; a.k = k; a.v = v; a.dout = dout; a.k_mid = k_mid; a.v_mid = v_mid; a.k_tail = k_tail; a.v_tail = v_tail;
     a.o = dq; a.lse = const_cast<float*>(lse); a.delta = delta; a.add = add_dq; a.add_nb = add_nb;
