@@ -350,15 +350,14 @@ def split_slots(nnz, chunk, slot_bytes, max_bytes):
     return max(0, min(int(max_bytes) // int(slot_bytes), 2 * (-(-int(nnz) // int(chunk)))))
 
 
-# resident CTAs per SM of the kernels that consume a plan (half of tensor memory in the forward; shared memory: 97 KB dK / dV,
-# 96 KB dQ at D = 128)
-_CTAS_PER_SM = {("fwd", 64): 2, ("fwd", 128): 2, ("bwd_kv", 64): 4, ("bwd_kv", 128): 2, ("bwd_q", 64): 4, ("bwd_q", 128): 2}
+# resident CTAs per SM of the kernels that consume a plan (half of tensor memory in the forward, all of it in the backward)
+_CTAS_PER_SM = {"fwd": 2, "bwd_kv": 1, "bwd_q": 1}
 
 
 def split_resident(q, kind, policy=None):
     if policy is not None and policy.resident_ctas is not None:
         return int(policy.resident_ctas)
-    return torch.cuda.get_device_properties(q.device).multi_processor_count * _CTAS_PER_SM[(kind, q.shape[-1])]
+    return torch.cuda.get_device_properties(q.device).multi_processor_count * _CTAS_PER_SM[kind]
 
 
 @N.device_guard

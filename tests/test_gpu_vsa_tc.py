@@ -1,4 +1,4 @@
-"""The tcgen05 kernels of the VSA2 fine branch (head dim 128) at the edges of their list walk: lists of 1 and 2 blocks, of odd
+"""The tcgen05 kernels of the VSA2 fine branch at the edges of their list walk: lists of 1 and 2 blocks, of odd
 length, around the 32-entry windows the load warp holds, and over every block; ragged blocks, a query block without a list.
 Against the CPU restatement in fp64. Tolerance: outputs and gradients are bf16 / fp16 (half a unit in the last place: 2^-9
 resp. 2^-12 relative) from products with P and dS rounded to the same type, a few such roundings each: 1e-2 resp. 2e-3 of the
@@ -12,11 +12,12 @@ pytestmark = pytest.mark.gpu
 LENGTHS = [0, 1, 2, 3, 30, 31, 32, 33, 34, 63, 64, 65, 66, 67]
 
 
+@pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("split", [False, True])
-def test_list_lengths(dtype, split):
+def test_list_lengths(D, dtype, split):
     from self_trainable_or_free_attn_b200 import vsa as V
-    nb, D = 67, 128
+    nb = 67
     g = torch.Generator().manual_seed(11)
     cnt = torch.randint(1, 65, (nb,), generator=g, dtype=torch.int32)
     cnt[::3] = 64
