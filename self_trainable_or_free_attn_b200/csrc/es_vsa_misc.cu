@@ -3,6 +3,8 @@
 // Reference: csrc/vsa/vsa2_kernels.h:179-302 of shaoshitong/self_trainable_or_free_attn (parameter structs of the same
 // stages) and tests/vsa_reference.py:28-87 (what they compute). Vectorised loads, warp shuffles and, for the two router
 // passes, mma.sync tiles; integer stages (top-k, CSR) are exact and deterministic.
+#include <cooperative_groups.h>
+
 #include <string>
 
 #include "es_api_internal.h"
@@ -82,15 +84,23 @@ struct RouterArgs {
 
 // MODE 0: lse2 of 64 pooled query rows over all pooled keys. MODE 1: block scores of the 64 / G query blocks of the tile:
 // score[i][j] = sum over the groups a of i and b of j of 2^(s - lse2), times the row normalisation; the G x G sums are
-// taken from a shared-memory copy of the probabilities in a fixed order (reproducible).
-template <typename T, int D, int MODE>
+// taken from a shared-memory copy of the probabilities in a fixed order (reproducible). GT: G as a compile-time constant for
+// R = 32, 16 and 8 (0: any power of two), so that the sums read 8 or 16 bytes at a time in the same order; the validity of a
+// tile's 64 keys is found once by 64 threads and handed round as two words (with every thread testing its 16 columns, integer
+// divisions were two thirds of the kernel). NB = 512, R = 16, 12 heads: LSE 58 us (137 before), scores
+// 95 us (225); NB = 624: 84 us (191) and 202 us (537).
+template <typename T, int D, int MODE, int GT>
 __global__ void __launch_bounds__(128) router_kernel(const RouterArgs a) {
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr uint32_t TILE = TB * D * 2;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int qt = blockIdx.x, bh = a.bh0 + blockIdx.y;
     const uint32_t sQ = smem_addr(smem), sK = sQ + TILE;                 // K: two stages
-    float* sP = reinterpret_cast<float*>(smem + 3 * TILE);               // MODE 1: [64][65] probabilities
+    uint32_t* sValid = reinterpret_cast<uint32_t*>(smem + 3 * TILE);     // [2 stages][2]: bit r = key r of the tile is valid
+    float* sP = reinterpret_cast<float*>(smem + 3 * TILE + 16);          // MODE 1: [64][SP] probabilities
+    constexpr int SP = 68;
+    const int G = GT ? GT : a.G, lg = 31 - __clz(G);                     // R divides 64: G is a power of two
+    auto valid_row = [&](int r) { return r < a.Lr && (r & (G - 1)) * a.R < a.blk_cnt[r >> lg]; };
     const T* q = static_cast<const T*>(a.qr) + ((size_t)bh * a.Lr_pad + (size_t)qt * TB) * D;
     const T* kbase = static_cast<const T*>(a.kr) + (size_t)bh * a.Lr_pad * D;
     const int nkt = a.Lr_pad / TB;
@@ -108,6 +118,10 @@ __global__ void __launch_bounds__(128) router_kernel(const RouterArgs a) {
         const uint32_t sKt = sK + (uint32_t)(kt & 1) * TILE;
         if (kt + 1 < nkt) load_tile<T, D>(sK + (uint32_t)((kt + 1) & 1) * TILE, kbase + (size_t)(kt + 1) * TB * D, D, tid);
         cp_commit();
+        if (warp < 2) {
+            const unsigned w = __ballot_sync(0xffffffffu, valid_row(kt * TB + tid));
+            if (lane == 0) sValid[(kt & 1) * 2 + warp] = w;
+        }
         cp_wait<1>();
         __syncthreads();
         if (kt == 0) {
@@ -127,14 +141,12 @@ __global__ void __launch_bounds__(128) router_kernel(const RouterArgs a) {
                 Elt<T>::mma(s[2 * np + 1], qa[ks], b[2], b[3]);
             }
         // validity of the pooled keys of this tile
+        const uint32_t vw[2] = {sValid[(kt & 1) * 2] >> (2 * (lane & 3)), sValid[(kt & 1) * 2 + 1] >> (2 * (lane & 3))};
         bool kv[8][2];
 #pragma unroll
         for (int i = 0; i < 8; ++i)
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const int r = kt * TB + i * 8 + 2 * (lane & 3) + u;
-                kv[i][u] = r < a.Lr && (r % a.G) * a.R < a.blk_cnt[r / a.G];
-            }
+            for (int u = 0; u < 2; ++u) kv[i][u] = (vw[i >> 2] >> ((i & 3) * 8 + u)) & 1u;
         if (MODE == 0) {
             float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
@@ -158,28 +170,45 @@ __global__ void __launch_bounds__(128) router_kernel(const RouterArgs a) {
             m0 = mn0; m1 = mn1;
         } else {
             // probabilities of this key tile -> shared memory, then fixed-order G x G sums
-            const int qrow0 = qt * TB + r0, qrow1 = qt * TB + r1;
-            const bool qv0 = qrow0 < a.Lr && (qrow0 % a.G) * a.R < a.blk_cnt[qrow0 / a.G];
-            const bool qv1 = qrow1 < a.Lr && (qrow1 % a.G) * a.R < a.blk_cnt[qrow1 / a.G];
+            const bool qv0 = valid_row(qt * TB + r0), qv1 = valid_row(qt * TB + r1);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const int c = i * 8 + 2 * (lane & 3);
-                sP[r0 * 65 + c] = (qv0 && kv[i][0]) ? exp2f(s[i][0] * a.scale_log2 - ls0) : 0.f;
-                sP[r0 * 65 + c + 1] = (qv0 && kv[i][1]) ? exp2f(s[i][1] * a.scale_log2 - ls0) : 0.f;
-                sP[r1 * 65 + c] = (qv1 && kv[i][0]) ? exp2f(s[i][2] * a.scale_log2 - ls1) : 0.f;
-                sP[r1 * 65 + c + 1] = (qv1 && kv[i][1]) ? exp2f(s[i][3] * a.scale_log2 - ls1) : 0.f;
+                *reinterpret_cast<float2*>(sP + r0 * SP + c) =
+                    make_float2((qv0 && kv[i][0]) ? exp2f(s[i][0] * a.scale_log2 - ls0) : 0.f,
+                                (qv0 && kv[i][1]) ? exp2f(s[i][1] * a.scale_log2 - ls0) : 0.f);
+                *reinterpret_cast<float2*>(sP + r1 * SP + c) =
+                    make_float2((qv1 && kv[i][0]) ? exp2f(s[i][2] * a.scale_log2 - ls1) : 0.f,
+                                (qv1 && kv[i][1]) ? exp2f(s[i][3] * a.scale_log2 - ls1) : 0.f);
             }
             __syncthreads();
-            const int per = TB / a.G;                        // blocks per tile side
+            const int per = TB >> lg;                        // blocks per tile side
             for (int e = tid; e < per * per; e += 128) {
-                const int bi = e / per, bj = e % per;
+                const int bi = e >> (6 - lg), bj = e & (per - 1);
                 const int qblk = qt * per + bi, kblk = kt * per + bj;
                 if (qblk < a.NB && kblk < a.NB) {
+                    const float* p0 = sP + bi * G * SP + bj * G;
                     float acc = 0.f;
-                    for (int x = 0; x < a.G; ++x)
-                        for (int y = 0; y < a.G; ++y) acc += sP[(bi * a.G + x) * 65 + bj * a.G + y];
+                    if (GT >= 4) {
+#pragma unroll
+                        for (int x = 0; x < GT; ++x)
+#pragma unroll
+                            for (int y = 0; y < GT; y += 4) {
+                                const float4 v = *reinterpret_cast<const float4*>(p0 + x * SP + y);
+                                acc += v.x; acc += v.y; acc += v.z; acc += v.w;
+                            }
+                    } else if (GT == 2) {
+#pragma unroll
+                        for (int x = 0; x < 2; ++x) {
+                            const float2 v = *reinterpret_cast<const float2*>(p0 + x * SP);
+                            acc += v.x; acc += v.y;
+                        }
+                    } else {
+                        for (int x = 0; x < G; ++x)
+                            for (int y = 0; y < G; ++y) acc += p0[x * SP + y];
+                    }
                     float norm;
-                    if (a.row_norm == 1) norm = 1.f / (float)(a.G * a.G);
+                    if (a.row_norm == 1) norm = 1.f / (float)(G * G);
                     else norm = 1.f / (float)((a.blk_cnt[qblk] + a.R - 1) / a.R);
                     a.scores[((size_t)blockIdx.y * a.NB + qblk) * a.NB + kblk] = acc * norm;
                 }
@@ -219,41 +248,69 @@ __device__ __forceinline__ uint32_t score_key(float x) {
     return (u & 0x80000000u) ? 0u : u;             // negative values (never produced by the router) order as zero
 }
 
-__global__ void __launch_bounds__(1024) topk_select_kernel(const TopkArgs a) {
-    __shared__ uint32_t hist[256];
-    __shared__ uint32_t s_prefix, s_need;
-    const int b = blockIdx.x, tid = threadIdx.x;
+// A cluster of eight CTAs per (b, h): each counts the digits of an eighth of the scores, reads the other seven histograms from
+// their shared memory and finds the digit for itself. One CTA per (b, h) left 136 of 148 SMs idle at 12 heads, and its thread
+// 0 walked the 256 bins; scores share their exponents, so the warps count into eight histograms. NB = 512, 12 heads:
+// 23 us (129 before).
+constexpr int SEL_CTAS = 8, SEL_COPIES = 8;
+__global__ void __cluster_dims__(SEL_CTAS, 1, 1) __launch_bounds__(1024) topk_select_kernel(const TopkArgs a) {
+    __shared__ uint32_t part[SEL_COPIES][256], hist[2][256], warp_sum[8], s_prefix, s_need;
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, rank = (int)cluster.block_rank();
     const float* sc = a.scores + (size_t)b * a.NB * a.NB;
-    const long long N = (long long)a.NB * a.NB;
-    if (tid == 0) { s_prefix = 0; s_need = (uint32_t)a.budget; }
-    __syncthreads();
-    if (a.budget <= 0) {
-        if (tid == 0) { a.state[b * 4] = (int)0xFFFFFFFFu; a.state[b * 4 + 1] = 0; }
+    const long long N = (long long)a.NB * a.NB, step = (N + SEL_CTAS - 1) / SEL_CTAS;
+    const long long lo = min(rank * step, N), hi = min(lo + step, N);
+    if (a.budget <= 0) {                               // the same for every CTA of the cluster
+        if (rank == 0 && tid == 0) { a.state[b * 4] = (int)0xFFFFFFFFu; a.state[b * 4 + 1] = 0; }
         return;
     }
+    if (tid == 0) { s_prefix = 0; s_need = (uint32_t)a.budget; }
+    uint32_t* mine = part[(tid >> 5) & (SEL_COPIES - 1)];
     for (int pass = 0; pass < 4; ++pass) {
         const int shift = 24 - 8 * pass;
-        if (tid < 256) hist[tid] = 0;
+        for (int i = tid; i < SEL_COPIES * 256; i += 1024) part[i >> 8][i & 255] = 0;
         __syncthreads();
-        const uint32_t prefix = s_prefix, mask = pass == 0 ? 0u : (0xFFFFFFFFu << (shift + 8));
-        for (long long i = tid; i < N; i += 1024) {
+        const uint32_t prefix = s_prefix, need = s_need, mask = pass == 0 ? 0u : (0xFFFFFFFFu << (shift + 8));
+#pragma unroll 4
+        for (long long i = lo + tid; i < hi; i += 1024) {
             const uint32_t key = score_key(sc[i]);
-            if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255], 1u);
+            if ((key & mask) == prefix) atomicAdd(&mine[(key >> shift) & 255], 1u);
         }
         __syncthreads();
-        if (tid == 0) {
-            uint32_t need = s_need, d = 255;
-            for (;; --d) {
-                if (hist[d] >= need) break;
-                need -= hist[d];
-                if (d == 0) break;
+        uint32_t* own = hist[pass & 1];                // the other buffer may still be read by a CTA that is one pass behind
+        if (tid < 256) {
+            uint32_t n = 0;
+#pragma unroll
+            for (int c = 0; c < SEL_COPIES; ++c) n += part[c][tid];
+            own[tid] = n;
+        }
+        cluster.sync();
+        // thread t holds digit 255 - t: the number of keys with a digit at least that large
+        uint32_t n = 0, incl = 0;
+        if (tid < 256) {
+#pragma unroll
+            for (int c = 0; c < SEL_CTAS; ++c) n += cluster.map_shared_rank(own, c)[255 - tid];
+            incl = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += x;
             }
-            s_prefix = prefix | (d << shift);
-            s_need = need;
+            if (lane == 31) warp_sum[tid >> 5] = incl;
+        }
+        __syncthreads();
+        if (tid < 256) {
+            for (int w = 0; w < (tid >> 5); ++w) incl += warp_sum[w];
+            if (incl >= need && incl - n < need) {     // exactly one digit
+                s_prefix = prefix | ((uint32_t)(255 - tid) << shift);
+                s_need = need - (incl - n);
+            }
         }
         __syncthreads();
     }
-    if (tid == 0) { a.state[b * 4] = (int)s_prefix; a.state[b * 4 + 1] = (int)s_need; }
+    if (rank == 0 && tid == 0) { a.state[b * 4] = (int)s_prefix; a.state[b * 4 + 1] = (int)s_need; }
+    cluster.sync();                                    // no CTA leaves while another reads its histogram
 }
 
 // one warp per row
@@ -349,20 +406,47 @@ __global__ void __launch_bounds__(128) topk_emit_rows_kernel(const TopkArgs a) {
     }
 }
 
-// one thread per column: count (pass 0) or emit the ascending query list (pass 1)
-__global__ void __launch_bounds__(128) topk_cols_kernel(const TopkArgs a, int pass) {
-    const int b = blockIdx.y, col = blockIdx.x * 128 + threadIdx.x, bh = a.bh0 + b;
-    if (col >= a.NB) return;
-    const uint32_t* bits = a.selbits + (size_t)b * a.NB * a.W + (col >> 5);
-    const uint32_t m = 1u << (col & 31);
+// One CTA per word (32 columns) of the bitmap, its 8 warps an eighth of the rows each: count (pass 0) or emit the ascending
+// query lists (pass 1). A warp takes 32 rows at a time, lane = row, and a vote per column turns them into that column's 32
+// rows; lane j keeps column j's count. One thread per column walking the rows took 79 us per pass at NB = 512, 12 heads;
+// this takes 7.
+__global__ void __launch_bounds__(256) topk_cols_kernel(const TopkArgs a, int pass) {
+    __shared__ int part[8][32];
+    const int b = blockIdx.y, w = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, bh = a.bh0 + b;
+    const uint32_t* bits = a.selbits + (size_t)b * a.NB * a.W + w;
+    const int per = ((a.NB + 255) / 256) * 32, lo = warp * per, hi = min(lo + per, a.NB);
+    const int col = w * 32 + lane;
+    int n = 0;
+    for (int r0 = lo; r0 < hi; r0 += 32) {
+        const uint32_t word = r0 + lane < hi ? bits[(size_t)(r0 + lane) * a.W] : 0u;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            const int c = __popc(__ballot_sync(0xffffffffu, (word >> j) & 1u));
+            n += lane == j ? c : 0;
+        }
+    }
+    part[warp][lane] = n;
+    __syncthreads();
     if (pass == 0) {
-        int n = 0;
-        for (int r = 0; r < a.NB; ++r) n += (bits[(size_t)r * a.W] & m) != 0;
-        a.colcnt[b * a.NB + col] = n;
-    } else {
-        int pos = a.k2q_ptr[(size_t)bh * (a.NB + 1) + col];
-        for (int r = 0; r < a.NB; ++r)
-            if (bits[(size_t)r * a.W] & m) a.k2q_idx[pos++] = r;
+        if (warp == 0 && col < a.NB) {
+            int t = 0;
+            for (int x = 0; x < 8; ++x) t += part[x][lane];
+            a.colcnt[b * a.NB + col] = t;
+        }
+        return;
+    }
+    int pos = col < a.NB ? a.k2q_ptr[(size_t)bh * (a.NB + 1) + col] : 0;
+    for (int x = 0; x < warp; ++x) pos += part[x][lane];
+    for (int r0 = lo; r0 < hi; r0 += 32) {
+        const uint32_t word = r0 + lane < hi ? bits[(size_t)(r0 + lane) * a.W] : 0u;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            const unsigned m = __ballot_sync(0xffffffffu, (word >> j) & 1u);
+            if (m == 0) continue;                      // uniform
+            const int at = __shfl_sync(0xffffffffu, pos, j);
+            if ((word >> j) & 1u) a.k2q_idx[at + __popc(m & ((1u << lane) - 1))] = r0 + lane;
+            pos += lane == j ? __popc(m) : 0;
+        }
     }
 }
 
@@ -642,19 +726,26 @@ extern "C" int es_vsa_pool(const void* q, const void* k, const void* v, void* qr
 
 template <int MODE>
 static int launch_router(const RouterArgs& a, int D, int dtype, int bh_count, cudaStream_t st) {
-    const size_t smem = (size_t)3 * TB * D * 2 + (MODE == 1 ? 64 * 65 * sizeof(float) : 0);
+    const size_t smem = (size_t)3 * TB * D * 2 + 16 + (MODE == 1 ? 64 * 68 * sizeof(float) : 0);
     const dim3 grid(a.Lr_pad / TB, bh_count);
-#define ROUTER_CASE(TT, DD)                                                                                             \
+#define ROUTER_LAUNCH(TT, DD, GG)                                                                                       \
     {                                                                                                                   \
-        cudaError_t e = cudaFuncSetAttribute(router_kernel<TT, DD, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        if (e != cudaSuccess) return set_error(-2, cudaGetErrorString(e));                                              \
-        router_kernel<TT, DD, MODE><<<grid, 128, smem, st>>>(a);                                                        \
+        if (int rc = opt_in_shared_memory((const void*)router_kernel<TT, DD, MODE, GG>, (int)smem)) return rc;          \
+        router_kernel<TT, DD, MODE, GG><<<grid, 128, smem, st>>>(a);                                                    \
+    }
+#define ROUTER_CASE(TT, DD)                          \
+    {                                                \
+        if (a.G == 2) ROUTER_LAUNCH(TT, DD, 2)       \
+        else if (a.G == 4) ROUTER_LAUNCH(TT, DD, 4)  \
+        else if (a.G == 8) ROUTER_LAUNCH(TT, DD, 8)  \
+        else ROUTER_LAUNCH(TT, DD, 0)                \
     }
     if (dtype == 0 && D == 128) ROUTER_CASE(__nv_bfloat16, 128)
     else if (dtype == 0) ROUTER_CASE(__nv_bfloat16, 64)
     else if (D == 128) ROUTER_CASE(__half, 128)
     else ROUTER_CASE(__half, 64)
 #undef ROUTER_CASE
+#undef ROUTER_LAUNCH
     ES_CHECK_LAUNCH("router_kernel");
     return 0;
 }
@@ -714,20 +805,20 @@ extern "C" int es_vsa_global_topk(const float* scores, int32_t NB, int32_t bh0, 
     a.colcnt = w; w += (size_t)bh_count * NB;
     a.selbits = reinterpret_cast<uint32_t*>(w);
     cudaStream_t st = (cudaStream_t)stream;
-    topk_select_kernel<<<bh_count, 1024, 0, st>>>(a);
+    topk_select_kernel<<<dim3(SEL_CTAS, bh_count), 1024, 0, st>>>(a);
     ES_CHECK_LAUNCH("topk_select_kernel");
-    const dim3 rows((NB + 3) / 4, bh_count), cols((NB + 127) / 128, bh_count);
+    const dim3 rows((NB + 3) / 4, bh_count), cols(a.W, bh_count);
     topk_count_kernel<<<rows, 128, 0, st>>>(a);
     ES_CHECK_LAUNCH("topk_count_kernel");
     topk_scan_kernel<<<bh_count, 1024, 0, st>>>(a, 0);
     ES_CHECK_LAUNCH("topk_scan_kernel");
     topk_emit_rows_kernel<<<rows, 128, 0, st>>>(a);
     ES_CHECK_LAUNCH("topk_emit_rows_kernel");
-    topk_cols_kernel<<<cols, 128, 0, st>>>(a, 0);
+    topk_cols_kernel<<<cols, 256, 0, st>>>(a, 0);
     ES_CHECK_LAUNCH("topk_cols_kernel");
     topk_scan_kernel<<<bh_count, 1024, 0, st>>>(a, 1);
     ES_CHECK_LAUNCH("topk_scan_kernel");
-    topk_cols_kernel<<<cols, 128, 0, st>>>(a, 1);
+    topk_cols_kernel<<<cols, 256, 0, st>>>(a, 1);
     ES_CHECK_LAUNCH("topk_cols_kernel");
     return 0;
 }
@@ -817,12 +908,12 @@ extern "C" int es_vsa_row_topk(const void* scores, int32_t NB, int32_t bh0, int3
     cudaStream_t st = (cudaStream_t)stream;
     row_topk_kernel<<<dim3(NB, bh_count), 128, 0, st>>>(a);
     ES_CHECK_LAUNCH("row_topk_kernel");
-    const dim3 cols((NB + 127) / 128, bh_count);
-    topk_cols_kernel<<<cols, 128, 0, st>>>(t, 0);
+    const dim3 cols(t.W, bh_count);
+    topk_cols_kernel<<<cols, 256, 0, st>>>(t, 0);
     ES_CHECK_LAUNCH("topk_cols_kernel");
     topk_scan_kernel<<<bh_count, 1024, 0, st>>>(t, 1);
     ES_CHECK_LAUNCH("topk_scan_kernel");
-    topk_cols_kernel<<<cols, 128, 0, st>>>(t, 1);
+    topk_cols_kernel<<<cols, 256, 0, st>>>(t, 1);
     ES_CHECK_LAUNCH("topk_cols_kernel");
     return 0;
 }
