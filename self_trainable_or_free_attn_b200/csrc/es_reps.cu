@@ -150,42 +150,44 @@ gram_reduce_kernel(float* __restrict__ parts, int nsplit, float norm) {
 }
 
 // G (from gram_reduce_kernel) regularised, then its Cholesky factor with clamped pivots (representatives.py:49-63,
-// 163-165), blocked: per panel of 16 columns one warp factors the 16 x 16 diagonal block in registers (a lane per row,
-// the pivot row's values by shuffle), every row below solves its 16 entries against that block, and the trailing matrix
-// takes the rank-16 update: three barriers per panel, 24 in all, against two per column in the unblocked form. One CTA
-// per head; the matrix lives in shared memory.
-constexpr int CH_PANEL = 16;
+// 163-165), one CTA per head, the matrix in shared memory, blocked by panels of 16 columns. What bounds it is one chain of
+// 128 square roots, divisions and broadcasts; everything else is kept off that chain:
+//   panel     every warp factors the 16 x 16 diagonal block for itself in registers (a lane per row, broadcasts by shuffle), and
+//             thread r solves its own row r of the panel in the same loop with the same broadcasts, so that the rows below the
+//             block cost one multiply-add per broadcast and no barrier; the panel's columns of the result leave from there;
+//   trailing  A -= L_panel L_panel^T on the lower triangle in 4 x 4 tiles from a transposed copy of the panel.
+// Two barriers per panel. An element takes its 128 multiply-adds in ascending order whatever the blocking, so the bits do not
+// depend on it. 26 us with two heads, 82 us with the rows below, the update and the stores as phases of their own.
+constexpr int CH_PANEL = 16, CH_LD = 132;
+constexpr int METRIC_SMEM = (HD + CH_PANEL) * CH_LD * (int)sizeof(float);
 __global__ void __launch_bounds__(256)
 metric_kernel(const float* __restrict__ parts, __nv_bfloat16* __restrict__ metric, float* __restrict__ gram_out,
               int nsplit) {
-    extern __shared__ float sm[];
-    float* A = sm;                 // [128][129]
-    float* Lm = A + HD * 129;      // [128][129]
-    float* sq = Lm + HD * 129;     // [128] square roots of the clamped pivots
+    extern __shared__ __align__(16) float sm[];
+    float* A = sm;                    // [128][CH_LD]
+    float* P = A + HD * CH_LD;        // [16][CH_LD]: the panel, transposed
     __shared__ float red[8];
     __shared__ float s_eps, s_diag;
     const int h = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const float* src = parts + (size_t)h * nsplit * HD * HD;
-    for (int e = tid * 4; e < HD * HD; e += 1024) {
-        const float4 x = *reinterpret_cast<const float4*>(src + e);
-        float* dst = A + (e >> 7) * 129 + (e & 127);
-        dst[0] = x.x; dst[1] = x.y; dst[2] = x.z; dst[3] = x.w;
-        float* dl = Lm + (e >> 7) * 129 + (e & 127);
-        dl[0] = 0.f; dl[1] = 0.f; dl[2] = 0.f; dl[3] = 0.f;
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+        const int e = (u * 256 + tid) * 4;
+        *reinterpret_cast<float4*>(A + (e >> 7) * CH_LD + (e & 127)) = *reinterpret_cast<const float4*>(src + e);
     }
     __syncthreads();
-    float dg = tid < HD ? A[tid * 129 + tid] : 0.f;
+    float dg = tid < HD ? A[tid * CH_LD + tid] : 0.f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) dg += __shfl_xor_sync(0xffffffffu, dg, o);
     if (lane == 0) red[warp] = dg;
     __syncthreads();
     if (tid == 0) s_diag = (((red[0] + red[1]) + (red[2] + red[3])) + ((red[4] + red[5]) + (red[6] + red[7]))) / HD;
     __syncthreads();
-    if (tid < HD) A[tid * 129 + tid] += 1e-3f * s_diag;
+    if (tid < HD) A[tid * CH_LD + tid] += 1e-3f * s_diag;
     __syncthreads();
     if (gram_out)
-        for (int e = tid; e < HD * HD; e += 256) gram_out[(size_t)h * HD * HD + e] = A[(e >> 7) * 129 + (e & 127)];
-    dg = tid < HD ? A[tid * 129 + tid] : 0.f;
+        for (int e = tid; e < HD * HD; e += 256) gram_out[(size_t)h * HD * HD + e] = A[(e >> 7) * CH_LD + (e & 127)];
+    dg = tid < HD ? A[tid * CH_LD + tid] : 0.f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) dg += __shfl_xor_sync(0xffffffffu, dg, o);
     __syncthreads();
@@ -196,67 +198,74 @@ metric_kernel(const float* __restrict__ parts, __nv_bfloat16* __restrict__ metri
     __syncthreads();
     const float eps = s_eps;
     for (int j0 = 0; j0 < HD; j0 += CH_PANEL) {
-        // (1) the diagonal block: lane i (and its duplicate i + 16) holds row j0 + i of the block
-        if (warp == 0) {
-            const int i = lane & 15, r = j0 + i;
-            float a[CH_PANEL];
+        if (tid < HD) {
+            const int i = lane & 15, r = tid;
+            if (warp * 32 + 31 >= j0) {                    // uniform over the warp: some row of it is not above the panel
+                float d[CH_PANEL], x[CH_PANEL];            // row i of the diagonal block; this thread's row of the panel
 #pragma unroll
-            for (int c = 0; c < CH_PANEL; ++c) a[c] = A[r * 129 + j0 + c];
-#pragma unroll
-            for (int j = 0; j < CH_PANEL; ++j) {
-                const float root = sqrtf(fmaxf(__shfl_sync(0xffffffffu, a[j], j), eps));
-                const float l = i >= j ? a[j] / root : 0.f;
-                a[j] = l;
-                if (lane == j) sq[j0 + j] = root;
-#pragma unroll
-                for (int c = j + 1; c < CH_PANEL; ++c) {
-                    const float lc = __shfl_sync(0xffffffffu, l, c);
-                    if (i >= c) a[c] -= l * lc;
+                for (int c = 0; c < CH_PANEL; c += 4) {
+                    *reinterpret_cast<float4*>(d + c) = *reinterpret_cast<const float4*>(A + (j0 + i) * CH_LD + j0 + c);
+                    *reinterpret_cast<float4*>(x + c) = *reinterpret_cast<const float4*>(A + r * CH_LD + j0 + c);
                 }
-            }
-            if (lane < 16) {
 #pragma unroll
-                for (int c = 0; c < CH_PANEL; ++c) Lm[r * 129 + j0 + c] = c <= i ? a[c] : 0.f;
+                for (int j = 0; j < CH_PANEL; ++j) {
+                    const float root = sqrtf(fmaxf(__shfl_sync(0xffffffffu, d[j], j), eps));
+                    const float l = d[j] / root;           // lanes above the pivot, and x right of the diagonal, hold values
+                    x[j] /= root;                          // that nothing reads
+#pragma unroll
+                    for (int c = j + 1; c < CH_PANEL; ++c) {
+                        const float lc = __shfl_sync(0xffffffffu, l, c);
+                        d[c] = fmaf(-l, lc, d[c]);
+                        x[c] = fmaf(-x[j], lc, x[c]);
+                    }
+                }
+                uint32_t w[CH_PANEL / 2];
+#pragma unroll
+                for (int c = 0; c < CH_PANEL; ++c) {
+                    x[c] = j0 + c <= r ? x[c] : 0.f;
+                    P[c * CH_LD + r] = x[c];
+                }
+#pragma unroll
+                for (int c = 0; c < CH_PANEL / 2; ++c) {
+                    const __nv_bfloat162 v = __floats2bfloat162_rn(x[2 * c], x[2 * c + 1]);
+                    w[c] = *reinterpret_cast<const uint32_t*>(&v);
+                }
+                uint4* dst = reinterpret_cast<uint4*>(metric + (size_t)h * HD * HD + r * HD + j0);
+                dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
+                dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
+            } else {
+                uint4* dst = reinterpret_cast<uint4*>(metric + (size_t)h * HD * HD + r * HD + j0);
+                dst[0] = dst[1] = make_uint4(0, 0, 0, 0);
             }
         }
         __syncthreads();
-        // (2) the rows below: L[r][j0 + j] = (A[r][j0 + j] - sum_{k < j} L[r][j0 + k] L[j0 + j][j0 + k]) / root_j
-        if (tid < HD && tid >= j0 + CH_PANEL) {
-            float x[CH_PANEL];
+        const int first = j0 + CH_PANEL, T = (HD - first) / 4;
+        for (int t = tid; t < T * (T + 1) / 2; t += 256) {
+            int tr = (int)((sqrtf(8.f * (float)t + 1.f) - 1.f) * 0.5f);      // tile (tr, tc), tc <= tr
+            if (tr * (tr + 1) / 2 > t) --tr;
+            if ((tr + 1) * (tr + 2) / 2 <= t) ++tr;
+            const int tc = t - tr * (tr + 1) / 2, R0 = first + 4 * tr, C0 = first + 4 * tc;
+            float4 acc[4];
 #pragma unroll
-            for (int c = 0; c < CH_PANEL; ++c) x[c] = A[tid * 129 + j0 + c];
+            for (int u = 0; u < 4; ++u) acc[u] = *reinterpret_cast<const float4*>(A + (R0 + u) * CH_LD + C0);
 #pragma unroll
-            for (int j = 0; j < CH_PANEL; ++j) {
-                float sacc = x[j];
+            for (int k = 0; k < CH_PANEL; ++k) {
+                const float4 b = *reinterpret_cast<const float4*>(P + k * CH_LD + C0);
+                const float4 a4 = *reinterpret_cast<const float4*>(P + k * CH_LD + R0);
+                const float a[4] = {a4.x, a4.y, a4.z, a4.w};
 #pragma unroll
-                for (int k2 = 0; k2 < j; ++k2) sacc -= x[k2] * Lm[(j0 + j) * 129 + j0 + k2];
-                x[j] = sacc / sq[j0 + j];
-            }
-#pragma unroll
-            for (int c = 0; c < CH_PANEL; ++c) Lm[tid * 129 + j0 + c] = x[c];
-        }
-        __syncthreads();
-        // (3) A -= L_panel L_panel^T on the lower triangle of the trailing block: two threads per row, columns alternating
-        {
-            const int r = tid >> 1;
-            if (r >= j0 + CH_PANEL) {
-                float lr[CH_PANEL];
-#pragma unroll
-                for (int k2 = 0; k2 < CH_PANEL; ++k2) lr[k2] = Lm[r * 129 + j0 + k2];
-                float* row = A + r * 129;
-                for (int c = j0 + CH_PANEL + (tid & 1); c <= r; c += 2) {
-                    const float* lc = Lm + c * 129 + j0;
-                    float sacc = row[c];
-#pragma unroll
-                    for (int k2 = 0; k2 < CH_PANEL; ++k2) sacc -= lr[k2] * lc[k2];
-                    row[c] = sacc;
+                for (int u = 0; u < 4; ++u) {
+                    acc[u].x = fmaf(-a[u], b.x, acc[u].x);
+                    acc[u].y = fmaf(-a[u], b.y, acc[u].y);
+                    acc[u].z = fmaf(-a[u], b.z, acc[u].z);
+                    acc[u].w = fmaf(-a[u], b.w, acc[u].w);
                 }
             }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) *reinterpret_cast<float4*>(A + (R0 + u) * CH_LD + C0) = acc[u];
         }
         __syncthreads();
     }
-    for (int e = tid; e < HD * HD; e += 256)
-        metric[(size_t)h * HD * HD + e] = __float2bfloat16_rn(Lm[(e >> 7) * 129 + (e & 127)]);
 }
 
 // ------------------------------------------------------------------------------------------------ probes
@@ -699,7 +708,7 @@ extern "C" int es_reps_metric(const void* q, float* gram_parts, float* gram, voi
     cudaStream_t st = (cudaStream_t)stream;
     gram_kernel<<<dim3(H, nsplit), 256, 0, st>>>((const __nv_bfloat16*)q, gram_parts, L, H, rps, nsplit);
     ES_CHECK_LAUNCH("gram");
-    const int smem = (2 * HD * 129 + HD) * (int)sizeof(float);
+    const int smem = METRIC_SMEM;
     if (int rc = opt_in_shared_memory((const void*)metric_kernel, smem)) return rc;
     const float scale = 1.0f / sqrtf((float)HD);
     gram_reduce_kernel<<<dim3(H, HD * HD / 1024), 256, 0, st>>>(gram_parts, nsplit, scale * scale / (float)L);
@@ -776,7 +785,7 @@ extern "C" int es_reps_metric_static(const void* q, float* gram, void* metric, v
     cudaStream_t st = (cudaStream_t)stream;
     gram_kernel<<<dim3(H, nsplit), 256, 0, st>>>((const __nv_bfloat16*)q, parts, L, H, rps, nsplit);
     ES_CHECK_LAUNCH("gram");
-    const int smem = (2 * HD * 129 + HD) * (int)sizeof(float);
+    const int smem = METRIC_SMEM;
     if (int rc = opt_in_shared_memory((const void*)metric_kernel, smem)) return rc;
     const float scale = 1.0f / sqrtf((float)HD);
     gram_reduce_kernel<<<dim3(H, HD * HD / 1024), 256, 0, st>>>(parts, nsplit, scale * scale / (float)L);
