@@ -94,8 +94,15 @@ int es_vsa_attn_bwd_q(const void* q, const void* k, const void* v, const void* d
 int es_vsa_fuse_fwd(const void* of, const void* oc, const void* gate, void* o, const int32_t* blk_cnt, int32_t BH, int32_t L,
                     int32_t D, int32_t NBc_pad, int32_t gate_mode, int32_t gate_act, int32_t dtype, void* stream);
 
+/* Dense attention of the block means (the coarse branch), a sequence of NB real rows in L = NB rounded up to 64: o [BH, L, D] and
+ * the natural-log lse, and the fp32 gradients [BH, L, D] of all three. Padded rows give 0 and -inf. */
+int es_vsa_coarse_fwd(const void* q, const void* k, const void* v, void* o, float* lse, int32_t BH, int32_t L, int32_t NB,
+                      int32_t D, int32_t dtype, void* stream);
+int es_vsa_coarse_bwd(const void* q, const void* k, const void* v, const void* dout, const float* lse, const float* delta,
+                      float* dq, float* dk, float* dv, int32_t BH, int32_t L, int32_t NB, int32_t D, int32_t dtype, void* stream);
+
 /* Backward of the fusion: dout_f (dO on valid rows, 0 elsewhere; may be NULL), delta_f [BH, L] = rowsum(dO * o_f),
- * dout_c [BH, NBc_pad, D] = sum over the block's valid rows of w * dO (rows >= NB are left to the caller),
+ * dout_c [BH, NBc_pad, D] = sum over the block's valid rows of w * dO (rows >= NB are zeroed),
  * delta_c [BH, NBc_pad] = rowsum(dout_c * o_c), dgate like gate. Replaces `fuse_bwd` (csrc/vsa/vsa2_kernels.h:295). */
 int es_vsa_fuse_bwd(const void* dout, const void* of, const void* oc, const void* gate, void* dout_f, float* delta_f,
                     void* dout_c, float* delta_c, void* dgate, const int32_t* blk_cnt, int32_t BH, int32_t L, int32_t D,

@@ -51,6 +51,8 @@ SIGNATURES = {
     "es_vsa_attn_bwd_kv": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _P],
     "es_vsa_attn_bwd_q": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _P],
     "es_vsa_fuse_fwd": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
+    "es_vsa_coarse_fwd": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
+    "es_vsa_coarse_bwd": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "es_vsa_fuse_bwd": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
     "es_vsa_finalize": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "es_vsa_split_plan_workspace_bytes": [_I, _I],

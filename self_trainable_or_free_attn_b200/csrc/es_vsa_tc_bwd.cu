@@ -56,6 +56,7 @@ struct BwdTcArgs {
     int add_nb;
     const int *row_ptr, *col_idx, *blk_cnt;
     int L, NB;
+    int rows;                      // coarse branch (no lists, row_ptr null): real rows of the sequence, the rest of L is padding
     float scale, scale_log2;
     // Split-KV task mode over the walked lists (es_vsa_tc_fwd.cu): slot >= 0 writes fp32 partial gradients to part0 / part1
     // [slot] [64, D] without the per-block add (the merge adds it once and zeroes the padded rows).
@@ -91,15 +92,17 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
         bh = t.x / a.NB; ob = t.x - bh * a.NB; beg = t.y; end = t.z; slot_out = t.w;
     } else {
         ob = blockIdx.x; bh = blockIdx.y; slot_out = -1;
-        beg = a.row_ptr[(size_t)bh * (a.NB + 1) + ob];
-        end = a.row_ptr[(size_t)bh * (a.NB + 1) + ob + 1];
+        beg = a.row_ptr ? a.row_ptr[(size_t)bh * (a.NB + 1) + ob] : 0;
+        end = a.row_ptr ? a.row_ptr[(size_t)bh * (a.NB + 1) + ob + 1] : a.NB;
     }
+    auto block_at = [&](int e) { return a.col_idx ? __ldg(a.col_idx + beg + e) : e; };
+    auto tokens_of = [&](int j) { return a.blk_cnt ? __ldg(a.blk_cnt + j) : min(TB, a.rows - TB * j); };
     const int n = end - beg, nt = (n + 1) >> 1;
     const uint32_t base = smem_u32(smem);
     BwdCtl* ctl = reinterpret_cast<BwdCtl*>(smem + C::CTL);
     volatile int* abort_flag = &ctl->abort;
     const int row0 = bh * a.L;                               // first row of this (b, h) in the [BH L, D] view
-    const int cnt_o = a.blk_cnt[ob];
+    const int cnt_o = tokens_of(ob);
     if (tid == 0) {
         mbar_init(smem_u32(&ctl->yfull), 1);
         for (int i = 0; i < NSLOT; ++i) {
@@ -148,11 +151,11 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
                     tma_load_2d(base + C::Y2 + d * Y_HALF, &tmY2, smem_u32(&ctl->yfull), 64 * d, row0 + ob * TB);
                 }
             }
-            int win = lane < n ? __ldg(a.col_idx + beg + lane) : 0;          // a window of 32 list entries
+            int win = lane < n ? block_at(lane) : 0;          // a window of 32 list entries
             uint32_t slot = 0, par = 1;
             for (int i = 0; i < nt && ok; ++i) {
                 const int e = 2 * i;
-                if (e > 0 && (e & 31) == 0) win = e + lane < n ? __ldg(a.col_idx + beg + e + lane) : 0;
+                if (e > 0 && (e & 31) == 0) win = e + lane < n ? block_at(e + lane) : 0;
                 const int j0 = __shfl_sync(0xffffffffu, win, e & 31), j1 = __shfl_sync(0xffffffffu, win, (e + 1) & 31);
                 const int nb = e + 1 < n ? 2 : 1;
 #pragma unroll 1
@@ -243,8 +246,8 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
             valid = e < n;
             off = dl = 0.f;
             if (!valid) return;
-            const int j = __ldg(a.col_idx + beg + e);
-            valid = (r & 63) < __ldg(a.blk_cnt + j);
+            const int j = block_at(e);
+            valid = (r & 63) < tokens_of(j);
             if (KV) {
                 const size_t g = (size_t)row0 + (size_t)j * TB + (r & 63);
                 const float l = __ldg(a.lse + g);
@@ -429,16 +432,17 @@ static int dispatch_bwd(const void* x1, const void* x2, const void* y1, const vo
 }
 
 // The caller has checked the pointers and sizes (D = 64 or 128). kv: the dK / dV pass (out0 = dK, out1 = dV), else the dQ pass
-// (out0 = dQ). tasks == nullptr: one CTA per (owner block, bh).
+// (out0 = dQ). tasks == nullptr: one CTA per (owner block, bh). row_ptr and tasks null: every block with every block, the
+// sequence's real rows are `rows`.
 int attn_bwd_tc(bool kv, const void* q, const void* k, const void* v, const void* dout, const float* lse, const float* delta,
                 void* out0, void* out1, float* f0, float* f1, const float* add0, const float* add1, int add_nb,
-                const int* row_ptr, const int* col_idx, const int* blk_cnt, int BH, int L, int D, int dtype, const int* tasks,
+                const int* row_ptr, const int* col_idx, const int* blk_cnt, int BH, int L, int rows, int D, int dtype, const int* tasks,
                 const int* task_info, int n_tasks, float* part0, float* part1, cudaStream_t st) {
     int* status = device_status_ptr();
     if (!status) return set_error(-2, "attn_bwd_tc: the device status word is not available on this device");
     const float scale = 1.f / sqrtf((float)D);
     const int wide = (((uintptr_t)out0 | (uintptr_t)out1 | (uintptr_t)f0 | (uintptr_t)f1 | (uintptr_t)part0 | (uintptr_t)part1) & 15) == 0;
-    const BwdTcArgs a{lse, delta, out0, out1, f0, f1, add0, add1, add_nb, row_ptr, col_idx, blk_cnt, L, L / TB, scale,
+    const BwdTcArgs a{lse, delta, out0, out1, f0, f1, add0, add1, add_nb, row_ptr, col_idx, blk_cnt, L, L / TB, rows, scale,
                       kLog2e * scale, tasks, task_info, part0, part1, status, wide};
     const dim3 grid = tasks ? dim3(n_tasks, 1) : dim3(L / TB, BH);
     return kv ? dispatch_bwd<true>(q, dout, k, v, a, BH, D, dtype, grid, st)

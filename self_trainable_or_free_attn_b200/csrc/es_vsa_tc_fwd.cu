@@ -50,6 +50,7 @@ struct FwdTcArgs {
     float* lse;
     const int *row_ptr, *col_idx, *blk_cnt;
     int L, NB;
+    int rows;                      // coarse branch (no lists, row_ptr null): real rows of the sequence, the rest of L is padding
     float scale_log2;
     // Split-KV task mode (es_vsa_split_plan), all null in the plain (block, bh) grid: tasks[t] = {row = bh * NB + block,
     // first edge, one past the last edge, slot}; slot < 0 writes o / lse, slot >= 0 writes the fp32 normalised partial
@@ -75,9 +76,11 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         bh = t.x / a.NB; qb = t.x - bh * a.NB; beg = t.y; end = t.z; slot_out = t.w;
     } else {
         qb = blockIdx.x; bh = blockIdx.y; slot_out = -1;
-        beg = a.row_ptr[(size_t)bh * (a.NB + 1) + qb];
-        end = a.row_ptr[(size_t)bh * (a.NB + 1) + qb + 1];
+        beg = a.row_ptr ? a.row_ptr[(size_t)bh * (a.NB + 1) + qb] : 0;
+        end = a.row_ptr ? a.row_ptr[(size_t)bh * (a.NB + 1) + qb + 1] : a.NB;
     }
+    auto block_at = [&](int e) { return a.col_idx ? __ldg(a.col_idx + beg + e) : e; };
+    auto tokens_of = [&](int j) { return a.blk_cnt ? __ldg(a.blk_cnt + j) : min(TB, a.rows - TB * j); };
     const int n = end - beg, nt = (n + 1) >> 1;
     const uint32_t base = smem_u32(smem);
     FwdCtl* ctl = reinterpret_cast<FwdCtl*>(smem + C::CTL);
@@ -121,14 +124,14 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                 for (int d = 0; d < D / 64; ++d)
                     tma_load_2d(base + C::Q + d * C::HALF, &tmQ, smem_u32(&ctl->qfull), 64 * d, row0 + qb * TB);
             }
-            int kwin = lane < n ? __ldg(a.col_idx + beg + lane) : 0, kbase = 0;   // a window of 32 list entries per tensor
+            int kwin = lane < n ? block_at(lane) : 0, kbase = 0;   // a window of 32 list entries per tensor
             int vwin = kwin, vbase = 0;
             uint32_t slot = 0, par = 1;
             auto put = [&](const CUtensorMap* m, int& win, int& wbase, int e) {
                 if (!ok || e >= n) return;
                 if ((e & ~31) != wbase) {
                     wbase = e & ~31;
-                    win = wbase + lane < n ? __ldg(a.col_idx + beg + wbase + lane) : 0;
+                    win = wbase + lane < n ? block_at(wbase + lane) : 0;
                 }
                 const int j = __shfl_sync(0xffffffffu, win, e & 31);
                 if (lane == 0) ok = mbar_wait(empty0 + 8 * slot, par, abort_flag, a.status, 401);
@@ -225,19 +228,19 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     } else {
         // ------------------------------------------------------------ softmax and epilogue
         const uint32_t tw = tmem + ((uint32_t)(32 * warp) << 16);
-        const int cnt_q = a.blk_cnt[qb];
+        const int cnt_q = tokens_of(qb);
         float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;      // offsets in use (log2) and row sums relative to them
         bool ok = *abort_flag == 0;
         int ca = 0, cb = 0;
-        if (n > 0) ca = __ldg(a.blk_cnt + __ldg(a.col_idx + beg));
-        if (n > 1) cb = __ldg(a.blk_cnt + __ldg(a.col_idx + beg + 1));
+        if (n > 0) ca = tokens_of(block_at(0));
+        if (n > 1) cb = tokens_of(block_at(1));
         // stmatrix: lane l gives the address of row (l & 7) of 8 x 8 matrix l >> 3: (rows 0-7, 8-15) x (chunk 2 j, 2 j + 1)
         const int prow = 16 * warp + (lane & 7) + ((lane >> 3) & 1) * 8;
         const uint32_t paddr = base + C::P + prow * 128, psw = prow & 7, pch = lane >> 4;
         for (int i = 0; i < nt && ok; ++i) {
             const int cnt_a = ca, cnt_b = cb;
-            ca = 2 * i + 2 < n ? __ldg(a.blk_cnt + __ldg(a.col_idx + beg + 2 * i + 2)) : 0;
-            cb = 2 * i + 3 < n ? __ldg(a.blk_cnt + __ldg(a.col_idx + beg + 2 * i + 3)) : 0;
+            ca = 2 * i + 2 < n ? tokens_of(block_at(2 * i + 2)) : 0;
+            cb = 2 * i + 3 < n ? tokens_of(block_at(2 * i + 3)) : 0;
             ok = mbar_wait_warp(smem_u32(&ctl->sfull), i & 1, abort_flag, a.status, 407);
             if (!ok) break;
             tc_fence_after();
@@ -410,13 +413,14 @@ static int launch_fwd(const void* q, const void* k, const void* v, FwdTcArgs a, 
     return 0;
 }
 
-// The caller has checked the pointers and sizes (D = 64 or 128). tasks == nullptr: one CTA per (query block, bh).
+// The caller has checked the pointers and sizes (D = 64 or 128). tasks == nullptr: one CTA per (query block, bh). row_ptr and
+// tasks null: every block attends to every block, the sequence's real rows are `rows`.
 int attn_fwd_tc(const void* q, const void* k, const void* v, void* o, float* lse, const int* row_ptr, const int* col_idx,
-                const int* blk_cnt, int BH, int L, int D, int dtype, const int* tasks, const int* task_info, int n_tasks,
+                const int* blk_cnt, int BH, int L, int rows, int D, int dtype, const int* tasks, const int* task_info, int n_tasks,
                 float* part_o, float* part_lse, cudaStream_t st) {
     int* status = device_status_ptr();
     if (!status) return set_error(-2, "attn_fwd_tc: the device status word is not available on this device");
-    const FwdTcArgs a{o, lse, row_ptr, col_idx, blk_cnt, L, L / TB, kLog2e / sqrtf((float)D), tasks, task_info, part_o, part_lse, status};
+    const FwdTcArgs a{o, lse, row_ptr, col_idx, blk_cnt, L, L / TB, rows, kLog2e / sqrtf((float)D), tasks, task_info, part_o, part_lse, status};
     const dim3 grid = tasks ? dim3(n_tasks, 1) : dim3(L / TB, BH);
     if (D == 64)
         return dtype == 0 ? launch_fwd<__nv_bfloat16, 64>(q, k, v, a, BH, grid, st) : launch_fwd<__half, 64>(q, k, v, a, BH, grid, st);

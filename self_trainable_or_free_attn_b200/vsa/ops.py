@@ -240,14 +240,24 @@ def attn_fwd(q, k, v, ptr, idx, cnt):
     return o, lse
 
 
-def _coarse_meta(B, H, nb, nbc_pad, device):
-    """Dense CSR over the 64-row tiles of the pooled sequence (shape-only metadata) and the tiles' valid counts."""
-    T = nbc_pad // 64
-    cnt = torch.clamp(nb - 64 * torch.arange(T, device=device), max=64).to(torch.int32).contiguous()
-    bh = torch.arange(B * H, device=device, dtype=torch.int64)
-    ptr = (bh[:, None] * (T * T) + torch.arange(T + 1, device=device, dtype=torch.int64)[None, :] * T)
-    idx = torch.arange(T, device=device, dtype=torch.int32).repeat(B * H * T).contiguous()
-    return cnt, ptr.to(torch.int32).reshape(B, H, T + 1).contiguous(), idx
+def _coarse_fwd(qc, kc, vc, nb):
+    """Dense attention of the block means [B, H, pad64(nb), D]: (O_c, lse)."""
+    B, H, L, D = qc.shape
+    o = torch.empty_like(qc)
+    lse = torch.empty(B, H, L, device=qc.device, dtype=torch.float32)
+    N.check(N.load().es_vsa_coarse_fwd(N.ptr(qc), N.ptr(kc), N.ptr(vc), N.ptr(o), N.ptr(lse), B * H, L, nb, D,
+                                       _DTYPES[qc.dtype], N.stream_ptr()), "es_vsa_coarse_fwd")
+    return o, lse
+
+
+def _coarse_bwd(qc, kc, vc, dout, lse, delta, nb):
+    """fp32 gradients (dq, dk, dv) of the block means."""
+    B, H, L, D = qc.shape
+    dq, dk, dv = (torch.empty(B, H, L, D, device=qc.device, dtype=torch.float32) for _ in range(3))
+    N.check(N.load().es_vsa_coarse_bwd(N.ptr(qc), N.ptr(kc), N.ptr(vc), N.ptr(dout), N.ptr(lse), N.ptr(delta), N.ptr(dq),
+                                       N.ptr(dk), N.ptr(dv), B * H, L, nb, D, _DTYPES[qc.dtype], N.stream_ptr()),
+            "es_vsa_coarse_bwd")
+    return dq, dk, dv
 
 
 def _bwd_kv(q, k, v, dout, lse, delta, ptr, idx, cnt, add_dk=None, add_dv=None, f32=False):
@@ -502,8 +512,8 @@ def _fuse_bwd(dout, of, oc, gate, blk_cnt, gate_act):
     nbc_pad = oc.shape[2]
     mode = _gate_mode(gate, dout)
     delta_f = torch.empty(B, H, L, device=dout.device, dtype=torch.float32)
-    dout_c = torch.zeros_like(oc)
-    delta_c = torch.zeros(B, H, nbc_pad, device=dout.device, dtype=torch.float32)
+    dout_c = torch.empty_like(oc)
+    delta_c = torch.empty(B, H, nbc_pad, device=dout.device, dtype=torch.float32)
     dgate = torch.empty_like(gate) if gate is not None else None
     N.check(N.load().es_vsa_fuse_bwd(N.ptr(dout), N.ptr(of), N.ptr(oc), N.ptr(gate), None, N.ptr(delta_f), N.ptr(dout_c),
                                      N.ptr(delta_c), N.ptr(dgate), N.ptr(blk_cnt), B * H, L, D, nbc_pad, mode, gate_act,
@@ -518,8 +528,7 @@ class _Function(torch.autograd.Function):
         B, H, L, D = q.shape
         nb = L // 64
         qr, kr, qc, kc, vc = pool_fwd(q, k, v, blk_cnt, R)
-        c_cnt, c_ptr, c_idx = _coarse_meta(B, H, nb, qc.shape[2], q.device)
-        oc, lse_c = attn_fwd(qc, kc, vc, c_ptr, c_idx, c_cnt)
+        oc, lse_c = _coarse_fwd(qc, kc, vc, nb)
         if sel_in is not None:
             sel = sel_in
         elif row_norm < 0:                               # original VSA: per-row top-K of the whole-block scores
@@ -533,7 +542,7 @@ class _Function(torch.autograd.Function):
                 "es_vsa_fuse_fwd")
         ctx.save_for_backward(q, k, v, gate, blk_cnt)
         # held as attributes, not saved tensors, so that backward can release them after their last use
-        ctx.inter = [qc, kc, vc, oc, lse_c, of, lse_f, sel, c_cnt, c_ptr, c_idx]
+        ctx.inter = [qc, kc, vc, oc, lse_c, of, lse_f, sel]
         ctx.has_gate = gate is not None
         ctx.gate_act = gate_act
         ctx.split = split
@@ -547,14 +556,13 @@ class _Function(torch.autograd.Function):
         if ctx.inter is None:
             raise RuntimeError("VSA backward frees its intermediates after the first backward; "
                                "re-run the forward instead of backward(retain_graph=True) twice")
-        qc, kc, vc, oc, lse_c, of, lse_f, sel, c_cnt, c_ptr, c_idx = ctx.inter
+        qc, kc, vc, oc, lse_c, of, lse_f, sel = ctx.inter
         dout = dout.contiguous()
         delta_f, dout_c, delta_c, dgate = _fuse_bwd(dout, of, oc, gate if ctx.has_gate else None, blk_cnt, ctx.gate_act)
         ctx.inter[5] = None
         del of
-        # coarse branch (dense over the block means) -> fp32 per-block gradients; the dense lists are their own inverse
-        dkc, dvc = _bwd_kv(qc, kc, vc, dout_c, lse_c, delta_c, c_ptr, c_idx, c_cnt, f32=True)
-        dqc = _bwd_q(qc, kc, vc, dout_c, lse_c, delta_c, c_ptr, c_idx, c_cnt, f32=True)
+        # coarse branch (dense over the block means) -> fp32 per-block gradients
+        dqc, dkc, dvc = _coarse_bwd(qc, kc, vc, dout_c, lse_c, delta_c, q.shape[2] // 64)
         # fine branch on the forward's selection, plus the unpooled coarse gradients (block gradient / count per token)
         dq, dk, dv = _fine_bwd(q, k, v, dout, lse_f, delta_f, sel, blk_cnt, dqc, dkc, dvc, ctx.split)
         ctx.inter = None
