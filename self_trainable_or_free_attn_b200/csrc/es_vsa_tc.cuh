@@ -84,15 +84,127 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* m, 
         : "memory");
 }
 
-// Token tensor [BH, L, D] as dims {D, BH L}; a box is 64 d x one 64-token block, 128-byte swizzled (8 KB).
-template <typename T> static int make_token_map(CUtensorMap* m, const void* ptr, int D, long long rows) {
+// Token tensor [BH, L, D] as dims {D, BH L}; a box is 64 d x one 64-token block, 128-byte swizzled (8 KB), or fewer rows.
+template <typename T> static int make_token_map(CUtensorMap* m, const void* ptr, int D, long long rows, int box_rows = 64) {
     cuuint64_t dims[2] = {(cuuint64_t)D, (cuuint64_t)rows};
     cuuint64_t strides[1] = {(cuuint64_t)D * 2};
-    cuuint32_t box[2] = {64, 64};
+    cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
     return encode_tensor_map(m, std::is_same<T, __half>::value ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
                                                                                 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
                              2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+// ---------------------------------------------------------------- 64 / RM / 1 representative tiers
+// Per query block every kv block is in one tier: A (its tokens; the CSR list and bits_a), B (bits_ab & ~bits_a: its RM group
+// means, bias log2(tokens of the group)) or C (~bits_ab: its block mean, bias log2(tokens)). The walk of a query block goes over
+// units of 64 columns: the list's blocks, then 64 / RM tier-B blocks at a time, gathered, then 64 consecutive block means at a
+// time, those of other tiers masked. (Gathering tier C would save tiles only where few blocks are left to it.)
+constexpr int PH_A = 1, PH_B = 2, PH_C = 4;
+constexpr int UNIT_RING = 8;                       // units whose column counts are staged at a time
+
+struct TierMaps {
+    const uint32_t *bits_a, *bits_ab;              // [BH, NB, W]
+    int W, RM, mid_stride, tail_stride, phases;
+};
+
+// One warp's walk over the tier-B blocks of a query block: 32 words (1024 blocks) of its bitmap row at a time, a word per lane.
+struct MidWalk {
+    const uint32_t *ra, *rab;
+    int NB, W, w0, before, total;                  // first word of the window, tier-B blocks before it and in it
+    uint32_t word, pre;                            // this lane's word, tier-B blocks in the words below it
+    __device__ __forceinline__ uint32_t live(int w) const {
+        const int left = NB - 32 * w;
+        return left >= 32 ? 0xFFFFFFFFu : left > 0 ? (1u << left) - 1u : 0u;
+    }
+    __device__ __forceinline__ void fill(int lane) {
+        const int w = w0 + lane;
+        word = w < W ? rab[w] & ~ra[w] & live(w) : 0u;
+        uint32_t incl = __popc(word);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += x;
+        }
+        pre = incl - __popc(word);
+        total = (int)__shfl_sync(0xffffffffu, incl, 31);
+    }
+    __device__ __forceinline__ void start(const TierMaps& t, int bh, int NB_, int qb, int lane) {
+        NB = NB_; W = t.W;
+        ra = t.bits_a + ((size_t)bh * NB + qb) * W;
+        rab = t.bits_ab + ((size_t)bh * NB + qb) * W;
+        w0 = before = 0;
+        fill(lane);
+    }
+    // Lane l < per: tier-B block number x0 + l of the query block, -1 past the last one. x0 never decreases.
+    __device__ __forceinline__ int blocks(int x0, int per, int lane) {
+        int id = -1;
+        while (true) {
+            const int rel = x0 + lane - before;
+            int l = 0;                             // the last lane whose word starts at or before the entry
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                if ((int)__shfl_sync(0xffffffffu, pre, l + o) <= rel) l += o;
+            uint32_t w = __shfl_sync(0xffffffffu, word, l);
+            const int k = rel - (int)__shfl_sync(0xffffffffu, pre, l);
+            if (lane < per && rel >= 0 && rel < total) {
+                for (int i = 0; i < k; ++i) w &= w - 1;
+                id = (w0 + l) * 32 + __ffs(w) - 1;
+            }
+            if (x0 + per <= before + total || w0 + 32 >= W) return id;
+            w0 += 32;
+            before += total;
+            fill(lane);
+        }
+    }
+};
+
+// Number of tier-B blocks of a query block and whether it has tier-C blocks (phases cleared are empty); one warp.
+__device__ __forceinline__ int2 tier_sizes(const TierMaps& t, int bh, int NB, int qb, int lane) {
+    MidWalk m;
+    m.NB = NB;
+    const uint32_t* ra = t.bits_a + ((size_t)bh * NB + qb) * t.W;
+    const uint32_t* rab = t.bits_ab + ((size_t)bh * NB + qb) * t.W;
+    int nB = 0, nC = 0;
+    for (int w = lane; w < t.W; w += 32) {
+        const uint32_t lv = m.live(w), wab = rab[w];
+        nB += __popc(wab & ~ra[w] & lv);
+        nC += (~wab & lv) != 0;
+    }
+    nB = __reduce_add_sync(0xffffffffu, nB);
+    nC = __reduce_add_sync(0xffffffffu, nC);
+    return make_int2((t.phases & PH_B) ? nB : 0, (t.phases & PH_C) ? nC : 0);
+}
+
+// Tokens behind the columns of a unit, 0 = masked, in two halves so that the loads can be on their way while the warp waits.
+// Tier B: lane l has the tokens of its block and writes its RM groups; tier C: two blocks a lane.
+__device__ __forceinline__ int2 unit_tokens(const int* blk_cnt, const TierMaps& t, int bh, int NB, int qb, bool mid, int id, int tile,
+                                            int lane) {
+    int n[2] = {0, 0};
+    if (mid) {
+        if (id >= 0) n[0] = __ldg(blk_cnt + id);
+    } else {
+        const uint32_t* rab = t.bits_ab + ((size_t)bh * NB + qb) * t.W;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int j = 64 * tile + 32 * h + lane;
+            if (j < NB) {
+                const int c = __ldg(blk_cnt + j);
+                n[h] = (__ldg(rab + 2 * tile + h) >> lane) & 1u ? 0 : c;
+            }
+        }
+    }
+    return make_int2(n[0], n[1]);
+}
+__device__ __forceinline__ void write_counts(uint8_t* dst, int2 n, int RM, bool mid, int lane) {
+    if (mid) {
+        const int R = 64 / RM;
+        if (lane < R)
+            for (int g = 0; g < RM; ++g) dst[lane * RM + g] = (uint8_t)min(max(n.x - g * R, 0), R);
+    } else {
+        dst[lane] = (uint8_t)n.x;
+        dst[32 + lane] = (uint8_t)n.y;
+    }
 }
 
 }  // namespace vsa

@@ -21,6 +21,9 @@
 // KB, 1,000 (830) clocks at 128 B/clock; the ring's five slots leave the X2 tile of the next iteration half an iteration of
 // lead. 32,768 tokens x 12 heads, 32 blocks per list: dK / dV 1.20 ms, dQ 1.09 ms (mma.sync: 2.27 and 1.68 ms); at D = 64 0.94
 // and 0.78 ms (1.29 and 0.91 ms), where M = D = 64 gradient products take half of the tensor pipe.
+//
+// BWD_TIER_Q, BWD_REP: the three tiers of resolution, see the modes below. 512 blocks x 12 heads, 32 + 102 blocks in tiers A and B:
+// dQ 2.19 ms, tables 1.91 ms (mma.sync: 2.63 and 3.32 ms).
 #include "es_vsa_tc.cuh"
 
 namespace es {
@@ -29,14 +32,20 @@ namespace vsa {
 namespace {
 constexpr int TB = 64;
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr int BW_THREADS = 320;
+constexpr int BW_THREADS = 320, BW_THREADS_TIER = 352;
 constexpr uint32_t Y_HALF = TB * 128, X_HALF = 128 * 128;                // 64 d of an owner / a walked tile
 constexpr uint32_t DS_BYTES = 128 * 128;                                 // P, dS: [128 rows][64 columns] 16-bit
-template <int D, bool KV> struct BwdCfg {
+// BWD_TIER_Q: the dQ pass over the units of all three tiers. BWD_REP: the dK / dV pass for 64 consecutive rows of a table of
+// representatives (group means, then block means) as the owner; it walks every query block, in fp32 tables and masked by the
+// tier of each (query block, table row).
+enum BwdMode { BWD_KV, BWD_Q, BWD_TIER_Q, BWD_REP };
+template <int D, int MODE> struct BwdCfg {
+    static constexpr bool KV = MODE == BWD_KV || MODE == BWD_REP;
     static constexpr int DH = D / 64, NSLOT = D == 128 ? 5 : 10;
     static constexpr uint32_t Y_TILE = DH * Y_HALF, X_TILE = DH * X_HALF;   // [d half][rows][128 B]
     static constexpr uint32_t Y1 = 0, Y2 = Y_TILE, DS = 2 * Y_TILE, P = DS + DS_BYTES;
-    static constexpr uint32_t RING = P + (KV ? DS_BYTES : 0u), CTL = RING + NSLOT * X_TILE, BYTES = CTL + 1024;
+    static constexpr uint32_t RING = P + (KV ? DS_BYTES : 0u), CTL = RING + NSLOT * X_TILE, COUNTS = CTL + 1024;
+    static constexpr uint32_t BYTES = COUNTS + (MODE == BWD_TIER_Q ? UNIT_RING * TB : 0);   // column counts of the units
     static constexpr int LD = D + 4;                                     // epilogue staging: floats per token row
 };
 
@@ -44,7 +53,8 @@ struct BwdCtl {
     uint64_t yfull, full[10], empty[10], sfull[2], pfull, pvdone, drain;
     uint32_t tmem_base;
     int abort;
-    alignas(16) float lse2[TB], delta[TB];       // dQ pass: the owner's rows
+    int2 tiers;                                  // BWD_TIER_Q: tier-B blocks, tier-C words of the query block
+    alignas(16) float lse2[TB], delta[TB];       // the owner's columns: minus their additive terms of the exponent; delta
 };
 static_assert(sizeof(BwdCtl) <= 1024, "control block");
 
@@ -63,6 +73,7 @@ struct BwdTcArgs {
     const int *tasks, *task_info;
     float *part0, *part1;
     int* status;
+    TierMaps tier;
     int wide;                      // every output pointer is 16-byte aligned
 };
 
@@ -76,11 +87,16 @@ __device__ __forceinline__ void store4(float* dst, float4 v, int wide) {
 }
 }  // namespace
 
-template <typename T, int D, bool KV>
-__global__ void __launch_bounds__(BW_THREADS, 1)
+template <typename T, int D, int MODE>
+__global__ void __launch_bounds__(MODE == BWD_TIER_Q ? BW_THREADS_TIER : BW_THREADS, 1)
 attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant__ CUtensorMap tmX2,
-                   const __grid_constant__ CUtensorMap tmY1, const __grid_constant__ CUtensorMap tmY2, const BwdTcArgs a) {
-    using C = BwdCfg<D, KV>;
+                   const __grid_constant__ CUtensorMap tmY1, const __grid_constant__ CUtensorMap tmY2,
+                   const __grid_constant__ CUtensorMap tmM1, const __grid_constant__ CUtensorMap tmM2,
+                   const __grid_constant__ CUtensorMap tmT1, const __grid_constant__ CUtensorMap tmT2, const BwdTcArgs a) {
+    // tmM, tmT: tables of group and of block means, walked (BWD_TIER_Q; tmM in boxes of RM rows) or the owner (BWD_REP)
+    constexpr bool TIER = MODE == BWD_TIER_Q, REP = MODE == BWD_REP;
+    using C = BwdCfg<D, MODE>;
+    constexpr bool KV = C::KV;
     constexpr int NSLOT = C::NSLOT, DH = C::DH;
     constexpr uint32_t Y_TILE = C::Y_TILE, X_TILE = C::X_TILE;
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -92,17 +108,23 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
         bh = t.x / a.NB; ob = t.x - bh * a.NB; beg = t.y; end = t.z; slot_out = t.w;
     } else {
         ob = blockIdx.x; bh = blockIdx.y; slot_out = -1;
+        // BWD_REP: ob is a tile of 64 table rows
         beg = a.row_ptr ? a.row_ptr[(size_t)bh * (a.NB + 1) + ob] : 0;
         end = a.row_ptr ? a.row_ptr[(size_t)bh * (a.NB + 1) + ob + 1] : a.NB;
     }
     auto block_at = [&](int e) { return a.col_idx ? __ldg(a.col_idx + beg + e) : e; };
     auto tokens_of = [&](int j) { return a.blk_cnt ? __ldg(a.blk_cnt + j) : min(TB, a.rows - TB * j); };
-    const int n = end - beg, nt = (n + 1) >> 1;
     const uint32_t base = smem_u32(smem);
     BwdCtl* ctl = reinterpret_cast<BwdCtl*>(smem + C::CTL);
     volatile int* abort_flag = &ctl->abort;
     const int row0 = bh * a.L;                               // first row of this (b, h) in the [BH L, D] view
-    const int cnt_o = tokens_of(ob);
+    uint8_t* counts = smem + C::COUNTS;
+    // BWD_REP: the owner's table and tile in it, and the first block that the tile covers
+    const int mid_tiles = REP && (a.tier.phases & PH_B) ? (a.NB * a.tier.RM + TB - 1) / TB : 0;
+    const bool rep_mid = REP && ob < mid_tiles;
+    const int rep_tile = rep_mid ? ob : ob - mid_tiles, rep_per = rep_mid ? TB / a.tier.RM : TB, rep_blk = rep_tile * rep_per;
+    const int rep_row0 = REP ? bh * (rep_mid ? a.tier.mid_stride : a.tier.tail_stride) + rep_tile * TB : 0;
+    const int cnt_o = REP ? min(TB, (rep_mid ? a.NB * a.tier.RM : a.NB) - rep_tile * TB) : tokens_of(ob);
     if (tid == 0) {
         mbar_init(smem_u32(&ctl->yfull), 1);
         for (int i = 0; i < NSLOT; ++i) {
@@ -126,6 +148,17 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
         ctl->lse2[r] = r < cnt_o && l != -INFINITY ? l * kLog2e : INFINITY;
         ctl->delta[r] = a.delta[g];
     }
+    if (REP && tid >= 64 && tid < 128) {
+        // additive term of a table row: log2 of the tokens it stands for, -inf for none
+        const int r = tid - 64, j = rep_blk + (rep_mid ? r / a.tier.RM : r), R = TB / a.tier.RM;
+        int c = j < a.NB ? __ldg(a.blk_cnt + j) : 0;
+        if (rep_mid) c = min(max(c - (r % a.tier.RM) * R, 0), R);
+        ctl->lse2[r] = -log2f((float)c);
+    }
+    if (TIER && warp == 9) {
+        const int2 t = tier_sizes(a.tier, bh, a.NB, ob, lane);
+        if (lane == 0) ctl->tiers = t;
+    }
     if (warp == 8) {
         tmem_alloc(smem_u32(&ctl->tmem_base), 512);
         tmem_relinquish();
@@ -134,37 +167,88 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = ctl->tmem_base;
+    // walked units of 64 rows: the list's blocks (every query block for BWD_REP), then the tiers' means as in the forward
+    const int nA = TIER && !(a.tier.phases & PH_A) ? 0 : end - beg;
+    const int nM = TIER ? nA + (ctl->tiers.x * a.tier.RM + TB - 1) / TB : nA;
+    const int n = TIER && ctl->tiers.y > 0 ? nM + (a.NB + TB - 1) / TB : nM;
+    const int nt = (n + 1) >> 1;
     constexpr uint32_t G1 = 256, G2 = 320;                   // accumulator columns
     const uint32_t full0 = smem_u32(&ctl->full[0]), empty0 = smem_u32(&ctl->empty[0]);
     uint32_t pseq = 0;                                       // load warp: tiles issued
 
-    if (warp == 9) {
+    if (warp == 9 || (TIER && warp == 10)) {
         // ------------------------------------------------------------ loads: Y1, Y2, then X1(i), X2(i)
+        // With tiers X1 and X2 have a warp each: a gathered unit is up to 64 small boxes per tensor.
+        const int x_first = TIER && warp == 10 ? 1 : 0, x_last = TIER && warp == 9 ? 0 : 1;
         bool ok = *abort_flag == 0;
         if (ok && nt > 0) {
             if (lane == 0) {
                 tma_prefetch_desc(&tmX1);
                 tma_prefetch_desc(&tmX2);
-                mbar_arrive_expect_tx(smem_u32(&ctl->yfull), 2 * Y_TILE);
-                for (int d = 0; d < DH; ++d) {
-                    tma_load_2d(base + C::Y1 + d * Y_HALF, &tmY1, smem_u32(&ctl->yfull), 64 * d, row0 + ob * TB);
-                    tma_load_2d(base + C::Y2 + d * Y_HALF, &tmY2, smem_u32(&ctl->yfull), 64 * d, row0 + ob * TB);
+                if (warp == 9) mbar_arrive_expect_tx(smem_u32(&ctl->yfull), 2 * Y_TILE);
+                for (int d = 0; warp == 9 && d < DH; ++d) {
+                    const CUtensorMap* y1 = !REP ? &tmY1 : rep_mid ? &tmM1 : &tmT1;
+                    const CUtensorMap* y2 = !REP ? &tmY2 : rep_mid ? &tmM2 : &tmT2;
+                    const int yrow = REP ? rep_row0 : row0 + ob * TB;
+                    tma_load_2d(base + C::Y1 + d * Y_HALF, y1, smem_u32(&ctl->yfull), 64 * d, yrow);
+                    tma_load_2d(base + C::Y2 + d * Y_HALF, y2, smem_u32(&ctl->yfull), 64 * d, yrow);
                 }
             }
-            int win = lane < n ? block_at(lane) : 0;          // a window of 32 list entries
-            uint32_t slot = 0, par = 1;
+            int win = lane < nA ? block_at(lane) : 0;          // a window of 32 list entries
+            MidWalk walk;
+            if (TIER) walk.start(a.tier, bh, a.NB, ob, lane);
             for (int i = 0; i < nt && ok; ++i) {
                 const int e = 2 * i;
-                if (e > 0 && (e & 31) == 0) win = e + lane < n ? block_at(e + lane) : 0;
+                if (e > 0 && (e & 31) == 0) win = e + lane < nA ? block_at(e + lane) : 0;
                 const int j0 = __shfl_sync(0xffffffffu, win, e & 31), j1 = __shfl_sync(0xffffffffu, win, (e + 1) & 31);
                 const int nb = e + 1 < n ? 2 : 1;
+                const bool lists = !TIER || e + nb <= nA;
+                int id[2] = {0, 0};
+                int2 tokens[2] = {};
+                if (TIER && !lists) {
+                    const int per = TB / a.tier.RM;
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) {
+                        if (e + b < nA || e + b >= n) continue;
+                        if (e + b < nM) id[b] = walk.blocks((e + b - nA) * per, per, lane);
+                        if (x_first == 0)
+                            tokens[b] = unit_tokens(a.blk_cnt, a.tier, bh, a.NB, ob, e + b < nM, id[b], e + b - nM, lane);
+                    }
+                }
 #pragma unroll 1
-                for (int x = 0; x < 2; ++x) {
+                for (int x = x_first; x <= x_last; ++x) {
+                    const uint32_t seq = 2 * i + x, slot = seq % NSLOT, par = ((seq / NSLOT) & 1) ^ 1;
                     if (lane == 0) ok = mbar_wait(empty0 + 8 * slot, par, abort_flag, a.status, 501);
                     ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
                     if (!ok) break;
+                    if (TIER && !lists && x == 0) {
+                        // the counts' slots are free: the P / dS warps are through all but the last two iterations
+#pragma unroll
+                        for (int b = 0; b < 2; ++b) {
+                            if (e + b >= nA && e + b < n)
+                                write_counts(counts + ((e + b) % UNIT_RING) * TB, tokens[b], a.tier.RM, e + b < nM, lane);
+                        }
+                        __syncwarp();
+                    }
                     if (lane == 0) mbar_arrive_expect_tx(full0 + 8 * slot, nb * Y_TILE);
                     __syncwarp();
+                    if (TIER && !lists) {
+#pragma unroll
+                        for (int b = 0; b < 2; ++b) {
+                            const uint32_t dst = base + C::RING + slot * X_TILE + b * Y_HALF, bar = full0 + 8 * slot;
+                            const int u = e + b;
+                            if (u >= nA && u < nM) {
+                                const int row = bh * a.tier.mid_stride + max(id[b], 0) * a.tier.RM;
+                                if (lane < TB / a.tier.RM)
+                                    for (int d = 0; d < DH; ++d)
+                                        tma_load_2d(dst + d * X_HALF + lane * a.tier.RM * 128, x ? &tmM2 : &tmM1, bar, 64 * d, row);
+                            } else if (u < n && lane < DH) {
+                                const CUtensorMap* m = u < nA ? (x ? &tmX2 : &tmX1) : (x ? &tmT2 : &tmT1);
+                                const int row = u < nA ? row0 + (b ? j1 : j0) * TB : bh * a.tier.tail_stride + (u - nM) * TB;
+                                tma_load_2d(dst + lane * X_HALF, m, bar, 64 * lane, row);
+                            }
+                        }
+                    } else
                     // the d halves of the first block, then of the second
                     if (lane < DH * nb) {
                         const int d = lane % DH, b = lane / DH;
@@ -172,8 +256,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
                                     full0 + 8 * slot, 64 * d, row0 + (b ? j1 : j0) * TB);
                     }
                     __syncwarp();
-                    ++pseq;
-                    if (++slot == NSLOT) { slot = 0; par ^= 1; }
+                    pseq = seq + 1;
                 }
             }
         }
@@ -201,7 +284,9 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
                     for (int ks = 0; ks < D / 16; ++ks)
                         umma_ss_lohi(d, xa + (((ks >> 2) * X_HALF + (ks & 3) * 32) >> 4), k_hi,
                                      yb + (((ks >> 2) * Y_HALF + (ks & 3) * 32) >> 4), k_hi, ID_S, ks > 0);
-                    if (!KV && x == 1) umma_commit(empty0 + 8 * s);   // the dQ pass needs V no more
+                    // the dQ pass needs V no more. (With tiers V goes with K at the end of the iteration: X1's and X2's load warps
+                    // wait on each other's slots, and a wait can only tell two consecutive rounds of a slot apart.)
+                    if (MODE == BWD_Q && x == 1) umma_commit(empty0 + 8 * s);
                     if (x == 1) umma_commit(smem_u32(&ctl->sfull[i & 1]));
                 }
                 __syncwarp();
@@ -225,6 +310,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
                                      (i > 0 || ks > 0) ? 1u : 0u);
                     umma_commit(empty0 + 8 * s);
                 }
+                if (TIER) umma_commit(empty0 + 8 * ((uint32_t)(2 * i + 1) % NSLOT));
                 umma_commit(smem_u32(&ctl->pvdone));
             }
             __syncwarp();
@@ -243,7 +329,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
         // the walked row's block, and in the dK / dV pass its offset and delta, one iteration ahead
         auto fetch = [&](int i, bool& valid, float& off, float& dl) {
             const int e = 2 * i + (r >> 6);
-            valid = e < n;
+            valid = e < nA;
             off = dl = 0.f;
             if (!valid) return;
             const int j = block_at(e);
@@ -256,16 +342,42 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
                 dl = __ldg(a.delta + g);
             }
         };
+        // BWD_REP: the tier word of (this warp's query block, the tile's columns): bit per block that is attended through it
+        auto fetch_bits = [&](int i) -> uint32_t {
+            const int e = 2 * i + (r >> 6), w = (rep_blk >> 5) + (rep_mid ? 0 : ch);
+            if (e >= nA || w >= a.tier.W) return 0u;
+            const size_t at = ((size_t)bh * a.NB + e) * a.tier.W + w;
+            const uint32_t wab = __ldg(a.tier.bits_ab + at);
+            return rep_mid ? (wab & ~__ldg(a.tier.bits_a + at)) >> (rep_blk & 31) : ~wab;
+        };
         bool nv = false;
         float noff = 0.f, ndl = 0.f;
-        if (nt > 0) fetch(0, nv, noff, ndl);
+        uint32_t nbits = 0;
+        if (nt > 0) {
+            fetch(0, nv, noff, ndl);
+            if (REP) nbits = fetch_bits(0);
+        }
         for (int i = 0; i < nt && ok; ++i) {
-            const bool valid = nv;
-            const float off = noff, dl = ndl;
-            if (i + 1 < nt) fetch(i + 1, nv, noff, ndl);
+            bool valid = nv;
+            float off = noff;
+            const float dl = ndl;
+            uint32_t use = 0xFFFFFFFFu;                      // bit c: this thread's column c is used by the row's block
+            if (REP) {
+                const int b = rep_mid ? (32 * ch + lane) / a.tier.RM : lane;
+                use = __ballot_sync(0xffffffffu, (nbits >> b) & 1u);
+            }
+            if (i + 1 < nt) {
+                fetch(i + 1, nv, noff, ndl);
+                if (REP) nbits = fetch_bits(i + 1);
+            }
             ok = mbar_wait_warp(smem_u32(&ctl->sfull[i & 1]), (i >> 1) & 1, abort_flag, a.status, 506);
             if (!ok) break;
             tc_fence_after();
+            if (TIER && 2 * i + (r >> 6) >= nA && 2 * i + (r >> 6) < n) {
+                const int c = counts[((2 * i + (r >> 6)) % UNIT_RING) * TB + (r & 63)];
+                valid = c > 0;
+                off = __log2f((float)max(c, 1));                // as in the forward
+            }
             uint32_t s[32], dp[32];
             tmem_ld32(tw + (i & 1) * 128 + 32 * ch, s);
             tmem_ld32(tw + (i & 1) * 128 + 64 + 32 * ch, dp);
@@ -277,11 +389,12 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
 #pragma unroll
             for (int c4 = 0; c4 < 8; ++c4) {
                 float4 o4 = make_float4(off, off, off, off), d4 = make_float4(dl, dl, dl, dl);
-                if (!KV) {
-                    o4 = lse4[c4];
-                    o4 = make_float4(-o4.x, -o4.y, -o4.z, -o4.w);
-                    d4 = dl4[c4];
+                if (!KV || REP) {
+                    const float4 l4 = lse4[c4];
+                    if (TIER || REP) o4 = make_float4(off - l4.x, off - l4.y, off - l4.z, off - l4.w);
+                    else o4 = make_float4(-l4.x, -l4.y, -l4.z, -l4.w);
                 }
+                if (!KV) d4 = dl4[c4];
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int c = 4 * c4 + 2 * h;
@@ -289,8 +402,8 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
                                                 h ? make_float2(o4.z, o4.w) : make_float2(o4.x, o4.y));
                     float2 p = make_float2(ex2_approx(x.x), ex2_approx(x.y));
                     // rows without a query / key are 0; a padded column only reaches its own (zeroed) gradient row
-                    p.x = valid ? p.x : 0.f;
-                    p.y = valid ? p.y : 0.f;
+                    p.x = valid && (!REP || ((use >> c) & 1u)) ? p.x : 0.f;
+                    p.y = valid && (!REP || ((use >> (c + 1)) & 1u)) ? p.y : 0.f;
                     const float2 g = make_float2(__uint_as_float(dp[c]) - (h ? d4.z : d4.x),
                                                  __uint_as_float(dp[c + 1]) - (h ? d4.w : d4.y));
                     const float gx = p.x * g.x, gy = p.y * g.y;
@@ -373,6 +486,12 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
                     store4(part + ((size_t)slot_out * TB + t) * D + d, v, a.wide);
                     continue;
                 }
+                if (REP) {
+                    // rows past the table's real size are left to the caller
+                    if (t < cnt_o)
+                        store4((rep_mid ? (x ? a.part1 : a.part0) : f) + ((size_t)rep_row0 + t) * D + d, v, a.wide);
+                    continue;
+                }
                 v.x += ad.x; v.y += ad.y; v.z += ad.z; v.w += ad.w;
                 if (t >= cnt_o) v = make_float4(0.f, 0.f, 0.f, 0.f);
                 const size_t g = ((size_t)row0 + (size_t)ob * TB + t) * D + d;
@@ -390,7 +509,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
 
     // ---------------------------------------------------------------- teardown
     __syncwarp();
-    if (warp == 9 && lane == 0 && *abort_flag) {
+    if (warp >= 9 && lane == 0 && *abort_flag) {
         // a wait gave up: give the loads of this warp a moment (100 us in all) to land before shared memory goes away
         const uint64_t t_end = global_timer_ns() + 100000ull;
         for (uint32_t back = 1; back <= (uint32_t)NSLOT && back <= pseq; ++back) {
@@ -407,28 +526,28 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
     }
 }
 
-template <typename T, int D, bool KV>
+template <typename T, int D, int MODE>
 static int launch_bwd(const void* x1, const void* x2, const void* y1, const void* y2, const BwdTcArgs& a, int BH, dim3 grid,
                       cudaStream_t st) {
     CUtensorMap t[4];
     const void* p[4] = {x1, x2, y1, y2};
     for (int i = 0; i < 4; ++i)
         if (int rc = make_token_map<T>(&t[i], p[i], D, (long long)BH * a.L)) return rc;
-    auto kern = attn_bwd_tc_kernel<T, D, KV>;
-    if (int rc = opt_in_shared_memory((const void*)kern, (int)BwdCfg<D, KV>::BYTES)) return rc;
-    kern<<<grid, BW_THREADS, BwdCfg<D, KV>::BYTES, st>>>(t[0], t[1], t[2], t[3], a);
+    auto kern = attn_bwd_tc_kernel<T, D, MODE>;
+    if (int rc = opt_in_shared_memory((const void*)kern, (int)BwdCfg<D, MODE>::BYTES)) return rc;
+    kern<<<grid, BW_THREADS, BwdCfg<D, MODE>::BYTES, st>>>(t[0], t[1], t[2], t[3], t[2], t[3], t[2], t[3], a);
     ES_CHECK_LAUNCH("attn_bwd_tc_kernel");
     return 0;
 }
 
-template <bool KV>
+template <int MODE>
 static int dispatch_bwd(const void* x1, const void* x2, const void* y1, const void* y2, const BwdTcArgs& a, int BH, int D,
                         int dtype, dim3 grid, cudaStream_t st) {
     if (D == 128)
-        return dtype == 0 ? launch_bwd<__nv_bfloat16, 128, KV>(x1, x2, y1, y2, a, BH, grid, st)
-                          : launch_bwd<__half, 128, KV>(x1, x2, y1, y2, a, BH, grid, st);
-    return dtype == 0 ? launch_bwd<__nv_bfloat16, 64, KV>(x1, x2, y1, y2, a, BH, grid, st)
-                      : launch_bwd<__half, 64, KV>(x1, x2, y1, y2, a, BH, grid, st);
+        return dtype == 0 ? launch_bwd<__nv_bfloat16, 128, MODE>(x1, x2, y1, y2, a, BH, grid, st)
+                          : launch_bwd<__half, 128, MODE>(x1, x2, y1, y2, a, BH, grid, st);
+    return dtype == 0 ? launch_bwd<__nv_bfloat16, 64, MODE>(x1, x2, y1, y2, a, BH, grid, st)
+                      : launch_bwd<__half, 64, MODE>(x1, x2, y1, y2, a, BH, grid, st);
 }
 
 // The caller has checked the pointers and sizes (D = 64 or 128). kv: the dK / dV pass (out0 = dK, out1 = dV), else the dQ pass
@@ -443,10 +562,67 @@ int attn_bwd_tc(bool kv, const void* q, const void* k, const void* v, const void
     const float scale = 1.f / sqrtf((float)D);
     const int wide = (((uintptr_t)out0 | (uintptr_t)out1 | (uintptr_t)f0 | (uintptr_t)f1 | (uintptr_t)part0 | (uintptr_t)part1) & 15) == 0;
     const BwdTcArgs a{lse, delta, out0, out1, f0, f1, add0, add1, add_nb, row_ptr, col_idx, blk_cnt, L, L / TB, rows, scale,
-                      kLog2e * scale, tasks, task_info, part0, part1, status, wide};
+                      kLog2e * scale, tasks, task_info, part0, part1, status, {}, wide};
     const dim3 grid = tasks ? dim3(n_tasks, 1) : dim3(L / TB, BH);
-    return kv ? dispatch_bwd<true>(q, dout, k, v, a, BH, D, dtype, grid, st)
-              : dispatch_bwd<false>(k, v, q, dout, a, BH, D, dtype, grid, st);
+    return kv ? dispatch_bwd<BWD_KV>(q, dout, k, v, a, BH, D, dtype, grid, st)
+              : dispatch_bwd<BWD_Q>(k, v, q, dout, a, BH, D, dtype, grid, st);
+}
+
+template <typename T, int D, int MODE>
+static int launch_tier_bwd(const void* x1, const void* x2, const void* y1, const void* y2, const void* k_mid, const void* v_mid,
+                           const void* k_tail, const void* v_tail, const BwdTcArgs& a, int BH, int grid_x, cudaStream_t st) {
+    CUtensorMap t[8];
+    const long long tok = (long long)BH * a.L, mid = (long long)BH * a.tier.mid_stride, tail = (long long)BH * a.tier.tail_stride;
+    const void* p[8] = {x1, x2, y1, y2, k_mid, v_mid, k_tail, v_tail};
+    const long long rows[8] = {tok, tok, tok, tok, mid, mid, tail, tail};
+    for (int i = 0; i < 8; ++i) {
+        if (MODE == BWD_REP && (i == 2 || i == 3)) { t[i] = t[i - 2]; continue; }            // the owner is a table
+        const int box = MODE == BWD_TIER_Q && (i == 4 || i == 5) ? a.tier.RM : TB;
+        if (int rc = make_token_map<T>(&t[i], p[i], D, rows[i], box)) return rc;
+    }
+    auto kern = attn_bwd_tc_kernel<T, D, MODE>;
+    if (int rc = opt_in_shared_memory((const void*)kern, (int)BwdCfg<D, MODE>::BYTES)) return rc;
+    kern<<<dim3(grid_x, BH), MODE == BWD_TIER_Q ? BW_THREADS_TIER : BW_THREADS, BwdCfg<D, MODE>::BYTES, st>>>(t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], a);
+    ES_CHECK_LAUNCH("attn_bwd_tc_kernel");
+    return 0;
+}
+
+template <int MODE>
+static int dispatch_tier_bwd(const void* x1, const void* x2, const void* y1, const void* y2, const void* k_mid, const void* v_mid,
+                             const void* k_tail, const void* v_tail, const BwdTcArgs& a, int BH, int D, int dtype, int grid_x,
+                             cudaStream_t st) {
+    if (D == 128)
+        return dtype == 0 ? launch_tier_bwd<__nv_bfloat16, 128, MODE>(x1, x2, y1, y2, k_mid, v_mid, k_tail, v_tail, a, BH, grid_x, st)
+                          : launch_tier_bwd<__half, 128, MODE>(x1, x2, y1, y2, k_mid, v_mid, k_tail, v_tail, a, BH, grid_x, st);
+    return dtype == 0 ? launch_tier_bwd<__nv_bfloat16, 64, MODE>(x1, x2, y1, y2, k_mid, v_mid, k_tail, v_tail, a, BH, grid_x, st)
+                      : launch_tier_bwd<__half, 64, MODE>(x1, x2, y1, y2, k_mid, v_mid, k_tail, v_tail, a, BH, grid_x, st);
+}
+
+// The three-tier dQ pass, and the gradients of the tables of representatives (fp32, like the tables); the caller has checked the
+// pointers and sizes.
+int tier_bwd_q_tc(const void* q, const void* k, const void* v, const void* k_mid, const void* v_mid, const void* k_tail,
+                  const void* v_tail, const void* dout, const float* lse, const float* delta, void* dq, const float* add, int add_nb,
+                  const int* row_ptr, const int* col_idx, const TierMaps& tier, const int* blk_cnt, int BH, int L, int D, int dtype,
+                  cudaStream_t st) {
+    int* status = device_status_ptr();
+    if (!status) return set_error(-2, "tier_bwd_q_tc: the device status word is not available on this device");
+    const float scale = 1.f / sqrtf((float)D);
+    const BwdTcArgs a{lse, delta, dq, nullptr, nullptr, nullptr, add, nullptr, add_nb, row_ptr, col_idx, blk_cnt, L, L / TB, 0, scale,
+                      kLog2e * scale, nullptr, nullptr, nullptr, nullptr, status, tier, ((uintptr_t)dq & 15) == 0};
+    return dispatch_tier_bwd<BWD_TIER_Q>(k, v, q, dout, k_mid, v_mid, k_tail, v_tail, a, BH, D, dtype, L / TB, st);
+}
+
+int tier_rep_bwd_tc(const void* q, const void* k_mid, const void* v_mid, const void* k_tail, const void* v_tail, const void* dout,
+                    const float* lse, const float* delta, float* dk_mid, float* dv_mid, float* dk_tail, float* dv_tail,
+                    const TierMaps& tier, const int* blk_cnt, int BH, int L, int D, int dtype, int tiles, cudaStream_t st) {
+    int* status = device_status_ptr();
+    if (!status) return set_error(-2, "tier_rep_bwd_tc: the device status word is not available on this device");
+    const float scale = 1.f / sqrtf((float)D);
+    const int wide = (((uintptr_t)dk_mid | (uintptr_t)dv_mid | (uintptr_t)dk_tail | (uintptr_t)dv_tail) & 15) == 0;
+    // no lists: every query block is walked; the group means' gradients travel as part0 / part1
+    const BwdTcArgs a{lse, delta, nullptr, nullptr, dk_tail, dv_tail, nullptr, nullptr, 0, nullptr, nullptr, blk_cnt, L, L / TB, 0,
+                      scale, kLog2e * scale, nullptr, nullptr, dk_mid, dv_mid, status, tier, wide};
+    return dispatch_tier_bwd<BWD_REP>(q, dout, nullptr, nullptr, k_mid, v_mid, k_tail, v_tail, a, BH, D, dtype, tiles, st);
 }
 
 }  // namespace vsa

@@ -21,6 +21,10 @@
 // read 56 KB (448) and P is written once (64): 0.53 ms for the 196,608 pairs of 32,768 tokens x 12 heads at 32 blocks per list.
 // Measured there, with the coarse branch's launch: 0.73 ms; the mma.sync kernel took 1.35 ms. Wan-1.3B 480p, 64 blocks per
 // list: 1.52 ms, 3.10 ms before. D = 64 at the first shape: 0.51 ms, 0.74 ms before.
+//
+// TIER: the same walk over three tiers of resolution (es_vsa_tc.cuh), one softmax over all; a mean's column has the bias log2 of
+// its tokens. K and V have a load warp each: one warp for both, with the token counts fetched in line, took 1.72 ms where this
+// takes 1.30 ms (512 blocks x 12 heads, 32 + 102 blocks in tiers A and B of every query block; mma.sync 2.34 ms).
 #include "es_vsa_tc.cuh"
 
 namespace es {
@@ -29,19 +33,21 @@ namespace vsa {
 namespace {
 constexpr int TB = 64;
 constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
-constexpr int FW_THREADS = 192;
+constexpr int FW_THREADS = 192, FW_THREADS_TIER = 224;
 
 template <int D> struct FwdCfg {
     static constexpr uint32_t HALF = TB * 128;                   // 64 rows x 64 d: one TMA box
     static constexpr uint32_t TILE = TB * D * 2;                 // one block: [d half][64 rows][128 B]
     static constexpr int NSLOT = 5;
     static constexpr uint32_t Q = 0, P = TILE, RING = P + 2 * HALF, CTL = RING + NSLOT * TILE;
-    static constexpr uint32_t BYTES = CTL + 256;
+    static constexpr uint32_t COUNTS = CTL + 256;                // tiers: [UNIT_RING][64] bytes
+    static constexpr uint32_t BYTES = CTL + 256, BYTES_TIER = COUNTS + UNIT_RING * TB;
 };
 struct FwdCtl {
     uint64_t qfull, full[5], empty[5], sfull, sfree, pfull, pvdone, drain;
     uint32_t tmem_base;
     int abort;
+    int2 tiers;                    // tier-B blocks, tier-C words of the query block
 };
 static_assert(sizeof(FwdCtl) <= 256, "control block");
 
@@ -59,13 +65,16 @@ struct FwdTcArgs {
     const int* task_info;
     float *part_o, *part_lse;
     int* status;
+    TierMaps tier;
 };
 }  // namespace
 
-template <typename T, int D>
-__global__ void __launch_bounds__(FW_THREADS, 2)
+template <typename T, int D, bool TIER>
+__global__ void __launch_bounds__(TIER ? FW_THREADS_TIER : FW_THREADS, 2)
 attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                   const __grid_constant__ CUtensorMap tmV, const FwdTcArgs a) {
+                   const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmKm,
+                   const __grid_constant__ CUtensorMap tmVm, const __grid_constant__ CUtensorMap tmKt,
+                   const __grid_constant__ CUtensorMap tmVt, const FwdTcArgs a) {
     using C = FwdCfg<D>;
     extern __shared__ __align__(1024) uint8_t smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -81,8 +90,8 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     }
     auto block_at = [&](int e) { return a.col_idx ? __ldg(a.col_idx + beg + e) : e; };
     auto tokens_of = [&](int j) { return a.blk_cnt ? __ldg(a.blk_cnt + j) : min(TB, a.rows - TB * j); };
-    const int n = end - beg, nt = (n + 1) >> 1;
     const uint32_t base = smem_u32(smem);
+    uint8_t* counts = smem + C::COUNTS;
     FwdCtl* ctl = reinterpret_cast<FwdCtl*>(smem + C::CTL);
     volatile int* abort_flag = &ctl->abort;
     if (tid == 0) {
@@ -101,6 +110,10 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         mbar_fence_init();
         fence_proxy_async_smem();
     }
+    if (TIER && warp == 5) {
+        const int2 t = tier_sizes(a.tier, bh, a.NB, qb, lane);
+        if (lane == 0) ctl->tiers = t;
+    }
     if (warp == 4) {
         tmem_alloc(smem_u32(&ctl->tmem_base), 256);
         tmem_relinquish();
@@ -109,51 +122,92 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = ctl->tmem_base;
+    // units of 64 columns: the list's blocks, then (tiers) gathered group means, then block means
+    const int nA = TIER && !(a.tier.phases & PH_A) ? 0 : end - beg;
+    const int nM = TIER ? nA + (ctl->tiers.x * a.tier.RM + TB - 1) / TB : nA;
+    const int n = TIER && ctl->tiers.y > 0 ? nM + (a.NB + TB - 1) / TB : nM;
+    const int nt = (n + 1) >> 1;
     const uint32_t full0 = smem_u32(&ctl->full[0]), empty0 = smem_u32(&ctl->empty[0]);
     const int row0 = bh * a.L;                               // first row of this (b, h) in the [BH L, D] view
-    uint32_t pseq = 0;                                       // load warp: tiles issued
+    uint32_t pseq = 0;                                       // load warps: one past the last tile issued
 
-    if (warp == 5) {
+    if (warp == 5 || (TIER && warp == 6)) {
         // ------------------------------------------------------------ loads: Q, K(0), then K(i + 1), V(i) for every i
+        // Tile numbers in the ring are in the order of use. With tiers K and V have a warp each: a gathered unit is up to 64 small
+        // boxes per tensor.
+        const bool k_warp = warp == 5, v_warp = !TIER || warp == 6;
         bool ok = *abort_flag == 0;
         if (ok && nt > 0) {
             if (lane == 0) {
                 tma_prefetch_desc(&tmK);
                 tma_prefetch_desc(&tmV);
-                mbar_arrive_expect_tx(smem_u32(&ctl->qfull), C::TILE);
-                for (int d = 0; d < D / 64; ++d)
-                    tma_load_2d(base + C::Q + d * C::HALF, &tmQ, smem_u32(&ctl->qfull), 64 * d, row0 + qb * TB);
-            }
-            int kwin = lane < n ? block_at(lane) : 0, kbase = 0;   // a window of 32 list entries per tensor
-            int vwin = kwin, vbase = 0;
-            uint32_t slot = 0, par = 1;
-            auto put = [&](const CUtensorMap* m, int& win, int& wbase, int e) {
-                if (!ok || e >= n) return;
-                if ((e & ~31) != wbase) {
-                    wbase = e & ~31;
-                    win = wbase + lane < n ? block_at(wbase + lane) : 0;
+                if (k_warp) {
+                    mbar_arrive_expect_tx(smem_u32(&ctl->qfull), C::TILE);
+                    for (int d = 0; d < D / 64; ++d)
+                        tma_load_2d(base + C::Q + d * C::HALF, &tmQ, smem_u32(&ctl->qfull), 64 * d, row0 + qb * TB);
                 }
-                const int j = __shfl_sync(0xffffffffu, win, e & 31);
+            }
+            int kwin = lane < nA ? block_at(lane) : 0, kbase = 0;   // a window of 32 list entries per tensor
+            int vwin = kwin, vbase = 0;
+            MidWalk walk;
+            if (TIER) walk.start(a.tier, bh, a.NB, qb, lane);
+            auto put = [&](bool is_v, int& win, int& wbase, int e) {
+                if (!ok || e >= n) return;
+                const uint32_t seq = is_v ? e + min(n, (e & ~1) + 4) : e + max(0, (e & ~1) - 2);
+                const uint32_t slot = seq % C::NSLOT, par = ((seq / C::NSLOT) & 1) ^ 1;
+                int j = 0, id = 0;
+                int2 tokens = make_int2(0, 0);
+                if (!TIER || e < nA) {
+                    if ((e & ~31) != wbase) {
+                        wbase = e & ~31;
+                        win = wbase + lane < nA ? block_at(wbase + lane) : 0;
+                    }
+                    j = __shfl_sync(0xffffffffu, win, e & 31);
+                } else {
+                    const int per = TB / a.tier.RM;
+                    if (e < nM) id = walk.blocks((e - nA) * per, per, lane);
+                    if (!is_v) tokens = unit_tokens(a.blk_cnt, a.tier, bh, a.NB, qb, e < nM, id, e - nM, lane);
+                }
                 if (lane == 0) ok = mbar_wait(empty0 + 8 * slot, par, abort_flag, a.status, 401);
                 ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
                 if (!ok) return;
-                if (lane == 0) {
-                    mbar_arrive_expect_tx(full0 + 8 * slot, C::TILE);
+                const uint32_t dst = base + C::RING + slot * C::TILE, bar = full0 + 8 * slot;
+                if (TIER && e >= nA) {
+                    // the counts of unit e - 8 have been read: the tile whose ring slot this is belonged to V(i - 3), i = e / 2
+                    if (!is_v) write_counts(counts + (e % UNIT_RING) * TB, tokens, a.tier.RM, e < nM, lane);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_expect_tx(bar, C::TILE);
+                    __syncwarp();
+                    if (e < nM) {
+                        const int row = bh * a.tier.mid_stride + max(id, 0) * a.tier.RM;
+                        if (lane < TB / a.tier.RM)
+                            for (int d = 0; d < D / 64; ++d)
+                                tma_load_2d(dst + d * C::HALF + lane * a.tier.RM * 128, is_v ? &tmVm : &tmKm, bar, 64 * d, row);
+                    } else if (lane < D / 64) {
+                        tma_load_2d(dst + lane * C::HALF, is_v ? &tmVt : &tmKt, bar, 64 * lane,
+                                    bh * a.tier.tail_stride + (e - nM) * TB);
+                    }
+                } else if (lane == 0) {
+                    mbar_arrive_expect_tx(bar, C::TILE);
 #pragma unroll
-                    for (int d = 0; d < D / 64; ++d)
-                        tma_load_2d(base + C::RING + slot * C::TILE + d * C::HALF, m, full0 + 8 * slot, 64 * d, row0 + j * TB);
+                    for (int d = 0; d < D / 64; ++d) tma_load_2d(dst + d * C::HALF, is_v ? &tmV : &tmK, bar, 64 * d, row0 + j * TB);
                 }
                 __syncwarp();
-                ++pseq;
-                if (++slot == C::NSLOT) { slot = 0; par ^= 1; }
+                pseq = seq + 1;
             };
-            put(&tmK, kwin, kbase, 0);
-            put(&tmK, kwin, kbase, 1);
+            if (k_warp) {
+                put(false, kwin, kbase, 0);
+                put(false, kwin, kbase, 1);
+            }
             for (int i = 0; i < nt; ++i) {
-                put(&tmK, kwin, kbase, 2 * i + 2);
-                put(&tmK, kwin, kbase, 2 * i + 3);
-                put(&tmV, vwin, vbase, 2 * i);
-                put(&tmV, vwin, vbase, 2 * i + 1);
+                if (k_warp) {
+                    put(false, kwin, kbase, 2 * i + 2);
+                    put(false, kwin, kbase, 2 * i + 3);
+                }
+                if (v_warp) {
+                    put(true, vwin, vbase, 2 * i);
+                    put(true, vwin, vbase, 2 * i + 1);
+                }
             }
         }
     } else if (warp == 4) {
@@ -231,16 +285,17 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const int cnt_q = tokens_of(qb);
         float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;      // offsets in use (log2) and row sums relative to them
         bool ok = *abort_flag == 0;
-        int ca = 0, cb = 0;
-        if (n > 0) ca = tokens_of(block_at(0));
-        if (n > 1) cb = tokens_of(block_at(1));
+        // columns of unit e that are not masked here (the means' come with their biases below)
+        auto width = [&](int e) { return e < nA ? tokens_of(block_at(e)) : e < n ? TB : 0; };
+        int ca = width(0), cb = width(1);
+        const float inv_scale = 1.f / a.scale_log2;
         // stmatrix: lane l gives the address of row (l & 7) of 8 x 8 matrix l >> 3: (rows 0-7, 8-15) x (chunk 2 j, 2 j + 1)
         const int prow = 16 * warp + (lane & 7) + ((lane >> 3) & 1) * 8;
         const uint32_t paddr = base + C::P + prow * 128, psw = prow & 7, pch = lane >> 4;
         for (int i = 0; i < nt && ok; ++i) {
             const int cnt_a = ca, cnt_b = cb;
-            ca = 2 * i + 2 < n ? tokens_of(block_at(2 * i + 2)) : 0;
-            cb = 2 * i + 3 < n ? tokens_of(block_at(2 * i + 3)) : 0;
+            ca = width(2 * i + 2);
+            cb = width(2 * i + 3);
             ok = mbar_wait_warp(smem_u32(&ctl->sfull), i & 1, abort_flag, a.status, 407);
             if (!ok) break;
             tc_fence_after();
@@ -257,6 +312,25 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                     const int c = (j & 7) * 8 + 2 * (lane & 3), cnt = j < 8 ? cnt_a : cnt_b;
                     if (c >= cnt) s[4 * j] = s[4 * j + 2] = 0xff800000u;
                     if (c + 1 >= cnt) s[4 * j + 1] = s[4 * j + 3] = 0xff800000u;
+                }
+            }
+            if (TIER) {
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    const int e = 2 * i + b;
+                    if (e < nA || e >= n) continue;
+                    const uint8_t* c8 = counts + (e % UNIT_RING) * TB + 2 * (lane & 3);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        // log2 of 0 .. 64, absolute error below 2^-21 (-inf for 0): a relative 3e-7 of P
+                        const uint32_t cc = *reinterpret_cast<const uint16_t*>(c8 + 8 * j);
+                        const float b0 = __log2f((float)(cc & 255u)) * inv_scale, b1 = __log2f((float)(cc >> 8)) * inv_scale;
+                        uint32_t* x = s + 32 * b + 4 * j;
+                        x[0] = __float_as_uint(__uint_as_float(x[0]) + b0);
+                        x[1] = __float_as_uint(__uint_as_float(x[1]) + b1);
+                        x[2] = __float_as_uint(__uint_as_float(x[2]) + b0);
+                        x[3] = __float_as_uint(__uint_as_float(x[3]) + b1);
+                    }
                 }
             }
             float x0 = -INFINITY, x1 = -INFINITY;
@@ -381,7 +455,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
     // ---------------------------------------------------------------- teardown
     __syncwarp();
-    if (warp == 5 && lane == 0 && *abort_flag) {
+    if (warp >= 5 && lane == 0 && *abort_flag) {
         // a wait gave up: give the loads of this warp a moment (100 us in all) to land before shared memory goes away
         const uint64_t t_end = global_timer_ns() + 100000ull;
         for (uint32_t back = 1; back <= (uint32_t)C::NSLOT && back <= pseq; ++back) {
@@ -406,9 +480,9 @@ static int launch_fwd(const void* q, const void* k, const void* v, FwdTcArgs a, 
     if ((rc = make_token_map<T>(&tq, q, D, rows)) || (rc = make_token_map<T>(&tk, k, D, rows)) ||
         (rc = make_token_map<T>(&tv, v, D, rows)))
         return rc;
-    auto kern = attn_fwd_tc_kernel<T, D>;
+    auto kern = attn_fwd_tc_kernel<T, D, false>;
     if ((rc = opt_in_shared_memory((const void*)kern, (int)FwdCfg<D>::BYTES))) return rc;
-    kern<<<grid, FW_THREADS, FwdCfg<D>::BYTES, st>>>(tq, tk, tv, a);
+    kern<<<grid, FW_THREADS, FwdCfg<D>::BYTES, st>>>(tq, tk, tv, tk, tv, tk, tv, a);
     ES_CHECK_LAUNCH("attn_fwd_tc_kernel");
     return 0;
 }
@@ -420,11 +494,42 @@ int attn_fwd_tc(const void* q, const void* k, const void* v, void* o, float* lse
                 float* part_o, float* part_lse, cudaStream_t st) {
     int* status = device_status_ptr();
     if (!status) return set_error(-2, "attn_fwd_tc: the device status word is not available on this device");
-    const FwdTcArgs a{o, lse, row_ptr, col_idx, blk_cnt, L, L / TB, rows, kLog2e / sqrtf((float)D), tasks, task_info, part_o, part_lse, status};
+    const FwdTcArgs a{o, lse, row_ptr, col_idx, blk_cnt, L, L / TB, rows, kLog2e / sqrtf((float)D), tasks, task_info, part_o, part_lse, status, {}};
     const dim3 grid = tasks ? dim3(n_tasks, 1) : dim3(L / TB, BH);
     if (D == 64)
         return dtype == 0 ? launch_fwd<__nv_bfloat16, 64>(q, k, v, a, BH, grid, st) : launch_fwd<__half, 64>(q, k, v, a, BH, grid, st);
     return dtype == 0 ? launch_fwd<__nv_bfloat16, 128>(q, k, v, a, BH, grid, st) : launch_fwd<__half, 128>(q, k, v, a, BH, grid, st);
+}
+
+template <typename T, int D>
+static int launch_tier_fwd(const void* q, const void* k, const void* v, const void* k_mid, const void* v_mid, const void* k_tail,
+                           const void* v_tail, const FwdTcArgs& a, int BH, cudaStream_t st) {
+    CUtensorMap t[7];
+    const long long tok = (long long)BH * a.L, mid = (long long)BH * a.tier.mid_stride, tail = (long long)BH * a.tier.tail_stride;
+    const void* p[7] = {q, k, v, k_mid, v_mid, k_tail, v_tail};
+    const long long rows[7] = {tok, tok, tok, mid, mid, tail, tail};
+    for (int i = 0; i < 7; ++i)
+        if (int rc = make_token_map<T>(&t[i], p[i], D, rows[i], i == 3 || i == 4 ? a.tier.RM : TB)) return rc;
+    auto kern = attn_fwd_tc_kernel<T, D, true>;
+    if (int rc = opt_in_shared_memory((const void*)kern, (int)FwdCfg<D>::BYTES_TIER)) return rc;
+    kern<<<dim3(a.NB, BH), FW_THREADS_TIER, FwdCfg<D>::BYTES_TIER, st>>>(t[0], t[1], t[2], t[3], t[4], t[5], t[6], a);
+    ES_CHECK_LAUNCH("attn_fwd_tc_kernel");
+    return 0;
+}
+
+// The three-tier forward; the caller has checked the pointers and sizes.
+int tier_fwd_tc(const void* q, const void* k, const void* v, const void* k_mid, const void* v_mid, const void* k_tail,
+                const void* v_tail, void* o, float* lse, const int* row_ptr, const int* col_idx, const TierMaps& tier,
+                const int* blk_cnt, int BH, int L, int D, int dtype, cudaStream_t st) {
+    int* status = device_status_ptr();
+    if (!status) return set_error(-2, "tier_fwd_tc: the device status word is not available on this device");
+    const FwdTcArgs a{o, lse, row_ptr, col_idx, blk_cnt, L, L / TB, 0, kLog2e / sqrtf((float)D), nullptr, nullptr, nullptr, nullptr,
+                      status, tier};
+    if (D == 64)
+        return dtype == 0 ? launch_tier_fwd<__nv_bfloat16, 64>(q, k, v, k_mid, v_mid, k_tail, v_tail, a, BH, st)
+                          : launch_tier_fwd<__half, 64>(q, k, v, k_mid, v_mid, k_tail, v_tail, a, BH, st);
+    return dtype == 0 ? launch_tier_fwd<__nv_bfloat16, 128>(q, k, v, k_mid, v_mid, k_tail, v_tail, a, BH, st)
+                      : launch_tier_fwd<__half, 128>(q, k, v, k_mid, v_mid, k_tail, v_tail, a, BH, st);
 }
 
 }  // namespace vsa
