@@ -64,9 +64,9 @@ struct Ctl {
     uint32_t tmem_base;
     int abort;
     int flag_part[4];
-    int redo;                          // some row left the range of the offset from a sample
     float l_part[2][BM];               // row sums of the two column halves
     float m_part[2][BM];               // row maxima of the two column halves (fallback sweep)
+    int redo;                          // some row left the range of the offset from a sample
 };
 static_assert(sizeof(Ctl) <= 3072, "control block");
 

@@ -326,53 +326,51 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
         const uint32_t tw = tmem + ((uint32_t)(32 * rq) << 16);
         const uint32_t prow = base + r * 128, psw = r & 7;
         bool ok = *abort_flag == 0;
-        // the walked row's block, and in the dK / dV pass its offset and delta, one iteration ahead
-        auto fetch = [&](int i, bool& valid, float& off, float& dl) {
+        // The walked row's block id is requested two iterations ahead and what hangs on it (the block's tokens, in the dK / dV
+        // pass the row's LSE and delta) one ahead, and nothing is computed from a loaded value before its own iteration: a warp
+        // issues in order, so one use of a load that is still on its way would stall the current iteration's exponentials.
+        auto walked = [&](int i) -> int {
             const int e = 2 * i + (r >> 6);
-            valid = e < nA;
-            off = dl = 0.f;
-            if (!valid) return;
-            const int j = block_at(e);
-            valid = (r & 63) < tokens_of(j);
+            return i < nt && e < nA ? block_at(e) : -1;
+        };
+        int n_blk = walked(0), n2_blk = walked(1), n_cnt = 0;
+        float n_lse = 0.f, n_delta = 0.f;
+        // BWD_REP: the tier words of (this warp's query block, the tile's columns)
+        uint32_t n_wa = 0, n_wab = 0;
+        const int rep_word = (rep_blk >> 5) + (rep_mid ? 0 : ch);
+        auto request = [&](int jb) {
+            if (jb < 0) return;
+            n_cnt = tokens_of(jb);
             if (KV) {
-                const size_t g = (size_t)row0 + (size_t)j * TB + (r & 63);
-                const float l = __ldg(a.lse + g);
-                valid = valid && l != -INFINITY;
-                off = -l * kLog2e;
-                dl = __ldg(a.delta + g);
+                const size_t g = (size_t)row0 + (size_t)jb * TB + (r & 63);
+                n_lse = __ldg(a.lse + g);
+                n_delta = __ldg(a.delta + g);
+            }
+            if (REP && rep_word < a.tier.W) {
+                const size_t at = ((size_t)bh * a.NB + jb) * a.tier.W + rep_word;
+                n_wab = __ldg(a.tier.bits_ab + at);
+                n_wa = __ldg(a.tier.bits_a + at);
             }
         };
-        // BWD_REP: the tier word of (this warp's query block, the tile's columns): bit per block that is attended through it
-        auto fetch_bits = [&](int i) -> uint32_t {
-            const int e = 2 * i + (r >> 6), w = (rep_blk >> 5) + (rep_mid ? 0 : ch);
-            if (e >= nA || w >= a.tier.W) return 0u;
-            const size_t at = ((size_t)bh * a.NB + e) * a.tier.W + w;
-            const uint32_t wab = __ldg(a.tier.bits_ab + at);
-            return rep_mid ? (wab & ~__ldg(a.tier.bits_a + at)) >> (rep_blk & 31) : ~wab;
-        };
-        bool nv = false;
-        float noff = 0.f, ndl = 0.f;
-        uint32_t nbits = 0;
-        if (nt > 0) {
-            fetch(0, nv, noff, ndl);
-            if (REP) nbits = fetch_bits(0);
-        }
+        request(n_blk);
         for (int i = 0; i < nt && ok; ++i) {
-            bool valid = nv;
-            float off = noff;
-            const float dl = ndl;
-            uint32_t use = 0xFFFFFFFFu;                      // bit c: this thread's column c is used by the row's block
-            if (REP) {
-                const int b = rep_mid ? (32 * ch + lane) / a.tier.RM : lane;
-                use = __ballot_sync(0xffffffffu, (nbits >> b) & 1u);
-            }
-            if (i + 1 < nt) {
-                fetch(i + 1, nv, noff, ndl);
-                if (REP) nbits = fetch_bits(i + 1);
-            }
+            const int blk = n_blk, cnt_w = n_cnt;
+            const float lse_w = n_lse, dl = n_delta;
+            const uint32_t wa = n_wa, wab = n_wab;
+            n_blk = n2_blk;
+            request(n_blk);
+            n2_blk = walked(i + 2);
             ok = mbar_wait_warp(smem_u32(&ctl->sfull[i & 1]), (i >> 1) & 1, abort_flag, a.status, 506);
             if (!ok) break;
             tc_fence_after();
+            bool valid = blk >= 0 && (r & 63) < cnt_w && (!KV || lse_w != -INFINITY);
+            float off = KV ? -lse_w * kLog2e : 0.f;
+            uint32_t use = 0xFFFFFFFFu;                      // bit c: this thread's column c is used by the row's block
+            if (REP) {
+                const uint32_t bits = blk < 0 || rep_word >= a.tier.W ? 0u : rep_mid ? (wab & ~wa) >> (rep_blk & 31) : ~wab;
+                const int b = rep_mid ? (32 * ch + lane) / a.tier.RM : lane;
+                use = __ballot_sync(0xffffffffu, (bits >> b) & 1u);
+            }
             if (TIER && 2 * i + (r >> 6) >= nA && 2 * i + (r >> 6) < n) {
                 const int c = counts[((2 * i + (r >> 6)) % UNIT_RING) * TB + (r & 63)];
                 valid = c > 0;
