@@ -15,15 +15,18 @@
 //   warps 0-7  P and dS: warp w owns rows 32 (w % 4) .. + 31 and columns 32 (w / 4) .. + 31
 //   warp 8     issues the MMAs; warp 9 issues the TMA loads
 // Tensor memory: (S, dP) of even and of odd iterations (4 x 64 columns), G1^T, G2^T (2 x 64). S and dP of iteration i + 1 are
-// computed while the warps work on iteration i. X tiles (32 KB at D = 128) go through a ring of five slots (ten at D = 64).
+// computed while the warps work on iteration i. X1 and X2 tiles (32 KB at D = 128) have a ring each, of three and two slots (five
+// and five at D = 64): the dQ passes free X2 as soon as dP has read it. Where the second products need both (dK / dV at D = 128),
+// one ring of five in the order of use is 3 % faster.
 //
-// What bounds it: shared memory. At D = 128 the MMAs read 96 KB per pair of blocks (72 KB in the dQ pass) and the loads fill 32
-// KB, 1,000 (830) clocks at 128 B/clock; the ring's five slots leave the X2 tile of the next iteration half an iteration of
-// lead. 32,768 tokens x 12 heads, 32 blocks per list: dK / dV 1.20 ms, dQ 1.09 ms (mma.sync: 2.27 and 1.68 ms); at D = 64 0.94
-// and 0.78 ms (1.29 and 0.91 ms), where M = D = 64 gradient products take half of the tensor pipe.
+// What bounds it: the hand-overs. The MMAs take 1,024 (768) clocks per two blocks at D = 128 and their operands 1,500 (1,150) of
+// shared memory's, of 3,300 (2,400) measured: a tile's load, its products, P / dS and the second products follow one another
+// with too few slots to have more than one and a half iterations on their way. 32,768 tokens x 12 heads, 32 blocks per list:
+// dK / dV 1.19 ms, dQ 0.88 ms (mma.sync: 2.27 and 1.68 ms); at D = 64 0.86 and 0.71 ms (1.29 and 0.91 ms), where M = D = 64
+// gradient products take half of the tensor pipe.
 //
 // BWD_TIER_Q, BWD_REP: the three tiers of resolution, see the modes below. 512 blocks x 12 heads, 32 + 102 blocks in tiers A and B:
-// dQ 2.19 ms, tables 1.91 ms (mma.sync: 2.63 and 3.32 ms).
+// dQ 1.85 ms, tables 1.7 ms (mma.sync: 2.63 and 3.32 ms).
 #include "es_vsa_tc.cuh"
 
 namespace es {
@@ -34,6 +37,7 @@ constexpr int TB = 64;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr int BW_THREADS = 320, BW_THREADS_TIER = 352;
 constexpr uint32_t Y_HALF = TB * 128, X_HALF = 128 * 128;                // 64 d of an owner / a walked tile
+constexpr int COUNT_RING = 16;                                           // units whose column counts are staged
 constexpr uint32_t DS_BYTES = 128 * 128;                                 // P, dS: [128 rows][64 columns] 16-bit
 // BWD_TIER_Q: the dQ pass over the units of all three tiers. BWD_REP: the dK / dV pass for 64 consecutive rows of a table of
 // representatives (group means, then block means) as the owner; it walks every query block, in fp32 tables and masked by the
@@ -41,11 +45,12 @@ constexpr uint32_t DS_BYTES = 128 * 128;                                 // P, d
 enum BwdMode { BWD_KV, BWD_Q, BWD_TIER_Q, BWD_REP };
 template <int D, int MODE> struct BwdCfg {
     static constexpr bool KV = MODE == BWD_KV || MODE == BWD_REP;
-    static constexpr int DH = D / 64, NSLOT = D == 128 ? 5 : 10;
+    static constexpr int DH = D / 64, N1 = D == 128 ? 3 : 5, N2 = D == 128 ? 2 : 5;   // slots of X1 and of X2
+    static constexpr bool SHARED = KV && D == 128;                       // one ring of N1 + N2 slots instead
     static constexpr uint32_t Y_TILE = DH * Y_HALF, X_TILE = DH * X_HALF;   // [d half][rows][128 B]
     static constexpr uint32_t Y1 = 0, Y2 = Y_TILE, DS = 2 * Y_TILE, P = DS + DS_BYTES;
-    static constexpr uint32_t RING = P + (KV ? DS_BYTES : 0u), CTL = RING + NSLOT * X_TILE, COUNTS = CTL + 1024;
-    static constexpr uint32_t BYTES = COUNTS + (MODE == BWD_TIER_Q ? UNIT_RING * TB : 0);   // column counts of the units
+    static constexpr uint32_t RING = P + (KV ? DS_BYTES : 0u), CTL = RING + (N1 + N2) * X_TILE, COUNTS = CTL + 1024;
+    static constexpr uint32_t BYTES = COUNTS + (MODE == BWD_TIER_Q ? COUNT_RING * TB : 0);   // column counts of the units
     static constexpr int LD = D + 4;                                     // epilogue staging: floats per token row
 };
 
@@ -97,7 +102,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
     constexpr bool TIER = MODE == BWD_TIER_Q, REP = MODE == BWD_REP;
     using C = BwdCfg<D, MODE>;
     constexpr bool KV = C::KV;
-    constexpr int NSLOT = C::NSLOT, DH = C::DH;
+    constexpr int N1 = C::N1, N2 = C::N2, DH = C::DH;
     constexpr uint32_t Y_TILE = C::Y_TILE, X_TILE = C::X_TILE;
     extern __shared__ __align__(1024) uint8_t smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -127,7 +132,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
     const int cnt_o = REP ? min(TB, (rep_mid ? a.NB * a.tier.RM : a.NB) - rep_tile * TB) : tokens_of(ob);
     if (tid == 0) {
         mbar_init(smem_u32(&ctl->yfull), 1);
-        for (int i = 0; i < NSLOT; ++i) {
+        for (int i = 0; i < N1 + N2; ++i) {
             mbar_init(smem_u32(&ctl->full[i]), 1);
             mbar_init(smem_u32(&ctl->empty[i]), 1);
         }
@@ -174,7 +179,10 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
     const int nt = (n + 1) >> 1;
     constexpr uint32_t G1 = 256, G2 = 320;                   // accumulator columns
     const uint32_t full0 = smem_u32(&ctl->full[0]), empty0 = smem_u32(&ctl->empty[0]);
-    uint32_t pseq = 0;                                       // load warp: tiles issued
+    int issued[2] = {0, 0};                                  // load warps: X1 and X2 tiles issued
+    // tile number i of X1 / X2: its index among the slots and barriers, and the phase of its full barrier
+    auto slot_of = [&](int x, int i) { return C::SHARED ? (2 * i + x) % (N1 + N2) : x ? N1 + i % N2 : i % N1; };
+    auto phase_of = [&](int x, int i) { return (uint32_t)(C::SHARED ? (2 * i + x) / (N1 + N2) : i / (x ? N2 : N1)) & 1u; };
 
     if (warp == 9 || (TIER && warp == 10)) {
         // ------------------------------------------------------------ loads: Y1, Y2, then X1(i), X2(i)
@@ -217,16 +225,16 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
                 }
 #pragma unroll 1
                 for (int x = x_first; x <= x_last; ++x) {
-                    const uint32_t seq = 2 * i + x, slot = seq % NSLOT, par = ((seq / NSLOT) & 1) ^ 1;
+                    const uint32_t slot = slot_of(x, i), par = phase_of(x, i) ^ 1;
                     if (lane == 0) ok = mbar_wait(empty0 + 8 * slot, par, abort_flag, a.status, 501);
                     ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
                     if (!ok) break;
                     if (TIER && !lists && x == 0) {
-                        // the counts' slots are free: the P / dS warps are through all but the last two iterations
+                        // the counts' slots are free: the tile this one replaces was released after iteration i - N1
 #pragma unroll
                         for (int b = 0; b < 2; ++b) {
                             if (e + b >= nA && e + b < n)
-                                write_counts(counts + ((e + b) % UNIT_RING) * TB, tokens[b], a.tier.RM, e + b < nM, lane);
+                                write_counts(counts + ((e + b) % COUNT_RING) * TB, tokens[b], a.tier.RM, e + b < nM, lane);
                         }
                         __syncwarp();
                     }
@@ -256,7 +264,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
                                     full0 + 8 * slot, 64 * d, row0 + (b ? j1 : j0) * TB);
                     }
                     __syncwarp();
-                    pseq = seq + 1;
+                    issued[x] = i + 1;
                 }
             }
         }
@@ -268,52 +276,88 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
         const uint32_t k_hi = (uint32_t)(dk0 >> 32), k_lo = (uint32_t)dk0, x_hi = (uint32_t)(dx0 >> 32), x_lo = (uint32_t)dx0;
         bool ok = *abort_flag == 0;
         if (nt > 0) ok = ok && mbar_wait_warp(smem_u32(&ctl->yfull), 0, abort_flag, a.status, 502);
-        // tile number s of the ring sits in slot s % NSLOT, its full barrier in phase (s / NSLOT) & 1
-        auto issue_s = [&](int i) {
-#pragma unroll 1
-            for (int x = 0; x < 2; ++x) {
-                const uint32_t seq = 2 * i + x, s = seq % NSLOT;
-                ok = ok && mbar_wait_warp(full0 + 8 * s, (seq / NSLOT) & 1, abort_flag, a.status, 503);
-                if (!ok) return;
-                tc_fence_after();
-                if (elect_one()) {
-                    const uint32_t xa = k_lo + ((base + C::RING + s * X_TILE) >> 4);
-                    const uint32_t yb = k_lo + ((base + (x ? C::Y2 : C::Y1)) >> 4);
-                    const uint32_t d = tmem + (i & 1) * 128 + x * 64;
+        auto ready = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_test_wait(bar, parity)) != 0; };
+        auto issue_s = [&](int x, int i) {                  // x = 0: S(i), x = 1: dP(i)
+            tc_fence_after();
+            if (elect_one()) {
+                const uint32_t slot = slot_of(x, i);
+                const uint32_t xa = k_lo + ((base + C::RING + slot * X_TILE) >> 4);
+                const uint32_t yb = k_lo + ((base + (x ? C::Y2 : C::Y1)) >> 4);
+                const uint32_t d = tmem + (i & 1) * 128 + x * 64;
 #pragma unroll
-                    for (int ks = 0; ks < D / 16; ++ks)
-                        umma_ss_lohi(d, xa + (((ks >> 2) * X_HALF + (ks & 3) * 32) >> 4), k_hi,
-                                     yb + (((ks >> 2) * Y_HALF + (ks & 3) * 32) >> 4), k_hi, ID_S, ks > 0);
-                    // the dQ pass needs V no more. (With tiers V goes with K at the end of the iteration: X1's and X2's load warps
-                    // wait on each other's slots, and a wait can only tell two consecutive rounds of a slot apart.)
-                    if (MODE == BWD_Q && x == 1) umma_commit(empty0 + 8 * s);
-                    if (x == 1) umma_commit(smem_u32(&ctl->sfull[i & 1]));
-                }
-                __syncwarp();
+                for (int ks = 0; ks < D / 16; ++ks)
+                    umma_ss_lohi(d, xa + (((ks >> 2) * X_HALF + (ks & 3) * 32) >> 4), k_hi,
+                                 yb + (((ks >> 2) * Y_HALF + (ks & 3) * 32) >> 4), k_hi, ID_S, ks > 0);
+                if (!KV && x == 1) umma_commit(empty0 + 8 * slot);    // the dQ passes need V no more
+                if (x == 1) umma_commit(smem_u32(&ctl->sfull[i & 1]));
             }
+            __syncwarp();
         };
-        if (nt > 0 && ok) issue_s(0);
-        for (int i = 0; i < nt && ok; ++i) {
-            if (i + 1 < nt) issue_s(i + 1);       // its S / dP columns were read before P and dS of iteration i - 1 were stored
-            ok = ok && mbar_wait_warp(smem_u32(&ctl->pfull), i & 1, abort_flag, a.status, 504);
-            if (!ok) break;
+        auto issue_g = [&](int i) {
             tc_fence_after();
             if (elect_one()) {
                 const int ksteps = 2 * i + 1 < n ? 8 : 4;      // an odd end has 64 rows: the other half of the slot is stale
 #pragma unroll 1
                 for (int x = 0; x < (KV ? 2 : 1); ++x) {
-                    const uint32_t s = (uint32_t)(2 * i + x) % NSLOT;
-                    const uint32_t xa = x_lo + ((base + C::RING + s * X_TILE) >> 4);
+                    const uint32_t slot = slot_of(x, i);
+                    const uint32_t xa = x_lo + ((base + C::RING + slot * X_TILE) >> 4);
                     const uint32_t pb = k_lo + ((base + (x ? C::P : C::DS)) >> 4);
                     for (int ks = 0; ks < ksteps; ++ks)
                         umma_ss_lohi(tmem + (x ? G2 : G1), xa + ((ks * 2048) >> 4), x_hi, pb + ((ks * 2048) >> 4), k_hi, ID_G,
                                      (i > 0 || ks > 0) ? 1u : 0u);
-                    umma_commit(empty0 + 8 * s);
+                    umma_commit(empty0 + 8 * slot);
                 }
-                if (TIER) umma_commit(empty0 + 8 * ((uint32_t)(2 * i + 1) % NSLOT));
                 umma_commit(smem_u32(&ctl->pvdone));
             }
             __syncwarp();
+        };
+        if (C::SHARED) {
+            // in the order of the ring (choosing as below is 2 to 6 % slower here)
+            auto issue_both = [&](int i) {
+                for (int x = 0; x < 2; ++x) {
+                    ok = ok && mbar_wait_warp(full0 + 8 * slot_of(x, i), phase_of(x, i), abort_flag, a.status, 504);
+                    if (ok) issue_s(x, i);
+                }
+            };
+            if (nt > 0) issue_both(0);
+            for (int i = 0; i < nt && ok; ++i) {
+                if (i + 1 < nt) issue_both(i + 1);
+                ok = ok && mbar_wait_warp(smem_u32(&ctl->pfull), i & 1, abort_flag, a.status, 509);
+                if (ok) issue_g(i);
+            }
+        }
+        // Whatever is ready goes next: in a fixed order the second products of one iteration waited for the X2 tile of the next
+        // but one, and that tile for the slot they free. S and dP of iteration i write the columns of i - 2, which the P / dS
+        // warps had read when they handed over P and dS of i - 2 (seen here before the second products of i - 2 were issued).
+        int si = 0, di = 0, gi = 0;                            // next S, dP and second products
+        uint32_t idle = 0, late = 0;
+        int64_t t0 = 0;
+        while (!C::SHARED && ok && gi < nt) {
+            bool did = false;
+            if (gi < di && ready(smem_u32(&ctl->pfull), gi & 1)) { issue_g(gi++); did = true; }
+            if (si < nt && si <= gi + 1 && ready(full0 + 8 * slot_of(0, si), phase_of(0, si))) { issue_s(0, si++); did = true; }
+            if (di < si && ready(full0 + 8 * slot_of(1, di), phase_of(1, di))) { issue_s(1, di++); did = true; }
+            if (did) {
+                idle = 0;
+                continue;
+            }
+            // a bounded wait, as mbar_wait
+            if (idle == 0) {
+                t0 = (int64_t)global_timer_ns();
+                late = 0;
+            }
+            if ((++idle & 255u) == 0) {
+                const bool gone = (int64_t)global_timer_ns() - t0 > (int64_t)kWaitLimitNs;
+                late = gone ? late + 1 : 0;
+                const bool stop = *abort_flag || *reinterpret_cast<volatile int*>(a.status) != 0 || late >= 2;
+                if (__any_sync(0xffffffffu, stop)) {
+                    if (lane == 0) {
+                        *abort_flag = 1;
+                        atomicCAS(a.status, 0, 503 + 1000 * (int)(blockIdx.x % 100000));
+                    }
+                    ok = false;
+                }
+            }
         }
         // every MMA issued above has finished before tensor memory is freed
         if (elect_one()) umma_commit(smem_u32(&ctl->drain));
@@ -372,7 +416,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
                 use = __ballot_sync(0xffffffffu, (bits >> b) & 1u);
             }
             if (TIER && 2 * i + (r >> 6) >= nA && 2 * i + (r >> 6) < n) {
-                const int c = counts[((2 * i + (r >> 6)) % UNIT_RING) * TB + (r & 63)];
+                const int c = counts[((2 * i + (r >> 6)) % COUNT_RING) * TB + (r & 63)];
                 valid = c > 0;
                 off = __log2f((float)max(c, 1));                // as in the forward
             }
@@ -510,10 +554,9 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
     if (warp >= 9 && lane == 0 && *abort_flag) {
         // a wait gave up: give the loads of this warp a moment (100 us in all) to land before shared memory goes away
         const uint64_t t_end = global_timer_ns() + 100000ull;
-        for (uint32_t back = 1; back <= (uint32_t)NSLOT && back <= pseq; ++back) {
-            const uint32_t sq = pseq - back;
-            while (!mbar_try_wait(full0 + 8 * (sq % NSLOT), (sq / NSLOT) & 1) && global_timer_ns() < t_end) {}
-        }
+        for (int x = 0; x < 2; ++x)
+            for (int i = max(0, issued[x] - N1); i < issued[x]; ++i)
+                while (!mbar_try_wait(full0 + 8 * slot_of(x, i), phase_of(x, i)) && global_timer_ns() < t_end) {}
     }
     __syncwarp();
     tc_fence_before();

@@ -149,12 +149,14 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             }
             int kwin = lane < nA ? block_at(lane) : 0, kbase = 0;   // a window of 32 list entries per tensor
             int vwin = kwin, vbase = 0;
+            uint32_t next_slot = 0, next_par = 1;
             MidWalk walk;
             if (TIER) walk.start(a.tier, bh, a.NB, qb, lane);
             auto put = [&](bool is_v, int& win, int& wbase, int e) {
                 if (!ok || e >= n) return;
-                const uint32_t seq = is_v ? e + min(n, (e & ~1) + 4) : e + max(0, (e & ~1) - 2);
-                const uint32_t slot = seq % C::NSLOT, par = ((seq / C::NSLOT) & 1) ^ 1;
+                // with one warp for both, the next slot; else the tile's number in the order of use
+                const uint32_t seq = !TIER ? pseq : is_v ? e + min(n, (e & ~1) + 4) : e + max(0, (e & ~1) - 2);
+                const uint32_t slot = TIER ? seq % C::NSLOT : next_slot, par = TIER ? ((seq / C::NSLOT) & 1) ^ 1 : next_par;
                 int j = 0, id = 0;
                 int2 tokens = make_int2(0, 0);
                 if (!TIER || e < nA) {
@@ -194,6 +196,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                 }
                 __syncwarp();
                 pseq = seq + 1;
+                if (!TIER && ++next_slot == C::NSLOT) { next_slot = 0; next_par ^= 1; }
             };
             if (k_warp) {
                 put(false, kwin, kbase, 0);
