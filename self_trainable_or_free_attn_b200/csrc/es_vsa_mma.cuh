@@ -52,10 +52,6 @@ __device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t& r0, uint32_t& r1,
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr));
 }
-__device__ __forceinline__ void ldsm4t(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr));
-}
 __device__ __forceinline__ void cp16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
@@ -87,12 +83,6 @@ template <int D> __device__ __forceinline__ void load_b_nk(uint32_t tile, int np
     const int row = np * 16 + ((lane >> 4) << 3) + (lane & 7), ch = 2 * ks + ((lane >> 3) & 1);
     ldsm4(tile + tile_off<D>(row, ch), b[0], b[1], b[2], b[3]);
 }
-// B fragments of the n tiles 2 dp and 2 dp + 1 for k step kt (16 rows of the tile), from a tile stored [k][n] (the "V" use).
-template <int D> __device__ __forceinline__ void load_b_kn(uint32_t tile, int kt, int dp, int lane, uint32_t (&b)[4]) {
-    const int row = kt * 16 + (((lane >> 3) & 1) << 3) + (lane & 7), ch = 2 * dp + (lane >> 4);
-    ldsm4t(tile + tile_off<D>(row, ch), b[0], b[1], b[2], b[3]);
-}
-
 __device__ __forceinline__ float quad_max(float x) {
     x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 1));
     return fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 2));
@@ -100,11 +90,6 @@ __device__ __forceinline__ float quad_max(float x) {
 __device__ __forceinline__ float quad_sum(float x) {
     x += __shfl_xor_sync(0xffffffffu, x, 1);
     return x + __shfl_xor_sync(0xffffffffu, x, 2);
-}
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
 }
 
 }  // namespace vsa
