@@ -49,9 +49,9 @@ constexpr uint32_t HALF_BYTES = TILE_BYTES / 2;  // one d half: 128 rows x 128 B
 constexpr uint32_t BLK_BYTES = BK * 128;         // 64 rows of one d half: one TMA box
 constexpr uint32_t SMEM_RING = 0;
 constexpr uint32_t SMEM_CTL = SMEM_RING + NSLOT * TILE_BYTES;
-constexpr uint32_t SMEM_BIAS = SMEM_CTL + 3072;                        // [NBIAS][128] floats
+constexpr uint32_t SMEM_BIAS = SMEM_CTL + 3584;                        // [NBIAS][128] floats
 constexpr uint32_t SMEM_MASS = SMEM_BIAS + NBIAS * 128 * 4;            // [NMASS][2 column halves][128 rows] floats
-constexpr uint32_t SMEM_ALLOC = SMEM_MASS + NMASS * 2 * BM * 4;        // 211,968 B: one CTA per SM
+constexpr uint32_t SMEM_ALLOC = SMEM_MASS + NMASS * 2 * BM * 4;        // 212,480 B: one CTA per SM
 
 struct Ctl {
     uint64_t qfull;
@@ -66,9 +66,10 @@ struct Ctl {
     int flag_part[4];
     float l_part[2][BM];               // row sums of the two column halves
     float m_part[2][BM];               // row maxima of the two column halves (fallback sweep)
+    float r_part[2][BM];               // dense: row sums of the rounded P
     int redo;                          // some row left the range of the offset from a sample
 };
-static_assert(sizeof(Ctl) <= 3072, "control block");
+static_assert(sizeof(Ctl) <= 3584, "control block");
 
 struct AttnArgs {
     const __nv_bfloat16* q;      // (L, H, 128)
@@ -645,7 +646,8 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
 
         // ---- epilogue: row sums of both column halves, then this thread's 64 columns of O
         ctl->l_part[ch][trow] = lsum.x + lsum.y;
-        if (DENSE) ctl->m_part[ch][trow] = rsum.x + rsum.y;    // every row has read its maxima by now (ofull came after)
+        // (not in m_part: with one or two iterations nothing keeps the other half's warp from still reading its maxima)
+        if (DENSE) ctl->r_part[ch][trow] = rsum.x + rsum.y;
         mbar_arrive(smem_u32(&ctl->lbar));
         ok = mbar_wait_warp(smem_u32(&ctl->lbar), FALLBACK ? 1 : 0, abort_flag, a.status, 307) && ok;
         const float l = ctl->l_part[0][trow] + ctl->l_part[1][trow];
@@ -654,7 +656,7 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
         if (nt > 0) ok = mbar_wait_warp(smem_u32(&ctl->ofull), 0, abort_flag, a.status, 303) && ok;
         if (ok) {
             tc_fence_after();
-            const float inv = COMPENSATE ? 1.0f / (1.0f + l) : DENSE ? 1.0f / (ctl->m_part[0][trow] + ctl->m_part[1][trow]) : 1.0f / l;
+            const float inv = COMPENSATE ? 1.0f / (1.0f + l) : DENSE ? 1.0f / (ctl->r_part[0][trow] + ctl->r_part[1][trow]) : 1.0f / l;
             bool finite = true;
             __nv_bfloat16* orow = a.out + ((size_t)row * a.H + h) * HD + 64 * ch;
 #pragma unroll
