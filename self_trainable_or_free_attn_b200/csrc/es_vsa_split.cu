@@ -132,8 +132,11 @@ __global__ void __launch_bounds__(128) split_merge_kernel(const MergeArgs a) {
         float lse = -INFINITY;
         if (FWD) {
             if (row < cnt || !a.mask_rows) {
-                float mx = -INFINITY;
-                for (int j = 0; j < c; ++j) mx = fmaxf(mx, a.part_lse[(size_t)(slot0 + j) * TB + row]);
+                float mx = -INFINITY;                          // NaN as soon as one partial is (fmaxf would drop it)
+                for (int j = 0; j < c; ++j) {
+                    const float x = a.part_lse[(size_t)(slot0 + j) * TB + row];
+                    mx = x > mx || x != x ? x : mx;
+                }
                 if (mx != -INFINITY) {
                     float sum = 0.f;
                     for (int j = 0; j < c; ++j) {

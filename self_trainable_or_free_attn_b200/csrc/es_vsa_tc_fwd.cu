@@ -414,7 +414,8 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             const int r0 = warp * 16 + (lane >> 2), r1 = r0 + 8;
             // a chunk of a split row writes every row (the merge masks the padded ones)
             const bool part = slot_out >= 0;
-            const bool ok0 = (part || r0 < cnt_q) && l0 > 0.f, ok1 = (part || r1 < cnt_q) && l1 > 0.f;
+            // a row sum of 0 is a row without a key; one that is NaN (a NaN or infinite logit) stays NaN in O and in the LSE
+            const bool ok0 = (part || r0 < cnt_q) && l0 != 0.f, ok1 = (part || r1 < cnt_q) && l1 != 0.f;
             const float i0 = ok0 ? 1.f / l0 : 0.f, i1 = ok1 ? 1.f / l1 : 0.f;
             T* out = static_cast<T*>(a.o) + ((size_t)row0 + (size_t)qb * TB) * D;
             float* po = part ? a.part_o + (size_t)slot_out * TB * D : nullptr;
@@ -444,8 +445,8 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             }
             if ((lane & 3) == 0) {
                 if (part) {
-                    a.part_lse[(size_t)slot_out * TB + r0] = l0 > 0.f ? m0 + log2f(l0) : -INFINITY;
-                    a.part_lse[(size_t)slot_out * TB + r1] = l1 > 0.f ? m1 + log2f(l1) : -INFINITY;
+                    a.part_lse[(size_t)slot_out * TB + r0] = ok0 ? m0 + log2f(l0) : -INFINITY;
+                    a.part_lse[(size_t)slot_out * TB + r1] = ok1 ? m1 + log2f(l1) : -INFINITY;
                 } else {
                     float* lse = a.lse + (size_t)row0 + (size_t)qb * TB;
                     lse[r0] = ok0 ? (m0 + log2f(l0)) * kLn2 : -INFINITY;
