@@ -58,7 +58,7 @@ struct BwdCtl {
     uint64_t yfull, full[10], empty[10], sfull[2], pfull, pvdone, drain;
     uint32_t tmem_base;
     int abort;
-    int2 tiers;                                  // BWD_TIER_Q: tier-B blocks, tier-C words of the query block
+    int2 tiers;                                  // BWD_TIER_Q: tier-B and tier-C blocks of the query block
     alignas(16) float lse2[TB], delta[TB];       // the owner's columns: minus their additive terms of the exponent; delta
 };
 static_assert(sizeof(BwdCtl) <= 1024, "control block");
@@ -175,7 +175,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
     // walked units of 64 rows: the list's blocks (every query block for BWD_REP), then the tiers' means as in the forward
     const int nA = TIER && !(a.tier.phases & PH_A) ? 0 : end - beg;
     const int nM = TIER ? nA + (ctl->tiers.x * a.tier.RM + TB - 1) / TB : nA;
-    const int n = TIER && ctl->tiers.y > 0 ? nM + (a.NB + TB - 1) / TB : nM;
+    const int n = TIER ? nM + tail_units(a.tier, a.NB, ctl->tiers.y) : nM;
     const int nt = (n + 1) >> 1;
     constexpr uint32_t G1 = 256, G2 = 320;                   // accumulator columns
     const uint32_t full0 = smem_u32(&ctl->full[0]), empty0 = smem_u32(&ctl->empty[0]);
@@ -203,7 +203,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
                 }
             }
             int win = lane < nA ? block_at(lane) : 0;          // a window of 32 list entries
-            MidWalk walk;
+            TierWalk walk;
             if (TIER) walk.start(a.tier, bh, a.NB, ob, lane);
             for (int i = 0; i < nt && ok; ++i) {
                 const int e = 2 * i;
@@ -211,57 +211,48 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
                 const int j0 = __shfl_sync(0xffffffffu, win, e & 31), j1 = __shfl_sync(0xffffffffu, win, (e + 1) & 31);
                 const int nb = e + 1 < n ? 2 : 1;
                 const bool lists = !TIER || e + nb <= nA;
-                int id[2] = {0, 0};
-                int2 tokens[2] = {};
-                if (TIER && !lists) {
-                    const int per = TB / a.tier.RM;
-#pragma unroll
-                    for (int b = 0; b < 2; ++b) {
-                        if (e + b < nA || e + b >= n) continue;
-                        if (e + b < nM) id[b] = walk.blocks((e + b - nA) * per, per, lane);
-                        if (x_first == 0)
-                            tokens[b] = unit_tokens(a.blk_cnt, a.tier, bh, a.NB, ob, e + b < nM, id[b], e + b - nM, lane);
-                    }
-                }
 #pragma unroll 1
                 for (int x = x_first; x <= x_last; ++x) {
-                    const uint32_t slot = slot_of(x, i), par = phase_of(x, i) ^ 1;
-                    if (lane == 0) ok = mbar_wait(empty0 + 8 * slot, par, abort_flag, a.status, 501);
-                    ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
-                    if (!ok) break;
-                    if (TIER && !lists && x == 0) {
-                        // the counts' slots are free: the tile this one replaces was released after iteration i - N1
-#pragma unroll
-                        for (int b = 0; b < 2; ++b) {
-                            if (e + b >= nA && e + b < n)
-                                write_counts(counts + ((e + b) % COUNT_RING) * TB, tokens[b], a.tier.RM, e + b < nM, lane);
-                        }
+                    const uint32_t slot = slot_of(x, i), par = phase_of(x, i) ^ 1, bar = full0 + 8 * slot;
+                    const uint32_t dst = base + C::RING + slot * X_TILE;
+                    if (lists) {
+                        if (lane == 0) ok = mbar_wait(empty0 + 8 * slot, par, abort_flag, a.status, 501);
+                        ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+                        if (!ok) break;
+                        if (lane == 0) mbar_arrive_expect_tx(bar, nb * Y_TILE);
                         __syncwarp();
-                    }
-                    if (lane == 0) mbar_arrive_expect_tx(full0 + 8 * slot, nb * Y_TILE);
-                    __syncwarp();
-                    if (TIER && !lists) {
-#pragma unroll
-                        for (int b = 0; b < 2; ++b) {
-                            const uint32_t dst = base + C::RING + slot * X_TILE + b * Y_HALF, bar = full0 + 8 * slot;
-                            const int u = e + b;
-                            if (u >= nA && u < nM) {
-                                const int row = bh * a.tier.mid_stride + max(id[b], 0) * a.tier.RM;
-                                if (lane < TB / a.tier.RM)
-                                    for (int d = 0; d < DH; ++d)
-                                        tma_load_2d(dst + d * X_HALF + lane * a.tier.RM * 128, x ? &tmM2 : &tmM1, bar, 64 * d, row);
-                            } else if (u < n && lane < DH) {
-                                const CUtensorMap* m = u < nA ? (x ? &tmX2 : &tmX1) : (x ? &tmT2 : &tmT1);
-                                const int row = u < nA ? row0 + (b ? j1 : j0) * TB : bh * a.tier.tail_stride + (u - nM) * TB;
-                                tma_load_2d(dst + lane * X_HALF, m, bar, 64 * lane, row);
-                            }
+                        // the d halves of the first block, then of the second
+                        if (lane < DH * nb) {
+                            const int d = lane % DH, b = lane / DH;
+                            tma_load_2d(dst + d * X_HALF + b * Y_HALF, x ? &tmX2 : &tmX1, bar, 64 * d, row0 + (b ? j1 : j0) * TB);
                         }
-                    } else
-                    // the d halves of the first block, then of the second
-                    if (lane < DH * nb) {
-                        const int d = lane % DH, b = lane / DH;
-                        tma_load_2d(base + C::RING + slot * X_TILE + d * X_HALF + b * Y_HALF, x ? &tmX2 : &tmX1,
-                                    full0 + 8 * slot, 64 * d, row0 + (b ? j1 : j0) * TB);
+                    } else {
+                        // unit by unit; one copy of the code that finds and loads a unit's means (two: 4 % slower)
+#pragma unroll 1
+                        for (int b = 0; b < nb; ++b) {
+                            const int u = e + b;
+                            int2 id = make_int2(-1, -1), tokens = make_int2(0, 0);
+                            if (u >= nA) {
+                                id = unit_blocks(walk, a.tier, bh, a.NB, ob, u < nM, u < nM ? u - nA : u - nM, lane);
+                                if (x == 0) tokens = unit_tokens(a.blk_cnt, a.tier, bh, a.NB, ob, u < nM, id, u - nM, lane);
+                            }
+                            if (b == 0) {
+                                if (lane == 0) ok = mbar_wait(empty0 + 8 * slot, par, abort_flag, a.status, 501);
+                                ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+                                if (!ok) break;
+                            }
+                            // the counts' slot is free: the tile this one replaces was released after iteration i - N1
+                            if (x == 0 && u >= nA) write_counts(counts + (u % COUNT_RING) * TB, tokens, a.tier.RM, u < nM, lane);
+                            __syncwarp();
+                            // one arrival, after the counts of both units (bytes may land before they are expected)
+                            if (lane == 0 && b + 1 == nb) mbar_arrive_expect_tx(bar, nb * Y_TILE);
+                            if (u >= nA)
+                                load_means<DH>(dst + b * Y_HALF, X_HALF, x ? &tmM2 : &tmM1, x ? &tmT2 : &tmT1, bar, a.tier, bh, u < nM, id,
+                                               u - nM, lane);
+                            else if (lane < DH)
+                                tma_load_2d(dst + lane * X_HALF, x ? &tmX2 : &tmX1, bar, 64 * lane, row0 + j0 * TB);
+                        }
+                        if (!ok) break;
                     }
                     __syncwarp();
                     issued[x] = i + 1;
@@ -618,7 +609,7 @@ static int launch_tier_bwd(const void* x1, const void* x2, const void* y1, const
     const long long rows[8] = {tok, tok, tok, tok, mid, mid, tail, tail};
     for (int i = 0; i < 8; ++i) {
         if (MODE == BWD_REP && (i == 2 || i == 3)) { t[i] = t[i - 2]; continue; }            // the owner is a table
-        const int box = MODE == BWD_TIER_Q && (i == 4 || i == 5) ? a.tier.RM : TB;
+        const int box = MODE != BWD_TIER_Q || i < 4 ? TB : i < 6 ? a.tier.RM : a.tier.tail_box();
         if (int rc = make_token_map<T>(&t[i], p[i], D, rows[i], box)) return rc;
     }
     auto kern = attn_bwd_tc_kernel<T, D, MODE>;

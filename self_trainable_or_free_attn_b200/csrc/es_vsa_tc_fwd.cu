@@ -23,8 +23,8 @@
 // list: 1.52 ms, 3.10 ms before. D = 64 at the first shape: 0.51 ms, 0.74 ms before.
 //
 // TIER: the same walk over three tiers of resolution (es_vsa_tc.cuh), one softmax over all; a mean's column has the bias log2 of
-// its tokens. K and V have a load warp each: one warp for both, with the token counts fetched in line, took 1.72 ms where this
-// takes 1.30 ms (512 blocks x 12 heads, 32 + 102 blocks in tiers A and B of every query block; mma.sync 2.34 ms).
+// its tokens. K and V have a load warp each, with one copy of the code that finds and loads a unit: 512 blocks x 12 heads, 32 + 102
+// blocks in tiers A and B of every query block, 1.25 ms (2.26 ms with that code inlined at six places, mma.sync 2.37 ms).
 #include "es_vsa_tc.cuh"
 
 namespace es {
@@ -47,7 +47,7 @@ struct FwdCtl {
     uint64_t qfull, full[5], empty[5], sfull, sfree, pfull, pvdone, drain;
     uint32_t tmem_base;
     int abort;
-    int2 tiers;                    // tier-B blocks, tier-C words of the query block
+    int2 tiers;                    // tier-B and tier-C blocks of the query block
 };
 static_assert(sizeof(FwdCtl) <= 256, "control block");
 
@@ -125,7 +125,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     // units of 64 columns: the list's blocks, then (tiers) gathered group means, then block means
     const int nA = TIER && !(a.tier.phases & PH_A) ? 0 : end - beg;
     const int nM = TIER ? nA + (ctl->tiers.x * a.tier.RM + TB - 1) / TB : nA;
-    const int n = TIER && ctl->tiers.y > 0 ? nM + (a.NB + TB - 1) / TB : nM;
+    const int n = TIER ? nM + tail_units(a.tier, a.NB, ctl->tiers.y) : nM;
     const int nt = (n + 1) >> 1;
     const uint32_t full0 = smem_u32(&ctl->full[0]), empty0 = smem_u32(&ctl->empty[0]);
     const int row0 = bh * a.L;                               // first row of this (b, h) in the [BH L, D] view
@@ -135,7 +135,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         // ------------------------------------------------------------ loads: Q, K(0), then K(i + 1), V(i) for every i
         // Tile numbers in the ring are in the order of use. With tiers K and V have a warp each: a gathered unit is up to 64 small
         // boxes per tensor.
-        const bool k_warp = warp == 5, v_warp = !TIER || warp == 6;
+        const bool k_warp = warp == 5;
         bool ok = *abort_flag == 0;
         if (ok && nt > 0) {
             if (lane == 0) {
@@ -150,15 +150,15 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             int kwin = lane < nA ? block_at(lane) : 0, kbase = 0;   // a window of 32 list entries per tensor
             int vwin = kwin, vbase = 0;
             uint32_t next_slot = 0, next_par = 1;
-            MidWalk walk;
+            TierWalk walk;
             if (TIER) walk.start(a.tier, bh, a.NB, qb, lane);
             auto put = [&](bool is_v, int& win, int& wbase, int e) {
                 if (!ok || e >= n) return;
                 // with one warp for both, the next slot; else the tile's number in the order of use
                 const uint32_t seq = !TIER ? pseq : is_v ? e + min(n, (e & ~1) + 4) : e + max(0, (e & ~1) - 2);
                 const uint32_t slot = TIER ? seq % C::NSLOT : next_slot, par = TIER ? ((seq / C::NSLOT) & 1) ^ 1 : next_par;
-                int j = 0, id = 0;
-                int2 tokens = make_int2(0, 0);
+                int j = 0;
+                int2 id = make_int2(-1, -1), tokens = make_int2(0, 0);
                 if (!TIER || e < nA) {
                     if ((e & ~31) != wbase) {
                         wbase = e & ~31;
@@ -166,8 +166,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                     }
                     j = __shfl_sync(0xffffffffu, win, e & 31);
                 } else {
-                    const int per = TB / a.tier.RM;
-                    if (e < nM) id = walk.blocks((e - nA) * per, per, lane);
+                    id = unit_blocks(walk, a.tier, bh, a.NB, qb, e < nM, e < nM ? e - nA : e - nM, lane);
                     if (!is_v) tokens = unit_tokens(a.blk_cnt, a.tier, bh, a.NB, qb, e < nM, id, e - nM, lane);
                 }
                 if (lane == 0) ok = mbar_wait(empty0 + 8 * slot, par, abort_flag, a.status, 401);
@@ -180,15 +179,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                     __syncwarp();
                     if (lane == 0) mbar_arrive_expect_tx(bar, C::TILE);
                     __syncwarp();
-                    if (e < nM) {
-                        const int row = bh * a.tier.mid_stride + max(id, 0) * a.tier.RM;
-                        if (lane < TB / a.tier.RM)
-                            for (int d = 0; d < D / 64; ++d)
-                                tma_load_2d(dst + d * C::HALF + lane * a.tier.RM * 128, is_v ? &tmVm : &tmKm, bar, 64 * d, row);
-                    } else if (lane < D / 64) {
-                        tma_load_2d(dst + lane * C::HALF, is_v ? &tmVt : &tmKt, bar, 64 * lane,
-                                    bh * a.tier.tail_stride + (e - nM) * TB);
-                    }
+                    load_means<D / 64>(dst, C::HALF, is_v ? &tmVm : &tmKm, is_v ? &tmVt : &tmKt, bar, a.tier, bh, e < nM, id, e - nM, lane);
                 } else if (lane == 0) {
                     mbar_arrive_expect_tx(bar, C::TILE);
 #pragma unroll
@@ -198,16 +189,15 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                 pseq = seq + 1;
                 if (!TIER && ++next_slot == C::NSLOT) { next_slot = 0; next_par ^= 1; }
             };
-            if (k_warp) {
+            if (TIER) {
+#pragma unroll 1
+                for (int e = 0; e < n && ok; ++e) put(!k_warp, kwin, kbase, e);
+            } else {
                 put(false, kwin, kbase, 0);
                 put(false, kwin, kbase, 1);
-            }
-            for (int i = 0; i < nt; ++i) {
-                if (k_warp) {
+                for (int i = 0; i < nt; ++i) {
                     put(false, kwin, kbase, 2 * i + 2);
                     put(false, kwin, kbase, 2 * i + 3);
-                }
-                if (v_warp) {
                     put(true, vwin, vbase, 2 * i);
                     put(true, vwin, vbase, 2 * i + 1);
                 }
@@ -513,7 +503,7 @@ static int launch_tier_fwd(const void* q, const void* k, const void* v, const vo
     const void* p[7] = {q, k, v, k_mid, v_mid, k_tail, v_tail};
     const long long rows[7] = {tok, tok, tok, mid, mid, tail, tail};
     for (int i = 0; i < 7; ++i)
-        if (int rc = make_token_map<T>(&t[i], p[i], D, rows[i], i == 3 || i == 4 ? a.tier.RM : TB)) return rc;
+        if (int rc = make_token_map<T>(&t[i], p[i], D, rows[i], i >= 5 ? a.tier.tail_box() : i >= 3 ? a.tier.RM : TB)) return rc;
     auto kern = attn_fwd_tc_kernel<T, D, true>;
     if (int rc = opt_in_shared_memory((const void*)kern, (int)FwdCfg<D>::BYTES_TIER)) return rc;
     kern<<<dim3(a.NB, BH), FW_THREADS_TIER, FwdCfg<D>::BYTES_TIER, st>>>(t[0], t[1], t[2], t[3], t[4], t[5], t[6], a);
