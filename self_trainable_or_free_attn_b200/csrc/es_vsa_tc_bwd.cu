@@ -38,10 +38,11 @@ constexpr float kLog2e = 1.4426950408889634f;
 constexpr int BW_THREADS = 320, BW_THREADS_TIER = 352;
 constexpr uint32_t Y_HALF = TB * 128, X_HALF = 128 * 128;                // 64 d of an owner / a walked tile
 constexpr int COUNT_RING = 16;                                           // units whose column counts are staged
+constexpr int REP_WORDS = 4096 / 32;                                     // the entry points take up to 4096 blocks
 constexpr uint32_t DS_BYTES = 128 * 128;                                 // P, dS: [128 rows][64 columns] 16-bit
 // BWD_TIER_Q: the dQ pass over the units of all three tiers. BWD_REP: the dK / dV pass for 64 consecutive rows of a table of
-// representatives (group means, then block means) as the owner; it walks every query block, in fp32 tables and masked by the
-// tier of each (query block, table row).
+// representatives (group means, then block means) as the owner; it walks the query blocks that use one of them, masked by the tier
+// of each (query block, table row), and writes fp32 tables.
 enum BwdMode { BWD_KV, BWD_Q, BWD_TIER_Q, BWD_REP };
 template <int D, int MODE> struct BwdCfg {
     static constexpr bool KV = MODE == BWD_KV || MODE == BWD_REP;
@@ -50,7 +51,8 @@ template <int D, int MODE> struct BwdCfg {
     static constexpr uint32_t Y_TILE = DH * Y_HALF, X_TILE = DH * X_HALF;   // [d half][rows][128 B]
     static constexpr uint32_t Y1 = 0, Y2 = Y_TILE, DS = 2 * Y_TILE, P = DS + DS_BYTES;
     static constexpr uint32_t RING = P + (KV ? DS_BYTES : 0u), CTL = RING + (N1 + N2) * X_TILE, COUNTS = CTL + 1024;
-    static constexpr uint32_t BYTES = COUNTS + (MODE == BWD_TIER_Q ? COUNT_RING * TB : 0);   // column counts of the units
+    // BWD_TIER_Q: column counts of the units; BWD_REP: a bit per query block
+    static constexpr uint32_t BYTES = COUNTS + (MODE == BWD_TIER_Q ? COUNT_RING * TB : MODE == BWD_REP ? REP_WORDS * 4 : 0);
     static constexpr int LD = D + 4;                                     // epilogue staging: floats per token row
 };
 
@@ -80,6 +82,20 @@ struct BwdTcArgs {
     int* status;
     TierMaps tier;
     int wide;                      // every output pointer is 16-byte aligned
+};
+
+// The set bits of a bitmap in shared memory, ascending.
+struct BitWalk {
+    const uint32_t* words;
+    int w;
+    uint32_t bits;
+    __device__ __forceinline__ BitWalk(const uint32_t* words_, bool any) : words(words_), w(0), bits(any ? words_[0] : 0u) {}
+    __device__ __forceinline__ int next() {                  // the caller knows that there is one
+        while (bits == 0) bits = words[++w];
+        const int b = __ffs(bits) - 1;
+        bits &= bits - 1;
+        return 32 * w + b;
+    }
 };
 
 __device__ __forceinline__ void store4(float* dst, float4 v, int wide) {
@@ -124,6 +140,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
     volatile int* abort_flag = &ctl->abort;
     const int row0 = bh * a.L;                               // first row of this (b, h) in the [BH L, D] view
     uint8_t* counts = smem + C::COUNTS;
+    uint32_t* use_words = reinterpret_cast<uint32_t*>(smem + C::COUNTS);
     // BWD_REP: the owner's table and tile in it, and the first block that the tile covers
     const int mid_tiles = REP && (a.tier.phases & PH_B) ? (a.NB * a.tier.RM + TB - 1) / TB : 0;
     const bool rep_mid = REP && ob < mid_tiles;
@@ -160,6 +177,27 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
         if (rep_mid) c = min(max(c - (r % a.tier.RM) * R, 0), R);
         ctl->lse2[r] = -log2f((float)c);
     }
+    if (REP) {
+        // bit i: query block i uses a row of this tile
+        const uint32_t* bit_row = a.tier.bits_ab + (size_t)bh * a.NB * a.tier.W;
+        const uint32_t* bit_row_a = a.tier.bits_a + (size_t)bh * a.NB * a.tier.W;
+        const int w0 = rep_blk >> 5, left = a.NB - rep_blk;
+        const uint32_t lo = left >= 32 ? 0xFFFFFFFFu : (1u << left) - 1u, hi = left >= 64 ? 0xFFFFFFFFu : left > 32 ? (1u << (left - 32)) - 1u : 0u;
+        const uint32_t mid_mask = (rep_per >= 32 ? 0xFFFFFFFFu : (1u << rep_per) - 1u) & lo;
+#pragma unroll 2
+        for (int w = warp; w < a.tier.W; w += BW_THREADS / 32) {
+            const int i = 32 * w + lane;
+            bool used = false;
+            if (i < a.NB) {
+                const size_t at = (size_t)i * a.tier.W + w0;
+                const uint32_t ab = __ldg(bit_row + at);
+                if (rep_mid) used = ((ab & ~__ldg(bit_row_a + at)) >> (rep_blk & 31)) & mid_mask;
+                else used = (~ab & lo) || (hi && (~__ldg(bit_row + at + 1) & hi));
+            }
+            const uint32_t word = __ballot_sync(0xffffffffu, used);
+            if (lane == 0) use_words[w] = word;
+        }
+    }
     if (TIER && warp == 9) {
         const int2 t = tier_sizes(a.tier, bh, a.NB, ob, lane);
         if (lane == 0) ctl->tiers = t;
@@ -172,8 +210,13 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = ctl->tmem_base;
-    // walked units of 64 rows: the list's blocks (every query block for BWD_REP), then the tiers' means as in the forward
-    const int nA = TIER && !(a.tier.phases & PH_A) ? 0 : end - beg;
+    // walked units of 64 rows: the list's blocks (the query blocks of the bitmap for BWD_REP), then the tiers' means as in the forward
+    int nA = TIER && !(a.tier.phases & PH_A) ? 0 : end - beg;
+    if (REP) {
+        int used = 0;
+        for (int w = lane; w < a.tier.W; w += 32) used += __popc(use_words[w]);
+        nA = __reduce_add_sync(0xffffffffu, used);
+    }
     const int nM = TIER ? nA + (ctl->tiers.x * a.tier.RM + TB - 1) / TB : nA;
     const int n = TIER ? nM + tail_units(a.tier, a.NB, ctl->tiers.y) : nM;
     const int nt = (n + 1) >> 1;
@@ -202,14 +245,22 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
                     tma_load_2d(base + C::Y2 + d * Y_HALF, y2, smem_u32(&ctl->yfull), 64 * d, yrow);
                 }
             }
-            int win = lane < nA ? block_at(lane) : 0;          // a window of 32 list entries
+            int win = !REP && lane < nA ? block_at(lane) : 0;  // a window of 32 list entries
+            BitWalk used(use_words, REP);
             TierWalk walk;
             if (TIER) walk.start(a.tier, bh, a.NB, ob, lane);
             for (int i = 0; i < nt && ok; ++i) {
                 const int e = 2 * i;
-                if (e > 0 && (e & 31) == 0) win = e + lane < nA ? block_at(e + lane) : 0;
-                const int j0 = __shfl_sync(0xffffffffu, win, e & 31), j1 = __shfl_sync(0xffffffffu, win, (e + 1) & 31);
                 const int nb = e + 1 < n ? 2 : 1;
+                int j0, j1;
+                if (REP) {
+                    j0 = used.next();
+                    j1 = nb > 1 ? used.next() : j0;
+                } else {
+                    if (e > 0 && (e & 31) == 0) win = e + lane < nA ? block_at(e + lane) : 0;
+                    j0 = __shfl_sync(0xffffffffu, win, e & 31);
+                    j1 = __shfl_sync(0xffffffffu, win, (e + 1) & 31);
+                }
                 const bool lists = !TIER || e + nb <= nA;
 #pragma unroll 1
                 for (int x = x_first; x <= x_last; ++x) {
@@ -364,8 +415,14 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
         // The walked row's block id is requested two iterations ahead and what hangs on it (the block's tokens, in the dK / dV
         // pass the row's LSE and delta) one ahead, and nothing is computed from a loaded value before its own iteration: a warp
         // issues in order, so one use of a load that is still on its way would stall the current iteration's exponentials.
-        auto walked = [&](int i) -> int {
+        BitWalk used(use_words, REP);
+        auto walked = [&](int i) -> int {                    // called for i = 0, 1, 2, ...
             const int e = 2 * i + (r >> 6);
+            if (REP) {
+                if (i >= nt) return -1;
+                const int j0 = used.next(), j1 = 2 * i + 1 < nA ? used.next() : -1;
+                return r >> 6 ? j1 : j0;
+            }
             return i < nt && e < nA ? block_at(e) : -1;
         };
         int n_blk = walked(0), n2_blk = walked(1), n_cnt = 0;
@@ -651,7 +708,7 @@ int tier_rep_bwd_tc(const void* q, const void* k_mid, const void* v_mid, const v
     if (!status) return set_error(-2, "tier_rep_bwd_tc: the device status word is not available on this device");
     const float scale = 1.f / sqrtf((float)D);
     const int wide = (((uintptr_t)dk_mid | (uintptr_t)dv_mid | (uintptr_t)dk_tail | (uintptr_t)dv_tail) & 15) == 0;
-    // no lists: every query block is walked; the group means' gradients travel as part0 / part1
+    // no lists: the kernel finds the query blocks to walk; the group means' gradients travel as part0 / part1
     const BwdTcArgs a{lse, delta, nullptr, nullptr, dk_tail, dv_tail, nullptr, nullptr, 0, nullptr, nullptr, blk_cnt, L, L / TB, 0,
                       scale, kLog2e * scale, nullptr, nullptr, dk_mid, dv_mid, status, tier, wide};
     return dispatch_tier_bwd<BWD_REP>(q, dout, nullptr, nullptr, k_mid, v_mid, k_tail, v_tail, a, BH, D, dtype, tiles, st);

@@ -69,3 +69,37 @@ def test_tier_walk(RM, D, nb):
     near(pick(grads[0]), torch.stack([ref_q[i] * ok[i, :, None] for i in rows]), 1e-2, "dq")
     near(grads[1].view(nb, 64, D), kd.grad * okd[..., None], 2e-2, "dk")
     near(grads[2].view(nb, 64, D), vd.grad * okd[..., None], 2e-2, "dv")
+
+
+@pytest.mark.parametrize("RM", [2, 4, 16])
+@pytest.mark.parametrize("nb", [1, 33, 64, 97, 130])
+def test_tables_that_few_query_blocks_use(RM, nb):
+    """The table gradients walk only the query blocks that use a row of the tile: none, one, two, an odd number, at the edges of the
+    bitmap's words. Tiers B and C alone, against the CPU restatement in fp64 (tolerances of the module)."""
+    from test_gpu_vsa_tiers import oracle_subset
+    from self_trainable_or_free_attn_b200.vsa import tiers as T
+    g = torch.Generator().manual_seed(nb + RM)
+    D = 64
+    cnt = torch.randint(1, 65, (nb,), generator=g, dtype=torch.int32)
+    ok = (torch.arange(64)[None] < cnt[:, None]).reshape(1, 1, -1, 1)
+    q, k, v, do = [(torch.randn(1, 1, nb * 64, D, generator=g) * ok).to(torch.bfloat16) for _ in range(4)]
+    b, c = torch.zeros(2, nb, nb, dtype=torch.bool)
+    edges = [i for i in (0, 31, 32, 63, 64, nb // 2, nb - 1) if i < nb]
+    for j in range(0, nb, 3):                                      # two of three column blocks are in neither tier
+        users = [edges[i] for i in torch.randperm(len(edges), generator=g)[: (j // 3) % 4].tolist()]
+        (b if (j // 3) % 2 else c)[users, j] = True
+    b[0, 0] = True
+    a = ~(b | c)
+    x = [t.cuda().requires_grad_(True) for t in (q, k, v)]
+    o, _ = T.rep_fine_attention(*x, cnt.cuda(), T.selection_from_masks(a[None, None].cuda(), (a | b)[None, None].cuda()), mid_reps=RM,
+                                phases=T.PHASE_B | T.PHASE_C)
+    grads = torch.autograd.grad(o, x, do.cuda())
+    ref = [t.double().requires_grad_(True) for t in (q, k, v)]
+    o_ref, _ = oracle_subset(ref, cnt, a[None, None] & False, b[None, None], c[None, None], mid_reps=RM)
+    ref_grads = torch.autograd.grad(o_ref, ref, do.double())
+    for name, got, exp, tol in zip(("o", "dq", "dk", "dv"), (o, *grads), (o_ref, *ref_grads), (1e-2, 2e-2, 2e-2, 2e-2)):
+        got, exp = got.detach().double().cpu(), exp.detach()
+        # nb = 1: one group or a few columns only, dq and dk are small differences
+        assert (got - exp).norm() <= tol * exp.norm() + (0.3 if nb == 1 else 0.0), (name, float((got - exp).norm() / exp.norm()))
+        if nb > 1:
+            assert torch.equal((got == 0).all(-1), (exp == 0).all(-1)), name
