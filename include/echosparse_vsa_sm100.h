@@ -7,7 +7,9 @@
  *   - token tensors are [BH, L, D] contiguous, L = NB * 64, D = 64 or 128, dtype 0 = bf16, 1 = fp16;
  *     blk_cnt [NB] int32 = valid tokens per 64-token block (1..64, valid tokens first); padded slots output 0;
  *   - CSR block lists: ptr [BH * (NB + 1)] int32 absolute offsets into idx, ids ascending per row;
- *   - lse [BH, L] fp32 is the natural-log LSE over the selected keys, -inf for rows without a key and for padded rows.
+ *   - lse [BH, L] fp32 is the natural-log LSE over the selected keys, -inf for rows without a key and for padded rows;
+ *   - every wait inside the attention kernels is bounded. A block of rows whose wait gave up is NaN in every output, and so is
+ *     what later attention calls of the device return until es_device_status (echosparse_sm100.h) has read and cleared the word.
  * Each declaration names the launcher / binding of the reference (shaoshitong/self_trainable_or_free_attn) it replaces.
  */
 #ifndef ECHOSPARSE_VSA_SM100_H

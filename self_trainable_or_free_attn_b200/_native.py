@@ -115,6 +115,17 @@ def device_status():
     return out.value
 
 
+def check_status(device=None):
+    """Raises NativeError if a kernel's bounded wait gave up on the device (default: the current one) since the last check; the
+    word is cleared. Synchronises the device."""
+    import torch
+    with torch.cuda.device(device):
+        code = device_status()
+    if code != 0:
+        raise NativeError(f"an attention kernel gave up a wait (status {code}: wait {code % 1000} in CTA {code // 1000}); the "
+                          f"outputs since the last check are not valid")
+
+
 def launch_count():
     return int(load().es_launch_count())
 

@@ -317,13 +317,8 @@ class EchoSparseAttention:
     def check_status(self):
         """Raises NativeError if a kernel's bounded wait gave up since the last check (the word is cleared). Synchronises
         the device, so call it where that is cheap: between videos, or once per denoising step."""
-        if self._device is None:
-            return
-        with torch.cuda.device(self._device):
-            code = _native.device_status()
-        if code != 0:
-            raise _native.NativeError(f"an attention kernel gave up a wait (status {code}: wait {code % 1000} in CTA "
-                                      f"{code // 1000}); the outputs since the last check are not valid")
+        if self._device is not None:
+            _native.check_status(self._device)
 
     def _bind(self, device):
         self.backend = backends.resolve(self.gpu, device)

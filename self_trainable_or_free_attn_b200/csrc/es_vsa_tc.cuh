@@ -103,6 +103,13 @@ template <typename T> static int make_token_map(CUtensorMap* m, const void* ptr,
                              2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
+// A CTA whose wait gave up, or that starts while the status word of an earlier one is set, leaves NaN in all it owns: its caller's
+// memory is not initialised, and without this could pass for a result until the word is read. The whole CTA, `words` 32-bit words.
+constexpr uint32_t kNaN16x2 = 0x7FFF7FFFu, kNaN32 = 0x7FFFFFFFu;      // bf16 and fp16 alike; fp32
+__device__ __forceinline__ void fill_nan(void* p, int words, uint32_t nan) {
+    for (int i = threadIdx.x; i < words; i += blockDim.x) static_cast<uint32_t*>(p)[i] = nan;
+}
+
 // ---------------------------------------------------------------- 64 / RM / 1 representative tiers
 // Per query block every kv block is in one tier: A (its tokens; the CSR list and bits_a), B (bits_ab & ~bits_a: its RM group
 // means, bias log2(tokens of the group)) or C (~bits_ab: its block mean, bias log2(tokens)). The walk of a query block goes over

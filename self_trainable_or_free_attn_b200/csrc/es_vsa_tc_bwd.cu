@@ -148,6 +148,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
     const int rep_row0 = REP ? bh * (rep_mid ? a.tier.mid_stride : a.tier.tail_stride) + rep_tile * TB : 0;
     const int cnt_o = REP ? min(TB, (rep_mid ? a.NB * a.tier.RM : a.NB) - rep_tile * TB) : tokens_of(ob);
     if (tid == 0) {
+        const int earlier = *reinterpret_cast<volatile int*>(a.status);      // (on its way during the set-up)
         mbar_init(smem_u32(&ctl->yfull), 1);
         for (int i = 0; i < N1 + N2; ++i) {
             mbar_init(smem_u32(&ctl->full[i]), 1);
@@ -157,7 +158,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
         mbar_init(smem_u32(&ctl->pfull), 256);
         mbar_init(smem_u32(&ctl->pvdone), 1);
         mbar_init(smem_u32(&ctl->drain), 1);
-        ctl->abort = (base & 1023u) ? 1 : 0;                 // the swizzled tiles need a 1024-byte aligned base
+        ctl->abort = (base & 1023u) || earlier ? 1 : 0;      // the swizzled tiles need a 1024-byte aligned base
         if (base & 1023u) atomicCAS(a.status, 0, 903);
         mbar_fence_init();
         fence_proxy_async_smem();
@@ -612,6 +613,17 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
     if (warp == 8) {
         tc_fence_after();
         tmem_dealloc(tmem, 512);
+    }
+    if (*abort_flag) {
+        for (int x = 0; x < (KV ? 2 : 1); ++x) {
+            float* part = x ? a.part1 : a.part0;
+            float* f = x ? a.f1 : a.f0;
+            const size_t row = (size_t)row0 + (size_t)ob * TB;
+            if (slot_out >= 0) fill_nan(part + (size_t)slot_out * TB * D, TB * D, kNaN32);
+            else if (REP) fill_nan((rep_mid ? part : f) + (size_t)rep_row0 * D, cnt_o * D, kNaN32);
+            else if (f) fill_nan(f + row * D, TB * D, kNaN32);
+            else fill_nan(static_cast<T*>(x ? a.d1 : a.d0) + row * D, TB * D / 2, kNaN16x2);
+        }
     }
 }
 

@@ -95,6 +95,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     FwdCtl* ctl = reinterpret_cast<FwdCtl*>(smem + C::CTL);
     volatile int* abort_flag = &ctl->abort;
     if (tid == 0) {
+        const int earlier = *reinterpret_cast<volatile int*>(a.status);      // (on its way during the set-up)
         mbar_init(smem_u32(&ctl->qfull), 1);
         for (int i = 0; i < C::NSLOT; ++i) {
             mbar_init(smem_u32(&ctl->full[i]), 1);
@@ -105,7 +106,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         mbar_init(smem_u32(&ctl->pfull), 128);
         mbar_init(smem_u32(&ctl->pvdone), 1);
         mbar_init(smem_u32(&ctl->drain), 1);
-        ctl->abort = (base & 1023u) ? 1 : 0;                 // the swizzled tiles need a 1024-byte aligned base
+        ctl->abort = (base & 1023u) || earlier ? 1 : 0;      // the swizzled tiles need a 1024-byte aligned base
         if (base & 1023u) atomicCAS(a.status, 0, 902);
         mbar_fence_init();
         fence_proxy_async_smem();
@@ -463,6 +464,12 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     if (warp == 4) {
         tc_fence_after();
         tmem_dealloc(tmem, 256);
+    }
+    if (*abort_flag) {
+        const size_t row = slot_out >= 0 ? (size_t)slot_out * TB : (size_t)row0 + (size_t)qb * TB;
+        if (slot_out >= 0) fill_nan(a.part_o + row * D, TB * D, kNaN32);
+        else fill_nan(static_cast<T*>(a.o) + row * D, TB * D / 2, kNaN16x2);
+        fill_nan((slot_out >= 0 ? a.part_lse : a.lse) + row, TB, kNaN32);
     }
 }
 
