@@ -5,6 +5,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <cmath>
 #include <string>
 #include <type_traits>
 
@@ -124,6 +125,12 @@ constexpr int UNIT_RING = 8;                       // units whose column counts 
 struct TierMaps {
     const uint32_t *bits_a, *bits_ab;              // [BH, NB, W]
     int W, RM, mid_stride, tail_stride, phases;
+    // Bias of a column that stands for n tokens, log2(n) over `unit`, rounded once; -inf for none. Lanes of a warp mostly ask for
+    // one or two values, which the constant cache serves at once.
+    float bias[65];
+    void set_bias(double unit) {
+        for (int n = 0; n <= 64; ++n) bias[n] = (float)(log2((double)n) / unit);
+    }
     __host__ __device__ bool gather_tail() const { return (phases & (PH_A | PH_B)) != (PH_A | PH_B); }
     __host__ __device__ int tail_box() const { return gather_tail() ? 1 : 64; }
 };

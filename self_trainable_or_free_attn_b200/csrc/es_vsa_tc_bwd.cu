@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(MODE == BWD_TIER_Q ? BW_THREADS_TIER : BW_THRE
 attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant__ CUtensorMap tmX2,
                    const __grid_constant__ CUtensorMap tmY1, const __grid_constant__ CUtensorMap tmY2,
                    const __grid_constant__ CUtensorMap tmM1, const __grid_constant__ CUtensorMap tmM2,
-                   const __grid_constant__ CUtensorMap tmT1, const __grid_constant__ CUtensorMap tmT2, const BwdTcArgs a) {
+                   const __grid_constant__ CUtensorMap tmT1, const __grid_constant__ CUtensorMap tmT2, const __grid_constant__ BwdTcArgs a) {
     // tmM, tmT: tables of group and of block means, walked (BWD_TIER_Q; tmM in boxes of RM rows) or the owner (BWD_REP)
     constexpr bool TIER = MODE == BWD_TIER_Q, REP = MODE == BWD_REP;
     using C = BwdCfg<D, MODE>;
@@ -176,7 +176,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
         const int r = tid - 64, j = rep_blk + (rep_mid ? r / a.tier.RM : r), R = TB / a.tier.RM;
         int c = j < a.NB ? __ldg(a.blk_cnt + j) : 0;
         if (rep_mid) c = min(max(c - (r % a.tier.RM) * R, 0), R);
-        ctl->lse2[r] = -log2f((float)c);
+        ctl->lse2[r] = -a.tier.bias[c];
     }
     if (REP) {
         // bit i: query block i uses a row of this tile
@@ -467,7 +467,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
             if (TIER && 2 * i + (r >> 6) >= nA && 2 * i + (r >> 6) < n) {
                 const int c = counts[((2 * i + (r >> 6)) % COUNT_RING) * TB + (r & 63)];
                 valid = c > 0;
-                off = __log2f((float)max(c, 1));                // as in the forward
+                off = a.tier.bias[max(c, 1)];
             }
             uint32_t s[32], dp[32];
             tmem_ld32(tw + (i & 1) * 128 + 32 * ch, s);
@@ -708,8 +708,9 @@ int tier_bwd_q_tc(const void* q, const void* k, const void* v, const void* k_mid
     int* status = device_status_ptr();
     if (!status) return set_error(-2, "tier_bwd_q_tc: the device status word is not available on this device");
     const float scale = 1.f / sqrtf((float)D);
-    const BwdTcArgs a{lse, delta, dq, nullptr, nullptr, nullptr, add, nullptr, add_nb, row_ptr, col_idx, blk_cnt, L, L / TB, 0, scale,
+    BwdTcArgs a{lse, delta, dq, nullptr, nullptr, nullptr, add, nullptr, add_nb, row_ptr, col_idx, blk_cnt, L, L / TB, 0, scale,
                       kLog2e * scale, nullptr, nullptr, nullptr, nullptr, status, tier, ((uintptr_t)dq & 15) == 0};
+    a.tier.set_bias(1.0);
     return dispatch_tier_bwd<BWD_TIER_Q>(k, v, q, dout, k_mid, v_mid, k_tail, v_tail, a, BH, D, dtype, L / TB, st);
 }
 
@@ -721,8 +722,9 @@ int tier_rep_bwd_tc(const void* q, const void* k_mid, const void* v_mid, const v
     const float scale = 1.f / sqrtf((float)D);
     const int wide = (((uintptr_t)dk_mid | (uintptr_t)dv_mid | (uintptr_t)dk_tail | (uintptr_t)dv_tail) & 15) == 0;
     // no lists: the kernel finds the query blocks to walk; the group means' gradients travel as part0 / part1
-    const BwdTcArgs a{lse, delta, nullptr, nullptr, dk_tail, dv_tail, nullptr, nullptr, 0, nullptr, nullptr, blk_cnt, L, L / TB, 0,
+    BwdTcArgs a{lse, delta, nullptr, nullptr, dk_tail, dv_tail, nullptr, nullptr, 0, nullptr, nullptr, blk_cnt, L, L / TB, 0,
                       scale, kLog2e * scale, nullptr, nullptr, dk_mid, dv_mid, status, tier, wide};
+    a.tier.set_bias(1.0);
     return dispatch_tier_bwd<BWD_REP>(q, dout, nullptr, nullptr, k_mid, v_mid, k_tail, v_tail, a, BH, D, dtype, tiles, st);
 }
 

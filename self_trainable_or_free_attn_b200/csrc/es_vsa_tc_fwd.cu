@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(TIER ? FW_THREADS_TIER : FW_THREADS, 2)
 attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmKm,
                    const __grid_constant__ CUtensorMap tmVm, const __grid_constant__ CUtensorMap tmKt,
-                   const __grid_constant__ CUtensorMap tmVt, const FwdTcArgs a) {
+                   const __grid_constant__ CUtensorMap tmVt, const __grid_constant__ FwdTcArgs a) {
     using C = FwdCfg<D>;
     extern __shared__ __align__(1024) uint8_t smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -282,7 +282,6 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         // columns of unit e that are not masked here (the means' come with their biases below)
         auto width = [&](int e) { return e < nA ? tokens_of(block_at(e)) : e < n ? TB : 0; };
         int ca = width(0), cb = width(1);
-        const float inv_scale = 1.f / a.scale_log2;
         // stmatrix: lane l gives the address of row (l & 7) of 8 x 8 matrix l >> 3: (rows 0-7, 8-15) x (chunk 2 j, 2 j + 1)
         const int prow = 16 * warp + (lane & 7) + ((lane >> 3) & 1) * 8;
         const uint32_t paddr = base + C::P + prow * 128, psw = prow & 7, pch = lane >> 4;
@@ -316,9 +315,8 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                     const uint8_t* c8 = counts + (e % UNIT_RING) * TB + 2 * (lane & 3);
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        // log2 of 0 .. 64, absolute error below 2^-21 (-inf for 0): a relative 3e-7 of P
                         const uint32_t cc = *reinterpret_cast<const uint16_t*>(c8 + 8 * j);
-                        const float b0 = __log2f((float)(cc & 255u)) * inv_scale, b1 = __log2f((float)(cc >> 8)) * inv_scale;
+                        const float b0 = a.tier.bias[cc & 255u], b1 = a.tier.bias[cc >> 8];
                         uint32_t* x = s + 32 * b + 4 * j;
                         x[0] = __float_as_uint(__uint_as_float(x[0]) + b0);
                         x[1] = __float_as_uint(__uint_as_float(x[1]) + b1);
@@ -524,8 +522,9 @@ int tier_fwd_tc(const void* q, const void* k, const void* v, const void* k_mid, 
                 const int* blk_cnt, int BH, int L, int D, int dtype, cudaStream_t st) {
     int* status = device_status_ptr();
     if (!status) return set_error(-2, "tier_fwd_tc: the device status word is not available on this device");
-    const FwdTcArgs a{o, lse, row_ptr, col_idx, blk_cnt, L, L / TB, 0, kLog2e / sqrtf((float)D), nullptr, nullptr, nullptr, nullptr,
-                      status, tier};
+    FwdTcArgs a{o, lse, row_ptr, col_idx, blk_cnt, L, L / TB, 0, kLog2e / sqrtf((float)D), nullptr, nullptr, nullptr, nullptr,
+                status, tier};
+    a.tier.set_bias(a.scale_log2);                            // S is scaled after the bias has been added
     if (D == 64)
         return dtype == 0 ? launch_tier_fwd<__nv_bfloat16, 64>(q, k, v, k_mid, v_mid, k_tail, v_tail, a, BH, st)
                           : launch_tier_fwd<__half, 64>(q, k, v, k_mid, v_mid, k_tail, v_tail, a, BH, st);

@@ -92,7 +92,7 @@ extern "C" int es_vsa_attn_bwd_q(const void* q, const void* k, const void* v, co
                                  int32_t L, int32_t D, int32_t dtype, void* stream);
 
 static TierMaps tier_maps(const int32_t* bits_a, const int32_t* bits_ab, int L, int RM, int mid_stride, int tail_stride, int phases) {
-    return {(const uint32_t*)bits_a, (const uint32_t*)bits_ab, (L / TB + 31) / 32, RM, mid_stride, tail_stride, phases};
+    return {(const uint32_t*)bits_a, (const uint32_t*)bits_ab, (L / TB + 31) / 32, RM, mid_stride, tail_stride, phases, {}};
 }
 
 extern "C" int es_vsa_tier_attn_fwd(const void* q, const void* k, const void* v, const void* k_mid, const void* v_mid,

@@ -103,3 +103,27 @@ def test_tables_that_few_query_blocks_use(RM, nb):
         assert (got - exp).norm() <= tol * exp.norm() + (0.3 if nb == 1 else 0.0), (name, float((got - exp).norm() / exp.norm()))
         if nb > 1:
             assert torch.equal((got == 0).all(-1), (exp == 0).all(-1)), name
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("phases", [2, 4])
+def test_bias_of_every_token_count(D, phases):
+    """With q = 0 and one block of n tokens per list the LSE is ln(n): the bias in fp32, its product with the scale, log2 e undone,
+    four roundings (2^-24 each) at most, and three more in the four columns' row sum. dV of that block's tokens is then dO's sum over
+    the query block over n: P is 1 (or the groups' shares) in both passes."""
+    from self_trainable_or_free_attn_b200.vsa import tiers as T
+    nb = 64
+    cnt = torch.arange(1, 65, dtype=torch.int32).cuda()
+    q = torch.zeros(1, 1, nb * 64, D, device="cuda", dtype=torch.bfloat16)
+    k, v, do = (torch.randn_like(q) for _ in range(3))
+    eye = torch.eye(nb, dtype=torch.bool)[None, None].cuda()
+    sel = T.selection_from_masks(eye & False, eye if phases == 2 else ~eye)
+    x = [t.requires_grad_(True) for t in (q, k, v)]
+    o, lse = T.rep_fine_attention(*x, cnt, sel, mid_reps=4, phases=phases)
+    want = cnt.double().log()
+    err = ((lse.view(nb, 64)[:, 0].double() - want).abs() / want.clamp(min=1)).max()
+    assert err <= (4 if phases == 4 else 7) * 2.0 ** -24, float(err * 2 ** 24)
+    dv = torch.autograd.grad(o, x, do)[2].view(nb, 64, D).double()
+    ok = (torch.arange(64, device="cuda")[None] < cnt[:, None]).double()[..., None]
+    exp = (do.view(nb, 64, D).double() * ok).sum(1, keepdim=True) / cnt[:, None, None] * ok
+    assert (dv - exp).norm() <= 4e-3 * exp.norm()
