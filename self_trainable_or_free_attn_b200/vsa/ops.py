@@ -9,8 +9,7 @@ argument meaning, layout contract and error behaviour:
   gate    : optional pre-activation, [B, H, L] or [B, H, L, D]. O = O_fine + act(gate) * O_coarse[block].
   blk_cnt : int32 [NB], 1..64.
 
-Every stage is a CUDA kernel of this library; torch is used for allocation and for the shape-only dense CSR of the coarse
-branch. The backward has one owner per output row in both passes (kv -> q lists for dK / dV, q -> kv lists for dQ), so
+Every stage is a CUDA kernel of this library; torch is used for allocation. The backward has one owner per output row in both passes (kv -> q lists for dK / dV, q -> kv lists for dQ), so
 gradients are reproducible bit for bit; the intermediates are released after the first backward (ops.py:520-522 there).
 """
 import math
