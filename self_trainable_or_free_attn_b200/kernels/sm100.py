@@ -145,10 +145,11 @@ def _tile_list_scratch(flags):
 
 @_timed
 def dense_attention(q, k, v, out, lse):
-    """Online-softmax attention over every block."""
+    """Online-softmax attention over every block. q, k, v, out: (L, H, 128) bf16; lse: (nq * 128, H) float32, log2."""
     L, H, hd = q.shape
-    assert hd == D
+    assert hd == D and k.shape == v.shape == out.shape == q.shape
     _cuda_bf16(q, k, v, out)
+    assert lse.shape == (_cdiv(L, BM) * BM, H) and lse.dtype == torch.float32 and lse.is_cuda and lse.is_contiguous()
     N.check(N.load().es_dense_attention(N.ptr(q), N.ptr(k), N.ptr(v), N.ptr(out), N.ptr(lse), L, H, N.stream_ptr()),
             "dense_attention")
 

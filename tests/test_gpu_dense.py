@@ -59,3 +59,15 @@ def test_short_sequences_repeat_their_bits(L):
         K.dense_attention(q, k, v, again, lse2)
         assert torch.equal(again, out) and torch.equal(lse2, lse)
     assert _native.device_status() == 0
+
+
+def test_wrong_shapes_are_refused():
+    """What the kernel would read or write out of range is refused on the host."""
+    from self_trainable_or_free_attn_b200 import backends
+    K = backends.kernels(backends.resolve("auto", DEV))
+    q = torch.zeros(130, 2, 128, device=DEV, dtype=torch.bfloat16)
+    lse = torch.empty(256, 2, device=DEV)
+    for bad in (dict(k=q[:129]), dict(v=q[:, :1].contiguous()), dict(out=q[:100]), dict(lse=lse[:130]), dict(lse=lse.double()),
+                dict(lse=torch.empty(2, 256, device=DEV).t())):
+        with pytest.raises(AssertionError):
+            K.dense_attention(**{**dict(q=q, k=q, v=q, out=torch.empty_like(q), lse=lse), **bad})
