@@ -17,7 +17,7 @@
 // Tensor memory: (S, dP) of even and of odd iterations (4 x 64 columns), G1^T, G2^T (2 x 64). S and dP of iteration i + 1 are
 // computed while the warps work on iteration i. X1 and X2 tiles (32 KB at D = 128) have a ring each, of three and two slots (five
 // and five at D = 64): the dQ passes free X2 as soon as dP has read it. Where the second products need both (dK / dV at D = 128),
-// one ring of five in the order of use is 3 % faster.
+// one ring of five in the order of use is 2 to 6 % faster.
 //
 // What bounds it: the hand-overs. The MMAs take 1,024 (768) clocks per two blocks at D = 128 and their operands 1,500 (1,150) of
 // shared memory's, of 3,300 (2,400) measured: a tile's load, its products, P / dS and the second products follow one another
@@ -26,7 +26,7 @@
 // gradient products take half of the tensor pipe.
 //
 // BWD_TIER_Q, BWD_REP: the three tiers of resolution, see the modes below. 512 blocks x 12 heads, 32 + 102 blocks in tiers A and B:
-// dQ 1.85 ms, tables 1.7 ms (mma.sync: 2.63 and 3.32 ms).
+// dQ 1.83 ms, tables 1.08 ms (mma.sync: 2.66 and 2.94 ms).
 #include "es_vsa_tc.cuh"
 
 namespace es {
