@@ -49,9 +49,9 @@ constexpr uint32_t HALF_BYTES = TILE_BYTES / 2;  // one d half: 128 rows x 128 B
 constexpr uint32_t BLK_BYTES = BK * 128;         // 64 rows of one d half: one TMA box
 constexpr uint32_t SMEM_RING = 0;
 constexpr uint32_t SMEM_CTL = SMEM_RING + NSLOT * TILE_BYTES;
-constexpr uint32_t SMEM_BIAS = SMEM_CTL + 3584;                        // [NBIAS][128] floats
+constexpr uint32_t SMEM_BIAS = SMEM_CTL + 5632;                        // [NBIAS][128] floats
 constexpr uint32_t SMEM_MASS = SMEM_BIAS + NBIAS * 128 * 4;            // [NMASS][2 column halves][128 rows] floats
-constexpr uint32_t SMEM_ALLOC = SMEM_MASS + NMASS * 2 * BM * 4;        // 212,480 B: one CTA per SM
+constexpr uint32_t SMEM_ALLOC = SMEM_MASS + NMASS * 2 * BM * 4;        // 214,528 B: one CTA per SM
 
 struct Ctl {
     uint64_t qfull;
@@ -67,12 +67,15 @@ struct Ctl {
     float l_part[2][BM];               // row sums of the two column halves
     float m_part[2][BM];               // row maxima of the two column halves (fallback sweep)
     float r_part[2][BM];               // dense: row sums of the rounded P
+    float e_part[2][BM];               // dense: what rounding took from a half's largest P above the sample's; its key, or -1
+    int key_part[2][BM];
     int redo;                          // some row left the range of the offset from a sample
 };
-static_assert(sizeof(Ctl) <= 3584, "control block");
+static_assert(sizeof(Ctl) <= 5632, "control block");
 
 struct AttnArgs {
     const __nv_bfloat16* q;      // (L, H, 128)
+    const __nv_bfloat16* v;      // (L, H, 128), dense mode only (elsewhere V comes through its tensor map alone)
     const uint8_t* keep;         // (H, nq, nb), compensation mode only
     __nv_bfloat16* out;
     const int* counts;           // (nq, H)
@@ -246,6 +249,7 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
     const int n = (n64 + 1) >> 1;                     // exact iterations: pairs of 64-token blocks
     // iterations of the fallback sweep: all, or for a sample one in 32 (1 to 8 of them) spread over the list
     const int nsweep = DENSE && sample ? min(n, min(max(n >> 5, 1), 8)) : n;
+    const bool find_top = DENSE && sample && n > nsweep;
     auto sweep_iter = [&](int i) { return DENSE && sample ? i * n / nsweep : i; };
     const int nvirt = FALLBACK ? 0 : a.nvirt;
     const int nref = (FALLBACK || COMPENSATE) ? 0 : a.nref;
@@ -472,6 +476,8 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
             mbar_arrive(smem_u32(&ctl->qfull));
         }
         float m = DENSE ? 0.f : a.offset[(size_t)row * a.H + h];
+        float best = 0.f;                          // dense: the largest logit found so far (at first the sample's) and its key
+        int best_key = -1;
         uint32_t uS[2] = {0, 0};
 
         if (FALLBACK) {
@@ -501,6 +507,7 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
             ok = mbar_wait_warp(smem_u32(&ctl->lbar), 0, abort_flag, a.status, 306) && ok;
             mx = fmaxf(ctl->m_part[0][trow], ctl->m_part[1][trow]);
             m = (mx == -INFINITY) ? 0.f : mx * a.scale_log2;
+            best = mx;
         }
 
         float2 lsum = make_float2(0.f, 0.f);
@@ -628,6 +635,35 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
             mbar_arrive(smem_u32(&ctl->pfull[buf]));
             acc = __fadd2_rn(acc, acc1);
             lsum = __fadd2_rn(lsum, acc);
+            if (DENSE && find_top) {
+                // a logit above the row's largest so far, and its key (P has left already: this is off the chain to PV)
+                const int lim = !has ? 0 : cur_blk == a.nb - 1 ? a.tail_valid : BK;
+                if (lim != BK) {
+#pragma unroll
+                    for (int c = 0; c < 64; ++c)
+                        if (c >= lim) s[c] = 0xff800000u;
+                }
+                float mx[8];
+#pragma unroll
+                for (int g = 0; g < 8; ++g) {
+                    const float* x = reinterpret_cast<const float*>(s) + 8 * g;
+                    mx[g] = fmaxf(fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3])), fmaxf(fmaxf(x[4], x[5]), fmaxf(x[6], x[7])));
+                }
+                const float top = fmaxf(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])), fmaxf(fmaxf(mx[4], mx[5]), fmaxf(mx[6], mx[7])));
+                const bool better = top > best;
+                if (__any_sync(0xffffffffu, better)) {
+                    best = better ? top : best;
+#pragma unroll
+                    for (int g = 0; g < 8; ++g) {
+                        const bool here = better && mx[g] == top;
+                        if (!__any_sync(0xffffffffu, here)) continue;
+                        int at = 0;
+#pragma unroll
+                        for (int c = 1; c < 8; ++c) at = __uint_as_float(s[8 * g + c]) == top ? c : at;
+                        best_key = here ? cur_blk * BK + 8 * g + at : best_key;
+                    }
+                }
+            }
             if (want_mass && exact) {
                 // per-block mass: every row leaves its sum over the block's columns in shared memory; the mass warp adds
                 // the 128 rows in a fixed order and stores the result (no atomics: the map is reproducible bit for bit). A
@@ -647,7 +683,12 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
         // ---- epilogue: row sums of both column halves, then this thread's 64 columns of O
         ctl->l_part[ch][trow] = lsum.x + lsum.y;
         // (not in m_part: with one or two iterations nothing keeps the other half's warp from still reading its maxima)
-        if (DENSE) ctl->r_part[ch][trow] = rsum.x + rsum.y;
+        if (DENSE) {
+            const float top = ex2_approx(fmaf(best, a.scale_log2, -m));      // the bits of the loop
+            ctl->r_part[ch][trow] = rsum.x + rsum.y;
+            ctl->e_part[ch][trow] = best_key < 0 ? 0.f : top - __uint_as_float(pack_bf16x2(top, 0.f) << 16);
+            ctl->key_part[ch][trow] = best_key;
+        }
         mbar_arrive(smem_u32(&ctl->lbar));
         ok = mbar_wait_warp(smem_u32(&ctl->lbar), FALLBACK ? 1 : 0, abort_flag, a.status, 307) && ok;
         const float l = ctl->l_part[0][trow] + ctl->l_part[1][trow];
@@ -656,18 +697,42 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
         if (nt > 0) ok = mbar_wait_warp(smem_u32(&ctl->ofull), 0, abort_flag, a.status, 303) && ok;
         if (ok) {
             tc_fence_after();
-            const float inv = COMPENSATE ? 1.0f / (1.0f + l) : DENSE ? 1.0f / (ctl->r_part[0][trow] + ctl->r_part[1][trow]) : 1.0f / l;
+            int top_key[2];
+            float e_top[2];
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                top_key[x] = DENSE ? ctl->key_part[x][trow] : -1;
+                e_top[x] = DENSE ? ctl->e_part[x][trow] : 0.f;
+            }
+            const float inv = COMPENSATE ? 1.0f / (1.0f + l)
+                              : DENSE ? 1.0f / ((ctl->r_part[0][trow] + ctl->r_part[1][trow]) + (e_top[0] + e_top[1])) : 1.0f / l;
             bool finite = true;
             __nv_bfloat16* orow = a.out + ((size_t)row * a.H + h) * HD + 64 * ch;
 #pragma unroll
             for (int part = 0; part < 2; ++part) {
                 uint32_t* o = &s[0];
+                uint4 vtop[2][4];                  // dense: this part of V at the two keys
+#pragma unroll
+                for (int x = 0; x < (DENSE ? 2 : 0); ++x) {
+                    const uint4* src = reinterpret_cast<const uint4*>(a.v + ((size_t)max(top_key[x], 0) * a.H + h) * HD + 64 * ch + 32 * part);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) vtop[x][c] = top_key[x] >= 0 ? __ldg(src + c) : make_uint4(0, 0, 0, 0);
+                }
                 if (nt > 0) {
                     tmem_ld32(lane_base + O_COL + 64 * ch + 32 * part, o);
                     tmem_wait_ld();
                 }
                 if (valid) {
                     if (DENSE) {
+#pragma unroll
+                        for (int x = 0; x < 2; ++x)
+#pragma unroll
+                            for (int c = 0; c < 16; ++c) {
+                                const uint4 w4 = vtop[x][c / 4];
+                                const uint32_t w = (c & 3) == 0 ? w4.x : (c & 3) == 1 ? w4.y : (c & 3) == 2 ? w4.z : w4.w;
+                                o[2 * c] = __float_as_uint(fmaf(e_top[x], __uint_as_float(w << 16), __uint_as_float(o[2 * c])));
+                                o[2 * c + 1] = __float_as_uint(fmaf(e_top[x], __uint_as_float(w & 0xFFFF0000u), __uint_as_float(o[2 * c + 1])));
+                            }
 #pragma unroll
                         for (int c = 0; c < 32; ++c) finite = finite && fabsf(__uint_as_float(o[c])) <= 3.0e38f;
                     }
@@ -763,11 +828,16 @@ attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
 // costs half as much tensor work again as the attention itself, and no offset has to be that exact: P is bf16 and the sums are
 // fp32, both as precise relative to any offset, as long as nothing leaves their exponent range. So the offset is the row's
 // maximum over a sample of the columns: the row sum then contains that maximum's own term 1, and the tile stands unless a row
-// sum passed 2^kSeedLimit or an output is not finite; only then is it done again with the maximum over all columns. The
-// outputs are divided by the sum of the rounded P, which cancels the rounding of a dominant term as an exact maximum (P = 1)
-// would: relative error against fp64 at 32,760 tokens x 12 heads 1.73e-3 with it, 1.93e-3 without, 1.72e-3 for two sweeps.
-// That shape takes 6.4 ms, 10.0 ms in two sweeps. (Flagged tiles, MODE 1, are those whose offset was far off, where a sample's
-// maximum often is too: 0.81 ms of a Wan-14B step with a sample first, 0.47 ms in two sweeps.)
+// sum passed 2^kSeedLimit or an output is not finite; only then is it done again with the maximum over all columns.
+// What an exact maximum gives besides is that the row's largest term is 1, so that its rounding costs nothing; a sample's maximum
+// rarely is the row's, and where few keys hold most of a row that is most of P's error. So the outputs are divided by the sum of the
+// rounded P, which cancels the rounding of a dominant term, and every half of a row remembers its largest logit above the sample's
+// and the key: the epilogue adds (P - rounded P) V[key]. Relative error against fp64, two sweeps / as here / without the remembered
+// terms: 32,760 tokens x 12 heads 1.716e-3 / 1.682e-3 / 1.726e-3; 9,360 tokens of random q, k with logits of deviation 3.2
+// 1.821e-3 / 1.773e-3 / 2.017e-3. Time of the first shape 9.7 / 6.2 / 5.6 ms, of 1,560 tokens 95 / 56 / 46 us (one iteration in four
+// searched: 6.1 ms, but 1.95e-3 on the random rows).
+// (Flagged tiles, MODE 1, are those whose offset was far off, where a sample's maximum often is too: 0.81 ms of a Wan-14B step with
+// a sample first, 0.47 ms in two sweeps.)
 __global__ void __launch_bounds__(NTHREADS, 1)
 dense_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const AttnArgs a) {
     bool again = false;
@@ -1003,7 +1073,7 @@ extern "C" int es_dense_attention(const void* q, const void* k, const void* v, v
     AttnCall c{};
     c.q = q; c.k = k; c.v = v;
     fill_common(c.a, L, H, 0.f);
-    c.a.out = (__nv_bfloat16*)out; c.a.lse = lse;
+    c.a.out = (__nv_bfloat16*)out; c.a.lse = lse; c.a.v = (const __nv_bfloat16*)v;
     fill_q(c);
     return launch_attention(c, 3, (cudaStream_t)stream);
 }

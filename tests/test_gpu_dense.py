@@ -71,3 +71,34 @@ def test_wrong_shapes_are_refused():
                 dict(lse=torch.empty(2, 256, device=DEV).t())):
         with pytest.raises(AssertionError):
             K.dense_attention(**{**dict(q=q, k=q, v=q, out=torch.empty_like(q), lse=lse), **bad})
+
+
+def _rows_fp64(q, k, v, h, rows):
+    s = q[rows, h].double() @ k[:, h].double().t() / 128 ** 0.5
+    return torch.softmax(s, 1) @ v[:, h].double(), torch.logsumexp(s, 1) * R.LOG2E
+
+
+@pytest.mark.parametrize("L", [2240, 4680, 9360])
+def test_no_less_precise_than_two_sweeps(L):
+    """Peaked rows (a few keys hold most of a row), far more keys than the sample has: the error against fp64 is no larger than
+    that of the kernel whose offset is the exact maximum, although most rows have their largest term outside the sample."""
+    from self_trainable_or_free_attn_b200 import backends
+    K = backends.kernels(backends.resolve("auto", DEV))
+    g = torch.Generator(device=DEV).manual_seed(L)
+    H = 2
+    q, k, v = [(torch.randn(L, H, 128, device=DEV, generator=g) * sc).to(torch.bfloat16) for sc in (1.8, 1.8, 1.0)]
+    nq, nb = R.cdiv(L, 128), R.cdiv(L, 64)
+    one, lse1, two, lse2 = torch.empty_like(q), torch.empty(nq * 128, H, device=DEV), torch.empty_like(q), torch.empty(nq * 128, H, device=DEV)
+    K.dense_attention(q, k, v, one, lse1)
+    blocks = torch.arange(nb, device=DEV, dtype=torch.int32).expand(nq, H, nb).contiguous()
+    K.exact_fallback(q, k, v, two, torch.full((nq, H), nb, device=DEV, dtype=torch.int32), blocks, lse2,
+                     torch.ones(nq, H, device=DEV, dtype=torch.int32))
+    err = []
+    for out, lse in ((one, lse1), (two, lse2)):
+        d = n = 0.0
+        for h in range(H):
+            ref, ref_lse = _rows_fp64(q, k, v, h, slice(0, L))
+            d, n = d + (out[:, h].double() - ref).square().sum(), n + ref.square().sum()
+            assert (lse[:L, h] - ref_lse).abs().max() <= 1e-4
+        err.append(float((d / n).sqrt()))
+    assert err[0] <= err[1], err
