@@ -492,7 +492,8 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
                 tc_fence_after();
                 tmem_ld32(lane_base + buf * 128 + 64 * ch, &s[0]);
                 tmem_ld32(lane_base + buf * 128 + 64 * ch + 32, &s[32]);
-                tmem_wait_ld();
+                tmem_wait_ld_regs(&s[0]);
+                tmem_wait_ld_regs(&s[32]);
                 tc_fence_before();
                 mbar_arrive(smem_u32(&ctl->pfull[buf]));
                 int lim = (blk == a.nb - 1) ? a.tail_valid : BK;
@@ -552,7 +553,8 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
             const uint32_t scol = lane_base + buf * 128 + 64 * ch;
             tmem_ld32(scol, &s[0]);
             tmem_ld32(scol + 32, &s[32]);
-            tmem_wait_ld();
+            tmem_wait_ld_regs(&s[0]);
+            tmem_wait_ld_regs(&s[32]);
             float2 acc = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
             uint32_t pk[32];
             if (exact) {
@@ -720,7 +722,7 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
                 }
                 if (nt > 0) {
                     tmem_ld32(lane_base + O_COL + 64 * ch + 32 * part, o);
-                    tmem_wait_ld();
+                    tmem_wait_ld_regs(o);
                 }
                 if (valid) {
                     if (DENSE) {

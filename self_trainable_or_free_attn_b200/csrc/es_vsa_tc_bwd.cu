@@ -472,7 +472,8 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
             uint32_t s[32], dp[32];
             tmem_ld32(tw + (i & 1) * 128 + 32 * ch, s);
             tmem_ld32(tw + (i & 1) * 128 + 64 + 32 * ch, dp);
-            tmem_wait_ld();
+            tmem_wait_ld_regs(s);
+            tmem_wait_ld_regs(dp);
             uint32_t pk[16], dk[16];
             const float2 sc = make_float2(a.scale_log2, a.scale_log2);
             const float4* lse4 = reinterpret_cast<const float4*>(ctl->lse2 + 32 * ch);

@@ -295,7 +295,8 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             uint32_t s[64];
             tmem_ld_16x64(tw, s);
             tmem_ld_16x64(tw + 64, s + 32);
-            tmem_wait_ld();
+            tmem_wait_ld_regs(s);
+            tmem_wait_ld_regs(s + 32);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&ctl->sfree));

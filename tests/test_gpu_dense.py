@@ -102,3 +102,36 @@ def test_no_less_precise_than_two_sweeps(L):
             assert (lse[:L, h] - ref_lse).abs().max() <= 1e-4
         err.append(float((d / n).sqrt()))
     assert err[0] <= err[1], err
+
+
+@pytest.mark.parametrize("L", [240, 8256, 32760])
+def test_tiles_that_start_again(L):
+    """A key outside the sample (one pair of blocks in 32, 1 to 8 of them, evenly spread) whose logits pass the sample's maximum by
+    more than 2^60 (head 0), or whose value makes the unnormalised output overflow (head 1): two iterations in all, a sample of two,
+    a sample of eight. Rows of the tiles in question and some others against fp64; tolerances as above."""
+    from self_trainable_or_free_attn_b200 import _native, backends
+    K = backends.kernels(backends.resolve("auto", DEV))
+    n = R.cdiv(L, 128)
+    sample = min(n, min(max(n >> 5, 1), 8))
+    columns = torch.cat([torch.arange(128) + 128 * (i * n // sample) for i in range(sample)])
+    key = next(c for c in range(L - 60, 0, -1) if not (columns == c).any())
+    g = torch.Generator(device=DEV).manual_seed(L)
+    q, k, v = [torch.randn(L, 2, 128, device=DEV, generator=g).to(torch.bfloat16) for _ in range(3)]
+    far = [L // 2, L // 3]
+    k[key, 0] = 80.0 * q[far[0], 0] / q[far[0], 0].float().norm()
+    k[key, 1] = 12.0 * q[far[1], 1] / q[far[1], 1].float().norm()
+    v[key, 1] = 1e38
+    out, lse = torch.full_like(q, 7.0), torch.zeros(n * 128, 2, device=DEV)
+    K.dense_attention(q, k, v, out, lse)
+    for h in range(2):
+        rows = sorted({*range(far[h] // 128 * 128, min(far[h] // 128 * 128 + 128, L)), *range(0, L, 97), L - 1})
+        ref, ref_lse = _rows_fp64(q, k, v, h, rows)
+        top = (q[far[h], h].float() @ k[columns[columns < L].to(DEV), h].float().t()).max() * (R.LOG2E / 128 ** 0.5)
+        gap = float(q[far[h], h].float() @ k[key, h].float()) * R.LOG2E / 128 ** 0.5 - float(top)
+        assert gap > (60 if h == 0 else 3), gap
+        got = out[rows, h].double()
+        assert torch.isfinite(got).all()
+        scale = ref.abs().max()
+        assert (got / scale - ref / scale).norm() <= 1e-2 * (ref / scale).norm() and (got - ref).abs().max() <= 3e-2 * scale
+        assert (lse[rows, h].double() - ref_lse).abs().max() <= 1e-4 * max(1.0, float(ref_lse.abs().max()) / 100)
+    assert _native.device_status() == 0
