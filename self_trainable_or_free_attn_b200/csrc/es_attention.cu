@@ -11,8 +11,8 @@
 // log2 l_r outside [-th, th].  There is no running maximum and no rescaling.
 //
 // FALLBACK = true is the online-softmax recomputation of flagged tiles (triton_ops.py:203-234): a sweep of QK MMAs
-// finds every row's maximum logit, then the same fixed-offset pipeline runs with that maximum as the offset, which is the online-softmax result without
-// rescaling steps.
+// finds every row's maximum logit, then the same fixed-offset pipeline runs with that maximum as the offset, which is the
+// online-softmax result without rescaling steps.
 //
 // Pipeline. An iteration covers 128 columns (two 64-token blocks, 128 block means, or 32 refine entries x 4).
 //   warps 0-7  softmax: warp w owns rows 32 (w % 4) .. +31 of the tile and columns 64 (w / 4) .. +63 of the iteration
