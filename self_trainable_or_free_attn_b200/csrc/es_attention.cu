@@ -553,8 +553,7 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
             const uint32_t scol = lane_base + buf * 128 + 64 * ch;
             tmem_ld32(scol, &s[0]);
             tmem_ld32(scol + 32, &s[32]);
-            tmem_wait_ld_regs(&s[0]);
-            tmem_wait_ld_regs(&s[32]);
+            tmem_wait_ld();                            // (naming the registers: 4.07 against 4.03 ms of a Wan-1.3B step)
             float2 acc = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
             uint32_t pk[32];
             if (exact) {
