@@ -86,6 +86,9 @@ full_scale_kernel(const float* __restrict__ m, float* __restrict__ lse, float* _
 // 64 blocks (cp.async, two stages, 16-byte chunks XOR-swizzled by the row) that all eight warps consume with ldmatrix:
 // S(16 sampled rows x 64 blocks) by mma.sync m16n8k16 over d. Reading the keys once per eight tiles with 16-byte accesses,
 // instead of once per tile with 4-byte ones, is what the kernel's time depends on (the keys of a head are 300 KB).
+// What bounds it now is issue: the products (mma.sync), the exponentials and the sums over the 16 rows, which a halving exchange
+// does with 14 shuffles per 64 blocks where every lane adding every column took 48: 591 x 40 tiles of 1,182 blocks 0.790 ->
+// 0.675 ms, 931 x 24 tiles of 1,861 blocks 1.227 -> 1.035 ms, 256 x 12 tiles of 512 blocks 66 -> 54 us.
 constexpr int EST_TILES = 8;
 __global__ void __launch_bounds__(256)
 estimate_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ km,
@@ -155,27 +158,34 @@ estimate_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __rest
                 Elt<__nv_bfloat16>::mma(acc[2 * np], afr[ks], b[0], b[1]);
                 Elt<__nv_bfloat16>::mma(acc[2 * np + 1], afr[ks], b[2], b[3]);
             }
-        // acc[i][0], acc[i][1]: row g, blocks 64 ct + 8 i + 2 tg, + 1; acc[i][2], acc[i][3]: row g + 8. After the sums over
-        // the 16 rows (the lanes with the same tg) every lane holds the estimates of blocks 8 i + 2 tg, + 1 for all i;
-        // the pair with i == g is the one this lane owns: 8 g + 2 tg = 2 lane.
-        float est0 = 0.f, est1 = 0.f;
+        // acc[i][0], acc[i][1]: row g, blocks 64 ct + 8 i + 2 tg, + 1; acc[i][2], acc[i][3]: row g + 8. Of the sums over the 16
+        // rows (the lanes with the same tg) the pair with i == g is the one this lane owns: 8 g + 2 tg = 2 lane. The sums are
+        // added in the same order in every lane: over g's lowest bit first.
+        float e[16];                                          // [2 i + x]
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            float e[2];
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
                 const int cc = ct * 64 + i * 8 + 2 * tg + x;
                 const float lb = (cc == nb - 1) ? lb_last : 6.0f;
                 const float e0 = v0 ? exp2f(fminf(acc[i][x] * scale_log2 - m0 + lb, 100.f)) : 0.f;
                 const float e1 = v1 ? exp2f(fminf(acc[i][2 + x] * scale_log2 - m1 + lb, 100.f)) : 0.f;
-                float s2 = e0 + e1;
-                s2 += __shfl_xor_sync(0xffffffffu, s2, 4);
-                s2 += __shfl_xor_sync(0xffffffffu, s2, 8);
-                s2 += __shfl_xor_sync(0xffffffffu, s2, 16);
-                e[x] = s2 * inv_ns;
+                e[2 * i + x] = e0 + e1;
             }
-            if (i == g) { est0 = e[0]; est1 = e[1]; }
+        // halving exchange over the bits of g: a lane hands on the columns whose i differs from its g in this bit
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+            const bool odd = (g >> b) & 1;
+#pragma unroll
+            for (int i = 0; i < 4 >> b; ++i)
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    const float keep_v = odd ? e[2 * (2 * i + 1) + x] : e[2 * (2 * i) + x];
+                    const float give = odd ? e[2 * (2 * i) + x] : e[2 * (2 * i + 1) + x];
+                    e[2 * i + x] = keep_v + __shfl_xor_sync(0xffffffffu, give, 4 << b);
+                }
         }
+        const float est0 = e[0] * inv_ns, est1 = e[1] * inv_ns;
         // kept blocks: their exact masses calibrate the estimates; the others receive their estimate
         if (in0) {
             if (kp0 != 0) { num += old0; den += est0; } else map[mbase + c0] = est0;
