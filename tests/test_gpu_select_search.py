@@ -1,6 +1,7 @@
 """The K-th largest key of a (tile, head): the search that ends with the first threshold that exactly K keys reach against the
-oracle's 31 halvings, bit for bit, over the lane counts of the warp kernel (8 .. 64 keys a lane) and rows where keys tie at the cut,
-are zero, NaN or infinite."""
+oracle's 31 halvings, bit for bit, over every lane count of the warp kernel (8, 16, 24, 32, 40, 48 and 64 keys a lane), the kernel
+of one CTA per (tile, head) that takes over above 2,048 blocks, and rows where keys tie at the cut, are zero, NaN or infinite. The
+plan packed from a selection gives its lists back."""
 import pytest
 import torch
 
@@ -10,8 +11,11 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
 
-@pytest.mark.parametrize("nb,k,r,sink", [(65, 7, 19, 1 << 30), (256, 1, 0, 1 << 30), (513, 500, 13, 511), (1182, 118, 355, 1 << 30),
-                                         (1281, 128, 384, 1 << 30), (1536, 1535, 1, 1 << 30), (1861, 223, 545, 1856), (2048, 2048, 0, 1 << 30)])
+@pytest.mark.parametrize("nb,k,r,sink", [(65, 7, 19, 1 << 30), (256, 1, 0, 1 << 30), (301, 30, 90, 297), (513, 500, 13, 511),
+                                         (1003, 100, 301, 1 << 30), (1024, 1, 1023, 1 << 30), (1182, 118, 355, 1 << 30),
+                                         (1281, 128, 384, 1 << 30), (1536, 1535, 1, 1 << 30), (1861, 223, 545, 1856),
+                                         (2048, 2048, 0, 1 << 30), (2049, 205, 615, 1 << 30), (2503, 0, 250, 2501),
+                                         (4096, 4000, 96, 1 << 30)])
 def test_selection_equals_the_oracle(nb, k, r, sink):
     from self_trainable_or_free_attn_b200.kernels import sm100 as K
     L, H = nb * 64 - 5, 2
@@ -38,3 +42,11 @@ def test_selection_equals_the_oracle(nb, k, r, sink):
     live = torch.arange(nb, device=DEV)[None, None] < counts[:, :, None]
     assert torch.equal(blocks[live], want[2][live])
     assert torch.equal(bits, want[3]) and torch.equal(refine, want[4])
+    # the plan of the selection, expanded again
+    exact = torch.zeros_like(bits)
+    K.pack_plan(keep, exact)
+    again = [torch.full_like(keep, 9), torch.zeros_like(counts), torch.zeros_like(blocks), torch.zeros_like(refine)]
+    listed = torch.zeros_like(counts)
+    K.rebuild_plan(exact, bits, *again, listed)
+    assert torch.equal(again[0], keep) and torch.equal(again[1], counts) and torch.equal(again[2][live], blocks[live])
+    assert torch.equal(again[3], refine) and torch.equal(listed, (refine < nb).sum(2).to(torch.int32))
