@@ -1,9 +1,10 @@
-// Block selection and plan bit masks: integer / bit work, one CTA per (query tile, head).
+// Block selection and plan bit masks: integer / bit work. Up to 2,048 kv blocks one warp per (query tile, head), above that one
+// CTA; plans are packed by one CTA and expanded by one warp per (query tile, head).
 //
 // select_blocks follows echosparse/kernels/triton_ops.py:58-105: values = mass x scale, the K-th largest value is
-// found exactly on the float bit patterns (the reference bisects; here a 4-pass 8-bit radix select over the same int32
-// keys gives the same key), ties at the threshold are all kept, forced blocks are added, the refine list is the R
-// largest raw masses among the blocks not kept (ties cut in ascending block order), lists come out ascending.
+// found exactly on the float bit patterns (the warp kernel bisects as the reference does, the CTA kernel finds the same key by a
+// 4-pass 8-bit radix select over the same int32 keys), ties at the threshold are all kept, forced blocks are added, the refine
+// list is the R largest raw masses among the blocks not kept (ties cut in ascending block order), lists come out ascending.
 // pack_plan / rebuild_plan follow echosparse/kernels/sm120.py:259-296.
 #include "es_api_internal.h"
 
@@ -12,11 +13,10 @@
 namespace es {
 
 constexpr int SEL_THREADS = 256;
-constexpr int SEL_MAX_ITEMS = 16;           // blocks per thread: nb <= 4096 (kernels are instantiated for 1, 2, 4, 8, 16)
+constexpr int ITEMS = 16;                   // blocks per thread of the CTA kernel: nb <= 4096
 
 // K-th largest of the non-negative int32 keys held as key[i] = keys of element i * 256 + tid (negative keys never
 // count). Returns 0 when fewer than K keys are non-negative, as the reference's bisection does.
-template <int ITEMS>
 __device__ int kth_largest_key(const int (&key)[ITEMS], int K, int* hist, int* bcast) {
     // hist: two histograms of 256 bins, bcast: two result triples; pass p uses copy p & 1 and clears the other one for pass
     // p + 1, so a pass needs two barriers (after the counting, after the digit is chosen). Both histograms are zero on
@@ -68,7 +68,6 @@ __device__ int kth_largest_key(const int (&key)[ITEMS], int K, int* hist, int* b
 // Ascending compaction of flagged elements in element order i * 256 + tid. Returns the total; `pos` gets each flagged
 // element's rank. One barrier pair for all ITEMS rounds: every warp posts its ITEMS ballot counts, then each thread adds
 // the counts of the rounds and warps before its own.
-template <int ITEMS>
 __device__ int compact_positions(const bool (&flag)[ITEMS], int (&pos)[ITEMS], int* warp_cnt) {
     constexpr int NW = SEL_THREADS / 32;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -96,7 +95,6 @@ __device__ int compact_positions(const bool (&flag)[ITEMS], int (&pos)[ITEMS], i
     return base;
 }
 
-template <int ITEMS>
 __global__ void __launch_bounds__(SEL_THREADS)
 select_kernel(const float* __restrict__ map, const uint8_t* __restrict__ keep_prev,
               const float* __restrict__ scale_exact, const float* __restrict__ scale_skip,
@@ -105,7 +103,7 @@ select_kernel(const float* __restrict__ map, const uint8_t* __restrict__ keep_pr
               int R, int nb, int L, int sink, int H, int nq) {
     __shared__ int hist[512];
     __shared__ int bcast[8];
-    __shared__ int warp_cnt[SEL_MAX_ITEMS * (SEL_THREADS / 32)];
+    __shared__ int warp_cnt[ITEMS * (SEL_THREADS / 32)];
     const int t = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
     const size_t base = ((size_t)h * nq + t) * nb;
     hist[tid] = 0;
@@ -135,7 +133,7 @@ select_kernel(const float* __restrict__ map, const uint8_t* __restrict__ keep_pr
         val[i] = v;
         key[i] = __float_as_int(v);
     }
-    const float thr = __int_as_float(kth_largest_key<ITEMS>(key, K, hist, bcast));
+    const float thr = __int_as_float(kth_largest_key(key, K, hist, bcast));
     bool keep[ITEMS];
     int rkey[ITEMS];
     float r2[ITEMS];
@@ -150,23 +148,23 @@ select_kernel(const float* __restrict__ map, const uint8_t* __restrict__ keep_pr
         r2[i] = r;
         rkey[i] = __float_as_int(r);
     }
-    const int rthr = kth_largest_key<ITEMS>(rkey, R, hist, bcast);
+    const int rthr = kth_largest_key(rkey, R, hist, bcast);
     bool ref[ITEMS];
     int pos[ITEMS];
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) ref[i] = rkey[i] >= rthr && r2[i] >= 0.f;
-    compact_positions<ITEMS>(ref, pos, warp_cnt);
+    compact_positions(ref, pos, warp_cnt);
     bool ref2[ITEMS];
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) ref2[i] = ref[i] && pos[i] < R;       // ties cut in ascending block order
-    const int nref = compact_positions<ITEMS>(ref2, pos, warp_cnt);
+    const int nref = compact_positions(ref2, pos, warp_cnt);
     int* rlist = refine + ((size_t)t * H + h) * rw;
     for (int j = nref + tid; j < rw; j += SEL_THREADS) rlist[j] = nb;             // padding
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i)
         if (ref2[i] && pos[i] < rw) rlist[pos[i]] = i * SEL_THREADS + tid;
 
-    const int nkeep = compact_positions<ITEMS>(keep, pos, warp_cnt);
+    const int nkeep = compact_positions(keep, pos, warp_cnt);
     int* blist = blocks + ((size_t)t * H + h) * nb;
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
@@ -206,53 +204,6 @@ pack_kernel(const uint8_t* __restrict__ keep, int* __restrict__ exact_bits, int 
         const unsigned b = __ballot_sync(0xffffffffu, bit);
         const int w = i * (SEL_THREADS / 32) + warp;
         if (lane == 0 && w < nw) words[w] = (int)b;
-    }
-}
-
-template <int ITEMS>
-__global__ void __launch_bounds__(SEL_THREADS)
-rebuild_kernel(const int* __restrict__ exact_bits, const int* __restrict__ skip_bits, int nw,
-               uint8_t* __restrict__ keep, int* __restrict__ counts, int* __restrict__ blocks,
-               int* __restrict__ refine, int rw, int* __restrict__ refine_counts, int* __restrict__ means,
-               int* __restrict__ mean_counts, int nb, int nq, int H) {
-    __shared__ int warp_cnt[SEL_MAX_ITEMS * (SEL_THREADS / 32)];
-    const int t = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
-    const int* ew = exact_bits + ((size_t)h * nq + t) * nw;
-    const int* sw = skip_bits + ((size_t)h * nq + t) * nw;
-    bool exact[ITEMS], refined[ITEMS], mean[ITEMS];
-#pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-        const int j = i * SEL_THREADS + tid;
-        const bool valid = j < nb;
-        const bool e = valid && ((ew[j >> 5 < nw ? j >> 5 : 0] >> (j & 31)) & 1);
-        const bool s = valid && ((sw[j >> 5 < nw ? j >> 5 : 0] >> (j & 31)) & 1);
-        exact[i] = e;
-        refined[i] = valid && s && !e;
-        mean[i] = valid && !s;
-    }
-    int pos[ITEMS];
-    const size_t lbase = ((size_t)t * H + h) * nb;
-    const int nmean = compact_positions<ITEMS>(mean, pos, warp_cnt);
-#pragma unroll
-    for (int i = 0; i < ITEMS; ++i)
-        if (mean[i]) means[lbase + pos[i]] = i * SEL_THREADS + tid;
-    const int nexact = compact_positions<ITEMS>(exact, pos, warp_cnt);
-#pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-        const int j = i * SEL_THREADS + tid;
-        if (exact[i]) blocks[lbase + pos[i]] = j;
-        if (j < nb) keep[((size_t)h * nq + t) * nb + j] = exact[i] ? 1 : 0;
-    }
-    const int nref = compact_positions<ITEMS>(refined, pos, warp_cnt);
-    int* rlist = refine + ((size_t)t * H + h) * rw;
-    for (int j = nref + tid; j < rw; j += SEL_THREADS) rlist[j] = nb;
-#pragma unroll
-    for (int i = 0; i < ITEMS; ++i)
-        if (refined[i] && pos[i] < rw) rlist[pos[i]] = i * SEL_THREADS + tid;
-    if (tid == 0) {
-        mean_counts[t * H + h] = nmean;
-        counts[t * H + h] = nexact;
-        refine_counts[t * H + h] = min(nref, rw);
     }
 }
 
@@ -423,7 +374,7 @@ extern "C" int es_select_blocks(const float* mass, const uint8_t* keep_prev, con
         return set_error(-1, "es_select_blocks: null pointer");
     if (L <= 0 || H <= 0) return set_error(-1, "es_select_blocks: L and H must be positive");
     const int nq = (L + 127) / 128, nb = (L + 63) / 64;
-    if (nb > SEL_THREADS * SEL_MAX_ITEMS) return set_error(-1, "es_select_blocks: more than 4096 kv blocks");
+    if (nb > SEL_THREADS * ITEMS) return set_error(-1, "es_select_blocks: more than 4096 kv blocks");
     if (rw < r) return set_error(-1, "es_select_blocks: refine width smaller than r");
     if (rw > 0 && !refine) return set_error(-1, "es_select_blocks: null refine list");
     if (nw * 32 < nb) return set_error(-1, "es_select_blocks: skip_bits has fewer than nb bits per tile");
@@ -446,17 +397,9 @@ extern "C" int es_select_blocks(const float* mass, const uint8_t* keep_prev, con
         ES_CHECK_LAUNCH("select_blocks");
         return 0;
     }
-    const int items = (nb + SEL_THREADS - 1) / SEL_THREADS;
-#define ES_SELECT_LAUNCH(N)                                                                                         \
-    select_kernel<N><<<dim3(nq, H), SEL_THREADS, 0, (cudaStream_t)stream>>>(mass, keep_prev, scale_exact, scale_skip, \
-                                                                             keep, counts, blocks, flags, skip_bits, \
-                                                                             nw, refine, rw, k, r, nb, L, sink, H, nq)
-    if (items <= 1) ES_SELECT_LAUNCH(1);
-    else if (items <= 2) ES_SELECT_LAUNCH(2);
-    else if (items <= 4) ES_SELECT_LAUNCH(4);
-    else if (items <= 8) ES_SELECT_LAUNCH(8);
-    else ES_SELECT_LAUNCH(16);
-#undef ES_SELECT_LAUNCH
+    select_kernel<<<dim3(nq, H), SEL_THREADS, 0, (cudaStream_t)stream>>>(mass, keep_prev, scale_exact, scale_skip, keep, counts,
+                                                                         blocks, flags, skip_bits, nw, refine, rw, k, r, nb, L,
+                                                                         sink, H, nq);
     ES_CHECK_LAUNCH("select_blocks");
     return 0;
 }
@@ -478,33 +421,18 @@ extern "C" int es_rebuild_plan(const int32_t* exact_bits, const int32_t* skip_bi
     if ((means == nullptr) != (mean_counts == nullptr))
         return set_error(-1, "es_rebuild_plan: give both the mean list and its counts, or neither");
     if (rw > 0 && !refine) return set_error(-1, "es_rebuild_plan: null refine list");
-    if (nb > SEL_THREADS * SEL_MAX_ITEMS) return set_error(-1, "es_rebuild_plan: more than 4096 kv blocks");
+    if (nb > SEL_THREADS * ITEMS) return set_error(-1, "es_rebuild_plan: more than 4096 kv blocks");
     if (nw * 32 < nb) return set_error(-1, "es_rebuild_plan: fewer than nb bits per tile");
-    if (nb <= 4096) {
-        const int ipl = (nb + 31) / 32, units = nq * H;
-        const dim3 grid((units + SELW_WARPS - 1) / SELW_WARPS);
+    const int ipl = (nb + 31) / 32, units = nq * H;
+    const dim3 grid((units + SELW_WARPS - 1) / SELW_WARPS);
 #define ES_REBUILDW_LAUNCH(N)                                                                                           \
     rebuild_warp_kernel<N><<<grid, SELW_WARPS * 32, 0, (cudaStream_t)stream>>>(exact_bits, skip_bits, nw, keep, counts,  \
                                                                                 blocks, refine, rw, refine_counts,      \
                                                                                 means, mean_counts, nb, nq, H)
-        if (ipl <= 16) ES_REBUILDW_LAUNCH(16);
-        else if (ipl <= 64) ES_REBUILDW_LAUNCH(64);
-        else ES_REBUILDW_LAUNCH(128);
+    if (ipl <= 16) ES_REBUILDW_LAUNCH(16);
+    else if (ipl <= 64) ES_REBUILDW_LAUNCH(64);
+    else ES_REBUILDW_LAUNCH(128);
 #undef ES_REBUILDW_LAUNCH
-        ES_CHECK_LAUNCH("rebuild_plan");
-        return 0;
-    }
-    const int items = (nb + SEL_THREADS - 1) / SEL_THREADS;
-#define ES_REBUILD_LAUNCH(N)                                                                                          \
-    rebuild_kernel<N><<<dim3(nq, H), SEL_THREADS, 0, (cudaStream_t)stream>>>(exact_bits, skip_bits, nw, keep, counts,  \
-                                                                              blocks, refine, rw, refine_counts, means, \
-                                                                              mean_counts, nb, nq, H)
-    if (items <= 1) ES_REBUILD_LAUNCH(1);
-    else if (items <= 2) ES_REBUILD_LAUNCH(2);
-    else if (items <= 4) ES_REBUILD_LAUNCH(4);
-    else if (items <= 8) ES_REBUILD_LAUNCH(8);
-    else ES_REBUILD_LAUNCH(16);
-#undef ES_REBUILD_LAUNCH
     ES_CHECK_LAUNCH("rebuild_plan");
     return 0;
 }
