@@ -212,9 +212,12 @@ pack_kernel(const uint8_t* __restrict__ keep, int* __restrict__ exact_bits, int 
 // largest key is then found the way the reference finds it (31 halvings of [0, 0x7F800001) on the int32 bit patterns,
 // triton_ops.py:43-54), each step one compare per held key and a warp sum: no shared memory, no atomics, no CTA barrier,
 // and every warp of a CTA works on a tile of its own. Word i of a bit mask is simply the ballot of round i.
-// Issue slots bound it (two searches of 31 steps over 37 or 59 keys a lane are most of its instructions), so a search ends
-// with the first threshold that exactly K keys reach: their smallest is the K-th largest. Distinct keys take about 14 steps,
-// ties at the cut all 31. Selection of 591 x 40 tiles of 1,182 blocks 0.545 -> 0.301 ms, of 256 x 12 tiles of 512 27.6 -> 19.0 us.
+// Its instructions bound it, not memory (591 x 40 tiles of 1,182 blocks: 60 % of the issue slots and 54 % of the ALU pipe with
+// four warps a scheduler, most stalls the latency of one compare and add to the next; 579 GB/s of DRAM), and a step of a search
+// compares every slot of a lane, empty ones too (40 at 1,182 blocks, 64 at 1,861). So a search ends with the first threshold that
+// exactly K keys reach: their smallest is the K-th largest. Distinct keys take about 14 steps, ties at the cut all 31. Against 31
+// steps always, us: 591 x 40 tiles of 1,182 blocks 513 -> 286 (masses that tie: 513 -> 384), 256 x 12 tiles of 512 blocks 27.4 ->
+// 19.2 (27.4 -> 27.4).
 constexpr int SELW_WARPS = 8;
 
 template <int IPL>
@@ -238,9 +241,13 @@ __device__ __forceinline__ int kth_largest_key_warp(const int (&key)[IPL], int K
     return lo;
 }
 
-// A lane that holds more than 40 keys reads the raw masses a second time for the refine list (from L2) instead of keeping them
-// beside the keys: with both it had the registers of one CTA per SM (931 x 24 tiles of 1,861 blocks: 1.40 -> 0.52 ms, the shorter
-// search included).
+// The refine list needs the raw masses once more. Whether a lane keeps them beside its keys or reads them again (from L2) is a
+// matter of registers, 128 a thread so that two CTAs share an SM. Random masses, us kept / read again (spilled bytes):
+//   24 slots, 350 x 40 tiles of 700 blocks  105.7 / 94.9 (0 / 0)      48 slots, 750 x 24 tiles of 1,500 blocks  264 / 286 (140 / 52)
+//   32 slots, 500 x 40 tiles of 1,000       257 / 191 (8 / 0)         64 slots, 931 x 24 tiles of 1,861         542 / 512 (576 / 92)
+//   40 slots, 591 x 40 tiles of 1,182       286 / 295 (12 / 16)
+// With 16 slots reading again is 0 to 9 % faster, with 8 even. Kept in 196 and 246 registers, one CTA per SM: 683 and 1,140 us with
+// 48 and 64 slots.
 template <int IPL>
 __global__ void __launch_bounds__(SELW_WARPS * 32, 2)
 select_warp_kernel(const float* __restrict__ map, const uint8_t* __restrict__ keep_prev,
@@ -259,7 +266,7 @@ select_warp_kernel(const float* __restrict__ map, const uint8_t* __restrict__ ke
     const bool fell_back = flags[t * H + h] != 0;
     const unsigned below = (1u << lane) - 1u;
 
-    constexpr bool KEEP_RAW = IPL <= 40;
+    constexpr bool KEEP_RAW = IPL == 40 || IPL == 48;
     float raw[KEEP_RAW ? IPL : 1];
     int key[IPL];
 #pragma unroll
