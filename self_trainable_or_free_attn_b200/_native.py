@@ -9,7 +9,7 @@ import functools
 import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
-# ECHOSPARSE_SM100_LIB selects another build of the same library (for example one compiled with other -D options).
+# ECHOSPARSE_SM100_LIB selects another build of the same library (for example an older one, to compare the two).
 LIB_PATH = os.environ.get("ECHOSPARSE_SM100_LIB") or os.path.join(_HERE, "_lib", "libechosparse_sm100.so")
 
 _P = ctypes.c_void_p

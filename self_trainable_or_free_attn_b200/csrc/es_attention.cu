@@ -103,34 +103,7 @@ struct AttnArgs {
     int* status;
 };
 
-// p = 2^x for a pair of columns. MUFU computes 16 exponentials per clock and SM, about as many clocks as the tensor
-// cores need for the same tile, so a share of the pairs can be computed on the FMA pipe instead: x = n + f with
-// n = floor(x), 2^f by a degree-4 polynomial (relative error 3e-6, far below the bf16 rounding of P), n added to the
-// exponent field.
-__device__ __forceinline__ float2 exp2_pair_mufu(float2 x) { return make_float2(ex2_approx(x.x), ex2_approx(x.y)); }
-__device__ __forceinline__ float2 exp2_pair_fma(float2 x) {
-    const float M = 12582912.0f;                               // 2^23 + 2^22: the integer part lands in the low mantissa bits
-    x.x = fmaxf(x.x, -126.0f);
-    x.y = fmaxf(x.y, -126.0f);
-    const float2 t = __fadd2_rd(x, make_float2(M, M));         // rounded down: f stays in [0, 1)
-    const float2 n = __fadd2_rn(t, make_float2(-M, -M));
-    const float2 f = __ffma2_rn(n, make_float2(-1.0f, -1.0f), x);
-    float2 p = make_float2(0.013426586054265499f, 0.013426586054265499f);
-    p = __ffma2_rn(p, f, make_float2(0.05224263295531273f, 0.05224263295531273f));
-    p = __ffma2_rn(p, f, make_float2(0.24128012359142303f, 0.24128012359142303f));
-    p = __ffma2_rn(p, f, make_float2(0.6930448412895203f, 0.6930448412895203f));
-    p = __ffma2_rn(p, f, make_float2(1.0f, 1.0f));
-    p.x = __int_as_float(__float_as_int(p.x) + (__float_as_int(t.x) << 23));
-    p.y = __int_as_float(__float_as_int(p.y) + (__float_as_int(t.y) << 23));
-    return p;
-}
-// Pair j (columns 2j, 2j+1) of a thread's 64 columns goes to the FMA pipe when bit (j & 7) of ES_EMU_PATTERN is set.
-// Measured on B200 with this kernel: 0x00 (all MUFU) 1.549 ms, 0x11 1.561 ms, 0x55 1.660 ms (Wan-1.3B shape), so the
-// default keeps every exponential on MUFU; the FMA path stays available for parts with a different balance.
-#ifndef ES_EMU_PATTERN
-#define ES_EMU_PATTERN 0x0
-#endif
-__device__ __forceinline__ constexpr bool emulate_pair(int j) { return (ES_EMU_PATTERN >> (j & 7)) & 1; }
+__device__ __forceinline__ float2 exp2_pair(float2 x) { return make_float2(ex2_approx(x.x), ex2_approx(x.y)); }
 
 // Order of a tile's iterations. The refine iterations (64 small TMA boxes per tile, slow to fill) are spread evenly among
 // the others instead of coming last, so that the ring refills during the cheap iterations in between: iteration i is the
@@ -564,7 +537,7 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
 #pragma unroll
                     for (int j = 0; j < 32; ++j) {
                         const float2 xv = __ffma2_rn(make_float2(__uint_as_float(s[2 * j]), __uint_as_float(s[2 * j + 1])), sc2, off2);
-                        const float2 p = emulate_pair(j) ? exp2_pair_fma(xv) : exp2_pair_mufu(xv);
+                        const float2 p = exp2_pair(xv);
                         if (j & 1) acc1 = __fadd2_rn(acc1, p); else acc = __fadd2_rn(acc, p);
                         pk[j] = pack_bf16x2(p.x, p.y);
                         if (DENSE) rsum = __fadd2_rn(rsum, make_float2(__uint_as_float(pk[j] << 16), __uint_as_float(pk[j] & 0xFFFF0000u)));
@@ -573,7 +546,7 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
 #pragma unroll
                     for (int j = 0; j < 32; ++j) {
                         const float2 xv = __ffma2_rn(make_float2(__uint_as_float(s[2 * j]), __uint_as_float(s[2 * j + 1])), sc2, off2);
-                        float2 p = exp2_pair_mufu(xv);
+                        float2 p = exp2_pair(xv);
                         p.x = 2 * j < lim ? p.x : 0.f;
                         p.y = 2 * j + 1 < lim ? p.y : 0.f;
                         acc = __fadd2_rn(acc, p);
@@ -604,7 +577,7 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
                     if (2 * j == last_c) xv.x += fix;
                     if (2 * j + 1 == last_c) xv.y += fix;
                     if (COMPENSATE) { xv.x = fminf(xv.x, 100.0f); xv.y = fminf(xv.y, 100.0f); }   // triton_ops.py:275
-                    float2 p = exp2_pair_mufu(xv);
+                    float2 p = exp2_pair(xv);
                     const uint32_t w = j < 16 ? w0 : w1;
                     p.x = ((w >> ((2 * j) & 31)) & 1u) ? 0.f : p.x;
                     p.y = ((w >> ((2 * j + 1) & 31)) & 1u) ? 0.f : p.y;
@@ -623,7 +596,7 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
                                                  make_float2(b4.x - m, b4.y - m));
                     const float2 x1 = __ffma2_rn(make_float2(__uint_as_float(s[c + 2]), __uint_as_float(s[c + 3])), sc2,
                                                  make_float2(b4.z - m, b4.w - m));
-                    const float2 p0 = exp2_pair_mufu(x0), p1 = exp2_pair_mufu(x1);
+                    const float2 p0 = exp2_pair(x0), p1 = exp2_pair(x1);
                     acc = __fadd2_rn(acc, p0);
                     acc1 = __fadd2_rn(acc1, p1);
                     pk[c / 2] = pack_bf16x2(p0.x, p0.y);
