@@ -18,6 +18,9 @@ void count_launch();
 // Lets `kernel` use `bytes` of dynamic shared memory on the current device (once per device and kernel). 0 or an error code.
 int opt_in_shared_memory(const void* kernel, int bytes);
 
+// Whether every pointer is a multiple of `bytes` (null ones pass): a vector access to anything else faults.
+template <typename... P> inline bool aligned(uintptr_t bytes, P... p) { return (((uintptr_t)p | ... | (uintptr_t)0) & (bytes - 1)) == 0; }
+
 int encode_tensor_map(CUtensorMap* m, CUtensorMapDataType dt, uint32_t rank, void* base, const cuuint64_t* dims,
                       const cuuint64_t* strides_bytes, const cuuint32_t* box, const cuuint32_t* elem_strides,
                       CUtensorMapSwizzle swizzle);

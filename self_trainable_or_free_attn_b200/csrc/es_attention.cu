@@ -999,7 +999,7 @@ extern "C" int es_sparse_attention(const void* q, const void* k, const void* v, 
     if (rw % 32 != 0) return set_error(-1, "es_sparse_attention: refine width must be a multiple of 32");
     if (rw > 0 && (!refine || !k_rep || !v_rep || !log_counts))
         return set_error(-1, "es_sparse_attention: refine list without representative tables");
-    if (rw > 0 && ((uintptr_t)refine & 15)) return set_error(-1, "es_sparse_attention: refine must be 16-byte aligned");
+    if (rw > 0 && !aligned(16, refine, log_counts)) return set_error(-1, "es_sparse_attention: refine and log_counts must be 16-byte aligned");
     c.a.refine = refine; c.a.rw = rw; c.a.nref = rw / 32;
     c.a.k_rep = (const __nv_bfloat16*)k_rep; c.a.v_rep = (const __nv_bfloat16*)v_rep; c.a.log_counts = log_counts;
     c.a.nb4 = (c.a.nb + 1) * 4;

@@ -702,7 +702,7 @@ extern "C" int es_reps_metric(const void* q, float* gram_parts, float* gram, voi
                               int32_t H, void* stream) {
     if (!q || !gram_parts || !metric || !probes) return set_error(-1, "es_reps_metric: null pointer");
     if (L <= 0 || H <= 0) return set_error(-1, "es_reps_metric: L and H must be positive");
-    if ((uintptr_t)q & 15) return set_error(-1, "es_reps_metric: q must be 16-byte aligned");
+    if (!aligned(16, q, gram_parts, metric)) return set_error(-1, "es_reps_metric: q, gram_parts and metric must be 16-byte aligned");
     const int nb = (L + 63) / 64;
     const int rps = gram_rows_per_split(L), nsplit = (L + rps - 1) / rps;
     cudaStream_t st = (cudaStream_t)stream;
@@ -728,7 +728,8 @@ extern "C" int es_reps_kmeans(const void* k, const void* v, const void* metric, 
     if (!k || !v || !metric || !probes || !k_rep || !v_rep || !log_counts)
         return set_error(-1, "es_reps_kmeans: null pointer");
     if (L <= 0 || H <= 0) return set_error(-1, "es_reps_kmeans: L and H must be positive");
-    if (((uintptr_t)k | (uintptr_t)metric) & 15) return set_error(-1, "es_reps_kmeans: k and metric must be 16-byte aligned");
+    if (!aligned(16, k, v, metric)) return set_error(-1, "es_reps_kmeans: k, v and metric must be 16-byte aligned");
+    if (!aligned(4, probes, k_rep, v_rep, k_mean, v_mean)) return set_error(-1, "es_reps_kmeans: probes, tables and means must be 4-byte aligned");
     if ((k_mean == nullptr) != (v_mean == nullptr)) return set_error(-1, "es_reps_kmeans: give both means or neither");
     const int nb = (L + 63) / 64;
     if (int rc = opt_in_shared_memory((const void*)kmeans_kernel, KM_SMEM)) return rc;
@@ -770,7 +771,7 @@ extern "C" int es_reps_metric_static(const void* q, float* gram, void* metric, v
                                      void* stream) {
     if (!q || !metric || !probes) return set_error(-1, "es_reps_metric_static: null pointer");
     if (L <= 0 || H <= 0) return set_error(-1, "es_reps_metric_static: L and H must be positive");
-    if ((uintptr_t)q & 15) return set_error(-1, "es_reps_metric_static: q must be 16-byte aligned");
+    if (!aligned(16, q, metric)) return set_error(-1, "es_reps_metric_static: q and metric must be 16-byte aligned");
     if (H > ES_STATIC_GRAM_PARTS)
         return set_error(-1, "es_reps_metric_static: more than 256 heads do not fit the built-in scratch; use es_reps_metric");
     float* parts = static_gram_parts();

@@ -257,6 +257,7 @@ extern "C" int es_estimate_skipped(const void* q, const void* k_mean, const uint
     if (!q || !k_mean || !keep || !offset || !lse || !mass || !scale_exact || !scale_skip)
         return set_error(-1, "es_estimate_skipped: null pointer");
     if (L <= 0 || H <= 0) return set_error(-1, "es_estimate_skipped: L and H must be positive");
+    if (!aligned(16, k_mean) || !aligned(4, q)) return set_error(-1, "es_estimate_skipped: k_mean must be 16-byte, q 4-byte aligned");
     const int nq = (L + 127) / 128, nb = (L + 63) / 64;
     const int tail = L - (nb - 1) * 64;
     estimate_kernel<<<dim3((nq + EST_TILES - 1) / EST_TILES, H), 256, 0, (cudaStream_t)stream>>>(

@@ -816,6 +816,7 @@ extern "C" int es_vsa_pool(const void* q, const void* k, const void* v, void* qr
     const int NB = L / TB, G = 64 / R;
     if (Lr_pad < NB * G || NBc_pad < NB) return set_error(-1, "es_vsa_pool: padded sizes smaller than the real ones");
     if ((vr || vc) && !v) return set_error(-1, "es_vsa_pool: v outputs without v");
+    if (!aligned(4, q, k, v, qr, kr, vr, qc, kc, vc)) return set_error(-1, "es_vsa_pool: tensors must be 4-byte aligned");
     PoolArgs a{q, k, v, qr, kr, vr, qc, kc, vc, blk_cnt, L, NB, R, G, Lr_pad, NBc_pad};
     cudaStream_t st = (cudaStream_t)stream;
     const int rows = max(max(NB, NBc_pad), (Lr_pad + G - 1) / G);
@@ -857,6 +858,7 @@ extern "C" int es_vsa_router_lse(const void* qr, const void* kr, float* lse2, co
     if (int rc = check_shape("es_vsa_router_lse", BH, NB * TB, D, dtype)) return rc;
     if (R < 1 || R > 64 || 64 % R != 0 || Lr_pad % TB != 0 || Lr_pad < NB * (64 / R))
         return set_error(-1, "es_vsa_router_lse: R must divide 64 and Lr_pad be a multiple of 64 covering NB * 64 / R");
+    if (!aligned(16, qr, kr)) return set_error(-1, "es_vsa_router_lse: qr and kr must be 16-byte aligned");
     RouterArgs a{qr, kr, lse2, nullptr, blk_cnt, NB, R, 64 / R, NB * (64 / R), Lr_pad, 0, 1, LOG2E / sqrtf((float)D)};
     return launch_router<0>(a, D, dtype, BH, (cudaStream_t)stream);
 }
@@ -870,6 +872,7 @@ extern "C" int es_vsa_router_scores(const void* qr, const void* kr, const float*
         return set_error(-1, "es_vsa_router_scores: R must divide 64 and Lr_pad be a multiple of 64 covering NB * 64 / R");
     if (bh0 < 0 || bh_count < 1 || bh0 + bh_count > BH) return set_error(-1, "es_vsa_router_scores: bad (b, h) range");
     if (row_norm != 0 && row_norm != 1) return set_error(-1, "es_vsa_router_scores: row_norm must be 0 or 1");
+    if (!aligned(16, qr, kr)) return set_error(-1, "es_vsa_router_scores: qr and kr must be 16-byte aligned");
     RouterArgs a{qr, kr, const_cast<float*>(lse2), scores, blk_cnt, NB, R, 64 / R, NB * (64 / R), Lr_pad, bh0, row_norm,
                  LOG2E / sqrtf((float)D)};
     return launch_router<1>(a, D, dtype, bh_count, (cudaStream_t)stream);
@@ -931,6 +934,7 @@ extern "C" int es_vsa_fuse_fwd(const void* of, const void* oc, const void* gate,
     if (int rc = check_shape("es_vsa_fuse_fwd", BH, L, D, dtype)) return rc;
     if (gate_mode < 0 || gate_mode > 2 || (gate_mode != 0 && !gate)) return set_error(-1, "es_vsa_fuse_fwd: bad gate mode");
     if (gate_act < 0 || gate_act > 1 || NBc_pad < L / TB) return set_error(-1, "es_vsa_fuse_fwd: bad gate_act or NBc_pad");
+    if (!aligned(4, of, oc, o, gate_mode == 2 ? gate : nullptr)) return set_error(-1, "es_vsa_fuse_fwd: tensors must be 4-byte aligned");
     FuseArgs a{};
     a.of = of; a.oc = oc; a.gate = gate; a.o = o; a.blk_cnt = blk_cnt; a.L = L; a.NB = L / TB; a.NBc_pad = NBc_pad;
     a.gate_mode = gate_mode; a.gate_act = gate_act;
@@ -950,6 +954,8 @@ extern "C" int es_vsa_fuse_bwd(const void* dout, const void* of, const void* oc,
     if (int rc = check_shape("es_vsa_fuse_bwd", BH, L, D, dtype)) return rc;
     if (gate_mode < 0 || gate_mode > 2 || (gate_mode != 0 && (!gate || !dgate))) return set_error(-1, "es_vsa_fuse_bwd: bad gate mode");
     if (gate_act < 0 || gate_act > 1 || NBc_pad < L / TB) return set_error(-1, "es_vsa_fuse_bwd: bad gate_act or NBc_pad");
+    if (!aligned(4, dout, of, oc, dout_f, dout_c, gate_mode == 2 ? gate : nullptr, gate_mode == 2 ? dgate : nullptr))
+        return set_error(-1, "es_vsa_fuse_bwd: tensors must be 4-byte aligned");
     FuseArgs a{};
     a.dout = dout; a.of = of; a.oc = oc; a.gate = gate; a.dout_f = dout_f; a.delta_f = delta_f; a.dout_c = dout_c;
     a.delta_c = delta_c; a.dgate = dgate; a.blk_cnt = blk_cnt; a.L = L; a.NB = L / TB; a.NBc_pad = NBc_pad;
@@ -968,6 +974,7 @@ extern "C" int es_vsa_finalize(const float* acc, const float* add, void* out, co
     if (!out || !blk_cnt) return set_error(-1, "es_vsa_finalize: null pointer");
     if (int rc = check_shape("es_vsa_finalize", BH, L, D, dtype)) return rc;
     if (add && add_nb < L / TB) return set_error(-1, "es_vsa_finalize: add_nb smaller than the block count");
+    if (!aligned(4, out)) return set_error(-1, "es_vsa_finalize: out must be 4-byte aligned");
     FinalArgs a{acc, add, out, blk_cnt, L, add_nb};
     cudaStream_t st = (cudaStream_t)stream;
     const dim3 grid(L / TB, BH);
@@ -981,6 +988,7 @@ extern "C" int es_vsa_block_scores(const void* qc, const void* kc, void* scores,
     if (!qc || !kc || !scores) return set_error(-1, "es_vsa_block_scores: null pointer");
     if (int rc = check_shape("es_vsa_block_scores", BH, NB * TB, D, dtype)) return rc;
     if (NBc_pad < NB || bh0 < 0 || bh_count < 1 || bh0 + bh_count > BH) return set_error(-1, "es_vsa_block_scores: bad sizes");
+    if (!aligned(4, qc, kc)) return set_error(-1, "es_vsa_block_scores: qc and kc must be 4-byte aligned");
     BlockScoreArgs a{qc, kc, scores, NB, NBc_pad, bh0, 1.0f / sqrtf((float)D)};
     cudaStream_t st = (cudaStream_t)stream;
     const dim3 grid((NB + 127) / 128, NB, bh_count);

@@ -218,6 +218,7 @@ extern "C" int es_vsa_split_merge_fwd(const float* part_o, const float* part_lse
     if (!part_o || !part_lse) return set_error(-1, "es_vsa_split_merge_fwd: null partials");
     if (L <= 0 || L % TB != 0 || (D != 64 && D != 128) || (dtype != 0 && dtype != 1))
         return set_error(-1, "es_vsa_split_merge_fwd: bad L, D or dtype");
+    if (!aligned(16, part_o, merges) || !aligned(8, o)) return set_error(-1, "es_vsa_split_merge_fwd: part_o and merges must be 16-byte, o 8-byte aligned");
     MergeArgs a{};
     a.merges = merges; a.info = info; a.blk_cnt = blk_cnt; a.part = part_o; a.part_lse = part_lse; a.out = o; a.lse = lse;
     a.L = L; a.NB = L / TB; a.mask_rows = mask_rows;
@@ -233,6 +234,8 @@ extern "C" int es_vsa_split_merge_sum(const float* part, const int32_t* merges, 
     if (L <= 0 || L % TB != 0 || (D != 64 && D != 128) || (dtype != 0 && dtype != 1))
         return set_error(-1, "es_vsa_split_merge_sum: bad L, D or dtype");
     if (add && add_nb < L / TB) return set_error(-1, "es_vsa_split_merge_sum: add_nb smaller than the block count");
+    if (!aligned(16, part, add, merges, out_f32) || !aligned(8, out))
+        return set_error(-1, "es_vsa_split_merge_sum: part, add, merges and out_f32 must be 16-byte, out 8-byte aligned");
     MergeArgs a{};
     a.merges = merges; a.info = info; a.blk_cnt = blk_cnt; a.part = part; a.add = add; a.add_nb = add_nb; a.out = out;
     a.out_f32 = out_f32; a.L = L; a.NB = L / TB;

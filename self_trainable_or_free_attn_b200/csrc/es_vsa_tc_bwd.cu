@@ -659,6 +659,8 @@ int attn_bwd_tc(bool kv, const void* q, const void* k, const void* v, const void
                 void* out0, void* out1, float* f0, float* f1, const float* add0, const float* add1, int add_nb,
                 const int* row_ptr, const int* col_idx, const int* blk_cnt, int BH, int L, int rows, int D, int dtype, const int* tasks,
                 const int* task_info, int n_tasks, float* part0, float* part1, cudaStream_t st) {
+    if (!aligned(4, out0, out1) || !aligned(8, f0, f1, part0, part1))
+        return set_error(-1, "attn_bwd_tc: 16-bit gradients must be 4-byte, fp32 gradients and partials 8-byte aligned");
     int* status = device_status_ptr();
     if (!status) return set_error(-2, "attn_bwd_tc: the device status word is not available on this device");
     const float scale = 1.f / sqrtf((float)D);
@@ -706,6 +708,7 @@ int tier_bwd_q_tc(const void* q, const void* k, const void* v, const void* k_mid
                   const void* v_tail, const void* dout, const float* lse, const float* delta, void* dq, const float* add, int add_nb,
                   const int* row_ptr, const int* col_idx, const TierMaps& tier, const int* blk_cnt, int BH, int L, int D, int dtype,
                   cudaStream_t st) {
+    if (!aligned(4, dq)) return set_error(-1, "tier_bwd_q_tc: dq must be 4-byte aligned");
     int* status = device_status_ptr();
     if (!status) return set_error(-2, "tier_bwd_q_tc: the device status word is not available on this device");
     const float scale = 1.f / sqrtf((float)D);
@@ -718,6 +721,7 @@ int tier_bwd_q_tc(const void* q, const void* k, const void* v, const void* k_mid
 int tier_rep_bwd_tc(const void* q, const void* k_mid, const void* v_mid, const void* k_tail, const void* v_tail, const void* dout,
                     const float* lse, const float* delta, float* dk_mid, float* dv_mid, float* dk_tail, float* dv_tail,
                     const TierMaps& tier, const int* blk_cnt, int BH, int L, int D, int dtype, int tiles, cudaStream_t st) {
+    if (!aligned(8, dk_mid, dv_mid, dk_tail, dv_tail)) return set_error(-1, "tier_rep_bwd_tc: the tables' gradients must be 8-byte aligned");
     int* status = device_status_ptr();
     if (!status) return set_error(-2, "tier_rep_bwd_tc: the device status word is not available on this device");
     const float scale = 1.f / sqrtf((float)D);

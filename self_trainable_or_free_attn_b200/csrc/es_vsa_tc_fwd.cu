@@ -492,6 +492,7 @@ static int launch_fwd(const void* q, const void* k, const void* v, FwdTcArgs a, 
 int attn_fwd_tc(const void* q, const void* k, const void* v, void* o, float* lse, const int* row_ptr, const int* col_idx,
                 const int* blk_cnt, int BH, int L, int rows, int D, int dtype, const int* tasks, const int* task_info, int n_tasks,
                 float* part_o, float* part_lse, cudaStream_t st) {
+    if (!aligned(4, o) || !aligned(8, part_o)) return set_error(-1, "attn_fwd_tc: o must be 4-byte, part_o 8-byte aligned");
     int* status = device_status_ptr();
     if (!status) return set_error(-2, "attn_fwd_tc: the device status word is not available on this device");
     const FwdTcArgs a{o, lse, row_ptr, col_idx, blk_cnt, L, L / TB, rows, kLog2e / sqrtf((float)D), tasks, task_info, part_o, part_lse, status, {}};
@@ -521,6 +522,7 @@ static int launch_tier_fwd(const void* q, const void* k, const void* v, const vo
 int tier_fwd_tc(const void* q, const void* k, const void* v, const void* k_mid, const void* v_mid, const void* k_tail,
                 const void* v_tail, void* o, float* lse, const int* row_ptr, const int* col_idx, const TierMaps& tier,
                 const int* blk_cnt, int BH, int L, int D, int dtype, cudaStream_t st) {
+    if (!aligned(4, o)) return set_error(-1, "tier_fwd_tc: o must be 4-byte aligned");
     int* status = device_status_ptr();
     if (!status) return set_error(-2, "tier_fwd_tc: the device status word is not available on this device");
     FwdTcArgs a{o, lse, row_ptr, col_idx, blk_cnt, L, L / TB, 0, kLog2e / sqrtf((float)D), nullptr, nullptr, nullptr, nullptr,

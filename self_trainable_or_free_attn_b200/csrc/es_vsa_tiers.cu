@@ -152,6 +152,7 @@ extern "C" int es_vsa_tier_unpool(const float* tok, const float* mid, const floa
     if (!out || !blk_cnt) return set_error(-1, "es_vsa_tier_unpool: null pointer");
     if (int rc = check_tier("es_vsa_tier_unpool", BH, L, D, dtype, mid_reps, 7, mid ? mid_stride : 1 << 30, tail ? tail_stride : 1 << 30)) return rc;
     if (add && add_nb < L / TB) return set_error(-1, "es_vsa_tier_unpool: add_nb smaller than the block count");
+    if (!aligned(4, out)) return set_error(-1, "es_vsa_tier_unpool: out must be 4-byte aligned");
     UnpoolArgs a{tok, mid, tail, add, out, blk_cnt, L, mid_reps, mid_stride, tail_stride, add_nb};
     cudaStream_t st = (cudaStream_t)stream;
     const dim3 grid(L / TB, BH);
