@@ -86,9 +86,10 @@ full_scale_kernel(const float* __restrict__ m, float* __restrict__ lse, float* _
 // 64 blocks (cp.async, two stages, 16-byte chunks XOR-swizzled by the row) that all eight warps consume with ldmatrix:
 // S(16 sampled rows x 64 blocks) by mma.sync m16n8k16 over d. Reading the keys once per eight tiles with 16-byte accesses,
 // instead of once per tile with 4-byte ones, is what the kernel's time depends on (the keys of a head are 300 KB).
-// What bounds it now is issue: the products (mma.sync), the exponentials and the sums over the 16 rows, which a halving exchange
-// does with 14 shuffles per 64 blocks where every lane adding every column took 48: 591 x 40 tiles of 1,182 blocks 0.790 ->
-// 0.675 ms, 931 x 24 tiles of 1,861 blocks 1.227 -> 1.035 ms, 256 x 12 tiles of 512 blocks 66 -> 54 us.
+// What bounds it now is the chain of a warp (products by mma.sync, exponentials, sums over the 16 rows) with four warps a
+// scheduler: 49 % of the issue slots, 579 GB/s of DRAM, stalls mostly fixed latencies and the results of ldmatrix, exponentials and
+// shuffles. So the sums are a halving exchange of 14 shuffles per 64 blocks where every lane adding every column took 48: 591 x 40
+// tiles of 1,182 blocks 0.790 -> 0.675 ms, 931 x 24 tiles of 1,861 blocks 1.227 -> 1.035 ms, 256 x 12 tiles of 512 blocks 66 -> 54 us.
 constexpr int EST_TILES = 8;
 __global__ void __launch_bounds__(256)
 estimate_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ km,
