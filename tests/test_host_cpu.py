@@ -192,8 +192,14 @@ def test_calls_under_way_together_list_their_tiles_in_scratch_of_their_own(monke
     monkeypatch.setattr(sm100, "_cuda_bf16", lambda *t: None)
     monkeypatch.setattr(sm100.N, "load", Library)
     monkeypatch.setattr(sm100.N, "stream_ptr", lambda: stream[0])
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
     call(*args)
     assert len(scratch) == 3 and None not in scratch and len(set(scratch)) == 3
     for n in range(1, 40):                                # every size another buffer, the last few kept
         sm100._tile_list_scratch(torch.zeros(n, dtype=torch.int32), 0)
         assert len(sm100._scratch.__dict__) <= sm100._SCRATCH_SIZES
+    kept = dict(sm100._scratch.__dict__)                  # a captured call neither takes a kept buffer nor leaves one behind
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    for buf in kept.values():
+        assert sm100._tile_list_scratch(buf[1:], 0).data_ptr() not in {b.data_ptr() for b in kept.values()}
+    assert sm100._scratch.__dict__ == kept
