@@ -139,9 +139,9 @@ _SCRATCH_SIZES = 8
 def _tile_list_scratch(flags, stream):
     """Device scratch for the list of flagged tiles (one int32 per tile and one for the count). The list and the kernel that walks
     it are two launches, so a call on another stream or from another thread has scratch of its own. A thread keeps the last few
-    (a tensor per call takes about 4 us of the host, two calls 5 % of a step of 4,152 tokens); what it drops, the allocator gives
-    out again in the order of the stream it was used on. A graph outlives that order: a captured call takes its scratch from the
-    graph's pool, and the graph keeps it."""
+    (0.6 us of the host a call, a tensor per call 1.5 and its release: a step of 4,152 tokens 162 -> 170 us with the latter); what it
+    drops, the allocator gives out again in the order of the stream it was used on. A graph outlives that order: a captured call
+    takes its scratch from the graph's pool, and the graph keeps it."""
     if torch.cuda.is_current_stream_capturing():
         return torch.empty(flags.numel() + 1, device=flags.device, dtype=torch.int32)
     pool = _scratch.__dict__
