@@ -71,6 +71,12 @@ int es_sparse_attention(const void* q, const void* k, const void* v, const void*
  * of the keys where that takes two (rounding differs); no lists and no scratch. */
 int es_dense_attention(const void* q, const void* k, const void* v, void* out, float* lse, int32_t L, int32_t H, void* stream);
 
+/* The same with device scratch of es_dense_scratch_bytes(L, H) bytes (16-byte aligned, on the current device; 0: none needed), which
+ * lets it cut tiles between CTAs where the tiles alone would leave SMs idle. A null scratch is es_dense_attention. */
+long long es_dense_scratch_bytes(int32_t L, int32_t H);
+int es_dense_attention_split(const void* q, const void* k, const void* v, void* out, float* lse, void* scratch,
+                             int64_t scratch_bytes, int32_t L, int32_t H, void* stream);
+
 /* Online-softmax attention over the block list for the tiles whose flag is set; writes out and lse of those tiles.
  * Replaces echosparse/kernels/triton_ops.py:237 `exact_fallback(q, k, v, out, counts, blocks, lse, flags)`.
  * tile_scratch: device scratch of ceil(L / 128) * H + 1 int32, or NULL. With it the flagged tiles are first listed (one

@@ -29,6 +29,8 @@ SIGNATURES = {
     "es_sparse_attention": [_P, _P, _P, _P, _P, _P, _I, _P, _P, _P, _I, _P, _P, _P, _P, _I, _P, _P, _P, _P, _I, _I, _F,
                             _P],
     "es_dense_attention": [_P, _P, _P, _P, _P, _I, _I, _P],
+    "es_dense_scratch_bytes": [_I, _I],
+    "es_dense_attention_split": [_P, _P, _P, _P, _P, _P, _I64, _I, _I, _P],
     "es_exact_fallback": [_P, _P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _P, _P],
     "es_compensate_fallback": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _P, _P],
     "es_block_means": [_P, _P, _P, _P, _I, _I, _P],
@@ -73,6 +75,7 @@ SIGNATURES = {
     "es_vsa_tier_unpool": [_P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
 }
 _RESTYPES = {"es_last_error": ctypes.c_char_p, "es_launch_count": ctypes.c_longlong,
+             "es_dense_scratch_bytes": ctypes.c_longlong,
              "es_vsa_topk_workspace_bytes": ctypes.c_longlong, "es_vsa_split_plan_workspace_bytes": ctypes.c_longlong,
              "es_vsa_topk_bits_offset": ctypes.c_longlong}
 

@@ -54,6 +54,22 @@ int opt_in_shared_memory(const void* kernel, int bytes) {
     return 0;
 }
 
+int prefer_shared_memory(const void* kernel) {
+    struct Done { int dev; const void* kernel; };
+    static std::mutex mu;
+    static std::vector<Done> done;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return set_error(-2, cudaGetErrorString(e));
+    std::lock_guard<std::mutex> lock(mu);
+    for (const Done& d : done)
+        if (d.dev == dev && d.kernel == kernel) return 0;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return set_error(-2, cudaGetErrorString(e));
+    done.push_back({dev, kernel});
+    return 0;
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);

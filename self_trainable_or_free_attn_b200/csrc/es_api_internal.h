@@ -18,6 +18,10 @@ void count_launch();
 // Lets `kernel` use `bytes` of dynamic shared memory on the current device (once per device and kernel). 0 or an error code.
 int opt_in_shared_memory(const void* kernel, int bytes);
 
+// Asks that an SM runs `kernel` (which uses little shared memory) with the largest shared-memory share, as the attention kernels
+// do: an SM changes its share only when it is empty, so kernels that agree on it may follow one another without draining it.
+int prefer_shared_memory(const void* kernel);
+
 // Whether every pointer is a multiple of `bytes` (null ones pass): a vector access to anything else faults.
 template <typename... P> inline bool aligned(uintptr_t bytes, P... p) { return (((uintptr_t)p | ... | (uintptr_t)0) & (bytes - 1)) == 0; }
 
@@ -31,5 +35,18 @@ int encode_tensor_map(CUtensorMap* m, CUtensorMapDataType dt, uint32_t rank, voi
         if (e__ != cudaSuccess) return es::set_error(-2, cudaGetErrorString(e__)); \
         es::count_launch();                                                       \
     } while (0)
+
+// Launches a kernel that may begin before the previous one on the stream has ended: it must call wait_prerequisites() before it
+// reads what that one wrote or writes what that one reads.
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+    cfg.attrs = &attr; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
 
 }  // namespace es

@@ -25,9 +25,12 @@
 // P (bf16 pairs) is written over the S columns it came from and is the A operand of PV. Two S buffers let QK of
 // iteration i + 1 run while the softmax warps work on iteration i; PV(i) and QK(i + 2) follow as soon as P(i) is stored.
 // K and V tiles (32 KB each, [d half][128 rows][128 B], four 8 KB TMA boxes; representative rows: 64 boxes of 512 B)
-// travel through a ring of NSLOT shared-memory slots, about three iterations ahead of the MMAs.
+// travel through a ring of NSLOT shared-memory slots, about three iterations ahead of the MMAs. With one CTA per SM nothing hides
+// a tile's start and end, so Q and O cross shared memory in whole lines: a tile of 32 iterations took 66,900 clocks with a row per
+// thread on both sides, 60,300 now (one launch of the fused step of 32,760 tokens, 47 iterations a tile: 1.315 -> 1.28 ms).
 #include "es_ptx.cuh"
 #include "es_api_internal.h"
+#include <algorithm>
 
 namespace es {
 
@@ -41,7 +44,11 @@ constexpr int NMASS = 8;      // sets of partial block masses in flight between 
 constexpr uint32_t TMEM_COLS = 512;
 constexpr uint32_t O_COL = 256, Q_COL = 384;
 constexpr int NSLOT = 6;      // K / V tiles in flight
+constexpr int Q_SLOT = NSLOT - 1;    // Q passes through this slot before its first K / V tile
 constexpr float kSeedLimit = 60.f;   // largest log2 row sum relative to a seeded offset (see dense_kernel)
+// Dense: a term below 1 / kTopShare of its row, which rounding changes by less than kTopLeast of the row (2^-9 / 64), stays rounded:
+// all terms' rounding together is some fifty times that.
+constexpr float kTopShare = 64.f, kTopLeast = 1.f / 32768.f;
 constexpr int NBIAS = 8;      // refine iterations whose column biases are staged in shared memory at a time
 
 constexpr uint32_t TILE_BYTES = 128 * HD * 2;    // 32 KB: [d half][128 rows][64 d], 128B-swizzled
@@ -54,7 +61,7 @@ constexpr uint32_t SMEM_MASS = SMEM_BIAS + NBIAS * 128 * 4;            // [NMASS
 constexpr uint32_t SMEM_ALLOC = SMEM_MASS + NMASS * 2 * BM * 4;        // 214,528 B: one CTA per SM
 
 struct Ctl {
-    uint64_t qfull;
+    uint64_t qload, qfull;             // Q in shared memory; Q in tensor memory (and its ring slot free)
     uint64_t full[NSLOT], empty[NSLOT];
     uint64_t sfull[2], pfull[2];
     uint64_t ofull, drain;
@@ -103,6 +110,19 @@ struct AttnArgs {
     int* status;
 };
 
+// How dense_kernel shares out its tiles (plan_dense chooses). CTA c takes the whole tiles c, c + grid, .. below `whole`; the
+// iterations of the tiles from there on are one line, of which it takes [edge(c), edge(c + 1)) (c < ctas). dense_merge_kernel
+// puts together the tiles that more than one CTA worked on.
+struct DenseSplit {
+    int n;                       // iterations of a tile
+    int whole, ctas;
+    int line;                    // iterations of the tiles that are cut
+    float* part;                 // [2 ctas] partial results; null: every tile is whole, one CTA per tile
+    __host__ __device__ int edge(int c) const { return (int)((unsigned)line * (unsigned)c / (unsigned)ctas); }   // line * ctas < 2^32
+};
+constexpr int PART_ROWS = 3;                                  // a partial result: m, l and the sum of the rounded P of every row,
+constexpr int PART_FLOATS = BM * (HD + PART_ROWS);            // then O as [d / 4][row][4]
+
 __device__ __forceinline__ float2 exp2_pair(float2 x) { return make_float2(ex2_approx(x.x), ex2_approx(x.y)); }
 
 // Order of a tile's iterations. The refine iterations (64 small TMA boxes per tile, slow to fill) are spread evenly among
@@ -139,10 +159,12 @@ struct SchedIter {
 
 // One (query tile, head): `tile` = head * nq + query tile. `again`: the CTA has run a tile before (its barriers exist).
 // Dense mode: `sample` takes the offset from a sample of the columns; true is returned when that did not do (dense_kernel).
+// The CTA runs iterations first .. last - 1 of the tile and leaves a partial result in `part`, or with null the outputs.
 template <int MODE>
-__device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmKm,
+__device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmKm,
                                                const CUtensorMap& tmVm, const CUtensorMap& tmKr, const CUtensorMap& tmVr,
-                                               const AttnArgs& a, const int tile, const bool again, const bool sample) {
+                                               const AttnArgs& a, const int tile, const bool again, const bool sample,
+                                               const int first = 0, const int last = 0, float* const part = nullptr) {
     constexpr bool COMPENSATE = MODE == 2;     // block-mean compensation of flagged tiles, added to out / lse in place
     constexpr bool DENSE = MODE == 3;          // online softmax over every block: no list, no flags
     constexpr bool FALLBACK = MODE == 1 || DENSE;    // the offset comes from a sweep; MODE 1: of flagged tiles, over their lists
@@ -154,19 +176,22 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
         if (a.flags[th_idx] == 0) return false;    // uniform over the CTA, before anything is allocated
     }
     // The tile's first global loads do not depend on one another: the list length, the first window of block ids (load
-    // warps) and this thread's half of its Q row (softmax warps) are requested here (in the fallback modes: once the tile
-    // is known to be flagged), before the status check, the barrier set-up and the tensor-memory allocation, whose
-    // latencies they then share instead of following them.
+    // warps) and this row's offset (softmax warps) are requested here (in the fallback modes: once the tile is known to be
+    // flagged), before the status check, the barrier set-up and the tensor-memory allocation, whose latencies they then
+    // share instead of following them.
     const int n64_early = COMPENSATE ? 0 : DENSE ? a.nb : __ldg(a.counts + th_idx);
     int win_early = 0;
-    uint4 q_early[8];
+    float m_early = 0.f;
     if (warp == LOADK_WARP || warp == LOADV_WARP) {
         if (!COMPENSATE && !DENSE && lane < a.nk) win_early = __ldg(a.blocks + (size_t)th_idx * a.nk + lane);
+        if (lane == 0) {
+            const bool is_v = warp == LOADV_WARP;
+            if (!COMPENSATE) tma_prefetch_desc(is_v ? &tmV : &tmK);
+            if (MODE == 0 || COMPENSATE) tma_prefetch_desc(is_v ? &tmVm : &tmKm);
+            if (MODE == 0) tma_prefetch_desc(is_v ? &tmVr : &tmKr);
+        }
     } else if (warp < NSOFT / 32) {
-        const int r0 = qb * BM + 32 * (warp & 3) + lane;
-        const uint4* src = reinterpret_cast<const uint4*>(a.q + ((size_t)(r0 < a.L ? r0 : 0) * a.H + h) * HD + 64 * (warp >> 2));
-#pragma unroll
-        for (int i = 0; i < 8; ++i) q_early[i] = r0 < a.L ? __ldg(src + i) : make_uint4(0, 0, 0, 0);
+        if (!FALLBACK) m_early = a.offset[((size_t)qb * BM + 32 * (warp & 3) + lane) * a.H + h];
     }
     // a wait has given up earlier (the status word is set until the host reads it): do not start more work
     if (*reinterpret_cast<volatile int*>(a.status) != 0) return false;
@@ -183,8 +208,9 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
         if (base & 1023u) atomicCAS(a.status, 0, 901);   // the swizzled tiles need a 1024-byte aligned base
         if (again) {
             // a CTA that walks a list of tiles makes its barriers anew for every tile
-            for (uint64_t* b = &ctl->qfull; b <= &ctl->sweepbar; ++b) mbar_inval(smem_u32(b));
+            for (uint64_t* b = &ctl->qload; b <= &ctl->sweepbar; ++b) mbar_inval(smem_u32(b));
         }
+        mbar_init(smem_u32(&ctl->qload), 1);
         mbar_init(smem_u32(&ctl->qfull), NSOFT);
         for (int i = 0; i < NSLOT; ++i) {
             mbar_init(smem_u32(&ctl->full[i]), 1);
@@ -219,10 +245,13 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
     const uint32_t tmem = ctl->tmem_base;
 
     const int n64 = n64_early;
-    const int n = (n64 + 1) >> 1;                     // exact iterations: pairs of 64-token blocks
+    const int n = DENSE ? last - first : (n64 + 1) >> 1;      // exact iterations: pairs of 64-token blocks
     // iterations of the fallback sweep: all, or for a sample one in 32 (1 to 8 of them) spread over the list
-    const int nsweep = DENSE && sample ? min(n, min(max(n >> 5, 1), 8)) : n;
-    const bool find_top = DENSE && sample && n > nsweep;
+    const int nsample = min(n, min(max(n >> 5, 1), 8));
+    // a sample of one iteration needs no sweep: it is a look at the logits of iteration 0, which stay for their own softmax
+    const bool first_is_sample = DENSE && sample && nsample == 1;
+    const int nsweep = first_is_sample ? 0 : DENSE && sample ? nsample : n;
+    const bool find_top = DENSE && sample && n > nsample;
     auto sweep_iter = [&](int i) { return DENSE && sample ? i * n / nsweep : i; };
     const int nvirt = FALLBACK ? 0 : a.nvirt;
     const int nref = (FALLBACK || COMPENSATE) ? 0 : a.nref;
@@ -242,7 +271,6 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
         const CUtensorMap* map_x = is_v ? &tmV : &tmK;       // exact blocks
         const CUtensorMap* map_m = is_v ? &tmVm : &tmKm;     // block means
         const CUtensorMap* map_r = is_v ? &tmVr : &tmKr;     // representative tables
-        if (lane == 0) { tma_prefetch_desc(map_x); tma_prefetch_desc(map_m); tma_prefetch_desc(map_r); }
         const int* rl = a.refine + (size_t)th_idx * a.rw;
         const uint32_t full0 = smem_u32(&ctl->full[0]), empty0 = smem_u32(&ctl->empty[0]);
         const uint32_t box_off = (uint32_t)(lane >> 1) * HALF_BYTES + (uint32_t)(lane & 1) * BLK_BYTES;   // lanes 0..3
@@ -258,7 +286,7 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
             if (i < 0) { kind = 0; idx = -i - 1; }        // a K tile of the fallback sweep
             else sched.decode(i, kind, idx);
             if (kind == 0) {
-                const int e = 2 * idx;
+                const int e = DENSE ? 2 * (first + idx) : 2 * idx;
                 if (DENSE) {
                     ra = e * BK;
                     rb = ra + BK;
@@ -277,7 +305,10 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
                 rb = ra + 64;
             }
             const uint32_t slot = seq % NSLOT, par = ((seq / NSLOT) & 1) ^ 1;
-            if (lane == 0) ok = mbar_wait(empty0 + 8 * slot, par, abort_flag, a.status, 101);
+            if (lane == 0) {
+                ok = mbar_wait(empty0 + 8 * slot, par, abort_flag, a.status, 101);
+                if (seq == Q_SLOT) ok = ok && mbar_wait(smem_u32(&ctl->qfull), 0, abort_flag, a.status, 103);
+            }
             ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;     // the other lanes sleep at the shuffle instead of polling
             if (!ok) return;
             const uint32_t dst = sRing + slot * TILE_BYTES, bar = full0 + 8 * slot;
@@ -305,29 +336,30 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
             }
             pseq = seq + 1;
         };
-        uint32_t base = 0;
-        if (FALLBACK) {
-            // The sweep's K tiles come first in the ring. A wait on a slot's `empty` barrier can only tell two consecutive
-            // rounds apart (one parity bit), so the V warp must not start polling while the ring is still rounds behind
-            // its first tile: it starts once the K warp has issued the last sweep tile.
-            if (!is_v) {
-                for (int i = 0; i < nsweep; ++i) put((uint32_t)i, -sweep_iter(i) - 1);
-                if (lane == 0) mbar_arrive(smem_u32(&ctl->sweepbar));
-            } else {
-                if (lane == 0) ok = mbar_wait(smem_u32(&ctl->sweepbar), 0, abort_flag, a.status, 102);
-                ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
-            }
-            base = (uint32_t)nsweep;
-            wbase = -1;
+        if (is_v) {
+            // Q through the ring's last slot. A thread's own row by plain loads is 32 lines to an instruction, 3,000 clocks a tile.
+            if (lane == 0) mbar_arrive_expect_tx(smem_u32(&ctl->qload), TILE_BYTES);
+            __syncwarp();
+            if (lane < 4) tma_load_3d(sRing + Q_SLOT * TILE_BYTES + box_off, &tmQ, smem_u32(&ctl->qload), box_x, qb * BM + (lane & 1) * BK, h);
         }
-        if (!is_v) {
-            // K(0), K(1), then K(i + 2) after every V(i)
-            if (nt > 0) put(base, 0);
-            if (nt > 1) put(base + 1, 1);
-            for (int i = 2; i < nt; ++i) put(base + 2 * i - 1, i);
-        } else {
-            // V(i) comes after the K tiles 0 .. min(i + 2, nt) - 1 and the V tiles before it
-            for (int i = 0; i < nt; ++i) put(base + (uint32_t)(min(i + 2, nt) + i), i);
+        // K: the sweep's tiles come first in the ring, then K(0), K(1) and K(i + 2) after every V(i). V(i) comes after the K tiles
+        // 0 .. min(i + 2, nt) - 1 and the V tiles before it. A wait on a slot's `empty` barrier can only tell two consecutive
+        // rounds apart (one parity bit), so the V warp must not start polling while the ring is still rounds behind its first
+        // tile: it starts once the K warp has issued the last sweep tile.
+        if (is_v && FALLBACK) {
+            if (lane == 0) ok = mbar_wait(smem_u32(&ctl->sweepbar), 0, abort_flag, a.status, 102);
+            ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+        }
+        const int sweeps = FALLBACK ? nsweep : 0, lead = is_v ? 0 : sweeps;
+#pragma unroll 1
+        for (int j = 0; j <= lead + nt; ++j) {
+            if (FALLBACK && !is_v && j == lead) {
+                if (lane == 0) mbar_arrive(smem_u32(&ctl->sweepbar));
+                wbase = -1;
+            }
+            if (j == lead + nt) break;
+            const int i = j - lead;
+            put((uint32_t)(i < 0 ? j : sweeps + (is_v ? min(i + 2, nt) + i : i < 2 ? i : 2 * i - 1)), i < 0 ? -sweep_iter(j) - 1 : i);
         }
     } else if (warp == MMA_WARP) {
         // ------------------------------------------------------------ MMAs: the warp runs uniformly, one elected lane issues
@@ -437,10 +469,12 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
         bool ok = true;
 
         // this thread's half of its Q row -> tensor memory (bf16 pairs, 32 columns), the A operand of every QK^T
+        ok = mbar_wait_warp(smem_u32(&ctl->qload), 0, abort_flag, a.status, 309);
         {
+            const uint8_t* src = smem_raw + SMEM_RING + Q_SLOT * TILE_BYTES + ch * HALF_BYTES + trow * 128;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                const uint4 w = q_early[i];
+                const uint4 w = *reinterpret_cast<const uint4*>(src + ((i ^ (trow & 7)) << 4));
                 s[4 * i] = w.x; s[4 * i + 1] = w.y; s[4 * i + 2] = w.z; s[4 * i + 3] = w.w;
             }
             tmem_st32(lane_base + Q_COL + 32 * ch, s);
@@ -448,27 +482,29 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
             tc_fence_before();
             mbar_arrive(smem_u32(&ctl->qfull));
         }
-        float m = DENSE ? 0.f : a.offset[(size_t)row * a.H + h];
+        float m = FALLBACK ? 0.f : m_early;
         float best = 0.f;                          // dense: the largest logit found so far (at first the sample's) and its key
         int best_key = -1;
         uint32_t uS[2] = {0, 0};
 
         if (FALLBACK) {
             float mx = -INFINITY;
-            for (int i = 0; i < nsweep && ok; ++i) {
-                const int buf = i & 1, e = 2 * sweep_iter(i) + ch;
+            for (int i = 0; i < (first_is_sample ? 1 : nsweep) && ok; ++i) {
+                const int buf = i & 1, e = 2 * (first + sweep_iter(i)) + ch;
                 const bool has = e < n64;
                 const int blk = DENSE ? e : list[has ? e : e - 1];
                 ok = ok && mbar_wait_warp(smem_u32(&ctl->sfull[buf]), uS[buf] & 1, abort_flag, a.status, 301);
                 if (!ok) break;
-                ++uS[buf];
+                if (!first_is_sample) ++uS[buf];
                 tc_fence_after();
                 tmem_ld32(lane_base + buf * 128 + 64 * ch, &s[0]);
                 tmem_ld32(lane_base + buf * 128 + 64 * ch + 32, &s[32]);
                 tmem_wait_ld_regs(&s[0]);
                 tmem_wait_ld_regs(&s[32]);
-                tc_fence_before();
-                mbar_arrive(smem_u32(&ctl->pfull[buf]));
+                if (!first_is_sample) {
+                    tc_fence_before();
+                    mbar_arrive(smem_u32(&ctl->pfull[buf]));
+                }
                 int lim = (blk == a.nb - 1) ? a.tail_valid : BK;
                 if (!has) lim = 0;
 #pragma unroll
@@ -479,9 +515,8 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
             ctl->m_part[ch][trow] = mx;
             mbar_arrive(smem_u32(&ctl->lbar));
             ok = mbar_wait_warp(smem_u32(&ctl->lbar), 0, abort_flag, a.status, 306) && ok;
-            mx = fmaxf(ctl->m_part[0][trow], ctl->m_part[1][trow]);
-            m = (mx == -INFINITY) ? 0.f : mx * a.scale_log2;
-            best = mx;
+            best = fmaxf(ctl->m_part[0][trow], ctl->m_part[1][trow]);
+            m = (best == -INFINITY) ? 0.f : best * a.scale_log2;
         }
 
         float2 lsum = make_float2(0.f, 0.f);
@@ -495,7 +530,7 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
         int kind = 0, idx = 0, blk = 0;
         auto block_of = [&](int kd, int ix) -> int {
             if (kd != 0) return 0;
-            const int e = 2 * ix + ch;
+            const int e = 2 * (first + ix) + ch;
             return DENSE ? e : __ldg(list + (e < n64 ? e : e - 1));
         };
         if (nt > 0) {
@@ -505,7 +540,7 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
         for (int i = 0; i < nt && ok; ++i) {
             const int buf = i & 1;
             const bool exact = kind == 0, pooled = kind == 1;
-            const bool has = !exact || 2 * idx + ch < n64;
+            const bool has = !exact || 2 * (first + idx) + ch < n64;
             const int cur_idx = idx, cur_blk = blk;
             int nkind = 0, nidx = 0, nblk = 0;
             walk.advance(sched);
@@ -626,16 +661,27 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
                 const float top = fmaxf(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])), fmaxf(fmaxf(mx[4], mx[5]), fmaxf(mx[6], mx[7])));
                 const bool better = top > best;
                 if (__any_sync(0xffffffffu, better)) {
-                    best = better ? top : best;
+                    // one that is no large part of what the row has by now needs no key, and the smaller one before it neither
+                    const bool large = better && ex2_approx(fmaf(top, a.scale_log2, -m)) * kTopShare >= lsum.x + lsum.y;
+                    int key = -1;
+                    if (__any_sync(0xffffffffu, large)) {
+                        // its column by halving: each level keeps the half of the candidates that holds the maximum
+                        const bool h5 = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) < top;
+                        const bool h4 = fmaxf(h5 ? mx[4] : mx[0], h5 ? mx[5] : mx[1]) < top;
+                        const float m0 = h5 ? mx[4] : mx[0], m2 = h5 ? mx[6] : mx[2];
+                        const bool h3 = (h4 ? m2 : m0) < top;
+                        uint32_t t[32];
 #pragma unroll
-                    for (int g = 0; g < 8; ++g) {
-                        const bool here = better && mx[g] == top;
-                        if (!__any_sync(0xffffffffu, here)) continue;
+                        for (int c = 0; c < 32; ++c) t[c] = h5 ? s[32 + c] : s[c];
+#pragma unroll
+                        for (int c = 0; c < 16; ++c) t[c] = h4 ? t[16 + c] : t[c];
                         int at = 0;
 #pragma unroll
-                        for (int c = 1; c < 8; ++c) at = __uint_as_float(s[8 * g + c]) == top ? c : at;
-                        best_key = here ? cur_blk * BK + 8 * g + at : best_key;
+                        for (int c = 0; c < 8; ++c) at = __uint_as_float(h3 ? t[8 + c] : t[c]) == top ? c : at;
+                        if (large) key = cur_blk * BK + 32 * h5 + 16 * h4 + 8 * h3 + at;
                     }
+                    best = better ? top : best;
+                    best_key = better ? key : best_key;
                 }
             }
             if (want_mass && exact) {
@@ -668,73 +714,106 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
         const float l = ctl->l_part[0][trow] + ctl->l_part[1][trow];
         // compensation: out = (out + sum e v) / (1 + sum e), lse += log2(1 + sum e) (triton_ops.py:280-282)
         const float lg = COMPENSATE ? log2f(1.0f + l) : log2f(l);
+        // dense: the V rows of the remembered keys, on their way while the last PV runs
+        int top_key[2];
+        float e_top[2];
+        uint4 vtop[2][8];
+#pragma unroll
+        for (int x = 0; x < (DENSE ? 2 : 0); ++x) {
+            e_top[x] = ctl->e_part[x][trow];
+            top_key[x] = fabsf(e_top[x]) > l * kTopLeast ? ctl->key_part[x][trow] : -1;
+            if (top_key[x] < 0) e_top[x] = 0.f;
+            const uint4* src = reinterpret_cast<const uint4*>(a.v + ((size_t)max(top_key[x], 0) * a.H + h) * HD + 64 * ch);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) vtop[x][c] = top_key[x] >= 0 ? __ldg(src + c) : make_uint4(0, 0, 0, 0);
+        }
         if (nt > 0) ok = mbar_wait_warp(smem_u32(&ctl->ofull), 0, abort_flag, a.status, 303) && ok;
         if (ok) {
             tc_fence_after();
-            int top_key[2];
-            float e_top[2];
-#pragma unroll
-            for (int x = 0; x < 2; ++x) {
-                top_key[x] = DENSE ? ctl->key_part[x][trow] : -1;
-                e_top[x] = DENSE ? ctl->e_part[x][trow] : 0.f;
-            }
-            const float inv = COMPENSATE ? 1.0f / (1.0f + l)
-                              : DENSE ? 1.0f / ((ctl->r_part[0][trow] + ctl->r_part[1][trow]) + (e_top[0] + e_top[1])) : 1.0f / l;
+            const float rounded = DENSE ? (ctl->r_part[0][trow] + ctl->r_part[1][trow]) + (e_top[0] + e_top[1]) : 0.f;
+            const float inv = COMPENSATE ? 1.0f / (1.0f + l) : DENSE ? 1.0f / rounded : 1.0f / l;
             bool finite = true;
-            __nv_bfloat16* orow = a.out + ((size_t)row * a.H + h) * HD + 64 * ch;
+            // The outputs are turned in shared memory, 32 rows of a column half per warp, in the ring (every K / V tile has been
+            // consumed): four whole lines to a store. A thread's own row at a time is 16 bytes of 32 lines, 4,000 clocks a tile; a
+            // TMA store keeps the CTA 1,000 clocks longer, until it has read its source.
+            uint8_t* stage = smem_raw + SMEM_RING + warp * (32 * 128);
+            auto chunk = [&](int r, int c) { return reinterpret_cast<uint4*>(stage + r * 128 + ((c ^ (r & 7)) << 4)); };
+            if (COMPENSATE) {
 #pragma unroll
-            for (int part = 0; part < 2; ++part) {
-                uint32_t* o = &s[0];
-                uint4 vtop[2][4];                  // dense: this part of V at the two keys
-#pragma unroll
-                for (int x = 0; x < (DENSE ? 2 : 0); ++x) {
-                    const uint4* src = reinterpret_cast<const uint4*>(a.v + ((size_t)max(top_key[x], 0) * a.H + h) * HD + 64 * ch + 32 * part);
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) vtop[x][c] = top_key[x] >= 0 ? __ldg(src + c) : make_uint4(0, 0, 0, 0);
+                for (int i = 0; i < 8; ++i) {              // the old outputs, four rows to a load
+                    const int r = 4 * i + (lane >> 3), grow = qb * BM + 32 * rq + r;
+                    if (grow < a.L) *chunk(r, lane & 7) = *reinterpret_cast<const uint4*>(a.out + ((size_t)grow * a.H + h) * HD + 64 * ch + 8 * (lane & 7));
                 }
+                __syncwarp();
+            }
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                uint32_t* o = &s[0];
                 if (nt > 0) {
-                    tmem_ld32(lane_base + O_COL + 64 * ch + 32 * part, o);
+                    tmem_ld32(lane_base + O_COL + 64 * ch + 32 * half, o);
                     tmem_wait_ld_regs(o);
                 }
-                if (valid) {
-                    if (DENSE) {
+                if (DENSE) {
 #pragma unroll
-                        for (int x = 0; x < 2; ++x)
+                    for (int x = 0; x < 2; ++x)
 #pragma unroll
-                            for (int c = 0; c < 16; ++c) {
-                                const uint4 w4 = vtop[x][c / 4];
-                                const uint32_t w = (c & 3) == 0 ? w4.x : (c & 3) == 1 ? w4.y : (c & 3) == 2 ? w4.z : w4.w;
-                                o[2 * c] = __float_as_uint(fmaf(e_top[x], __uint_as_float(w << 16), __uint_as_float(o[2 * c])));
-                                o[2 * c + 1] = __float_as_uint(fmaf(e_top[x], __uint_as_float(w & 0xFFFF0000u), __uint_as_float(o[2 * c + 1])));
-                            }
-#pragma unroll
-                        for (int c = 0; c < 32; ++c) finite = finite && fabsf(__uint_as_float(o[c])) <= 3.0e38f;
-                    }
-#pragma unroll
-                    for (int c = 0; c < 32; c += 8) {
-                        uint4 w;
-                        if (COMPENSATE) {
-                            const uint4 old = *reinterpret_cast<const uint4*>(orow + 32 * part + c);
-                            const uint32_t ow[4] = {old.x, old.y, old.z, old.w};
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                o[c + 2 * e] = __float_as_uint(__uint_as_float(o[c + 2 * e]) + __uint_as_float(ow[e] << 16));
-                                o[c + 2 * e + 1] = __float_as_uint(__uint_as_float(o[c + 2 * e + 1]) + __uint_as_float(ow[e] & 0xFFFF0000u));
-                            }
+                        for (int c = 0; c < 16; ++c) {
+                            const uint4 w4 = vtop[x][4 * half + c / 4];
+                            const uint32_t w = (c & 3) == 0 ? w4.x : (c & 3) == 1 ? w4.y : (c & 3) == 2 ? w4.z : w4.w;
+                            o[2 * c] = __float_as_uint(fmaf(e_top[x], __uint_as_float(w << 16), __uint_as_float(o[2 * c])));
+                            o[2 * c + 1] = __float_as_uint(fmaf(e_top[x], __uint_as_float(w & 0xFFFF0000u), __uint_as_float(o[2 * c + 1])));
                         }
-                        w.x = pack_bf16x2(__uint_as_float(o[c]) * inv, __uint_as_float(o[c + 1]) * inv);
-                        w.y = pack_bf16x2(__uint_as_float(o[c + 2]) * inv, __uint_as_float(o[c + 3]) * inv);
-                        w.z = pack_bf16x2(__uint_as_float(o[c + 4]) * inv, __uint_as_float(o[c + 5]) * inv);
-                        w.w = pack_bf16x2(__uint_as_float(o[c + 6]) * inv, __uint_as_float(o[c + 7]) * inv);
-                        if (nt == 0) w = make_uint4(0, 0, 0, 0);
-                        *reinterpret_cast<uint4*>(orow + 32 * part + c) = w;
+#pragma unroll
+                    for (int c = 0; c < 32; ++c) finite = finite && fabsf(__uint_as_float(o[c])) <= 3.0e38f;
+                }
+                if (DENSE && part != nullptr) {
+                    if (valid) {
+#pragma unroll
+                        for (int c = 0; c < 32; c += 4)
+                            *reinterpret_cast<uint4*>(part + PART_ROWS * BM + (16 * ch + 8 * half + c / 4) * (4 * BM) + 4 * trow) =
+                                make_uint4(o[c], o[c + 1], o[c + 2], o[c + 3]);
                     }
+                    continue;
+                }
+#pragma unroll
+                for (int c = 0; c < 32; c += 8) {
+                    uint4 w;
+                    uint4* dst = chunk(lane, 4 * half + c / 8);
+                    if (COMPENSATE) {
+                        const uint4 old = *dst;
+                        const uint32_t ow[4] = {old.x, old.y, old.z, old.w};
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            o[c + 2 * e] = __float_as_uint(__uint_as_float(o[c + 2 * e]) + __uint_as_float(ow[e] << 16));
+                            o[c + 2 * e + 1] = __float_as_uint(__uint_as_float(o[c + 2 * e + 1]) + __uint_as_float(ow[e] & 0xFFFF0000u));
+                        }
+                    }
+                    w.x = pack_bf16x2(__uint_as_float(o[c]) * inv, __uint_as_float(o[c + 1]) * inv);
+                    w.y = pack_bf16x2(__uint_as_float(o[c + 2]) * inv, __uint_as_float(o[c + 3]) * inv);
+                    w.z = pack_bf16x2(__uint_as_float(o[c + 4]) * inv, __uint_as_float(o[c + 5]) * inv);
+                    w.w = pack_bf16x2(__uint_as_float(o[c + 6]) * inv, __uint_as_float(o[c + 7]) * inv);
+                    if (nt == 0) w = make_uint4(0, 0, 0, 0);
+                    *dst = w;
+                }
+            }
+            if (!(DENSE && part != nullptr)) {
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int r = 4 * i + (lane >> 3), grow = qb * BM + 32 * rq + r;
+                    if (grow < a.L) *reinterpret_cast<uint4*>(a.out + ((size_t)grow * a.H + h) * HD + 64 * ch + 8 * (lane & 7)) = *chunk(r, lane & 7);
                 }
             }
             tc_fence_before();
             if (ch == 0) {
                 // rows past L keep the "no offset" value, as echosparse/kernels/sm120.py:96
-                a.lse[(size_t)row * a.H + h] = valid ? m + lg : 1e30f;
+                if (DENSE && part != nullptr) {
+                    part[trow] = m;
+                    part[BM + trow] = l;
+                    part[2 * BM + trow] = rounded;
+                } else {
+                    a.lse[(size_t)row * a.H + h] = valid ? m + lg : 1e30f;
+                }
             }
             if (DENSE && sample) {
                 // the maximum of the sample was no usable offset for some row: the tile is done again in two sweeps
@@ -759,6 +838,10 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
 
     // ---------------------------------------------------------------- teardown
     __syncwarp();
+    if (warp == LOADV_WARP && lane == 0 && *abort_flag) {            // Q may still be on its way
+        const uint64_t t_end = global_timer_ns() + 100000ull;
+        while (!mbar_try_wait(smem_u32(&ctl->qload), 0) && global_timer_ns() < t_end) {}
+    }
     if ((warp == LOADK_WARP || warp == LOADV_WARP) && lane == 0 && *abort_flag) {
         // a wait gave up somewhere: give the loads this warp issued a moment (100 us in all) to land before the CTA's
         // shared memory goes away; a tile that was never issued cannot hold the CTA back
@@ -780,11 +863,12 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmK, const CUt
 
 template <int MODE>
 __global__ void __launch_bounds__(NTHREADS, 1)
-attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
+attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                 const __grid_constant__ CUtensorMap tmV,
                  const __grid_constant__ CUtensorMap tmKm, const __grid_constant__ CUtensorMap tmVm,
                  const __grid_constant__ CUtensorMap tmKr, const __grid_constant__ CUtensorMap tmVr, const AttnArgs a) {
     if (MODE == 0 || a.tile_list == nullptr) {
-        attention_tile<MODE>(tmK, tmV, tmKm, tmVm, tmKr, tmVr, a, (int)blockIdx.x, false, false);
+        attention_tile<MODE>(tmQ, tmK, tmV, tmKm, tmVm, tmKr, tmVr, a, (int)blockIdx.x, false, false);
         return;
     }
     // fallback modes with a tile list: a grid of one CTA per SM walks the flagged tiles, instead of one CTA per tile of
@@ -792,7 +876,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     const int count = *a.tile_count;
     bool again = false;
     for (int e = blockIdx.x; e < count; e += gridDim.x) {
-        attention_tile<MODE>(tmK, tmV, tmKm, tmVm, tmKr, tmVr, a, a.tile_list[e], again, false);
+        attention_tile<MODE>(tmQ, tmK, tmV, tmKm, tmVm, tmKr, tmVr, a, a.tile_list[e], again, false);
         again = true;
         __syncthreads();
     }
@@ -812,13 +896,113 @@ attention_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
 // searched: 6.1 ms, but 1.95e-3 on the random rows).
 // (Flagged tiles, MODE 1, are those whose offset was far off, where a sample's maximum often is too: 0.81 ms of a Wan-14B step with
 // a sample first, 0.47 ms in two sweeps.)
+//
+// Few tiles, or a few more than the SMs, leave most SMs idle: 1,560 tokens of 12 heads are 156 tiles on 148 SMs, two waves of which
+// the second is nearly empty. So the last tiles are cut by iterations (plan_dense): each piece takes its own offset from its own
+// columns and leaves m, the row sums and O in fp32, and a second kernel adds the pieces of a tile in their order. One launch after
+// the other, us, whole tiles / cut: 1,560 tokens x 12 heads 44.5 / 36.1, x 1 head 23.0 / 14.1, 4,096 x 1 44.2 / 20.9, 6,000 x 4
+// 120 / 91, 8,000 x 12 485 / 422; 4,096 tokens x 8 heads (1.73 waves of 32 iterations) stay whole: 87.7 / 93.0.
 __global__ void __launch_bounds__(NTHREADS, 1)
-dense_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const AttnArgs a) {
-    bool again = false;
-    do {
+dense_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+             const __grid_constant__ CUtensorMap tmV, const AttnArgs a, const DenseSplit d) {
+    const int c = blockIdx.x, whole = d.part ? d.whole : (int)gridDim.x;
+    int x = 0, end = 0;                                   // this CTA's stretch of the cut tiles' iterations
+    if (d.part && c < d.ctas) { x = d.edge(c); end = d.edge(c + 1); }
+    int next = c, tile = 0, first = 0, last = d.n;
+    float* part = nullptr;
+    bool redo = false;
+    for (bool again = false;; again = true) {
+        if (!redo) {
+            if (next < whole) {
+                tile = next;
+                next += gridDim.x;
+            } else if (x < end) {
+                const int t = x / d.n;
+                tile = d.whole + t;
+                first = x - t * d.n;
+                last = min(d.n, end - t * d.n);
+                x = t * d.n + last;
+                // a piece that ends a tile goes to the CTA's first slot, one that only starts it to its second
+                part = last - first == d.n ? nullptr : d.part + (size_t)(2 * c + (first == 0)) * PART_FLOATS;
+            } else {
+                break;
+            }
+        }
         if (again) __syncthreads();
-        again = attention_tile<3>(tmK, tmV, tmK, tmV, tmK, tmV, a, (int)blockIdx.x, again, !again);
-    } while (again);
+        redo = attention_tile<3>(tmQ, tmK, tmV, tmK, tmV, tmK, tmV, a, tile, again, !redo, first, last, part);
+    }
+    launch_dependents();
+}
+
+// The pieces of a cut tile, added in their order: block (t, y) does MERGE_COLS columns of the t-th cut tile, one row per thread.
+constexpr int MERGE_COLS = 8;
+__global__ void __launch_bounds__(BM)
+dense_merge_kernel(const AttnArgs a, const DenseSplit d) {
+    constexpr int N4 = MERGE_COLS / 4, AT_ONCE = 4;
+    const int t = blockIdx.x, x0 = t * d.n, x1 = x0 + d.n, trow = threadIdx.x;
+    wait_prerequisites();
+    const int tile = d.whole + t, qb = tile % a.nq, h = tile / a.nq, row = qb * BM + trow;
+    int c = (int)((unsigned)x0 * (unsigned)d.ctas / (unsigned)d.line);        // the first CTA with a piece of the tile
+    while (c > 0 && d.edge(c) > x0) --c;
+    while (d.edge(c + 1) <= x0) ++c;
+    const int next = d.edge(c + 1);
+    if (next >= x1) return;                               // one CTA did the whole tile
+    // pieces c, c + 1, ..: the first is in its CTA's second slot if the CTA's stretch starts at or before the tile's first
+    // iteration, the others, which start inside the tile, are in the first
+    const float* p = d.part + (size_t)(2 * c + (d.edge(c) <= x0)) * PART_FLOATS;
+    float M = -INFINITY, l = 0.f, r = 0.f;
+    float4 o[N4];
+#pragma unroll
+    for (int i = 0; i < N4; ++i) o[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    bool more = true;
+    while (more) {
+        float mp[AT_ONCE], lp[AT_ONCE], rp[AT_ONCE];
+        float4 v[AT_ONCE][N4];
+#pragma unroll
+        for (int u = 0; u < AT_ONCE; ++u) {
+            mp[u] = lp[u] = rp[u] = 0.f;
+#pragma unroll
+            for (int i = 0; i < N4; ++i) v[u][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (more) {
+                mp[u] = p[trow]; lp[u] = p[BM + trow]; rp[u] = p[2 * BM + trow];
+                const float4* po = reinterpret_cast<const float4*>(p + PART_ROWS * BM) + (size_t)N4 * blockIdx.y * BM + trow;
+#pragma unroll
+                for (int i = 0; i < N4; ++i) v[u][i] = po[i * BM];
+                ++c;
+                p = d.part + (size_t)(2 * c) * PART_FLOATS;
+                more = c < d.ctas && d.edge(c) < x1;
+            }
+        }
+        float Mn = M;
+#pragma unroll
+        for (int u = 0; u < AT_ONCE; ++u)
+            if (lp[u] != 0.f) Mn = fmaxf(Mn, mp[u]);      // a piece whose logits are all -inf has no maximum
+        const float w0 = l != 0.f ? exp2f(M - Mn) : 0.f;
+        l *= w0; r *= w0;
+#pragma unroll
+        for (int i = 0; i < N4; ++i) o[i] = make_float4(o[i].x * w0, o[i].y * w0, o[i].z * w0, o[i].w * w0);
+#pragma unroll
+        for (int u = 0; u < AT_ONCE; ++u) {
+            const float w = lp[u] != 0.f ? exp2f(mp[u] - Mn) : 0.f;
+            l = fmaf(w, lp[u], l);
+            r = fmaf(w, rp[u], r);
+#pragma unroll
+            for (int i = 0; i < N4; ++i)
+                o[i] = make_float4(fmaf(w, v[u][i].x, o[i].x), fmaf(w, v[u][i].y, o[i].y), fmaf(w, v[u][i].z, o[i].z), fmaf(w, v[u][i].w, o[i].w));
+        }
+        M = Mn;
+    }
+    if (M == -INFINITY) M = 0.f;
+    const bool valid = row < a.L;
+    if (blockIdx.y == 0) a.lse[(size_t)row * a.H + h] = valid ? M + log2f(l) : 1e30f;
+    if (!valid) return;
+    const float inv = 1.0f / r;
+    uint4* dst = reinterpret_cast<uint4*>(a.out + ((size_t)row * a.H + h) * HD + MERGE_COLS * blockIdx.y);
+#pragma unroll
+    for (int i = 0; i < MERGE_COLS / 8; ++i)
+        dst[i] = make_uint4(pack_bf16x2(o[2 * i].x * inv, o[2 * i].y * inv), pack_bf16x2(o[2 * i].z * inv, o[2 * i].w * inv),
+                            pack_bf16x2(o[2 * i + 1].x * inv, o[2 * i + 1].y * inv),
+                            pack_bf16x2(o[2 * i + 1].z * inv, o[2 * i + 1].w * inv));
 }
 
 // Tiles whose flag is set, in ascending tile number (head * nq + tile): one CTA, ordered compaction by prefix sums. The
@@ -886,7 +1070,35 @@ static int make_map(CUtensorMap* m, const void* ptr, int rows, int H, int box_ro
 struct AttnCall {
     const void *q, *k, *v, *k_mean, *v_mean;
     AttnArgs a;
+    DenseSplit split;            // dense mode
+    int sms;
 };
+
+// Times in iterations of a dense tile (1.17 us at 12 heads of 1,560 tokens): what a piece costs besides its own, and a merging
+// launch where the cut tiles are fewer than a wave (3 us) and where they are one or two waves (7 us).
+constexpr int PIECE_COST = 5, MERGE_FEW = 3, MERGE_MANY = 7;
+
+// One wave of whole tiles after the other, or the tiles of the last wave cut into the same number of pieces each, or those of the
+// last two waves cut without regard to their ends, so that a CTA works on two or three tiles: whichever these counts say is shortest.
+static DenseSplit plan_dense(int tiles, int nb, int sms) {
+    DenseSplit d{};
+    d.n = (nb + 1) / 2;
+    const int waves = tiles / sms, rest = tiles % sms;
+    int best = (waves + (rest > 0)) * (d.n + PIECE_COST) * 19 / 20;       // cut only where that saves a twentieth
+    if (rest == 0 || 2ll * sms * sms * d.n >= 1ll << 32) return d;
+    const int pieces = std::min(sms / rest, d.n);
+    if (pieces > 1) {
+        const int t = waves * (d.n + PIECE_COST) + (d.n + pieces - 1) / pieces + PIECE_COST + MERGE_FEW;
+        if (t < best) {
+            best = t;
+            d.whole = waves * sms; d.line = rest * d.n; d.ctas = rest * pieces;
+        }
+    }
+    const int lead = std::max(waves - 1, 0), cut = tiles - lead * sms, ctas = std::min(sms, cut * d.n);
+    const int t = lead * (d.n + PIECE_COST) + (cut * d.n + ctas - 1) / ctas + 2 * PIECE_COST + MERGE_MANY;
+    if (t < best) { d.whole = lead * sms; d.line = cut * d.n; d.ctas = ctas; }
+    return d;
+}
 
 static int launch_attention(const AttnCall& c, int mode, cudaStream_t stream) {
     const AttnArgs& a = c.a;
@@ -894,8 +1106,9 @@ static int launch_attention(const AttnCall& c, int mode, cudaStream_t stream) {
     if (a.status == nullptr) return set_error(-2, "attention: the device status word is not available on this device");
     if (((uintptr_t)c.q | (uintptr_t)c.k | (uintptr_t)c.v | (uintptr_t)a.out) & 15)
         return set_error(-1, "attention: q, k, v, out must be 16-byte aligned");
-    CUtensorMap tk, tv, tkm, tvm, tkr, tvr;
+    CUtensorMap tq, tk, tv, tkm, tvm, tkr, tvr;
     int rc;
+    if ((rc = make_map(&tq, c.q, a.L, a.H, BK))) return rc;
     if ((rc = make_map(&tk, c.k, a.L, a.H, BK))) return rc;
     if ((rc = make_map(&tv, c.v, a.L, a.H, BK))) return rc;
     if (c.k_mean) {
@@ -913,10 +1126,17 @@ static int launch_attention(const AttnCall& c, int mode, cudaStream_t stream) {
     }
     if (mode == 3) {
         if ((rc = opt_in_shared_memory((const void*)dense_kernel, (int)SMEM_ALLOC))) return rc;
-        dense_kernel<<<a.nq * a.H, NTHREADS, SMEM_ALLOC, stream>>>(tk, tv, a);
-        const cudaError_t e3 = cudaGetLastError();
+        const DenseSplit& d = c.split;
+        dense_kernel<<<!d.part ? a.nq * a.H : d.whole ? c.sms : d.ctas, NTHREADS, SMEM_ALLOC, stream>>>(tq, tk, tv, a, d);
+        cudaError_t e3 = cudaGetLastError();
         if (e3 != cudaSuccess) return set_error(-2, cudaGetErrorString(e3));
         count_launch();
+        if (d.part) {
+            if ((rc = prefer_shared_memory((const void*)dense_merge_kernel))) return rc;
+            if ((e3 = launch_dependent(dense_merge_kernel, dim3(d.line / d.n, HD / MERGE_COLS), dim3(BM), 0, stream, a, d)) != cudaSuccess)
+                return set_error(-2, cudaGetErrorString(e3));
+            count_launch();
+        }
         return 0;
     }
     auto kern = mode == 0 ? attention_kernel<0> : mode == 1 ? attention_kernel<1> : attention_kernel<2>;
@@ -941,7 +1161,7 @@ static int launch_attention(const AttnCall& c, int mode, cudaStream_t stream) {
             return set_error(-2, "attention: cannot read the SM count");
         grid = sms < grid ? sms : grid;
     }
-    kern<<<grid, NTHREADS, SMEM_ALLOC, stream>>>(tk, tv, tkm, tvm, tkr, tvr, a);
+    kern<<<grid, NTHREADS, SMEM_ALLOC, stream>>>(tq, tk, tv, tkm, tvm, tkr, tvr, a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return set_error(-2, cudaGetErrorString(e));
     count_launch();
@@ -1041,13 +1261,45 @@ extern "C" int es_compensate_fallback(const void* q, const void* k_mean, const v
     return launch_attention(c, 2, (cudaStream_t)stream);
 }
 
-extern "C" int es_dense_attention(const void* q, const void* k, const void* v, void* out, float* lse, int32_t L, int32_t H,
-                                  void* stream) {
-    if (!q || !k || !v || !out || !lse) return set_error(-1, "es_dense_attention: null pointer");
+static int dense_sms(int* sms) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return set_error(-2, "es_dense_attention: cannot read the SM count");
+    return 0;
+}
+
+extern "C" long long es_dense_scratch_bytes(int32_t L, int32_t H) {
+    int sms = 0;
+    if (L <= 0 || H <= 0 || dense_sms(&sms)) return 0;
+    return 2ll * plan_dense((L + BM - 1) / BM * H, (L + BK - 1) / BK, sms).ctas * PART_FLOATS * (long long)sizeof(float);
+}
+
+static int dense_call(const char* who, const void* q, const void* k, const void* v, void* out, float* lse, void* scratch,
+                      long long scratch_bytes, int32_t L, int32_t H, void* stream) {
+    if (!q || !k || !v || !out || !lse) return set_error(-1, who);
+    if (!aligned(16, scratch)) return set_error(-1, "es_dense_attention_split: scratch must be 16-byte aligned");
     AttnCall c{};
     c.q = q; c.k = k; c.v = v;
     fill_common(c.a, L, H, 0.f);
     c.a.out = (__nv_bfloat16*)out; c.a.lse = lse; c.a.v = (const __nv_bfloat16*)v;
     fill_q(c);
+    c.split.n = (c.a.nb + 1) / 2;
+    if (scratch && L > 0 && H > 0) {
+        if (int rc = dense_sms(&c.sms)) return rc;
+        const DenseSplit d = plan_dense(c.a.nq * H, c.a.nb, c.sms);
+        if (2ll * d.ctas * PART_FLOATS * (long long)sizeof(float) > scratch_bytes)
+            return set_error(-1, "es_dense_attention_split: scratch is smaller than es_dense_scratch_bytes says");
+        if (d.ctas > 0) { c.split = d; c.split.part = static_cast<float*>(scratch); }
+    }
     return launch_attention(c, 3, (cudaStream_t)stream);
+}
+
+extern "C" int es_dense_attention(const void* q, const void* k, const void* v, void* out, float* lse, int32_t L, int32_t H,
+                                  void* stream) {
+    return dense_call("es_dense_attention: null pointer", q, k, v, out, lse, nullptr, 0, L, H, stream);
+}
+
+extern "C" int es_dense_attention_split(const void* q, const void* k, const void* v, void* out, float* lse, void* scratch,
+                                        int64_t scratch_bytes, int32_t L, int32_t H, void* stream) {
+    return dense_call("es_dense_attention_split: null pointer", q, k, v, out, lse, scratch, scratch_bytes, L, H, stream);
 }

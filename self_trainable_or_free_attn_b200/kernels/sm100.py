@@ -161,8 +161,12 @@ def dense_attention(q, k, v, out, lse):
     assert hd == D and k.shape == v.shape == out.shape == q.shape
     _cuda_bf16(q, k, v, out)
     assert lse.shape == (_cdiv(L, BM) * BM, H) and lse.dtype == torch.float32 and lse.is_cuda and lse.is_contiguous()
-    N.check(N.load().es_dense_attention(N.ptr(q), N.ptr(k), N.ptr(v), N.ptr(out), N.ptr(lse), L, H, N.stream_ptr()),
-            "dense_attention")
+    lib = N.load()
+    # partial results of tiles that several CTAs work on (0 bytes: every tile is one CTA's)
+    size = lib.es_dense_scratch_bytes(L, H)
+    scratch = torch.empty(size, device=q.device, dtype=torch.uint8) if size else None
+    N.check(lib.es_dense_attention_split(N.ptr(q), N.ptr(k), N.ptr(v), N.ptr(out), N.ptr(lse), N.ptr(scratch), size, L, H,
+                                         N.stream_ptr()), "dense_attention")
 
 
 @_timed
