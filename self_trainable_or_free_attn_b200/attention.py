@@ -378,10 +378,10 @@ class EchoSparseAttention:
             out = torch.empty_like(q[0])
             self.K.dense_attention(q[0].contiguous(), k[0].contiguous(), v[0].contiguous(), out, buf.dense_lse)
             return out[None]
-        with torch.cuda.device(q.device):
-            return self._step(q[0].contiguous(), k[0].contiguous(), v[0].contiguous(), step, branch, layer,
-                              NO_SINK if sink is None else sink)[None]
+        return self._step(q[0].contiguous(), k[0].contiguous(), v[0].contiguous(), step, branch, layer,
+                          NO_SINK if sink is None else sink)[None]
 
+    @_native.device_guard
     def _step(self, q, k, v, step, branch, layer, sink):
         L, H, D = q.shape
         K = self.K

@@ -546,12 +546,15 @@ class _Function(torch.autograd.Function):
         ctx.gate_act = gate_act
         ctx.split = split
         ctx.mark_non_differentiable(sel.q2k_ptr, sel.q2k_idx, sel.k2q_ptr, sel.k2q_idx)
+        ctx.set_materialize_grads(False)                 # no zero-filled gradients of the four lists
         return o, sel.q2k_ptr, sel.q2k_idx, sel.k2q_ptr, sel.k2q_idx
 
     @staticmethod
     @N.device_guard
     def backward(ctx, dout, *unused):
         q, k, v, gate, blk_cnt = ctx.saved_tensors
+        if dout is None:
+            return (None,) * 11
         if ctx.inter is None:
             raise RuntimeError("VSA backward frees its intermediates after the first backward; "
                                "re-run the forward instead of backward(retain_graph=True) twice")
@@ -635,11 +638,14 @@ class _FineFunction(torch.autograd.Function):
         ctx.split = split
         ctx.save_for_backward(q, k, v, blk_cnt, of, lse, sel.q2k_ptr, sel.q2k_idx, sel.k2q_ptr, sel.k2q_idx)
         ctx.mark_non_differentiable(lse)
+        ctx.set_materialize_grads(False)
         return of, lse
 
     @staticmethod
     @N.device_guard
     def backward(ctx, dout, dlse):
+        if dout is None:
+            return (None,) * 6
         q, k, v, blk_cnt, of, lse, qp, qi, kp, ki = ctx.saved_tensors
         B, H, L, D = q.shape
         dout = dout.contiguous()

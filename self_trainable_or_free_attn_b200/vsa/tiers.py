@@ -183,11 +183,14 @@ class _TierFineFunction(torch.autograd.Function):
         ctx.save_for_backward(q, k, v, blk_cnt, of, lse, *tab)
         ctx.sel, ctx.mid_reps, ctx.phases = sel, mid_reps, phases
         ctx.mark_non_differentiable(lse)
+        ctx.set_materialize_grads(False)
         return of, lse
 
     @staticmethod
     @N.device_guard
     def backward(ctx, dout, dlse):
+        if dout is None:
+            return (None,) * 7
         q, k, v, blk_cnt, of, lse, *tab = ctx.saved_tensors
         B, H, L, D = q.shape
         dout = dout.contiguous()
