@@ -13,7 +13,7 @@
 // M = 64 product, which uses half of the tensor pipe.)
 //
 //   warps 0-7  P and dS: warp w owns rows 32 (w % 4) .. + 31 and columns 32 (w / 4) .. + 31
-//   warp 8     issues the MMAs; warp 9 issues the TMA loads
+//   warp 8     issues the MMAs; warps 9 and 10 issue the TMA loads (X1 and X2; warp 9 alone where they share a ring)
 // Tensor memory: (S, dP) of even and of odd iterations (4 x 64 columns), G1^T, G2^T (2 x 64). S and dP of iteration i + 1 are
 // computed while the warps work on iteration i. X1 and X2 tiles (32 KB at D = 128) have a ring each, of three and two slots (five
 // and five at D = 64): the dQ passes free X2 as soon as dP has read it. Where the second products need both (dK / dV at D = 128),
@@ -22,7 +22,7 @@
 // What bounds it: the hand-overs. The MMAs take 1,024 (768) clocks per two blocks at D = 128 and their operands 1,500 (1,150) of
 // shared memory's, of 3,300 (2,400) measured: a tile's load, its products, P / dS and the second products follow one another
 // with too few slots to have more than one and a half iterations on their way. 32,768 tokens x 12 heads, 32 blocks per list:
-// dK / dV 1.19 ms, dQ 0.88 ms (mma.sync: 2.27 and 1.68 ms); at D = 64 0.86 and 0.71 ms (1.29 and 0.91 ms), where M = D = 64
+// dK / dV 1.14 ms, dQ 0.85 ms (mma.sync: 2.27 and 1.68 ms); at D = 64 0.86 and 0.71 ms (1.29 and 0.91 ms), where M = D = 64
 // gradient products take half of the tensor pipe.
 //
 // BWD_TIER_Q, BWD_REP: the three tiers of resolution, see the modes below. 512 blocks x 12 heads, 32 + 102 blocks in tiers A and B:
@@ -35,7 +35,6 @@ namespace vsa {
 namespace {
 constexpr int TB = 64;
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr int BW_THREADS = 320, BW_THREADS_TIER = 352;
 constexpr uint32_t Y_HALF = TB * 128, X_HALF = 128 * 128;                // 64 d of an owner / a walked tile
 constexpr int COUNT_RING = 16;                                           // units whose column counts are staged
 constexpr int REP_WORDS = 4096 / 32;                                     // the entry points take up to 4096 blocks
@@ -47,7 +46,8 @@ enum BwdMode { BWD_KV, BWD_Q, BWD_TIER_Q, BWD_REP };
 template <int D, int MODE> struct BwdCfg {
     static constexpr bool KV = MODE == BWD_KV || MODE == BWD_REP;
     static constexpr int DH = D / 64, N1 = D == 128 ? 3 : 5, N2 = D == 128 ? 2 : 5;   // slots of X1 and of X2
-    static constexpr bool SHARED = KV && D == 128;                       // one ring of N1 + N2 slots instead
+    static constexpr bool SHARED = KV && D == 128;                       // one ring of N1 + N2 slots instead, filled by one warp
+    static constexpr int THREADS = SHARED ? 320 : 352;
     static constexpr uint32_t Y_TILE = DH * Y_HALF, X_TILE = DH * X_HALF;   // [d half][rows][128 B]
     static constexpr uint32_t Y1 = 0, Y2 = Y_TILE, DS = 2 * Y_TILE, P = DS + DS_BYTES;
     static constexpr uint32_t RING = P + (KV ? DS_BYTES : 0u), CTL = RING + (N1 + N2) * X_TILE, COUNTS = CTL + 1024;
@@ -109,7 +109,7 @@ __device__ __forceinline__ void store4(float* dst, float4 v, int wide) {
 }  // namespace
 
 template <typename T, int D, int MODE>
-__global__ void __launch_bounds__(MODE == BWD_TIER_Q ? BW_THREADS_TIER : BW_THREADS, 1)
+__global__ void __launch_bounds__((BwdCfg<D, MODE>::THREADS), 1)
 attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant__ CUtensorMap tmX2,
                    const __grid_constant__ CUtensorMap tmY1, const __grid_constant__ CUtensorMap tmY2,
                    const __grid_constant__ CUtensorMap tmM1, const __grid_constant__ CUtensorMap tmM2,
@@ -149,7 +149,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
     const int cnt_o = REP ? min(TB, (rep_mid ? a.NB * a.tier.RM : a.NB) - rep_tile * TB) : tokens_of(ob);
     if (tid == 0) {
         const int earlier = *reinterpret_cast<volatile int*>(a.status);      // (on its way during the set-up)
-        mbar_init(smem_u32(&ctl->yfull), 1);
+        mbar_init(smem_u32(&ctl->yfull), 2);
         for (int i = 0; i < N1 + N2; ++i) {
             mbar_init(smem_u32(&ctl->full[i]), 1);
             mbar_init(smem_u32(&ctl->empty[i]), 1);
@@ -186,7 +186,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
         const uint32_t lo = left >= 32 ? 0xFFFFFFFFu : (1u << left) - 1u, hi = left >= 64 ? 0xFFFFFFFFu : left > 32 ? (1u << (left - 32)) - 1u : 0u;
         const uint32_t mid_mask = (rep_per >= 32 ? 0xFFFFFFFFu : (1u << rep_per) - 1u) & lo;
 #pragma unroll 2
-        for (int w = warp; w < a.tier.W; w += BW_THREADS / 32) {
+        for (int w = warp; w < a.tier.W; w += C::THREADS / 32) {
             const int i = 32 * w + lane;
             bool used = false;
             if (i < a.NB) {
@@ -228,23 +228,19 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
     auto slot_of = [&](int x, int i) { return C::SHARED ? (2 * i + x) % (N1 + N2) : x ? N1 + i % N2 : i % N1; };
     auto phase_of = [&](int x, int i) { return (uint32_t)(C::SHARED ? (2 * i + x) / (N1 + N2) : i / (x ? N2 : N1)) & 1u; };
 
-    if (warp == 9 || (TIER && warp == 10)) {
-        // ------------------------------------------------------------ loads: Y1, Y2, then X1(i), X2(i)
-        // With tiers X1 and X2 have a warp each: a gathered unit is up to 64 small boxes per tensor.
-        const int x_first = TIER && warp == 10 ? 1 : 0, x_last = TIER && warp == 9 ? 0 : 1;
+    if (warp == 9 || warp == 10) {
+        // ------------------------------------------------------------ loads: Y1, X1(i) by warp 9, Y2, X2(i) by warp 10 or, into one
+        // ring, all by warp 9. A tile's load is 600 clocks of a warp: with one warp for both dQ took 0.94 ms instead of 0.91; two
+        // warps into the one ring made dK / dV slower, 1.24 -> 1.285 ms.
+        const int x_first = warp - 9, x_last = C::SHARED ? 1 : x_first;
         bool ok = *abort_flag == 0;
         if (ok && nt > 0) {
-            if (lane == 0) {
-                tma_prefetch_desc(&tmX1);
-                tma_prefetch_desc(&tmX2);
-                if (warp == 9) mbar_arrive_expect_tx(smem_u32(&ctl->yfull), 2 * Y_TILE);
-                for (int d = 0; warp == 9 && d < DH; ++d) {
-                    const CUtensorMap* y1 = !REP ? &tmY1 : rep_mid ? &tmM1 : &tmT1;
-                    const CUtensorMap* y2 = !REP ? &tmY2 : rep_mid ? &tmM2 : &tmT2;
-                    const int yrow = REP ? rep_row0 : row0 + ob * TB;
-                    tma_load_2d(base + C::Y1 + d * Y_HALF, y1, smem_u32(&ctl->yfull), 64 * d, yrow);
-                    tma_load_2d(base + C::Y2 + d * Y_HALF, y2, smem_u32(&ctl->yfull), 64 * d, yrow);
-                }
+            for (int x = x_first; x <= x_last && lane == 0; ++x) {
+                const CUtensorMap* y = !REP ? (x ? &tmY2 : &tmY1) : rep_mid ? (x ? &tmM2 : &tmM1) : (x ? &tmT2 : &tmT1);
+                const int yrow = REP ? rep_row0 : row0 + ob * TB;
+                tma_prefetch_desc(x ? &tmX2 : &tmX1);
+                mbar_arrive_expect_tx(smem_u32(&ctl->yfull), Y_TILE);
+                for (int d = 0; d < DH; ++d) tma_load_2d(base + (x ? C::Y2 : C::Y1) + d * Y_HALF, y, smem_u32(&ctl->yfull), 64 * d, yrow);
             }
             int win = !REP && lane < nA ? block_at(lane) : 0;  // a window of 32 list entries
             BitWalk used(use_words, REP);
@@ -355,7 +351,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
             __syncwarp();
         };
         if (C::SHARED) {
-            // in the order of the ring (choosing as below is 2 to 6 % slower here)
+            // in the order of the ring (choosing as below is 8 % slower here)
             auto issue_both = [&](int i) {
                 for (int x = 0; x < 2; ++x) {
                     ok = ok && mbar_wait_warp(full0 + 8 * slot_of(x, i), phase_of(x, i), abort_flag, a.status, 504);
@@ -518,6 +514,18 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
             fence_proxy_async_smem();
             mbar_arrive(smem_u32(&ctl->pfull));
         }
+        // the per-block gradients to add, on their way during the last products (fetched where they are added they cost a tile 1,500 clocks: dK / dV 1.24 -> 1.19 ms)
+        float4 adds[KV ? 2 : 1];
+        const float inv = 1.f / (float)cnt_o;
+#pragma unroll
+        for (int x = 0; x < (KV ? 2 : 1); ++x) {
+            const float* add = x ? a.add1 : a.add0;
+            adds[x] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (add && slot_out < 0) {
+                const float* src = add + ((size_t)bh * a.add_nb + ob) * D + 4 * (lane % (D / 4));
+                adds[x] = make_float4(__ldg(src) * inv, __ldg(src + 1) * inv, __ldg(src + 2) * inv, __ldg(src + 3) * inv);
+            }
+        }
         if (nt > 0) ok = ok && mbar_wait_warp(smem_u32(&ctl->pvdone), (nt - 1) & 1, abort_flag, a.status, 508);
         // all products have finished and every load has been consumed: the ring holds the transposed gradients now,
         // [64 tokens][LD] floats each
@@ -554,18 +562,11 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
         }
         tc_fence_before();
         asm volatile("bar.sync 1, 256;" ::: "memory");
-        const float inv = 1.f / (float)cnt_o;
 #pragma unroll
         for (int x = 0; x < (KV ? 2 : 1); ++x) {
             const float mul = x ? 1.f : a.scale;
-            const float* add = x ? a.add1 : a.add0;
+            const float4 ad = adds[x];
             const int d = 4 * (lane % (D / 4));                  // D / 4 lanes share a token
-            float4 ad = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (add && slot_out < 0) {
-                const float* src = add + ((size_t)bh * a.add_nb + ob) * D + d;
-                ad = make_float4(__ldg(src), __ldg(src + 1), __ldg(src + 2), __ldg(src + 3));
-                ad.x *= inv; ad.y *= inv; ad.z *= inv; ad.w *= inv;
-            }
             float* part = x ? a.part1 : a.part0;
             float* f = x ? a.f1 : a.f0;
             T* e = static_cast<T*>(x ? a.d1 : a.d0);
@@ -637,7 +638,7 @@ static int launch_bwd(const void* x1, const void* x2, const void* y1, const void
         if (int rc = make_token_map<T>(&t[i], p[i], D, (long long)BH * a.L)) return rc;
     auto kern = attn_bwd_tc_kernel<T, D, MODE>;
     if (int rc = opt_in_shared_memory((const void*)kern, (int)BwdCfg<D, MODE>::BYTES)) return rc;
-    kern<<<grid, BW_THREADS, BwdCfg<D, MODE>::BYTES, st>>>(t[0], t[1], t[2], t[3], t[2], t[3], t[2], t[3], a);
+    kern<<<grid, BwdCfg<D, MODE>::THREADS, BwdCfg<D, MODE>::BYTES, st>>>(t[0], t[1], t[2], t[3], t[2], t[3], t[2], t[3], a);
     ES_CHECK_LAUNCH("attn_bwd_tc_kernel");
     return 0;
 }
@@ -686,7 +687,7 @@ static int launch_tier_bwd(const void* x1, const void* x2, const void* y1, const
     }
     auto kern = attn_bwd_tc_kernel<T, D, MODE>;
     if (int rc = opt_in_shared_memory((const void*)kern, (int)BwdCfg<D, MODE>::BYTES)) return rc;
-    kern<<<dim3(grid_x, BH), MODE == BWD_TIER_Q ? BW_THREADS_TIER : BW_THREADS, BwdCfg<D, MODE>::BYTES, st>>>(t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], a);
+    kern<<<dim3(grid_x, BH), BwdCfg<D, MODE>::THREADS, BwdCfg<D, MODE>::BYTES, st>>>(t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], a);
     ES_CHECK_LAUNCH("attn_bwd_tc_kernel");
     return 0;
 }
