@@ -80,6 +80,10 @@ struct Ctl {
 };
 static_assert(sizeof(Ctl) <= 5632, "control block");
 
+// Fallback modes: tiles whose flags a CTA looks at in one go, and the most of them that are its own.
+constexpr int WALK_TILES = 64 * NTHREADS, WALK_MINE = 256;
+static_assert(WALK_TILES / 8 + (WALK_MINE + 32) * 4 <= NMASS * 2 * BM * 4, "the walk's lists take the block masses' room");
+
 struct AttnArgs {
     const __nv_bfloat16* q;      // (L, H, 128)
     const __nv_bfloat16* v;      // (L, H, 128), dense mode only (elsewhere V comes through its tensor map alone)
@@ -105,8 +109,7 @@ struct AttnArgs {
     int tail_valid;              // tokens of the last block
     float tail_log2;             // log2(tail_valid)
     int nvirt, nref;             // mean iterations (128 blocks each), refine iterations (32 list entries each)
-    const int* tile_list;        // fallback modes: tiles to process (head * nq + tile), ascending, or null: every CTA tests its flag
-    const int* tile_count;       // entries of tile_list
+    int walk;                    // fallback modes: CTAs find the flagged tiles and share them; 0: one CTA per tile tests its flag
     int* status;
 };
 
@@ -237,7 +240,7 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
     if (warp == MMA_WARP) {
         tmem_alloc(smem_u32(&ctl->tmem_base), TMEM_COLS);
         // a CTA that may allocate again (for its next tile, or for the same one in two sweeps) keeps its permit
-        if ((MODE == 0 || (MODE != 3 && a.tile_list == nullptr)) && !again) tmem_relinquish();
+        if ((MODE == 0 || (MODE != 3 && !a.walk)) && !again) tmem_relinquish();
         tc_fence_before();
     }
     __syncthreads();
@@ -867,18 +870,67 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                  const __grid_constant__ CUtensorMap tmV,
                  const __grid_constant__ CUtensorMap tmKm, const __grid_constant__ CUtensorMap tmVm,
                  const __grid_constant__ CUtensorMap tmKr, const __grid_constant__ CUtensorMap tmVr, const AttnArgs a) {
-    if (MODE == 0 || a.tile_list == nullptr) {
+    if (MODE == 0 || !a.walk) {
         attention_tile<MODE>(tmQ, tmK, tmV, tmKm, tmVm, tmKr, tmVr, a, (int)blockIdx.x, false, false);
         return;
     }
-    // fallback modes with a tile list: a grid of one CTA per SM walks the flagged tiles, instead of one CTA per tile of
-    // which all but a fraction of a percent would find their flag clear and leave
-    const int count = *a.tile_count;
+    // Fallback modes, one CTA per SM: every CTA finds the flagged tiles (a fraction of a percent of all, as a rule) and takes every
+    // gridDim-th, counted in the order of the tile numbers so that the CTAs at work share a head's K and V in L2. All read all
+    // flags, 94 KB at 591 tiles x 40 heads, in coalesced loads, into a bit per tile in tile order: 2 us. A kernel of its own that made
+    // the list took 25 us there, 0.10 ms of a Wan-14B step, and 2.3 us and a launch at 4,152 tokens x 2 heads.
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint32_t* bits = reinterpret_cast<uint32_t*>(smem_raw + SMEM_MASS);       // the block masses' room: these modes have none
+    int* mine = reinterpret_cast<int*>(bits + WALK_TILES / 32);
+    int* warp_sum = mine + WALK_MINE;
+    constexpr int PER = WALK_TILES / 32 / NTHREADS;                          // words of a thread
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, total = a.nq * a.H;
+    const int step = min(WALK_TILES, (WALK_MINE - 1) * (int)gridDim.x);
+    int found = 0;                                                           // flagged tiles before this range
     bool again = false;
-    for (int e = blockIdx.x; e < count; e += gridDim.x) {
-        attention_tile<MODE>(tmQ, tmK, tmV, tmKm, tmVm, tmKr, tmVr, a, a.tile_list[e], again, false);
-        again = true;
+    for (int e0 = 0; e0 < total; e0 += step) {
+        for (int w = tid; w < WALK_TILES / 32; w += NTHREADS) bits[w] = 0;
         __syncthreads();
+#pragma unroll 8
+        for (int f = tid; f < total; f += NTHREADS) {
+            const int e = (f % a.H) * a.nq + f / a.H - e0;                   // flags are (tile, head), tile numbers head * nq + tile
+            if (__ldg(a.flags + f) != 0 && e >= 0 && e < step) atomicOr(bits + (e >> 5), 1u << (e & 31));
+        }
+        __syncthreads();
+        uint32_t w[PER];
+        int n = 0;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            w[i] = bits[tid * PER + i];
+            n += __popc(w[i]);
+        }
+        int incl = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        if (lane == 31) warp_sum[warp] = incl;
+        __syncthreads();
+        int rank = found + incl - n, count = 0;
+        for (int i = 0; i < NTHREADS / 32; ++i) {
+            if (i < warp) rank += warp_sum[i];
+            count += warp_sum[i];
+        }
+        // ranks blockIdx, blockIdx + grid, .. are this CTA's; the first of the range goes to mine[0]
+        const int grid = gridDim.x, lead = ((int)blockIdx.x - found % grid + grid) % grid;
+#pragma unroll
+        for (int i = 0; i < PER; ++i)
+            for (uint32_t m = w[i]; m != 0; m &= m - 1, ++rank) {
+                const int at = rank - found - lead;
+                if (at >= 0 && at % grid == 0) mine[at / grid] = e0 + 32 * (tid * PER + i) + __ffs(m) - 1;
+            }
+        __syncthreads();
+        for (int t = 0; lead + t * grid < count; ++t) {
+            attention_tile<MODE>(tmQ, tmK, tmV, tmKm, tmVm, tmKr, tmVr, a, mine[t], again, false);
+            again = true;
+            __syncthreads();
+        }
+        found += count;
     }
 }
 
@@ -1005,47 +1057,6 @@ dense_merge_kernel(const AttnArgs a, const DenseSplit d) {
                             pack_bf16x2(o[2 * i + 1].z * inv, o[2 * i + 1].w * inv));
 }
 
-// Tiles whose flag is set, in ascending tile number (head * nq + tile): one CTA, ordered compaction by prefix sums. The
-// flags are stored tile-major (nq, H); they are copied to shared memory with coalesced loads first (STAGED; 94 KB at 591
-// tiles x 40 heads) and walked head-major from there.
-template <bool STAGED>
-__global__ void __launch_bounds__(1024)
-flag_list_kernel(const int* __restrict__ flags, int nq, int H, int* __restrict__ list, int* __restrict__ count) {
-    extern __shared__ int staged[];
-    __shared__ int warp_sum[32];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n = nq * H, per = (n + 1023) / 1024, b0 = tid * per;
-    if (STAGED) {
-        for (int i = tid; i < n; i += 1024) staged[i] = flags[i];
-        __syncthreads();
-    }
-    const int* f = STAGED ? staged : flags;
-    int mine = 0;
-    for (int b = b0; b < min(b0 + per, n); ++b) mine += f[(b % nq) * H + b / nq] != 0;
-    int incl = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-    }
-    if (lane == 31) warp_sum[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        int w = warp_sum[lane];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += v;
-        }
-        warp_sum[lane] = w;
-    }
-    __syncthreads();
-    int pos = incl - mine + (warp > 0 ? warp_sum[warp - 1] : 0);
-    for (int b = b0; b < min(b0 + per, n); ++b)
-        if (f[(b % nq) * H + b / nq] != 0) list[pos++] = b;
-    if (tid == 1023) *count = pos;
-}
-
 // ---------------------------------------------------------------------------------------------- host side
 // Representative tables (H, rows, 128) bf16 viewed as dims {128 d, rows, H}; a box is 64 d x 4 rows (one block's four rows).
 static int make_rep_map(CUtensorMap* m, const void* ptr, int rows, int H) {
@@ -1142,20 +1153,7 @@ static int launch_attention(const AttnCall& c, int mode, cudaStream_t stream) {
     auto kern = mode == 0 ? attention_kernel<0> : mode == 1 ? attention_kernel<1> : attention_kernel<2>;
     if ((rc = opt_in_shared_memory((const void*)kern, (int)SMEM_ALLOC))) return rc;
     int grid = a.nq * a.H;
-    if (mode != 0 && a.tile_list != nullptr) {
-        // the flagged tiles as a list, then one CTA per SM walking it
-        const int flag_bytes = a.nq * a.H * (int)sizeof(int);
-        if (flag_bytes <= 200 * 1024) {
-            if ((rc = opt_in_shared_memory((const void*)flag_list_kernel<true>, flag_bytes))) return rc;
-            flag_list_kernel<true><<<1, 1024, flag_bytes, stream>>>(a.flags, a.nq, a.H, const_cast<int*>(a.tile_list),
-                                                                     const_cast<int*>(a.tile_count));
-        } else {
-            flag_list_kernel<false><<<1, 1024, 0, stream>>>(a.flags, a.nq, a.H, const_cast<int*>(a.tile_list),
-                                                             const_cast<int*>(a.tile_count));
-        }
-        cudaError_t e0 = cudaGetLastError();
-        if (e0 != cudaSuccess) return set_error(-2, cudaGetErrorString(e0));
-        count_launch();
+    if (mode != 0 && a.walk) {
         int dev = 0, sms = 0;
         if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
             return set_error(-2, "attention: cannot read the SM count");
@@ -1238,7 +1236,7 @@ extern "C" int es_exact_fallback(const void* q, const void* k, const void* v, vo
     c.a.out = (__nv_bfloat16*)out; c.a.counts = counts; c.a.blocks = blocks; c.a.nk = nk;
     c.a.offset = lse; c.a.lse = lse; c.a.flags = const_cast<int32_t*>(flags); c.a.mass = nullptr;
     c.a.nvirt = 0; c.a.nref = 0;
-    if (tile_scratch) { c.a.tile_count = tile_scratch; c.a.tile_list = tile_scratch + 1; }
+    c.a.walk = tile_scratch != nullptr;
     fill_q(c);
     return launch_attention(c, 1, (cudaStream_t)stream);
 }
@@ -1256,7 +1254,7 @@ extern "C" int es_compensate_fallback(const void* q, const void* k_mean, const v
     c.a.offset = lse; c.a.lse = lse; c.a.flags = const_cast<int32_t*>(flags); c.a.mass = nullptr;
     c.a.keep = keep;
     c.a.nvirt = (c.a.nb + 127) / 128; c.a.nref = 0;
-    if (tile_scratch) { c.a.tile_count = tile_scratch; c.a.tile_list = tile_scratch + 1; }
+    c.a.walk = tile_scratch != nullptr;
     fill_q(c);
     return launch_attention(c, 2, (cudaStream_t)stream);
 }

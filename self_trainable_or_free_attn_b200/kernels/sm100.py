@@ -137,8 +137,8 @@ _SCRATCH_SIZES = 8
 
 
 def _tile_list_scratch(flags, stream):
-    """Device scratch for the list of flagged tiles (one int32 per tile and one for the count). The list and the kernel that walks
-    it are two launches, so a call on another stream or from another thread has scratch of its own. A thread keeps the last few
+    """Device scratch that the C ABI asks for where flagged tiles are walked (one int32 per tile and one more; the kernels find the
+    tiles by themselves now and leave it alone). A call on another stream or from another thread has scratch of its own. A thread keeps the last few
     (0.6 us of the host a call, a tensor per call 1.5 and its release: a step of 4,152 tokens 162 -> 170 us with the latter); what it
     drops, the allocator gives out again in the order of the stream it was used on. A graph outlives that order: a captured call
     takes its scratch from the graph's pool, and the graph keeps it."""
