@@ -149,6 +149,33 @@ gram_reduce_kernel(float* __restrict__ parts, int nsplit, float norm) {
     *reinterpret_cast<float4*>(src) = r;              // the slot of split 0: only this thread reads or writes these elements
 }
 
+// ------------------------------------------------------------------------------------------------ probes
+// Probe i of a head = scale * mean of the query rows of 64-row block floor(i (nb - 1) / 63 + 0.5) (representatives.py:36-46): 64
+// threads, two dimensions each, PROBES_PER_CTA of them in a CTA. The probes need only q, so they are more CTAs of the launch that
+// makes the metric, beside its one chain per head. As a kernel of their own (a dimension per thread, a few loads on their way)
+// they took 57 us a branch at Wan-14B, 20 us at Wan-1.3B, 6.7 us and a launch at 4,152 tokens.
+constexpr int PROBES_PER_CTA = 4;
+__device__ __forceinline__ void probe_block(const __nv_bfloat16* __restrict__ q, __nv_bfloat16* __restrict__ probes, int cta, int L,
+                                            int H, int nb, float scale) {
+    const int at = cta * PROBES_PER_CTA + (threadIdx.x >> 6), d = 2 * (threadIdx.x & 63), i = at % NP, h = at / NP;
+    const int blk = (int)((float)(i * (nb - 1)) / (float)(NP - 1) + 0.5f), n = min(64, L - blk * 64);
+    const __nv_bfloat16* src = q + ((size_t)blk * 64 * H + h) * HD + d;
+    float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+    for (int r0 = 0; r0 < 64; r0 += 32) {
+        uint32_t w[32];
+#pragma unroll
+        for (int r = 0; r < 32; ++r) w[r] = r0 + r < n ? __ldg(reinterpret_cast<const uint32_t*>(src + (size_t)(r0 + r) * H * HD)) : 0u;
+#pragma unroll
+        for (int r = 0; r < 32; ++r)
+            if (r0 + r < n) { s0 += bf_lo(w[r]); s1 += bf_hi(w[r]); }
+    }
+    const float c = fmaxf((float)n, 1.0f);
+    probes[(size_t)at * HD + d] = __float2bfloat16_rn(s0 * scale / c);
+    probes[(size_t)at * HD + d + 1] = __float2bfloat16_rn(s1 * scale / c);
+}
+
+// ------------------------------------------------------------------------------------------------ metric
 // G (from gram_reduce_kernel) regularised, then its Cholesky factor with clamped pivots (representatives.py:49-63,
 // 163-165), one CTA per head, the matrix in shared memory, blocked by panels of 16 columns. What bounds it is one chain of
 // 128 square roots, divisions and broadcasts; everything else is kept off that chain:
@@ -162,7 +189,11 @@ constexpr int CH_PANEL = 16, CH_LD = 132;
 constexpr int METRIC_SMEM = (HD + CH_PANEL) * CH_LD * (int)sizeof(float);
 __global__ void __launch_bounds__(256)
 metric_kernel(const float* __restrict__ parts, __nv_bfloat16* __restrict__ metric, float* __restrict__ gram_out,
-              int nsplit) {
+              int nsplit, const __nv_bfloat16* __restrict__ q, __nv_bfloat16* __restrict__ probes, int L, int H, float scale) {
+    if ((int)blockIdx.x >= H) {
+        probe_block(q, probes, (int)blockIdx.x - H, L, H, (L + 63) / 64, scale);
+        return;
+    }
     extern __shared__ __align__(16) float sm[];
     float* A = sm;                    // [128][CH_LD]
     float* P = A + HD * CH_LD;        // [16][CH_LD]: the panel, transposed
@@ -266,21 +297,6 @@ metric_kernel(const float* __restrict__ parts, __nv_bfloat16* __restrict__ metri
         }
         __syncthreads();
     }
-}
-
-// ------------------------------------------------------------------------------------------------ probes
-// Probe i of a head = scale * mean of the query rows of 64-row block floor(i (nb - 1) / 63 + 0.5) (representatives.py:36-46).
-__global__ void __launch_bounds__(HD)
-probe_kernel(const __nv_bfloat16* __restrict__ q, __nv_bfloat16* __restrict__ probes, int L, int H, int nb, float scale) {
-    const int i = blockIdx.x, h = blockIdx.y, d = threadIdx.x;
-    const int blk = (int)((float)(i * (nb - 1)) / (float)(NP - 1) + 0.5f);
-    float s = 0.f;
-    int n = 0;
-    for (int r = 0; r < 64; ++r) {
-        const int row = blk * 64 + r;
-        if (row < L) { s += __bfloat162float(q[((size_t)row * H + h) * HD + d]); ++n; }
-    }
-    probes[((size_t)h * NP + i) * HD + d] = __float2bfloat16_rn(s * scale / fmaxf((float)n, 1.0f));
 }
 
 // ------------------------------------------------------------------------------------------------ k-means
@@ -703,7 +719,6 @@ extern "C" int es_reps_metric(const void* q, float* gram_parts, float* gram, voi
     if (!q || !gram_parts || !metric || !probes) return set_error(-1, "es_reps_metric: null pointer");
     if (L <= 0 || H <= 0) return set_error(-1, "es_reps_metric: L and H must be positive");
     if (!aligned(16, q, gram_parts, metric)) return set_error(-1, "es_reps_metric: q, gram_parts and metric must be 16-byte aligned");
-    const int nb = (L + 63) / 64;
     const int rps = gram_rows_per_split(L), nsplit = (L + rps - 1) / rps;
     cudaStream_t st = (cudaStream_t)stream;
     gram_kernel<<<dim3(H, nsplit), 256, 0, st>>>((const __nv_bfloat16*)q, gram_parts, L, H, rps, nsplit);
@@ -713,10 +728,9 @@ extern "C" int es_reps_metric(const void* q, float* gram_parts, float* gram, voi
     const float scale = 1.0f / sqrtf((float)HD);
     gram_reduce_kernel<<<dim3(H, HD * HD / 1024), 256, 0, st>>>(gram_parts, nsplit, scale * scale / (float)L);
     ES_CHECK_LAUNCH("gram_reduce");
-    metric_kernel<<<H, 256, smem, st>>>(gram_parts, (__nv_bfloat16*)metric, gram, nsplit);
+    metric_kernel<<<H + NP / PROBES_PER_CTA * H, 256, smem, st>>>(gram_parts, (__nv_bfloat16*)metric, gram, nsplit, (const __nv_bfloat16*)q,
+                                                                  (__nv_bfloat16*)probes, L, H, scale);
     ES_CHECK_LAUNCH("metric");
-    probe_kernel<<<dim3(NP, H), HD, 0, st>>>((const __nv_bfloat16*)q, (__nv_bfloat16*)probes, L, H, nb, scale);
-    ES_CHECK_LAUNCH("probes");
     return 0;
 }
 
@@ -782,7 +796,6 @@ extern "C" int es_reps_metric_static(const void* q, float* gram, void* metric, v
     if (nsplit > usual) nsplit = usual;
     const int rps = (((L + nsplit - 1) / nsplit + 63) / 64) * 64;
     nsplit = (L + rps - 1) / rps;
-    const int nb = (L + 63) / 64;
     cudaStream_t st = (cudaStream_t)stream;
     gram_kernel<<<dim3(H, nsplit), 256, 0, st>>>((const __nv_bfloat16*)q, parts, L, H, rps, nsplit);
     ES_CHECK_LAUNCH("gram");
@@ -791,9 +804,8 @@ extern "C" int es_reps_metric_static(const void* q, float* gram, void* metric, v
     const float scale = 1.0f / sqrtf((float)HD);
     gram_reduce_kernel<<<dim3(H, HD * HD / 1024), 256, 0, st>>>(parts, nsplit, scale * scale / (float)L);
     ES_CHECK_LAUNCH("gram_reduce");
-    metric_kernel<<<H, 256, smem, st>>>(parts, (__nv_bfloat16*)metric, gram, nsplit);
+    metric_kernel<<<H + NP / PROBES_PER_CTA * H, 256, smem, st>>>(parts, (__nv_bfloat16*)metric, gram, nsplit, (const __nv_bfloat16*)q,
+                                                                  (__nv_bfloat16*)probes, L, H, scale);
     ES_CHECK_LAUNCH("metric");
-    probe_kernel<<<dim3(NP, H), HD, 0, st>>>((const __nv_bfloat16*)q, (__nv_bfloat16*)probes, L, H, nb, scale);
-    ES_CHECK_LAUNCH("probes");
     return 0;
 }
