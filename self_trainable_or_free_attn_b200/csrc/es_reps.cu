@@ -8,6 +8,7 @@
 //
 // The Gram matrix is accumulated as per-split partial sums that the Cholesky kernel adds in a fixed order, so the
 // metric is reproducible bit for bit (the reference adds with atomics).
+#include "es_ptx.cuh"
 #include "es_api_internal.h"
 
 #include <cuda_bf16.h>
@@ -45,77 +46,110 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// parts[h][split] = sum over the split's rows of q_r q_r^T (bf16 products, float32 sums). The rows stream through two
-// 64-row shared-memory tiles (cp.async); both MMA operands are transposed views of the same tile (ldmatrix.trans): warp
-// (wm, wn) owns the 32 x 64 patch at (32 wm, 64 wn) of the 128 x 128 result.
-constexpr int GS = 136;           // bf16 row stride of a row tile: 272 B, conflict-free for ldmatrix
-__global__ void __launch_bounds__(256)
-gram_kernel(const __nv_bfloat16* __restrict__ q, float* __restrict__ parts, int L, int H, int rows_per_split,
-            int nsplit) {
-    __shared__ __align__(16) __nv_bfloat16 tile[2][64 * GS];
+// parts[h][split] = sum over the split's rows of q_r q_r^T (bf16 products, float32 sums in tensor memory). A 64-row tile of Q
+// ([d half][64 rows][128 B], by TMA, rows past L zero) is both operands of a tcgen05.mma, MN-major: A = Q^T, B = Q. The tensor pipe
+// needs 256 clocks a tile of 16 KB, less than HBM takes to bring it, so the ring is there to keep loads on their way: six tiles,
+// two CTAs per SM: 0.132 ms for 75,600 tokens x 40 heads, 5.9 TB/s (mma.sync from two cp.async tiles: 0.364 ms), and the same error
+// against fp64 (3.4e-6, the float32 sums over a split).
+//   warps 0-3  the result: row m of the accumulator is stored as column m (the matrix is symmetric), a whole line per store
+//   warp 4     MMAs; warp 5 loads
+constexpr int GRAM_SLOTS = 6;
+constexpr uint32_t GRAM_HALF = 64 * 128, GRAM_TILE = 2 * GRAM_HALF, GRAM_CTL = GRAM_SLOTS * GRAM_TILE, GRAM_SMEM = GRAM_CTL + 256;
+struct GramCtl {
+    uint64_t full[GRAM_SLOTS], empty[GRAM_SLOTS], done;
+    uint32_t tmem_base;
+    int abort;
+};
+static_assert(sizeof(GramCtl) <= 256, "control block");
+
+__global__ void __launch_bounds__(192, 2)
+gram_kernel(const __grid_constant__ CUtensorMap tmQ, float* __restrict__ parts, int L, int rows_per_split, int nsplit, int* status) {
+    extern __shared__ __align__(1024) uint8_t gram_smem[];
     const int h = blockIdx.x, sp = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int wm = warp >> 1, wn = warp & 1, g = lane >> 2, tg = lane & 3;
-    float acc[2][8][4];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-#pragma unroll
-            for (int x = 0; x < 4; ++x) acc[i][j][x] = 0.f;
-    const int r_begin = sp * rows_per_split, r_end = min(L, r_begin + rows_per_split);
-    const int nchunk = (r_end - r_begin + 63) / 64;
-    auto load = [&](int c, int buf) {
-        // 64 rows x 256 B: thread -> row tid / 4 (+ 0), four 16-byte pieces
-#pragma unroll
-        for (int x = 0; x < 4; ++x) {
-            const int rr = tid >> 2, c16 = (tid & 3) * 4 + x;
-            const int row = r_begin + c * 64 + rr;
-            const bool okr = row < r_end;
-            cp_async16_zfill((uint32_t)__cvta_generic_to_shared(&tile[buf][rr * GS + c16 * 8]),
-                             q + ((size_t)(okr ? row : 0) * H + h) * HD + c16 * 8, okr ? 16 : 0);
+    const uint32_t base = smem_u32(gram_smem);
+    GramCtl* ctl = reinterpret_cast<GramCtl*>(gram_smem + GRAM_CTL);
+    volatile int* abort_flag = &ctl->abort;
+    // a split is a multiple of 64 rows, so that only rows past L fill up its last tile
+    const int r_begin = sp * rows_per_split, nt = (min(L - r_begin, rows_per_split) + 63) / 64;
+    if (tid == 0) {
+        for (int i = 0; i < GRAM_SLOTS; ++i) {
+            mbar_init(smem_u32(&ctl->full[i]), 1);
+            mbar_init(smem_u32(&ctl->empty[i]), 1);
         }
-        cp_async_commit();
-    };
-    if (nchunk > 0) load(0, 0);
-    const int lj = lane & 7, lm = lane >> 3;
-    for (int c = 0; c < nchunk; ++c) {
-        if (c + 1 < nchunk) { load(c + 1, (c + 1) & 1); cp_async_wait<1>(); } else { cp_async_wait<0>(); }
-        __syncthreads();
-        const uint32_t tb = (uint32_t)__cvta_generic_to_shared(&tile[c & 1][0]);
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks) {
-            const int k0 = ks * 16;
-            uint32_t a[2][4];
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                // A[m][k] = tile[k][m]: matrices (m lo, k lo), (m hi, k lo), (m lo, k hi), (m hi, k hi)
-                const int row = k0 + lj + (lm >> 1) * 8, col = 32 * wm + 16 * i + (lm & 1) * 8;
-                ldmatrix_x4_trans(tb + (uint32_t)(row * GS + col) * 2, a[i][0], a[i][1], a[i][2], a[i][3]);
-            }
-#pragma unroll
-            for (int jp = 0; jp < 4; ++jp) {
-                // B[k][n] = tile[k][n]: matrices (k lo, n0), (k hi, n0), (k lo, n0 + 8), (k hi, n0 + 8)
-                const int row = k0 + lj + (lm & 1) * 8, col = 64 * wn + 16 * jp + (lm >> 1) * 8;
-                uint32_t b0, b1, b2, b3;
-                ldmatrix_x4_trans(tb + (uint32_t)(row * GS + col) * 2, b0, b1, b2, b3);
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    mma16816(acc[i][2 * jp], a[i][0], a[i][1], a[i][2], a[i][3], b0, b1);
-                    mma16816(acc[i][2 * jp + 1], a[i][0], a[i][1], a[i][2], a[i][3], b2, b3);
-                }
-            }
-        }
-        __syncthreads();
+        mbar_init(smem_u32(&ctl->done), 1);
+        ctl->abort = (base & 1023u) ? 1 : 0;              // the swizzled tiles need a 1024-byte aligned base
+        if (base & 1023u) atomicCAS(status, 0, 904);
+        mbar_fence_init();
+        fence_proxy_async_smem();
     }
-    float* out = parts + ((size_t)h * nsplit + sp) * HD * HD;
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int m = 32 * wm + 16 * i + g, nn = 64 * wn + 8 * j + 2 * tg;
-            *reinterpret_cast<float2*>(out + m * HD + nn) = make_float2(acc[i][j][0], acc[i][j][1]);
-            *reinterpret_cast<float2*>(out + (m + 8) * HD + nn) = make_float2(acc[i][j][2], acc[i][j][3]);
+    if (warp == 4) {
+        tmem_alloc(smem_u32(&ctl->tmem_base), HD);
+        tmem_relinquish();
+        tc_fence_before();
+    }
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = ctl->tmem_base, full0 = smem_u32(&ctl->full[0]), empty0 = smem_u32(&ctl->empty[0]);
+    bool ok = *abort_flag == 0;
+    int issued = 0;
+    if (warp == 5) {
+        for (int c = 0; c < nt && ok; ++c) {
+            const uint32_t slot = c % GRAM_SLOTS, bar = full0 + 8 * slot;
+            ok = mbar_wait_warp(empty0 + 8 * slot, ((c / GRAM_SLOTS) & 1) ^ 1, abort_flag, status, 601);
+            if (!ok) break;
+            if (lane == 0) mbar_arrive_expect_tx(bar, GRAM_TILE);
+            __syncwarp();
+            if (lane < 2) tma_load_3d(base + slot * GRAM_TILE + lane * GRAM_HALF, &tmQ, bar, 64 * lane, r_begin + 64 * c, h);
+            issued = c + 1;
         }
+    } else if (warp == 4) {
+        constexpr uint32_t IDESC = umma_idesc_bf16(HD, HD, 1) | (1u << 15);      // both operands MN-major
+        const uint64_t d0 = umma_desc_sw128(0, GRAM_HALF, 1024);
+        const uint32_t d_hi = (uint32_t)(d0 >> 32), d_lo = (uint32_t)d0;
+        for (int c = 0; c < nt && ok; ++c) {
+            const uint32_t slot = c % GRAM_SLOTS;
+            ok = mbar_wait_warp(full0 + 8 * slot, (c / GRAM_SLOTS) & 1, abort_flag, status, 602);
+            if (!ok) break;
+            tc_fence_after();
+            if (elect_one()) {
+                const uint32_t t = d_lo + ((base + slot * GRAM_TILE) >> 4);
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks)
+                    umma_ss_lohi(tmem, t + ((ks * 2048) >> 4), d_hi, t + ((ks * 2048) >> 4), d_hi, IDESC, (c > 0 || ks > 0) ? 1u : 0u);
+                umma_commit(empty0 + 8 * slot);
+            }
+            __syncwarp();
+        }
+        // after the last product, or what was issued of them: tensor memory is freed below
+        if (elect_one()) umma_commit(smem_u32(&ctl->done));
+        __syncwarp();
+        mbar_wait(smem_u32(&ctl->done), 0, abort_flag, status, 603);
+    } else {
+        ok = ok && mbar_wait_warp(smem_u32(&ctl->done), 0, abort_flag, status, 604) && *abort_flag == 0;
+        tc_fence_after();
+        float* out = parts + ((size_t)h * nsplit + sp) * HD * HD + 32 * warp + lane;
+#pragma unroll 1
+        for (int p = 0; p < HD / 32; ++p) {
+            uint32_t r[32];
+            tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16) + 32 * p, r);
+            tmem_wait_ld_regs(r);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) out[(32 * p + j) * HD] = ok ? __uint_as_float(r[j]) : NAN;
+        }
+        tc_fence_before();
+    }
+    __syncwarp();
+    if (warp == 5 && lane == 0 && *abort_flag) {
+        // a wait gave up: give the loads a moment (100 us in all) to land before shared memory goes away
+        const uint64_t t_end = global_timer_ns() + 100000ull;
+        for (int c = max(0, issued - GRAM_SLOTS); c < issued; ++c)
+            while (!mbar_try_wait(full0 + 8 * (c % GRAM_SLOTS), (c / GRAM_SLOTS) & 1) && global_timer_ns() < t_end) {}
+    }
+    __syncthreads();
+    if (warp == 4) {
+        tc_fence_after();
+        tmem_dealloc(tmem, HD);
+    }
 }
 
 // ------------------------------------------------------------------------------------------------ metric
@@ -150,29 +184,29 @@ gram_reduce_kernel(float* __restrict__ parts, int nsplit, float norm) {
 }
 
 // ------------------------------------------------------------------------------------------------ probes
-// Probe i of a head = scale * mean of the query rows of 64-row block floor(i (nb - 1) / 63 + 0.5) (representatives.py:36-46): 64
-// threads, two dimensions each, PROBES_PER_CTA of them in a CTA. The probes need only q, so they are more CTAs of the launch that
-// makes the metric, beside its one chain per head. As a kernel of their own (a dimension per thread, a few loads on their way)
-// they took 57 us a branch at Wan-14B, 20 us at Wan-1.3B, 6.7 us and a launch at 4,152 tokens.
-constexpr int PROBES_PER_CTA = 4;
+// Probe i of a head = scale * mean of the query rows of 64-row block floor(i (nb - 1) / 63 + 0.5) (representatives.py:36-46): a warp
+// each, four dimensions a lane, 32 rows requested at a time. The probes need only q, so they are more CTAs of the launch that makes
+// the metric, beside its one chain per head. As a kernel of their own (a dimension per thread, a few loads on their way) they took
+// 57 us a branch at Wan-14B, 20 us at Wan-1.3B, 6.7 us and a launch at 4,152 tokens.
+constexpr int PROBES_PER_CTA = 8;
 __device__ __forceinline__ void probe_block(const __nv_bfloat16* __restrict__ q, __nv_bfloat16* __restrict__ probes, int cta, int L,
                                             int H, int nb, float scale) {
-    const int at = cta * PROBES_PER_CTA + (threadIdx.x >> 6), d = 2 * (threadIdx.x & 63), i = at % NP, h = at / NP;
+    const int at = cta * PROBES_PER_CTA + (threadIdx.x >> 5), d = 4 * (threadIdx.x & 31), i = at % NP, h = at / NP;
     const int blk = (int)((float)(i * (nb - 1)) / (float)(NP - 1) + 0.5f), n = min(64, L - blk * 64);
     const __nv_bfloat16* src = q + ((size_t)blk * 64 * H + h) * HD + d;
-    float s0 = 0.f, s1 = 0.f;
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int r0 = 0; r0 < 64; r0 += 32) {
-        uint32_t w[32];
+        uint2 w[32];
 #pragma unroll
-        for (int r = 0; r < 32; ++r) w[r] = r0 + r < n ? __ldg(reinterpret_cast<const uint32_t*>(src + (size_t)(r0 + r) * H * HD)) : 0u;
+        for (int r = 0; r < 32; ++r) w[r] = r0 + r < n ? __ldg(reinterpret_cast<const uint2*>(src + (size_t)(r0 + r) * H * HD)) : make_uint2(0u, 0u);
 #pragma unroll
         for (int r = 0; r < 32; ++r)
-            if (r0 + r < n) { s0 += bf_lo(w[r]); s1 += bf_hi(w[r]); }
+            if (r0 + r < n) { s[0] += bf_lo(w[r].x); s[1] += bf_hi(w[r].x); s[2] += bf_lo(w[r].y); s[3] += bf_hi(w[r].y); }
     }
     const float c = fmaxf((float)n, 1.0f);
-    probes[(size_t)at * HD + d] = __float2bfloat16_rn(s0 * scale / c);
-    probes[(size_t)at * HD + d + 1] = __float2bfloat16_rn(s1 * scale / c);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) probes[(size_t)at * HD + d + e] = __float2bfloat16_rn(s[e] * scale / c);
 }
 
 // ------------------------------------------------------------------------------------------------ metric
@@ -702,6 +736,22 @@ kmeans_kernel(const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restri
 
 using namespace es;
 
+static int launch_gram(const void* q, float* parts, int L, int H, int rows_per_split, int nsplit, cudaStream_t st) {
+    int* status = device_status_ptr();
+    if (!status) return set_error(-2, "es_reps_metric: the device status word is not available on this device");
+    // (L, H, 128) bf16 viewed as dims {128 d, L, H}; a box is 64 d x 64 rows, 128-byte swizzled
+    CUtensorMap tq;
+    cuuint64_t dims[3] = {(cuuint64_t)HD, (cuuint64_t)L, (cuuint64_t)H};
+    cuuint64_t strides[2] = {(cuuint64_t)H * HD * 2, (cuuint64_t)HD * 2};
+    cuuint32_t box[3] = {64, 64, 1}, estr[3] = {1, 1, 1};
+    if (int rc = encode_tensor_map(&tq, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(q), dims, strides, box, estr,
+                                   CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
+    if (int rc = opt_in_shared_memory((const void*)gram_kernel, (int)GRAM_SMEM)) return rc;
+    gram_kernel<<<dim3(H, nsplit), 192, GRAM_SMEM, st>>>(tq, parts, L, rows_per_split, nsplit, status);
+    ES_CHECK_LAUNCH("gram");
+    return 0;
+}
+
 // Rows of q per Gram partial, as the reference splits them (representatives.py:160).
 static int gram_rows_per_split(int L) { return ((((L + 31) / 32) + 63) / 64) * 64; }
 
@@ -721,8 +771,7 @@ extern "C" int es_reps_metric(const void* q, float* gram_parts, float* gram, voi
     if (!aligned(16, q, gram_parts, metric)) return set_error(-1, "es_reps_metric: q, gram_parts and metric must be 16-byte aligned");
     const int rps = gram_rows_per_split(L), nsplit = (L + rps - 1) / rps;
     cudaStream_t st = (cudaStream_t)stream;
-    gram_kernel<<<dim3(H, nsplit), 256, 0, st>>>((const __nv_bfloat16*)q, gram_parts, L, H, rps, nsplit);
-    ES_CHECK_LAUNCH("gram");
+    if (int rc = launch_gram(q, gram_parts, L, H, rps, nsplit, st)) return rc;
     const int smem = METRIC_SMEM;
     if (int rc = opt_in_shared_memory((const void*)metric_kernel, smem)) return rc;
     const float scale = 1.0f / sqrtf((float)HD);
@@ -797,8 +846,7 @@ extern "C" int es_reps_metric_static(const void* q, float* gram, void* metric, v
     const int rps = (((L + nsplit - 1) / nsplit + 63) / 64) * 64;
     nsplit = (L + rps - 1) / rps;
     cudaStream_t st = (cudaStream_t)stream;
-    gram_kernel<<<dim3(H, nsplit), 256, 0, st>>>((const __nv_bfloat16*)q, parts, L, H, rps, nsplit);
-    ES_CHECK_LAUNCH("gram");
+    if (int rc = launch_gram(q, parts, L, H, rps, nsplit, st)) return rc;
     const int smem = METRIC_SMEM;
     if (int rc = opt_in_shared_memory((const void*)metric_kernel, smem)) return rc;
     const float scale = 1.0f / sqrtf((float)HD);
