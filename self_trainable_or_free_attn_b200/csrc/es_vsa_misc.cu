@@ -87,18 +87,23 @@ struct RouterArgs {
 // taken from a shared-memory copy of the probabilities in a fixed order (reproducible). GT: G as a compile-time constant for
 // R = 32, 16 and 8 (0: any power of two), so that the sums read 8 or 16 bytes at a time in the same order; the validity of a
 // tile's 64 keys is found once by 64 threads and handed round as two words (with every thread testing its 16 columns, integer
-// divisions were two thirds of the kernel). NB = 512, R = 16, 12 heads: LSE 58 us (137 before), scores
-// 95 us (225); NB = 624: 84 us (191) and 202 us (537).
+// divisions were two thirds of the kernel). NB = 512, R = 16, 12 heads: LSE 57 us (137 before), scores
+// 91 us (225); NB = 624: 84 us (191) and 128 us (537; 202 with three CTAs per SM).
+template <int D> constexpr bool ROUTER_P_OVER_Q = TB * D * 2 >= 64 * 64 * 4;
 template <typename T, int D, int MODE, int GT>
-__global__ void __launch_bounds__(128) router_kernel(const RouterArgs a) {
+__global__ void __launch_bounds__(128, 4) router_kernel(const RouterArgs a) {
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr uint32_t TILE = TB * D * 2;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int qt = blockIdx.x, bh = a.bh0 + blockIdx.y;
     const uint32_t sQ = smem_addr(smem), sK = sQ + TILE;                 // K: two stages
     uint32_t* sValid = reinterpret_cast<uint32_t*>(smem + 3 * TILE);     // [2 stages][2]: bit r = key r of the tile is valid
-    float* sP = reinterpret_cast<float*>(smem + 3 * TILE + 16);          // MODE 1: [64][SP] probabilities
-    constexpr int SP = 68;
+    // MODE 1: [64][64] probabilities, in the place of the Q tile (its fragments are in registers) where that is as large, so that
+    // four CTAs fit an SM. At 39 tiles x 12 heads three leave 24 of 468 CTAs to a second round.
+    float* sP = reinterpret_cast<float*>(smem + (ROUTER_P_OVER_Q<D> ? 0 : 3 * TILE + 16));
+    // element (r, c): a row's chunks of 4 are exchanged by the row, so that neither the fragments' pairs (four rows to a half warp)
+    // nor the chunks read back meet in a bank
+    auto at_p = [&](int r, int c) { return sP + r * 64 + (((c >> 2) ^ ((r & 3) << 1)) << 2) + (c & 3); };
     const int G = GT ? GT : a.G, lg = 31 - __clz(G);                     // R divides 64: G is a power of two
     auto valid_row = [&](int r) { return r < a.Lr && (r & (G - 1)) * a.R < a.blk_cnt[r >> lg]; };
     const T* q = static_cast<const T*>(a.qr) + ((size_t)bh * a.Lr_pad + (size_t)qt * TB) * D;
@@ -113,6 +118,7 @@ __global__ void __launch_bounds__(128) router_kernel(const RouterArgs a) {
         const float* lse = a.lse2 + (size_t)bh * a.Lr_pad + (size_t)qt * TB;
         ls0 = lse[r0]; ls1 = lse[r1];
     }
+    const bool qv0 = MODE == 1 && valid_row(qt * TB + r0), qv1 = MODE == 1 && valid_row(qt * TB + r1);
     uint32_t qa[D / 16][4];
     for (int kt = 0; kt < nkt; ++kt) {
         const uint32_t sKt = sK + (uint32_t)(kt & 1) * TILE;
@@ -127,6 +133,7 @@ __global__ void __launch_bounds__(128) router_kernel(const RouterArgs a) {
         if (kt == 0) {
 #pragma unroll
             for (int ks = 0; ks < D / 16; ++ks) load_a<D>(sQ, warp * 16, ks, lane, qa[ks]);
+            if (MODE == 1 && ROUTER_P_OVER_Q<D>) __syncthreads();        // the tile's room is the probabilities' from here on
         }
         float s[8][4];
 #pragma unroll
@@ -170,14 +177,13 @@ __global__ void __launch_bounds__(128) router_kernel(const RouterArgs a) {
             m0 = mn0; m1 = mn1;
         } else {
             // probabilities of this key tile -> shared memory, then fixed-order G x G sums
-            const bool qv0 = valid_row(qt * TB + r0), qv1 = valid_row(qt * TB + r1);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const int c = i * 8 + 2 * (lane & 3);
-                *reinterpret_cast<float2*>(sP + r0 * SP + c) =
+                *reinterpret_cast<float2*>(at_p(r0, c)) =
                     make_float2((qv0 && kv[i][0]) ? exp2f(s[i][0] * a.scale_log2 - ls0) : 0.f,
                                 (qv0 && kv[i][1]) ? exp2f(s[i][1] * a.scale_log2 - ls0) : 0.f);
-                *reinterpret_cast<float2*>(sP + r1 * SP + c) =
+                *reinterpret_cast<float2*>(at_p(r1, c)) =
                     make_float2((qv1 && kv[i][0]) ? exp2f(s[i][2] * a.scale_log2 - ls1) : 0.f,
                                 (qv1 && kv[i][1]) ? exp2f(s[i][3] * a.scale_log2 - ls1) : 0.f);
             }
@@ -187,25 +193,24 @@ __global__ void __launch_bounds__(128) router_kernel(const RouterArgs a) {
                 const int bi = e >> (6 - lg), bj = e & (per - 1);
                 const int qblk = qt * per + bi, kblk = kt * per + bj;
                 if (qblk < a.NB && kblk < a.NB) {
-                    const float* p0 = sP + bi * G * SP + bj * G;
                     float acc = 0.f;
                     if (GT >= 4) {
 #pragma unroll
                         for (int x = 0; x < GT; ++x)
 #pragma unroll
                             for (int y = 0; y < GT; y += 4) {
-                                const float4 v = *reinterpret_cast<const float4*>(p0 + x * SP + y);
+                                const float4 v = *reinterpret_cast<const float4*>(at_p(bi * GT + x, bj * GT + y));
                                 acc += v.x; acc += v.y; acc += v.z; acc += v.w;
                             }
                     } else if (GT == 2) {
 #pragma unroll
                         for (int x = 0; x < 2; ++x) {
-                            const float2 v = *reinterpret_cast<const float2*>(p0 + x * SP);
+                            const float2 v = *reinterpret_cast<const float2*>(at_p(bi * 2 + x, bj * 2));
                             acc += v.x; acc += v.y;
                         }
                     } else {
                         for (int x = 0; x < G; ++x)
-                            for (int y = 0; y < G; ++y) acc += p0[x * SP + y];
+                            for (int y = 0; y < G; ++y) acc += *at_p(bi * G + x, bj * G + y);
                     }
                     float norm;
                     if (a.row_norm == 1) norm = 1.f / (float)(G * G);
@@ -828,7 +833,7 @@ extern "C" int es_vsa_pool(const void* q, const void* k, const void* v, void* qr
 
 template <int MODE>
 static int launch_router(const RouterArgs& a, int D, int dtype, int bh_count, cudaStream_t st) {
-    const size_t smem = (size_t)3 * TB * D * 2 + 16 + (MODE == 1 ? 64 * 68 * sizeof(float) : 0);
+    const size_t smem = (size_t)3 * TB * D * 2 + 16 + (MODE == 1 && D == 64 ? 64 * 64 * sizeof(float) : 0);
     const dim3 grid(a.Lr_pad / TB, bh_count);
 #define ROUTER_LAUNCH(TT, DD, GG)                                                                                       \
     {                                                                                                                   \
