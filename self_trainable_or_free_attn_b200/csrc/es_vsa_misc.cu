@@ -242,7 +242,6 @@ struct TopkArgs {
     int NB, W, bh0;
     long long budget;       // clamped to NB * NB
     int *q2k_ptr, *q2k_idx, *k2q_ptr, *k2q_idx;
-    int* state;             // [bh_count, 4]: threshold key, equal entries to take
     int *gtcnt, *eqcnt, *eqbase, *colcnt;     // [bh_count, NB] each
     uint32_t* selbits;      // [bh_count, NB, W]
 };
@@ -258,18 +257,24 @@ __device__ __forceinline__ uint32_t score_key(float x) {
 // 0 walked the 256 bins; scores share their exponents, so the warps count into eight histograms. NB = 512, 12 heads:
 // 23 us (129 before).
 constexpr int SEL_CTAS = 8, SEL_COPIES = 8;
-__global__ void __cluster_dims__(SEL_CTAS, 1, 1) __launch_bounds__(1024) topk_select_kernel(const TopkArgs a) {
-    __shared__ uint32_t part[SEL_COPIES][256], hist[2][256], warp_sum[8], s_prefix, s_need;
+struct SelectShared {
+    uint32_t part[SEL_COPIES][256], hist[2][256], warp_sum[8], prefix, need;
+};
+// The threshold key and how many entries equal to it are taken, for every thread of the cluster.
+__device__ __forceinline__ void topk_select(const TopkArgs& a, SelectShared& sh, uint32_t& thr, int& take_equal) {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
+    auto& part = sh.part;
+    auto& hist = sh.hist;
+    auto& warp_sum = sh.warp_sum;
+    uint32_t &s_prefix = sh.prefix, &s_need = sh.need;
     const int b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, rank = (int)cluster.block_rank();
     const float* sc = a.scores + (size_t)b * a.NB * a.NB;
     const long long N = (long long)a.NB * a.NB, step = (N + SEL_CTAS - 1) / SEL_CTAS;
     const long long lo = min(rank * step, N), hi = min(lo + step, N);
-    if (a.budget <= 0) {                               // the same for every CTA of the cluster
-        if (rank == 0 && tid == 0) { a.state[b * 4] = (int)0xFFFFFFFFu; a.state[b * 4 + 1] = 0; }
-        return;
-    }
+    thr = 0xFFFFFFFFu;
+    take_equal = 0;
+    if (a.budget <= 0) return;                         // the same for every CTA of the cluster
     if (tid == 0) { s_prefix = 0; s_need = (uint32_t)a.budget; }
     uint32_t* mine = part[(tid >> 5) & (SEL_COPIES - 1)];
     for (int pass = 0; pass < 4; ++pass) {
@@ -314,123 +319,82 @@ __global__ void __cluster_dims__(SEL_CTAS, 1, 1) __launch_bounds__(1024) topk_se
         }
         __syncthreads();
     }
-    if (rank == 0 && tid == 0) { a.state[b * 4] = (int)s_prefix; a.state[b * 4 + 1] = (int)s_need; }
-    cluster.sync();                                    // no CTA leaves while another reads its histogram
+    thr = s_prefix;
+    take_equal = (int)s_need;
 }
 
-// one warp per row
-__global__ void __launch_bounds__(128) topk_count_kernel(const TopkArgs a) {
-    const int b = blockIdx.y, row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (row >= a.NB) return;
-    const uint32_t thr = (uint32_t)a.state[b * 4];
-    const float* sc = a.scores + ((size_t)b * a.NB + row) * a.NB;
-    int gt = 0, eq = 0;
-    for (int j = lane; j < a.NB; j += 32) {
-        const uint32_t key = score_key(sc[j]);
-        gt += key > thr; eq += key == thr;
+// Exclusive prefix of v over the 1024 threads of a CTA.
+__device__ __forceinline__ int scan_1024(int v, int* warp_total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += x;
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        gt += __shfl_xor_sync(0xffffffffu, gt, o);
-        eq += __shfl_xor_sync(0xffffffffu, eq, o);
-    }
-    if (lane == 0) { a.gtcnt[b * a.NB + row] = gt; a.eqcnt[b * a.NB + row] = eq; }
+    if (lane == 31) warp_total[warp] = incl;
+    __syncthreads();
+    const int before = incl - v + __reduce_add_sync(0xffffffffu, lane < warp ? warp_total[lane] : 0);
+    __syncthreads();
+    return before;
 }
 
-// one CTA per (b, h): exclusive scans over the rows (kind 0: rows -> eqbase and q2k_ptr; kind 1: columns -> k2q_ptr)
-__global__ void __launch_bounds__(1024) topk_scan_kernel(const TopkArgs a, int kind) {
-    __shared__ int part[1024];
-    const int b = blockIdx.x, tid = threadIdx.x, bh = a.bh0 + b;
-    const int per = (a.NB + 1023) / 1024, lo = tid * per, hi = min(lo + per, a.NB);
-    const int need = a.state[b * 4 + 1];
-    const long long base = (long long)bh * a.budget;
-    auto scan = [&](int v) -> int {          // exclusive prefix of v over the threads
-        part[tid] = v;
-        __syncthreads();
-        for (int o = 1; o < 1024; o <<= 1) {
-            const int x = tid >= o ? part[tid - o] : 0;
-            __syncthreads();
-            part[tid] += x;
-            __syncthreads();
-        }
-        const int r = part[tid] - v;
-        __syncthreads();
-        return r;
-    };
-    if (kind == 0) {
-        int se = 0;
-        for (int r = lo; r < hi; ++r) se += a.eqcnt[b * a.NB + r];
-        int eb = scan(se);
-        int sc = 0;
-        for (int r = lo; r < hi; ++r) {
-            a.eqbase[b * a.NB + r] = eb;
-            const int e = a.eqcnt[b * a.NB + r];
-            sc += a.gtcnt[b * a.NB + r] + max(0, min(e, need - eb));
-            eb += e;
-        }
-        int pos = scan(sc);
-        eb = a.eqbase[b * a.NB + (lo < a.NB ? lo : 0)];
-        for (int r = lo; r < hi; ++r) {
-            a.q2k_ptr[(size_t)bh * (a.NB + 1) + r] = (int)(base + pos);
-            const int e = a.eqcnt[b * a.NB + r];
-            pos += a.gtcnt[b * a.NB + r] + max(0, min(e, need - eb));
-            eb += e;
-        }
-        if (tid == 1023) a.q2k_ptr[(size_t)bh * (a.NB + 1) + a.NB] = (int)(base + pos);   // the last thread ends at the total
-    } else {
-        int sc = 0;
-        for (int r = lo; r < hi; ++r) sc += a.colcnt[b * a.NB + r];
-        int pos = scan(sc);
-        for (int r = lo; r < hi; ++r) {
-            a.k2q_ptr[(size_t)bh * (a.NB + 1) + r] = (int)(base + pos);
-            pos += a.colcnt[b * a.NB + r];
-        }
-        if (tid == 1023) a.k2q_ptr[(size_t)bh * (a.NB + 1) + a.NB] = (int)(base + pos);
+// Column counts -> k2q_ptr of one (b, h), by the 1024 threads of a CTA.
+__device__ __forceinline__ void scan_columns(const TopkArgs& a, int b, int* warp_total) {
+    const int tid = threadIdx.x, bh = a.bh0 + b, per = (a.NB + 1023) / 1024, lo = tid * per, hi = min(lo + per, a.NB);
+    int n = 0;
+    for (int r = lo; r < hi; ++r) n += __ldcg(a.colcnt + b * a.NB + r);
+    int pos = scan_1024(n, warp_total) + (int)((long long)bh * a.budget);
+    for (int r = lo; r < hi; ++r) {
+        a.k2q_ptr[(size_t)bh * (a.NB + 1) + r] = pos;
+        pos += __ldcg(a.colcnt + b * a.NB + r);
     }
+    if (tid == 1023) a.k2q_ptr[(size_t)bh * (a.NB + 1) + a.NB] = pos;            // the last thread ends at the total
 }
-
-// one warp per row: the ascending kv list and the selection bits
-__global__ void __launch_bounds__(128) topk_emit_rows_kernel(const TopkArgs a) {
-    const int b = blockIdx.y, row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, bh = a.bh0 + b;
-    if (row >= a.NB) return;
-    const uint32_t thr = (uint32_t)a.state[b * 4];
-    const int need = a.state[b * 4 + 1];
-    const float* sc = a.scores + ((size_t)b * a.NB + row) * a.NB;
-    int eqrank = a.eqbase[b * a.NB + row];
-    int pos = a.q2k_ptr[(size_t)bh * (a.NB + 1) + row];
-    for (int j0 = 0; j0 < a.NB; j0 += 32) {
-        const int j = j0 + lane;
-        const uint32_t key = j < a.NB ? score_key(sc[j]) : 0u;
-        const bool gt = j < a.NB && key > thr, eq = j < a.NB && key == thr;
-        const unsigned em = __ballot_sync(0xffffffffu, eq);
-        const bool take = gt || (eq && eqrank + __popc(em & ((1u << lane) - 1)) < need);
-        const unsigned tm = __ballot_sync(0xffffffffu, take);
-        if (take) a.q2k_idx[pos + __popc(tm & ((1u << lane) - 1))] = j;
-        if (lane == 0) a.selbits[((size_t)b * a.NB + row) * a.W + (j0 >> 5)] = tm;
-        pos += __popc(tm);
-        eqrank += __popc(em);
-    }
+__global__ void __launch_bounds__(1024) topk_scan_kernel(const TopkArgs a) {
+    __shared__ int warp_total[32];
+    scan_columns(a, blockIdx.x, warp_total);
 }
 
 // One CTA per word (32 columns) of the bitmap, its 8 warps an eighth of the rows each: count (pass 0) or emit the ascending
 // query lists (pass 1). A warp takes 32 rows at a time, lane = row, and a vote per column turns them into that column's 32
 // rows; lane j keeps column j's count. One thread per column walking the rows took 79 us per pass at NB = 512, 12 heads;
 // this takes 7.
-__global__ void __launch_bounds__(256) topk_cols_kernel(const TopkArgs a, int pass) {
-    __shared__ int part[8][32];
-    const int b = blockIdx.y, w = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, bh = a.bh0 + b;
+__device__ __forceinline__ int count_columns(const TopkArgs& a, int b, int w, int warp, int lane) {
     const uint32_t* bits = a.selbits + (size_t)b * a.NB * a.W + w;
     const int per = ((a.NB + 255) / 256) * 32, lo = warp * per, hi = min(lo + per, a.NB);
-    const int col = w * 32 + lane;
     int n = 0;
     for (int r0 = lo; r0 < hi; r0 += 32) {
-        const uint32_t word = r0 + lane < hi ? bits[(size_t)(r0 + lane) * a.W] : 0u;
+        const uint32_t word = r0 + lane < hi ? __ldcg(bits + (size_t)(r0 + lane) * a.W) : 0u;
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
             const int c = __popc(__ballot_sync(0xffffffffu, (word >> j) & 1u));
             n += lane == j ? c : 0;
         }
     }
-    part[warp][lane] = n;
+    return n;
+}
+__device__ __forceinline__ void emit_columns(const TopkArgs& a, int b, int w, int warp, int lane, const int (&part)[8][32]) {
+    const uint32_t* bits = a.selbits + (size_t)b * a.NB * a.W + w;
+    const int per = ((a.NB + 255) / 256) * 32, lo = warp * per, hi = min(lo + per, a.NB), col = w * 32 + lane;
+    int pos = col < a.NB ? __ldcg(a.k2q_ptr + (size_t)(a.bh0 + b) * (a.NB + 1) + col) : 0;
+    for (int x = 0; x < warp; ++x) pos += part[x][lane];
+    for (int r0 = lo; r0 < hi; r0 += 32) {
+        const uint32_t word = r0 + lane < hi ? __ldcg(bits + (size_t)(r0 + lane) * a.W) : 0u;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            const unsigned m = __ballot_sync(0xffffffffu, (word >> j) & 1u);
+            if (m == 0) continue;                      // uniform
+            const int at = __shfl_sync(0xffffffffu, pos, j);
+            if ((word >> j) & 1u) a.k2q_idx[at + __popc(m & ((1u << lane) - 1))] = r0 + lane;
+            pos += lane == j ? __popc(m) : 0;
+        }
+    }
+}
+__global__ void __launch_bounds__(256) topk_cols_kernel(const TopkArgs a, int pass) {
+    __shared__ int part[8][32];
+    const int b = blockIdx.y, w = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, col = w * 32 + lane;
+    part[warp][lane] = count_columns(a, b, w, warp, lane);
     __syncthreads();
     if (pass == 0) {
         if (warp == 0 && col < a.NB) {
@@ -440,18 +404,98 @@ __global__ void __launch_bounds__(256) topk_cols_kernel(const TopkArgs a, int pa
         }
         return;
     }
-    int pos = col < a.NB ? a.k2q_ptr[(size_t)bh * (a.NB + 1) + col] : 0;
-    for (int x = 0; x < warp; ++x) pos += part[x][lane];
-    for (int r0 = lo; r0 < hi; r0 += 32) {
-        const uint32_t word = r0 + lane < hi ? bits[(size_t)(r0 + lane) * a.W] : 0u;
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-            const unsigned m = __ballot_sync(0xffffffffu, (word >> j) & 1u);
-            if (m == 0) continue;                      // uniform
-            const int at = __shfl_sync(0xffffffffu, pos, j);
-            if ((word >> j) & 1u) a.k2q_idx[at + __popc(m & ((1u << lane) - 1))] = r0 + lane;
-            pos += lane == j ? __popc(m) : 0;
+    emit_columns(a, b, w, warp, lane, part);
+}
+
+// The whole of the global top-k in one launch, a cluster per (b, h): threshold, counts per row, row pointers, lists and bitmap,
+// and the lists of the columns. What one CTA leaves for the others of its cluster (counts, pointers, the bitmap) goes through
+// global memory, written before a cluster barrier and read past it from L2. As seven launches (selection, counts, scan, rows,
+// column counts, scan, columns) it took 28.6 us and six gaps at NB = 100, 8 heads, 20.1 now; 54.6 / 50.3 at NB = 512, 12 heads.
+__global__ void __cluster_dims__(SEL_CTAS, 1, 1) __launch_bounds__(1024) topk_kernel(const TopkArgs a) {
+    __shared__ SelectShared sh;
+    __shared__ int warp_total[32];
+    __shared__ int colpart[4][8][32];
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = (int)cluster.block_rank(), bh = a.bh0 + b;
+    uint32_t thr;
+    int need;
+    topk_select(a, sh, thr, need);
+    const float* scores = a.scores + (size_t)b * a.NB * a.NB;
+    const int row0 = rank * 32 + warp;                 // a warp's rows: row0, row0 + 256, ..
+    for (int row = row0; row < a.NB; row += 32 * SEL_CTAS) {
+        const float* sc = scores + (size_t)row * a.NB;
+        int gt = 0, eq = 0;
+#pragma unroll 4
+        for (int j = lane; j < a.NB; j += 32) {
+            const uint32_t key = score_key(sc[j]);
+            gt += key > thr; eq += key == thr;
         }
+        gt = __reduce_add_sync(0xffffffffu, gt);
+        eq = __reduce_add_sync(0xffffffffu, eq);
+        if (lane == 0) { a.gtcnt[b * a.NB + row] = gt; a.eqcnt[b * a.NB + row] = eq; }
+    }
+    cluster.sync();
+    if (rank == 0) {                                   // scans over the rows: equal entries before a row, row pointers
+        const int per = (a.NB + 1023) / 1024, lo = min(tid * per, a.NB), hi = min(lo + per, a.NB);
+        int equal = 0, n = 0;
+        for (int r = lo; r < hi; ++r) equal += __ldcg(a.eqcnt + b * a.NB + r);
+        const int eb0 = scan_1024(equal, warp_total);
+        for (int r = lo, eb = eb0; r < hi; ++r) {
+            const int e = __ldcg(a.eqcnt + b * a.NB + r);
+            n += __ldcg(a.gtcnt + b * a.NB + r) + max(0, min(e, need - eb));
+            eb += e;
+        }
+        int pos = scan_1024(n, warp_total) + (int)((long long)bh * a.budget);
+        for (int r = lo, eb = eb0; r < hi; ++r) {
+            const int e = __ldcg(a.eqcnt + b * a.NB + r);
+            a.eqbase[b * a.NB + r] = eb;
+            a.q2k_ptr[(size_t)bh * (a.NB + 1) + r] = pos;
+            pos += __ldcg(a.gtcnt + b * a.NB + r) + max(0, min(e, need - eb));
+            eb += e;
+        }
+        if (tid == 1023) a.q2k_ptr[(size_t)bh * (a.NB + 1) + a.NB] = pos;        // the last thread ends at the total
+    }
+    cluster.sync();
+    for (int row = row0; row < a.NB; row += 32 * SEL_CTAS) {
+        const float* sc = scores + (size_t)row * a.NB;
+        int eqrank = __ldcg(a.eqbase + b * a.NB + row), pos = __ldcg(a.q2k_ptr + (size_t)bh * (a.NB + 1) + row);
+#pragma unroll 4
+        for (int j0 = 0; j0 < a.NB; j0 += 32) {
+            const int j = j0 + lane;
+            const uint32_t key = j < a.NB ? score_key(sc[j]) : 0u;
+            const bool gt = j < a.NB && key > thr, eq = j < a.NB && key == thr;
+            const unsigned em = __ballot_sync(0xffffffffu, eq);
+            const bool take = gt || (eq && eqrank + __popc(em & ((1u << lane) - 1)) < need);
+            const unsigned tm = __ballot_sync(0xffffffffu, take);
+            if (take) a.q2k_idx[pos + __popc(tm & ((1u << lane) - 1))] = j;
+            if (lane == 0) a.selbits[((size_t)b * a.NB + row) * a.W + (j0 >> 5)] = tm;
+            pos += __popc(tm);
+            eqrank += __popc(em);
+        }
+    }
+    cluster.sync();
+    // columns: words rank, rank + 8, .. of the bitmap's rows, four at a time with eight warps each
+    const int w8 = warp & 7, quarter = warp >> 3;
+    for (int pass = 0; pass < 2; ++pass) {
+        for (int w0 = rank; w0 < a.W; w0 += 4 * SEL_CTAS) {
+            const int w = w0 + SEL_CTAS * quarter;
+            if (w < a.W) colpart[quarter][w8][lane] = count_columns(a, b, w, w8, lane);
+            __syncthreads();
+            if (w < a.W && pass == 1) emit_columns(a, b, w, w8, lane, colpart[quarter]);
+            const int col = w * 32 + lane;
+            if (w < a.W && pass == 0 && w8 == 0 && col < a.NB) {
+                int t = 0;
+#pragma unroll
+                for (int x = 0; x < 8; ++x) t += colpart[quarter][x][lane];
+                a.colcnt[b * a.NB + col] = t;
+            }
+            __syncthreads();
+        }
+        if (pass == 1) break;
+        cluster.sync();
+        if (rank == 0) scan_columns(a, b, warp_total);
+        cluster.sync();
     }
 }
 
@@ -907,28 +951,15 @@ extern "C" int es_vsa_global_topk(const float* scores, int32_t NB, int32_t bh0, 
     a.scores = scores; a.NB = NB; a.W = (NB + 31) / 32; a.bh0 = bh0; a.budget = budget;
     a.q2k_ptr = q2k_ptr; a.q2k_idx = q2k_idx; a.k2q_ptr = k2q_ptr; a.k2q_idx = k2q_idx;
     int* w = static_cast<int*>(workspace);
-    a.state = w; w += (size_t)bh_count * 4;
+    w += (size_t)bh_count * 4;                         // (unused)
     a.gtcnt = w; w += (size_t)bh_count * NB;
     a.eqcnt = w; w += (size_t)bh_count * NB;
     a.eqbase = w; w += (size_t)bh_count * NB;
     a.colcnt = w; w += (size_t)bh_count * NB;
     a.selbits = reinterpret_cast<uint32_t*>(w);
     cudaStream_t st = (cudaStream_t)stream;
-    topk_select_kernel<<<dim3(SEL_CTAS, bh_count), 1024, 0, st>>>(a);
-    ES_CHECK_LAUNCH("topk_select_kernel");
-    const dim3 rows((NB + 3) / 4, bh_count), cols(a.W, bh_count);
-    topk_count_kernel<<<rows, 128, 0, st>>>(a);
-    ES_CHECK_LAUNCH("topk_count_kernel");
-    topk_scan_kernel<<<bh_count, 1024, 0, st>>>(a, 0);
-    ES_CHECK_LAUNCH("topk_scan_kernel");
-    topk_emit_rows_kernel<<<rows, 128, 0, st>>>(a);
-    ES_CHECK_LAUNCH("topk_emit_rows_kernel");
-    topk_cols_kernel<<<cols, 256, 0, st>>>(a, 0);
-    ES_CHECK_LAUNCH("topk_cols_kernel");
-    topk_scan_kernel<<<bh_count, 1024, 0, st>>>(a, 1);
-    ES_CHECK_LAUNCH("topk_scan_kernel");
-    topk_cols_kernel<<<cols, 256, 0, st>>>(a, 1);
-    ES_CHECK_LAUNCH("topk_cols_kernel");
+    topk_kernel<<<dim3(SEL_CTAS, bh_count), 1024, 0, st>>>(a);
+    ES_CHECK_LAUNCH("topk_kernel");
     return 0;
 }
 
@@ -1015,7 +1046,7 @@ extern "C" int es_vsa_row_topk(const void* scores, int32_t NB, int32_t bh0, int3
     t.NB = NB; t.W = (NB + 31) / 32; t.bh0 = bh0; t.budget = (long long)NB * K;
     t.q2k_ptr = q2k_ptr; t.q2k_idx = q2k_idx; t.k2q_ptr = k2q_ptr; t.k2q_idx = k2q_idx;
     int* w = static_cast<int*>(workspace);
-    t.state = w; w += (size_t)bh_count * 4;
+    w += (size_t)bh_count * 4;                         // (unused)
     t.gtcnt = w; w += (size_t)bh_count * NB;
     t.eqcnt = w; w += (size_t)bh_count * NB;
     t.eqbase = w; w += (size_t)bh_count * NB;
@@ -1028,7 +1059,7 @@ extern "C" int es_vsa_row_topk(const void* scores, int32_t NB, int32_t bh0, int3
     const dim3 cols(t.W, bh_count);
     topk_cols_kernel<<<cols, 256, 0, st>>>(t, 0);
     ES_CHECK_LAUNCH("topk_cols_kernel");
-    topk_scan_kernel<<<bh_count, 1024, 0, st>>>(t, 1);
+    topk_scan_kernel<<<bh_count, 1024, 0, st>>>(t);
     ES_CHECK_LAUNCH("topk_scan_kernel");
     topk_cols_kernel<<<cols, 256, 0, st>>>(t, 1);
     ES_CHECK_LAUNCH("topk_cols_kernel");
