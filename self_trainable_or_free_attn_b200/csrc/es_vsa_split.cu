@@ -28,28 +28,33 @@ struct PlanArgs {
     int BH, NB, chunk, max_slots, min_len, resident, budget;
     double rel_mean, tail_frac;
     int *tasks, *merges, *info;
-    int* work;            // [3 * NR] chunk counts, their inclusive sums over the eligible rows, split flags
+    int* work;            // [3 * NR] chunk counts, (unused), split flags
 };
 
+// PER: rows of a thread where they fit its registers (8 for up to 8,192 rows; all their loads are on their way together and nothing
+// goes through `work`), or 0.
+template <int PER>
 __global__ void __launch_bounds__(1024) split_plan_kernel(const PlanArgs a) {
-    __shared__ int part[1024];
+    __shared__ int warp_total[32];
     __shared__ int s_total;
     const int tid = threadIdx.x, NR = a.BH * a.NB;
     const int per = (NR + 1023) / 1024, lo = min(tid * per, NR), hi = min(lo + per, NR);
     int* cnt = a.work;
-    int* incl = a.work + NR;
     int* flag = a.work + 2 * NR;
-    auto scan = [&](int v) -> int {          // exclusive prefix over the threads; the total lands in s_total
-        part[tid] = v;
-        __syncthreads();
-        for (int o = 1; o < 1024; o <<= 1) {
-            const int x = tid >= o ? part[tid - o] : 0;
-            __syncthreads();
-            part[tid] += x;
-            __syncthreads();
+    // exclusive prefix over the threads, the total in s_total: shuffles and two barriers (20 barriers a scan in shared memory, five
+    // scans: 20.5 us a plan of 6,144 rows, 16.2 with these, 12.8 with the rows in registers as well)
+    auto scan = [&](int v) -> int {
+        const int lane = tid & 31, warp = tid >> 5;
+        int incl = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += x;
         }
-        if (tid == 1023) s_total = part[1023];
-        const int r = part[tid] - v;
+        if (lane == 31) warp_total[warp] = incl;
+        __syncthreads();
+        const int r = incl - v + __reduce_add_sync(0xffffffffu, lane < warp ? warp_total[lane] : 0);
+        if (tid == 1023) s_total = r + v;
         __syncthreads();
         return r;
     };
@@ -58,15 +63,43 @@ __global__ void __launch_bounds__(1024) split_plan_kernel(const PlanArgs a) {
     if (a.tail_frac > 0.0) gthr = max(gthr, (int)ceil(a.tail_frac * (double)W / (double)a.resident));
     // chunks of the eligible rows, and how many rows are eligible
     int my_c = 0, my_e = 0;
-    for (int r = lo; r < hi; ++r) {
-        const int bh = r / a.NB, i = r - bh * a.NB;
-        const int* hp = a.ptr + (size_t)bh * (a.NB + 1);
-        const int n = hp[i + 1] - hp[i];
+    int r_beg[PER ? PER : 1], r_n[PER ? PER : 1], r_cnt[PER ? PER : 1], r_nnz[PER ? PER : 1];
+    uint32_t r_split = 0;
+    if (PER) {
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            const int r = lo + k, bh = r / a.NB, i = r - bh * a.NB;
+            const int* hp = a.ptr + (size_t)bh * (a.NB + 1);
+            r_beg[k] = r_n[k] = r_nnz[k] = 0;
+            if (r < hi) {
+                r_beg[k] = hp[i];
+                r_n[k] = hp[i + 1];
+                if (a.rel_mean > 0.0) r_nnz[k] = hp[a.NB] - hp[0];
+            }
+        }
+    }
+    auto row = [&](int n, int nnz) -> int {       // chunks of an eligible row, or 0
         int thr = gthr;
-        if (a.rel_mean > 0.0) thr = max(thr, (int)ceil(a.rel_mean * (double)(hp[a.NB] - hp[0]) / (double)a.NB));
+        if (a.rel_mean > 0.0) thr = max(thr, (int)ceil(a.rel_mean * (double)nnz / (double)a.NB));
         const int c = n >= thr ? (n + a.chunk - 1) / a.chunk : 0;
-        cnt[r] = c;
         my_c += c; my_e += n >= thr;
+        return c;
+    };
+    if (PER) {
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            r_cnt[k] = 0;
+            if (lo + k < hi) {
+                r_n[k] -= r_beg[k];
+                r_cnt[k] = row(r_n[k], r_nnz[k]);
+            }
+        }
+    } else {
+        for (int r = lo; r < hi; ++r) {
+            const int bh = r / a.NB, i = r - bh * a.NB;
+            const int* hp = a.ptr + (size_t)bh * (a.NB + 1);
+            cnt[r] = row(hp[i + 1] - hp[i], a.rel_mean > 0.0 ? hp[a.NB] - hp[0] : 0);
+        }
     }
     int run = scan(my_c);
     scan(my_e);
@@ -74,12 +107,18 @@ __global__ void __launch_bounds__(1024) split_plan_kernel(const PlanArgs a) {
     const bool within = E <= a.budget;
     // split flags; slots of the split rows; number of direct rows before each row
     int my_slots = 0, my_split = 0, my_direct = 0;
-    for (int r = lo; r < hi; ++r) {
-        run += cnt[r];
-        incl[r] = run;
-        const bool split = within && cnt[r] > 0 && run <= a.max_slots;
-        flag[r] = split;
-        my_slots += split ? cnt[r] : 0; my_split += split; my_direct += !split;
+    auto decide = [&](int c) -> bool {
+        run += c;
+        const bool split = within && c > 0 && run <= a.max_slots;
+        my_slots += split ? c : 0; my_split += split; my_direct += !split;
+        return split;
+    };
+    if (PER) {
+#pragma unroll
+        for (int k = 0; k < PER; ++k)
+            if (lo + k < hi) r_split |= (uint32_t)decide(r_cnt[k]) << k;
+    } else {
+        for (int r = lo; r < hi; ++r) flag[r] = decide(cnt[r]);
     }
     int slot = scan(my_slots);
     const int t_split = s_total;
@@ -89,18 +128,25 @@ __global__ void __launch_bounds__(1024) split_plan_kernel(const PlanArgs a) {
     const int n_direct = s_total;
     int4* tasks = reinterpret_cast<int4*>(a.tasks);
     int4* merges = reinterpret_cast<int4*>(a.merges);
-    for (int r = lo; r < hi; ++r) {
-        const int bh = r / a.NB, i = r - bh * a.NB;
-        const int* rp = a.ptr + (size_t)bh * (a.NB + 1) + i;
-        const int beg = rp[0], n = rp[1] - beg;
-        if (flag[r]) {
-            const int c = cnt[r];
+    auto emit = [&](int r, int beg, int n, int c, bool split) {
+        if (split) {
             for (int j = 0; j < c; ++j)
                 tasks[slot + j] = make_int4(r, beg + (int)((long long)j * n / c), beg + (int)((long long)(j + 1) * n / c), slot + j);
             merges[mrow++] = make_int4(r, slot, c, 0);
             slot += c;
         } else {
             tasks[t_split + drow++] = make_int4(r, beg, beg + n, -1);
+        }
+    };
+    if (PER) {
+#pragma unroll
+        for (int k = 0; k < PER; ++k)
+            if (lo + k < hi) emit(lo + k, r_beg[k], r_n[k], r_cnt[k], (r_split >> k) & 1u);
+    } else {
+        for (int r = lo; r < hi; ++r) {
+            const int bh = r / a.NB;
+            const int* rp = a.ptr + (size_t)bh * (a.NB + 1) + (r - bh * a.NB);
+            emit(r, rp[0], rp[1] - rp[0], cnt[r], flag[r]);
         }
     }
     if (tid == 0) {
@@ -205,7 +251,8 @@ extern "C" int es_vsa_split_plan(const int32_t* ptr, int32_t BH, int32_t NB, int
     if (((uintptr_t)tasks | (uintptr_t)merges) & 15) return set_error(-1, "es_vsa_split_plan: tasks and merges must be 16-byte aligned");
     PlanArgs a{ptr, BH, NB, chunk, max_slots, min_len, resident, budget, rel_mean, tail_frac, tasks, merges, info,
                static_cast<int*>(workspace)};
-    split_plan_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(a);
+    if ((long long)BH * NB <= 8 * 1024) split_plan_kernel<8><<<1, 1024, 0, (cudaStream_t)stream>>>(a);
+    else split_plan_kernel<0><<<1, 1024, 0, (cudaStream_t)stream>>>(a);
     ES_CHECK_LAUNCH("split_plan_kernel");
     return 0;
 }
