@@ -42,13 +42,13 @@ constexpr int NTHREADS = NSOFT + 128;
 constexpr int MMA_WARP = NSOFT / 32, LOADK_WARP = MMA_WARP + 1, LOADV_WARP = MMA_WARP + 2, MASS_WARP = MMA_WARP + 3;
 constexpr int NMASS = 8;      // sets of partial block masses in flight between the softmax warps and the mass warp
 constexpr uint32_t TMEM_COLS = 512;
-constexpr uint32_t O_COL = 256, Q_COL = 384;
+constexpr uint32_t O_COL = 256, Q_COL = 384, R_COL = 448;   // R: dense, the row sums of the rounded P
 constexpr int NSLOT = 6;      // K / V tiles in flight
 constexpr int Q_SLOT = NSLOT - 1;    // Q passes through this slot before its first K / V tile
 constexpr float kSeedLimit = 60.f;   // largest log2 row sum relative to a seeded offset (see dense_kernel)
-// Dense: a term below 1 / kTopShare of its row, which rounding changes by less than kTopLeast of the row (2^-9 / 64), stays rounded:
-// all terms' rounding together is some fifty times that.
-constexpr float kTopShare = 64.f, kTopLeast = 1.f / 32768.f;
+// Dense: a term below 1 / kTopShare of its row, which rounding changes by less than kTopLeast of the row (2^-9 / 256), stays rounded:
+// all terms' rounding together is some two hundred times that.
+constexpr float kTopShare = 256.f, kTopLeast = 1.f / 131072.f;
 constexpr int NBIAS = 8;      // refine iterations whose column biases are staged in shared memory at a time
 
 constexpr uint32_t TILE_BYTES = 128 * HD * 2;    // 32 KB: [d half][128 rows][64 d], 128B-swizzled
@@ -73,12 +73,17 @@ struct Ctl {
     int flag_part[4];
     float l_part[2][BM];               // row sums of the two column halves
     float m_part[2][BM];               // row maxima of the two column halves (fallback sweep)
-    float r_part[2][BM];               // dense: row sums of the rounded P
     float e_part[2][BM];               // dense: what rounding took from a half's largest P above the sample's; its key, or -1
     int key_part[2][BM];
     int redo;                          // some row left the range of the offset from a sample
 };
 static_assert(sizeof(Ctl) <= 5632, "control block");
+
+// Dense mode: 16 columns of ones as the B operand of one more product per k-step of PV, whose result is the row sum of the rounded P
+// (unpacking and adding it took a tenth of the softmax warps' instructions: 32,760 tokens x 12 heads 7.11 -> 6.93 ms). Four sums take
+// turns: the tensor core cuts off what it adds, and one sum over 256 iterations was 4e-5 short, 0.03 % of the error against fp64.
+constexpr uint32_t SMEM_ONES = (SMEM_MASS + 1023) / 1024 * 1024, ONES_BYTES = 2048;
+static_assert(SMEM_ONES + ONES_BYTES <= SMEM_ALLOC, "the ones take the block masses' room");
 
 // Fallback modes: tiles whose flags a CTA looks at in one go, and the most of them that are its own.
 constexpr int WALK_TILES = 64 * NTHREADS, WALK_MINE = 256;
@@ -237,6 +242,10 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
         mbar_fence_init();
         fence_proxy_async_smem();
     }
+    if (DENSE && warp == MASS_WARP) {
+        for (uint32_t e = lane; e < ONES_BYTES / 4; e += 32) reinterpret_cast<uint32_t*>(smem_raw + SMEM_ONES)[e] = 0x3F803F80u;
+        fence_proxy_async_smem();
+    }
     if (warp == MMA_WARP) {
         tmem_alloc(smem_u32(&ctl->tmem_base), TMEM_COLS);
         // a CTA that may allocate again (for its next tile, or for the same one in two sweeps) keeps its permit
@@ -368,6 +377,7 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
         // ------------------------------------------------------------ MMAs: the warp runs uniformly, one elected lane issues
         constexpr uint32_t IDESC = umma_idesc_bf16(BM, 128, 0);        // S = Q K^T: A (Q) from tensor memory, B K-major
         constexpr uint32_t IDESC_PV = umma_idesc_bf16(BM, HD, 1);      // O += P V: A (P) from tensor memory, B MN-major
+        constexpr uint32_t IDESC_R = umma_idesc_bf16(BM, 16, 0);       // dense: R += P 1
         // Shared-memory descriptors: everything but the start address is a constant of the layout, so the words are built
         // once and an MMA costs one add. K-major (K): LBO 16, SBO 1024; MN-major (V): LBO = one d half, SBO 1024.
         const uint64_t dk0 = umma_desc_sw128(0, 16, 1024), dv0 = umma_desc_sw128(0, HALF_BYTES, 1024);
@@ -427,6 +437,12 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
                     umma_ts_lohi(tmem + O_COL, p + (ks < 4 ? ks * 8 : 64 + (ks - 4) * 8),
                                  vb_lo + (uint32_t)((ks * 2048) >> 4), v_hi, IDESC_PV,
                                  (i > 0 || ks > 0) ? 1u : 0u);
+                if (DENSE) {
+#pragma unroll
+                    for (int ks = 0; ks < 8; ++ks)
+                        umma_ts_lohi(tmem + R_COL + 16 * (i & 3), p + (ks < 4 ? ks * 8 : 64 + (ks - 4) * 8), k_lo0 + ((smem_u32(smem_raw) + SMEM_ONES) >> 4),
+                                     k_hi, IDESC_R, (i > 3 || ks > 0) ? 1u : 0u);
+                }
                 umma_commit(empty0 + 8 * slot);
                 if (i + 1 == nt) umma_commit(smem_u32(&ctl->ofull));
             }
@@ -488,6 +504,7 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
         float m = FALLBACK ? 0.f : m_early;
         float best = 0.f;                          // dense: the largest logit found so far (at first the sample's) and its key
         int best_key = -1;
+        float p_best = 1.f;                        // its P, rounded (1 for the sample's maximum, the offset)
         uint32_t uS[2] = {0, 0};
 
         if (FALLBACK) {
@@ -523,7 +540,6 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
         }
 
         float2 lsum = make_float2(0.f, 0.f);
-        float2 rsum = make_float2(0.f, 0.f);       // dense: the row sum of P as rounded for PV
         const int* bits = a.skip_bits + ((size_t)h * a.nq + qb) * a.nw;
         const bool want_mass = !FALLBACK && !COMPENSATE && a.mass != nullptr;
         const float2 sc2 = make_float2(a.scale_log2, a.scale_log2);
@@ -578,7 +594,6 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
                         const float2 p = exp2_pair(xv);
                         if (j & 1) acc1 = __fadd2_rn(acc1, p); else acc = __fadd2_rn(acc, p);
                         pk[j] = pack_bf16x2(p.x, p.y);
-                        if (DENSE) rsum = __fadd2_rn(rsum, make_float2(__uint_as_float(pk[j] << 16), __uint_as_float(pk[j] & 0xFFFF0000u)));
                     }
                 } else {
 #pragma unroll
@@ -589,7 +604,6 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
                         p.y = 2 * j + 1 < lim ? p.y : 0.f;
                         acc = __fadd2_rn(acc, p);
                         pk[j] = pack_bf16x2(p.x, p.y);
-                        if (DENSE) rsum = __fadd2_rn(rsum, make_float2(__uint_as_float(pk[j] << 16), __uint_as_float(pk[j] & 0xFFFF0000u)));
                     }
                 }
             } else if (pooled) {
@@ -649,42 +663,55 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
             lsum = __fadd2_rn(lsum, acc);
             if (DENSE && find_top) {
                 // a logit above the row's largest so far, and its key (P has left already: this is off the chain to PV)
-                const int lim = !has ? 0 : cur_blk == a.nb - 1 ? a.tail_valid : BK;
-                if (lim != BK) {
+                // rounding keeps the order: a larger logit has a P that rounds to no less than the best one's, and P is packed already
+                uint32_t pm[4];
 #pragma unroll
-                    for (int c = 0; c < 64; ++c)
-                        if (c >= lim) s[c] = 0xff800000u;
+                for (int x = 0; x < 4; ++x) {
+                    pm[x] = max_bf16x2(pk[8 * x], pk[8 * x + 1]);
+#pragma unroll
+                    for (int y = 2; y < 8; ++y) pm[x] = max_bf16x2(pm[x], pk[8 * x + y]);
                 }
-                float mx[8];
+                pm[0] = max_bf16x2(max_bf16x2(pm[0], pm[1]), max_bf16x2(pm[2], pm[3]));
+                const float p_top = fmaxf(__uint_as_float(pm[0] << 16), __uint_as_float(pm[0] & 0xFFFF0000u));
+                if (__any_sync(0xffffffffu, p_top >= p_best)) {
+                    const int lim = !has ? 0 : cur_blk == a.nb - 1 ? a.tail_valid : BK;
+                    if (lim != BK) {
 #pragma unroll
-                for (int g = 0; g < 8; ++g) {
-                    const float* x = reinterpret_cast<const float*>(s) + 8 * g;
-                    mx[g] = fmaxf(fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3])), fmaxf(fmaxf(x[4], x[5]), fmaxf(x[6], x[7])));
-                }
-                const float top = fmaxf(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])), fmaxf(fmaxf(mx[4], mx[5]), fmaxf(mx[6], mx[7])));
-                const bool better = top > best;
-                if (__any_sync(0xffffffffu, better)) {
-                    // one that is no large part of what the row has by now needs no key, and the smaller one before it neither
-                    const bool large = better && ex2_approx(fmaf(top, a.scale_log2, -m)) * kTopShare >= lsum.x + lsum.y;
-                    int key = -1;
-                    if (__any_sync(0xffffffffu, large)) {
-                        // its column by halving: each level keeps the half of the candidates that holds the maximum
-                        const bool h5 = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) < top;
-                        const bool h4 = fmaxf(h5 ? mx[4] : mx[0], h5 ? mx[5] : mx[1]) < top;
-                        const float m0 = h5 ? mx[4] : mx[0], m2 = h5 ? mx[6] : mx[2];
-                        const bool h3 = (h4 ? m2 : m0) < top;
-                        uint32_t t[32];
-#pragma unroll
-                        for (int c = 0; c < 32; ++c) t[c] = h5 ? s[32 + c] : s[c];
-#pragma unroll
-                        for (int c = 0; c < 16; ++c) t[c] = h4 ? t[16 + c] : t[c];
-                        int at = 0;
-#pragma unroll
-                        for (int c = 0; c < 8; ++c) at = __uint_as_float(h3 ? t[8 + c] : t[c]) == top ? c : at;
-                        if (large) key = cur_blk * BK + 32 * h5 + 16 * h4 + 8 * h3 + at;
+                        for (int c = 0; c < 64; ++c)
+                            if (c >= lim) s[c] = 0xff800000u;
                     }
-                    best = better ? top : best;
-                    best_key = better ? key : best_key;
+                    float mx[8];
+#pragma unroll
+                    for (int g = 0; g < 8; ++g) {
+                        const float* x = reinterpret_cast<const float*>(s) + 8 * g;
+                        mx[g] = fmaxf(fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3])), fmaxf(fmaxf(x[4], x[5]), fmaxf(x[6], x[7])));
+                    }
+                    const float top = fmaxf(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])), fmaxf(fmaxf(mx[4], mx[5]), fmaxf(mx[6], mx[7])));
+                    const bool better = top > best;
+                    if (__any_sync(0xffffffffu, better)) {
+                        // one that is no large part of what the row has by now needs no key, and the smaller one before it neither
+                        const bool large = better && ex2_approx(fmaf(top, a.scale_log2, -m)) * kTopShare >= lsum.x + lsum.y;
+                        int key = -1;
+                        if (__any_sync(0xffffffffu, large)) {
+                            // its column by halving: each level keeps the half of the candidates that holds the maximum
+                            const bool h5 = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) < top;
+                            const bool h4 = fmaxf(h5 ? mx[4] : mx[0], h5 ? mx[5] : mx[1]) < top;
+                            const float m0 = h5 ? mx[4] : mx[0], m2 = h5 ? mx[6] : mx[2];
+                            const bool h3 = (h4 ? m2 : m0) < top;
+                            uint32_t t[32];
+#pragma unroll
+                            for (int c = 0; c < 32; ++c) t[c] = h5 ? s[32 + c] : s[c];
+#pragma unroll
+                            for (int c = 0; c < 16; ++c) t[c] = h4 ? t[16 + c] : t[c];
+                            int at = 0;
+#pragma unroll
+                            for (int c = 0; c < 8; ++c) at = __uint_as_float(h3 ? t[8 + c] : t[c]) == top ? c : at;
+                            if (large) key = cur_blk * BK + 32 * h5 + 16 * h4 + 8 * h3 + at;
+                        }
+                        best = better ? top : best;
+                        best_key = better ? key : best_key;
+                        p_best = better ? __uint_as_float(pack_bf16x2(ex2_approx(fmaf(top, a.scale_log2, -m)), 0.f) << 16) : p_best;
+                    }
                 }
             }
             if (want_mass && exact) {
@@ -708,7 +735,6 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
         // (not in m_part: with one or two iterations nothing keeps the other half's warp from still reading its maxima)
         if (DENSE) {
             const float top = ex2_approx(fmaf(best, a.scale_log2, -m));      // the bits of the loop
-            ctl->r_part[ch][trow] = rsum.x + rsum.y;
             ctl->e_part[ch][trow] = best_key < 0 ? 0.f : top - __uint_as_float(pack_bf16x2(top, 0.f) << 16);
             ctl->key_part[ch][trow] = best_key;
         }
@@ -733,7 +759,8 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
         if (nt > 0) ok = mbar_wait_warp(smem_u32(&ctl->ofull), 0, abort_flag, a.status, 303) && ok;
         if (ok) {
             tc_fence_after();
-            const float rounded = DENSE ? (ctl->r_part[0][trow] + ctl->r_part[1][trow]) + (e_top[0] + e_top[1]) : 0.f;
+            float rounded = DENSE ? e_top[0] + e_top[1] : 0.f;
+            for (int x = 0; x < (DENSE ? min(nt, 4) : 0); ++x) rounded += tmem_ld1(lane_base + R_COL + 16 * x);
             const float inv = COMPENSATE ? 1.0f / (1.0f + l) : DENSE ? 1.0f / rounded : 1.0f / l;
             bool finite = true;
             // The outputs are turned in shared memory, 32 rows of a column half per warp, in the ring (every K / V tile has been
