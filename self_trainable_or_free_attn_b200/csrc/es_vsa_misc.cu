@@ -14,7 +14,7 @@ namespace es {
 namespace vsa {
 
 // ---------------------------------------------------------------------------------------------- pooling
-// One CTA per (block, bh): means of the R-token router groups of q and k (optionally v) over their valid tokens, and the
+// Means of the R-token router groups of q and k (optionally v) over their valid tokens, and the
 // block means of q, k, v, fp32 sums rounded once to the element type. Empty groups and the padding rows of the pooled
 // tensors are zero.
 struct PoolArgs {
@@ -24,51 +24,61 @@ struct PoolArgs {
     int L, NB, R, G, Lr_pad, NBc_pad;
 };
 
-template <typename T, int D>
+//
+// One CTA per (block, bh, tensor). RT = R for the group sizes in use (4 .. 32): all 64 rows are requested before the first is added;
+// 0: any R, a row after the other. The sums are the same in both. 512 blocks x 12 heads, us: 49.8, three
+// tensors one after the other and a few rows at a time 72.3; 100 blocks x 8 heads, D = 64: 3.2, 10.4.
+template <typename T, int D, int RT>
 __global__ void __launch_bounds__(D / 2) pool_kernel(const PoolArgs a) {
-    const int blk = blockIdx.x, bh = blockIdx.y, c = 2 * threadIdx.x;
-    const int tiles_c = a.NBc_pad, rows_r = a.Lr_pad;
-    const void* src[3] = {a.q, a.k, a.v};
-    void* dst_r[3] = {a.qr, a.kr, a.vr};
-    void* dst_c[3] = {a.qc, a.kc, a.vc};
+    const int blk = blockIdx.x, bh = blockIdx.y, t = blockIdx.z, c = 2 * threadIdx.x;
+    const int tiles_c = a.NBc_pad, rows_r = a.Lr_pad, R = RT ? RT : a.R, G = TB / R;
+    const void* src = t == 0 ? a.q : t == 1 ? a.k : a.v;
+    T* dst_r = static_cast<T*>(t == 0 ? a.qr : t == 1 ? a.kr : a.vr);
+    T* dst_c = static_cast<T*>(t == 0 ? a.qc : t == 1 ? a.kc : a.vc);
+    auto put = [&](T* row, float x, float y) { *reinterpret_cast<uint32_t*>(row + c) = Elt<T>::pack(x, y); };
     if (blk >= a.NB) {                       // padding rows of the pooled tensors
-#pragma unroll
-        for (int t = 0; t < 3; ++t) {
-            if (blk < tiles_c && dst_c[t])
-                *reinterpret_cast<uint32_t*>(static_cast<T*>(dst_c[t]) + ((size_t)bh * tiles_c + blk) * D + c) = 0u;
-            if (dst_r[t])
-                for (int r = blk * a.G; r < (blk + 1) * a.G; ++r)
-                    if (r < rows_r)
-                        *reinterpret_cast<uint32_t*>(static_cast<T*>(dst_r[t]) + ((size_t)bh * rows_r + r) * D + c) = 0u;
-        }
+        if (blk < tiles_c && dst_c) put(dst_c + ((size_t)bh * tiles_c + blk) * D, 0.f, 0.f);
+        if (dst_r)
+            for (int r = blk * G; r < min((blk + 1) * G, rows_r); ++r) put(dst_r + ((size_t)bh * rows_r + r) * D, 0.f, 0.f);
         return;
     }
+    if (!src || !(dst_r || dst_c)) return;
     const int cnt = a.blk_cnt[blk];
+    const T* x = static_cast<const T*>(src) + ((size_t)bh * a.L + (size_t)blk * TB) * D + c;
+    auto row = [&](int r) { return __ldg(reinterpret_cast<const uint32_t*>(x + (size_t)r * D)); };
+    float bx = 0.f, by = 0.f;
+    auto group = [&](int g, float sx, float sy) {
+        bx += sx; by += sy;
+        const int n = min(cnt - g * R, R);
+        const float inv = n > 0 ? 1.f / (float)n : 0.f;
+        if (dst_r) put(dst_r + ((size_t)bh * rows_r + blk * G + g) * D, sx * inv, sy * inv);
+    };
+    if (RT) {
+        uint32_t w[TB];
 #pragma unroll
-    for (int t = 0; t < 3; ++t) {
-        if (!src[t]) continue;
-        const T* x = static_cast<const T*>(src[t]) + ((size_t)bh * a.L + (size_t)blk * TB) * D + c;
-        float bx = 0.f, by = 0.f;
-        for (int g = 0; g < a.G; ++g) {
+        for (int r = 0; r < TB; ++r) w[r] = r < cnt ? row(r) : 0u;
+#pragma unroll
+        for (int g = 0; g < TB / (RT ? RT : TB); ++g) {
             float sx = 0.f, sy = 0.f;
-            const int lo = g * a.R, hi = min(lo + a.R, cnt);
-            for (int r = lo; r < hi; ++r) {
-                const float2 w = Elt<T>::unpack(*reinterpret_cast<const uint32_t*>(x + (size_t)r * D));
-                sx += w.x; sy += w.y;
+#pragma unroll
+            for (int r = 0; r < RT; ++r) {
+                const float2 f = Elt<T>::unpack(w[(g * RT + r) % TB]);
+                sx += f.x; sy += f.y;
             }
-            bx += sx; by += sy;
-            if (dst_r[t]) {
-                const float inv = hi > lo ? 1.f / (float)(hi - lo) : 0.f;
-                *reinterpret_cast<uint32_t*>(static_cast<T*>(dst_r[t]) + ((size_t)bh * rows_r + blk * a.G + g) * D + c) =
-                    Elt<T>::pack(sx * inv, sy * inv);
-            }
+            group(g, sx, sy);
         }
-        if (dst_c[t]) {
-            const float inv = 1.f / (float)cnt;
-            *reinterpret_cast<uint32_t*>(static_cast<T*>(dst_c[t]) + ((size_t)bh * tiles_c + blk) * D + c) =
-                Elt<T>::pack(bx * inv, by * inv);
+    } else {
+        for (int g = 0; g < G; ++g) {
+            float sx = 0.f, sy = 0.f;
+            for (int r = g * R; r < min((g + 1) * R, cnt); ++r) {
+                const float2 f = Elt<T>::unpack(row(r));
+                sx += f.x; sy += f.y;
+            }
+            group(g, sx, sy);
         }
     }
+    const float inv = 1.f / (float)cnt;
+    if (dst_c) put(dst_c + ((size_t)bh * tiles_c + blk) * D, bx * inv, by * inv);
 }
 
 // ---------------------------------------------------------------------------------------------- router
@@ -869,8 +879,20 @@ extern "C" int es_vsa_pool(const void* q, const void* k, const void* v, void* qr
     PoolArgs a{q, k, v, qr, kr, vr, qc, kc, vc, blk_cnt, L, NB, R, G, Lr_pad, NBc_pad};
     cudaStream_t st = (cudaStream_t)stream;
     const int rows = max(max(NB, NBc_pad), (Lr_pad + G - 1) / G);
-    const dim3 grid(rows, BH);
-    VSA_LAUNCH(pool_kernel, grid, D / 2, 0, a);
+    const dim3 grid(rows, BH, 3);
+#define POOL_CASE(TT, DD)                                                          \
+    {                                                                              \
+        if (R == 16) pool_kernel<TT, DD, 16><<<grid, DD / 2, 0, st>>>(a);          \
+        else if (R == 8) pool_kernel<TT, DD, 8><<<grid, DD / 2, 0, st>>>(a);       \
+        else if (R == 32) pool_kernel<TT, DD, 32><<<grid, DD / 2, 0, st>>>(a);     \
+        else if (R == 4) pool_kernel<TT, DD, 4><<<grid, DD / 2, 0, st>>>(a);       \
+        else pool_kernel<TT, DD, 0><<<grid, DD / 2, 0, st>>>(a);                   \
+    }
+    if (dtype == 0 && D == 128) POOL_CASE(__nv_bfloat16, 128)
+    else if (dtype == 0) POOL_CASE(__nv_bfloat16, 64)
+    else if (D == 128) POOL_CASE(__half, 128)
+    else POOL_CASE(__half, 64)
+#undef POOL_CASE
     ES_CHECK_LAUNCH("pool_kernel");
     return 0;
 }
