@@ -252,6 +252,7 @@ struct TopkArgs {
     int NB, W, bh0;
     long long budget;       // clamped to NB * NB
     int *q2k_ptr, *q2k_idx, *k2q_ptr, *k2q_idx;
+    int* state;             // [bh_count, 4]: threshold key, equal entries to take (where stages are launches)
     int *gtcnt, *eqcnt, *eqbase, *colcnt;     // [bh_count, NB] each
     uint32_t* selbits;      // [bh_count, NB, W]
 };
@@ -361,10 +362,77 @@ __device__ __forceinline__ void scan_columns(const TopkArgs& a, int b, int* warp
     }
     if (tid == 1023) a.k2q_ptr[(size_t)bh * (a.NB + 1) + a.NB] = pos;            // the last thread ends at the total
 }
-__global__ void __launch_bounds__(1024) topk_scan_kernel(const TopkArgs a) {
-    __shared__ int warp_total[32];
-    scan_columns(a, blockIdx.x, warp_total);
+// Equal entries before a row and row pointers of one (b, h), by the 1024 threads of a CTA.
+__device__ __forceinline__ void scan_rows(const TopkArgs& a, int b, int need, int* warp_total) {
+    const int tid = threadIdx.x, bh = a.bh0 + b;
+    const int per = (a.NB + 1023) / 1024, lo = min(tid * per, a.NB), hi = min(lo + per, a.NB);
+    int equal = 0, n = 0;
+    for (int r = lo; r < hi; ++r) equal += __ldcg(a.eqcnt + b * a.NB + r);
+    const int eb0 = scan_1024(equal, warp_total);
+    for (int r = lo, eb = eb0; r < hi; ++r) {
+        const int e = __ldcg(a.eqcnt + b * a.NB + r);
+        n += __ldcg(a.gtcnt + b * a.NB + r) + max(0, min(e, need - eb));
+        eb += e;
+    }
+    int pos = scan_1024(n, warp_total) + (int)((long long)bh * a.budget);
+    for (int r = lo, eb = eb0; r < hi; ++r) {
+        const int e = __ldcg(a.eqcnt + b * a.NB + r);
+        a.eqbase[b * a.NB + r] = eb;
+        a.q2k_ptr[(size_t)bh * (a.NB + 1) + r] = pos;
+        pos += __ldcg(a.gtcnt + b * a.NB + r) + max(0, min(e, need - eb));
+        eb += e;
+    }
+    if (tid == 1023) a.q2k_ptr[(size_t)bh * (a.NB + 1) + a.NB] = pos;        // the last thread ends at the total
 }
+
+// One CTA per (b, h): kind 0 rows, kind 1 columns.
+__global__ void __launch_bounds__(1024) topk_scan_kernel(const TopkArgs a, int kind) {
+    __shared__ int warp_total[32];
+    if (kind == 0) scan_rows(a, blockIdx.x, a.state[blockIdx.x * 4 + 1], warp_total);
+    else scan_columns(a, blockIdx.x, warp_total);
+}
+
+// one warp per row
+__global__ void __launch_bounds__(128) topk_count_kernel(const TopkArgs a) {
+    const int b = blockIdx.y, row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (row >= a.NB) return;
+    const uint32_t thr = (uint32_t)a.state[b * 4];
+    const float* sc = a.scores + ((size_t)b * a.NB + row) * a.NB;
+    int gt = 0, eq = 0;
+    for (int j = lane; j < a.NB; j += 32) {
+        const uint32_t key = score_key(sc[j]);
+        gt += key > thr; eq += key == thr;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        gt += __shfl_xor_sync(0xffffffffu, gt, o);
+        eq += __shfl_xor_sync(0xffffffffu, eq, o);
+    }
+    if (lane == 0) { a.gtcnt[b * a.NB + row] = gt; a.eqcnt[b * a.NB + row] = eq; }
+}
+
+// one warp per row: the ascending kv list and the selection bits
+__global__ void __launch_bounds__(128) topk_emit_rows_kernel(const TopkArgs a) {
+    const int b = blockIdx.y, row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, bh = a.bh0 + b;
+    if (row >= a.NB) return;
+    const uint32_t thr = (uint32_t)a.state[b * 4];
+    const int need = a.state[b * 4 + 1];
+    const float* sc = a.scores + ((size_t)b * a.NB + row) * a.NB;
+    int eqrank = a.eqbase[b * a.NB + row];
+    int pos = a.q2k_ptr[(size_t)bh * (a.NB + 1) + row];
+    for (int j0 = 0; j0 < a.NB; j0 += 32) {
+        const int j = j0 + lane;
+        const uint32_t key = j < a.NB ? score_key(sc[j]) : 0u;
+        const bool gt = j < a.NB && key > thr, eq = j < a.NB && key == thr;
+        const unsigned em = __ballot_sync(0xffffffffu, eq);
+        const bool take = gt || (eq && eqrank + __popc(em & ((1u << lane) - 1)) < need);
+        const unsigned tm = __ballot_sync(0xffffffffu, take);
+        if (take) a.q2k_idx[pos + __popc(tm & ((1u << lane) - 1))] = j;
+        if (lane == 0) a.selbits[((size_t)b * a.NB + row) * a.W + (j0 >> 5)] = tm;
+        pos += __popc(tm);
+        eqrank += __popc(em);
+    }
+}
+
 
 // One CTA per word (32 columns) of the bitmap, its 8 warps an eighth of the rows each: count (pass 0) or emit the ascending
 // query lists (pass 1). A warp takes 32 rows at a time, lane = row, and a vote per column turns them into that column's 32
@@ -417,10 +485,20 @@ __global__ void __launch_bounds__(256) topk_cols_kernel(const TopkArgs a, int pa
     emit_columns(a, b, w, warp, lane, part);
 }
 
+// The selection alone, a cluster per (b, h).
+__global__ void __cluster_dims__(SEL_CTAS, 1, 1) __launch_bounds__(1024) topk_select_kernel(const TopkArgs a) {
+    __shared__ SelectShared sh;
+    uint32_t thr;
+    int need;
+    topk_select(a, sh, thr, need);
+    if (blockIdx.x == 0 && threadIdx.x == 0) { a.state[blockIdx.y * 4] = (int)thr; a.state[blockIdx.y * 4 + 1] = need; }
+    cooperative_groups::this_cluster().sync();         // no CTA leaves while another reads its histogram
+}
+
 // The whole of the global top-k in one launch, a cluster per (b, h): threshold, counts per row, row pointers, lists and bitmap,
 // and the lists of the columns. What one CTA leaves for the others of its cluster (counts, pointers, the bitmap) goes through
-// global memory, written before a cluster barrier and read past it from L2. As seven launches (selection, counts, scan, rows,
-// column counts, scan, columns) it took 28.6 us and six gaps at NB = 100, 8 heads, 20.1 now; 54.6 / 50.3 at NB = 512, 12 heads.
+// global memory, written before a cluster barrier and read past it from L2. Where eight CTAs per head are enough (the rule is at
+// es_vsa_global_topk) this saves six launches.
 __global__ void __cluster_dims__(SEL_CTAS, 1, 1) __launch_bounds__(1024) topk_kernel(const TopkArgs a) {
     __shared__ SelectShared sh;
     __shared__ int warp_total[32];
@@ -446,26 +524,7 @@ __global__ void __cluster_dims__(SEL_CTAS, 1, 1) __launch_bounds__(1024) topk_ke
         if (lane == 0) { a.gtcnt[b * a.NB + row] = gt; a.eqcnt[b * a.NB + row] = eq; }
     }
     cluster.sync();
-    if (rank == 0) {                                   // scans over the rows: equal entries before a row, row pointers
-        const int per = (a.NB + 1023) / 1024, lo = min(tid * per, a.NB), hi = min(lo + per, a.NB);
-        int equal = 0, n = 0;
-        for (int r = lo; r < hi; ++r) equal += __ldcg(a.eqcnt + b * a.NB + r);
-        const int eb0 = scan_1024(equal, warp_total);
-        for (int r = lo, eb = eb0; r < hi; ++r) {
-            const int e = __ldcg(a.eqcnt + b * a.NB + r);
-            n += __ldcg(a.gtcnt + b * a.NB + r) + max(0, min(e, need - eb));
-            eb += e;
-        }
-        int pos = scan_1024(n, warp_total) + (int)((long long)bh * a.budget);
-        for (int r = lo, eb = eb0; r < hi; ++r) {
-            const int e = __ldcg(a.eqcnt + b * a.NB + r);
-            a.eqbase[b * a.NB + r] = eb;
-            a.q2k_ptr[(size_t)bh * (a.NB + 1) + r] = pos;
-            pos += __ldcg(a.gtcnt + b * a.NB + r) + max(0, min(e, need - eb));
-            eb += e;
-        }
-        if (tid == 1023) a.q2k_ptr[(size_t)bh * (a.NB + 1) + a.NB] = pos;        // the last thread ends at the total
-    }
+    if (rank == 0) scan_rows(a, b, need, warp_total);
     cluster.sync();
     for (int row = row0; row < a.NB; row += 32 * SEL_CTAS) {
         const float* sc = scores + (size_t)row * a.NB;
@@ -973,15 +1032,37 @@ extern "C" int es_vsa_global_topk(const float* scores, int32_t NB, int32_t bh0, 
     a.scores = scores; a.NB = NB; a.W = (NB + 31) / 32; a.bh0 = bh0; a.budget = budget;
     a.q2k_ptr = q2k_ptr; a.q2k_idx = q2k_idx; a.k2q_ptr = k2q_ptr; a.k2q_idx = k2q_idx;
     int* w = static_cast<int*>(workspace);
-    w += (size_t)bh_count * 4;                         // (unused)
+    a.state = w; w += (size_t)bh_count * 4;
     a.gtcnt = w; w += (size_t)bh_count * NB;
     a.eqcnt = w; w += (size_t)bh_count * NB;
     a.eqbase = w; w += (size_t)bh_count * NB;
     a.colcnt = w; w += (size_t)bh_count * NB;
     a.selbits = reinterpret_cast<uint32_t*>(w);
     cudaStream_t st = (cudaStream_t)stream;
-    topk_kernel<<<dim3(SEL_CTAS, bh_count), 1024, 0, st>>>(a);
-    ES_CHECK_LAUNCH("topk_kernel");
+    // One launch where it is gaps and launches that count and every cluster has its place at once (eight SMs each, 18 on 148); beyond,
+    // the stages are launches of their own, whose rows and columns go to all SMs. One call after the other, us, one launch / seven:
+    // 64 blocks x 12 heads 21.0 / 26.7, 256 x 12 26.3 / 32.4, 400 x 8 43.5 / 42.9 (and six launches of the host), 624 x 12 74.5 /
+    // 66.4, 1,600 x 1 324 / 171, 64 x 24 37.5 / 28.5.
+    if (NB <= 384 && bh_count <= 18) {
+        topk_kernel<<<dim3(SEL_CTAS, bh_count), 1024, 0, st>>>(a);
+        ES_CHECK_LAUNCH("topk_kernel");
+        return 0;
+    }
+    topk_select_kernel<<<dim3(SEL_CTAS, bh_count), 1024, 0, st>>>(a);
+    ES_CHECK_LAUNCH("topk_select_kernel");
+    const dim3 rows((NB + 3) / 4, bh_count), cols(a.W, bh_count);
+    topk_count_kernel<<<rows, 128, 0, st>>>(a);
+    ES_CHECK_LAUNCH("topk_count_kernel");
+    topk_scan_kernel<<<bh_count, 1024, 0, st>>>(a, 0);
+    ES_CHECK_LAUNCH("topk_scan_kernel");
+    topk_emit_rows_kernel<<<rows, 128, 0, st>>>(a);
+    ES_CHECK_LAUNCH("topk_emit_rows_kernel");
+    topk_cols_kernel<<<cols, 256, 0, st>>>(a, 0);
+    ES_CHECK_LAUNCH("topk_cols_kernel");
+    topk_scan_kernel<<<bh_count, 1024, 0, st>>>(a, 1);
+    ES_CHECK_LAUNCH("topk_scan_kernel");
+    topk_cols_kernel<<<cols, 256, 0, st>>>(a, 1);
+    ES_CHECK_LAUNCH("topk_cols_kernel");
     return 0;
 }
 
@@ -1081,7 +1162,7 @@ extern "C" int es_vsa_row_topk(const void* scores, int32_t NB, int32_t bh0, int3
     const dim3 cols(t.W, bh_count);
     topk_cols_kernel<<<cols, 256, 0, st>>>(t, 0);
     ES_CHECK_LAUNCH("topk_cols_kernel");
-    topk_scan_kernel<<<bh_count, 1024, 0, st>>>(t);
+    topk_scan_kernel<<<bh_count, 1024, 0, st>>>(t, 1);
     ES_CHECK_LAUNCH("topk_scan_kernel");
     topk_cols_kernel<<<cols, 256, 0, st>>>(t, 1);
     ES_CHECK_LAUNCH("topk_cols_kernel");

@@ -1,4 +1,4 @@
-"""The global top-k's one cluster per head, against a stable sort."""
+"""The global top-k, as one cluster per head and as a launch per stage, against a stable sort."""
 import pytest
 import torch
 
@@ -6,15 +6,15 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
-# one block; a word and one column; rows of 256 warps and one more; more words than the 32 a cluster has at a time, more rows than
-# threads (1,100)
-@pytest.mark.parametrize("nb", [1, 33, 257, 1100])
+# one launch: one block; a word and one column; rows of 256 warps and one more; the largest. Seven: one block more, more rows than
+# threads, more heads than clusters at once
+@pytest.mark.parametrize("nb,H", [(1, 3), (33, 18), (257, 3), (384, 2), (385, 2), (1100, 3), (33, 19)])
 @pytest.mark.parametrize("kind", ["random", "ties", "zeros"])
-def test_lists_match_a_stable_sort(nb, kind):
+def test_lists_match_a_stable_sort(nb, H, kind):
     """Score descending, ties to the smaller flat index: the lists are whole numbers and have to be equal."""
     from self_trainable_or_free_attn_b200.vsa import ops
     g = torch.Generator(device=DEV).manual_seed(nb)
-    B, H = 1, 3
+    B = 1
     s = torch.rand(B, H, nb, nb, device=DEV, generator=g)
     if kind == "ties":
         s = (s * 7).floor() / 7
