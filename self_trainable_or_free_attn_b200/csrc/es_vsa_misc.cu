@@ -718,9 +718,9 @@ __device__ __forceinline__ void store_piece(void* p, const uint32_t (&w)[4], int
 }
 
 // One CTA per (block, bh), 16 bytes a thread and row, four rows of a thread in flight. Bound by HBM: 32,768 tokens x 12 heads,
-// D = 128, a gate per token: 43 us (84 before).
+// D = 128, a gate per token: 38 us, twelve CTAs per SM (43 with nine).
 template <typename T, int D>
-__global__ void __launch_bounds__(128) fuse_fwd_kernel(const FuseArgs a) {
+__global__ void __launch_bounds__(128, 12) fuse_fwd_kernel(const FuseArgs a) {
     constexpr int CH = D / 8, ROWS = 128 / CH;                 // 16-byte pieces per row, rows per pass
     const int blk = blockIdx.x, bh = blockIdx.y, c = 8 * (threadIdx.x % CH), r0 = threadIdx.x / CH;
     const int cnt = a.blk_cnt[blk];
@@ -832,8 +832,11 @@ __device__ __forceinline__ void fuse_bwd_rows(const FuseArgs& a, const int blk, 
     }
 }
 
-template <typename T, int D>
-__global__ void __launch_bounds__(256) fuse_bwd_kernel(const FuseArgs a) {
+// Four CTAs per SM (64 registers), three with an elementwise gate at D = 128. 512 blocks x 12 heads, bf16, us, against one kernel for
+// all modes (99 registers at D = 128, two CTAs per SM): token gate 96 -> 63, none 62 -> 42, elementwise 94 -> 85 (four CTAs: 99);
+// at D = 64 39 -> 32 and, elementwise, 45 -> 43 (three: 48).
+template <typename T, int D, int GATE>
+__global__ void __launch_bounds__(256, GATE == 2 && D == 128 ? 3 : 4) fuse_bwd_kernel(const FuseArgs a) {
     constexpr int LR = D / 8, GROUPS = 256 / LR;
     __shared__ __align__(16) float part[GROUPS][D];
     const int blk = blockIdx.x, bh = blockIdx.y, tid = threadIdx.x, grp = tid / LR, c = 8 * (tid % LR);
@@ -851,9 +854,7 @@ __global__ void __launch_bounds__(256) fuse_bwd_kernel(const FuseArgs a) {
     float sum[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) sum[i] = 0.f;
-    if (a.gate_mode == 0) fuse_bwd_rows<T, D, 0>(a, blk, bh, cnt, ow, sum);
-    else if (a.gate_mode == 1) fuse_bwd_rows<T, D, 1>(a, blk, bh, cnt, ow, sum);
-    else fuse_bwd_rows<T, D, 2>(a, blk, bh, cnt, ow, sum);
+    fuse_bwd_rows<T, D, GATE>(a, blk, bh, cnt, ow, sum);
     *reinterpret_cast<float4*>(&part[grp][c]) = make_float4(sum[0], sum[1], sum[2], sum[3]);
     *reinterpret_cast<float4*>(&part[grp][c + 4]) = make_float4(sum[4], sum[5], sum[6], sum[7]);
     __syncthreads();
@@ -1103,7 +1104,17 @@ extern "C" int es_vsa_fuse_bwd(const void* dout, const void* of, const void* oc,
                (gate_mode == 2 ? (uintptr_t)gate | (uintptr_t)dgate : 0)) & 15) == 0;
     cudaStream_t st = (cudaStream_t)stream;
     const dim3 grid(NBc_pad, BH);
-    VSA_LAUNCH(fuse_bwd_kernel, grid, 256, 0, a);
+#define FUSE_BWD_CASE(TT, DD)                                                              \
+    {                                                                                      \
+        if (gate_mode == 0) fuse_bwd_kernel<TT, DD, 0><<<grid, 256, 0, st>>>(a);           \
+        else if (gate_mode == 1) fuse_bwd_kernel<TT, DD, 1><<<grid, 256, 0, st>>>(a);      \
+        else fuse_bwd_kernel<TT, DD, 2><<<grid, 256, 0, st>>>(a);                          \
+    }
+    if (dtype == 0 && D == 128) FUSE_BWD_CASE(__nv_bfloat16, 128)
+    else if (dtype == 0) FUSE_BWD_CASE(__nv_bfloat16, 64)
+    else if (D == 128) FUSE_BWD_CASE(__half, 128)
+    else FUSE_BWD_CASE(__half, 64)
+#undef FUSE_BWD_CASE
     ES_CHECK_LAUNCH("fuse_bwd_kernel");
     return 0;
 }
