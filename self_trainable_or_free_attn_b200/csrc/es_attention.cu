@@ -27,7 +27,7 @@
 // K and V tiles (32 KB each, [d half][128 rows][128 B], four 8 KB TMA boxes; representative rows: 64 boxes of 512 B)
 // travel through a ring of NSLOT shared-memory slots, about three iterations ahead of the MMAs. With one CTA per SM nothing hides
 // a tile's start and end, so Q and O cross shared memory in whole lines: a tile of 32 iterations took 66,900 clocks with a row per
-// thread on both sides, 60,300 now (one launch of the fused step of 32,760 tokens, 47 iterations a tile: 1.315 -> 1.28 ms).
+// thread on both sides, 60,300 now (the fused step of 32,760 tokens x 12 heads, 47 iterations a tile: 1.316 -> 1.301 ms).
 #include "es_ptx.cuh"
 #include "es_api_internal.h"
 #include <algorithm>
@@ -970,8 +970,8 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 // rarely is the row's, and where few keys hold most of a row that is most of P's error. So the outputs are divided by the sum of the
 // rounded P, which cancels the rounding of a dominant term, and every half of a row remembers its largest logit above the sample's
 // and the key: the epilogue adds (P - rounded P) V[key]. Relative error against fp64, two sweeps / as here / without the remembered
-// terms: 32,760 tokens x 12 heads 1.716e-3 / 1.682e-3 / 1.726e-3; 9,360 tokens of random q, k with logits of deviation 3.2
-// 1.821e-3 / 1.773e-3 / 2.017e-3. Time of the first shape 9.7 / 6.2 / 5.6 ms, of 1,560 tokens 95 / 56 / 46 us (one iteration in four
+// terms: 32,760 tokens x 12 heads 1.716e-3 / 1.681e-3 / 1.726e-3; 9,360 tokens of random q, k with logits of deviation 3.2
+// 1.821e-3 / 1.763e-3 / 2.017e-3. Time of the first shape, when this was chosen, 9.7 / 6.2 / 5.6 ms, of 1,560 tokens 95 / 56 / 46 us (one iteration in four
 // searched: 6.1 ms, but 1.95e-3 on the random rows).
 // (Flagged tiles, MODE 1, are those whose offset was far off, where a sample's maximum often is too: 0.81 ms of a Wan-14B step with
 // a sample first, 0.47 ms in two sweeps.)
