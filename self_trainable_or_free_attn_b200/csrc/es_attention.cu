@@ -42,7 +42,7 @@ constexpr int NTHREADS = NSOFT + 128;
 constexpr int MMA_WARP = NSOFT / 32, LOADK_WARP = MMA_WARP + 1, LOADV_WARP = MMA_WARP + 2, MASS_WARP = MMA_WARP + 3;
 constexpr int NMASS = 8;      // sets of partial block masses in flight between the softmax warps and the mass warp
 constexpr uint32_t TMEM_COLS = 512;
-constexpr uint32_t O_COL = 256, Q_COL = 384, R_COL = 448;   // R: dense, the row sums of the rounded P
+constexpr uint32_t O_COL = 256, Q_COL = 384;
 constexpr int NSLOT = 6;      // K / V tiles in flight
 constexpr int Q_SLOT = NSLOT - 1;    // Q passes through this slot before its first K / V tile
 constexpr float kSeedLimit = 60.f;   // largest log2 row sum relative to a seeded offset (see dense_kernel)
@@ -73,17 +73,12 @@ struct Ctl {
     int flag_part[4];
     float l_part[2][BM];               // row sums of the two column halves
     float m_part[2][BM];               // row maxima of the two column halves (fallback sweep)
+    float r_part[2][BM];               // dense: row sums of the rounded P
     float e_part[2][BM];               // dense: what rounding took from a half's largest P above the sample's; its key, or -1
     int key_part[2][BM];
     int redo;                          // some row left the range of the offset from a sample
 };
 static_assert(sizeof(Ctl) <= 5632, "control block");
-
-// Dense mode: 16 columns of ones as the B operand of one more product per k-step of PV, whose result is the row sum of the rounded P
-// (unpacking and adding it took a tenth of the softmax warps' instructions: 32,760 tokens x 12 heads 7.11 -> 6.93 ms). Four sums take
-// turns: the tensor core cuts off what it adds, and one sum over 256 iterations was 4e-5 short, 0.03 % of the error against fp64.
-constexpr uint32_t SMEM_ONES = (SMEM_MASS + 1023) / 1024 * 1024, ONES_BYTES = 2048;
-static_assert(SMEM_ONES + ONES_BYTES <= SMEM_ALLOC, "the ones take the block masses' room");
 
 // Fallback modes: tiles whose flags a CTA looks at in one go, and the most of them that are its own.
 constexpr int WALK_TILES = 64 * NTHREADS, WALK_MINE = 256;
@@ -242,10 +237,6 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
         mbar_fence_init();
         fence_proxy_async_smem();
     }
-    if (DENSE && warp == MASS_WARP) {
-        for (uint32_t e = lane; e < ONES_BYTES / 4; e += 32) reinterpret_cast<uint32_t*>(smem_raw + SMEM_ONES)[e] = 0x3F803F80u;
-        fence_proxy_async_smem();
-    }
     if (warp == MMA_WARP) {
         tmem_alloc(smem_u32(&ctl->tmem_base), TMEM_COLS);
         // a CTA that may allocate again (for its next tile, or for the same one in two sweeps) keeps its permit
@@ -377,7 +368,6 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
         // ------------------------------------------------------------ MMAs: the warp runs uniformly, one elected lane issues
         constexpr uint32_t IDESC = umma_idesc_bf16(BM, 128, 0);        // S = Q K^T: A (Q) from tensor memory, B K-major
         constexpr uint32_t IDESC_PV = umma_idesc_bf16(BM, HD, 1);      // O += P V: A (P) from tensor memory, B MN-major
-        constexpr uint32_t IDESC_R = umma_idesc_bf16(BM, 16, 0);       // dense: R += P 1
         // Shared-memory descriptors: everything but the start address is a constant of the layout, so the words are built
         // once and an MMA costs one add. K-major (K): LBO 16, SBO 1024; MN-major (V): LBO = one d half, SBO 1024.
         const uint64_t dk0 = umma_desc_sw128(0, 16, 1024), dv0 = umma_desc_sw128(0, HALF_BYTES, 1024);
@@ -437,12 +427,6 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
                     umma_ts_lohi(tmem + O_COL, p + (ks < 4 ? ks * 8 : 64 + (ks - 4) * 8),
                                  vb_lo + (uint32_t)((ks * 2048) >> 4), v_hi, IDESC_PV,
                                  (i > 0 || ks > 0) ? 1u : 0u);
-                if (DENSE) {
-#pragma unroll
-                    for (int ks = 0; ks < 8; ++ks)
-                        umma_ts_lohi(tmem + R_COL + 16 * (i & 3), p + (ks < 4 ? ks * 8 : 64 + (ks - 4) * 8), k_lo0 + ((smem_u32(smem_raw) + SMEM_ONES) >> 4),
-                                     k_hi, IDESC_R, (i > 3 || ks > 0) ? 1u : 0u);
-                }
                 umma_commit(empty0 + 8 * slot);
                 if (i + 1 == nt) umma_commit(smem_u32(&ctl->ofull));
             }
@@ -540,6 +524,10 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
         }
 
         float2 lsum = make_float2(0.f, 0.f);
+        // dense: the row sum of P as rounded for PV, in rounded float32 adds. Taken by the tensor core along with PV (a product with
+        // ones, no faster: 6.93 ms for 32,760 tokens x 12 heads, 6.89 so) it was cut off at every add: the sum of 65,536 terms 1e-5
+        // short, of 119,056 2e-5, in every row on the same side.
+        float2 rsum = make_float2(0.f, 0.f);
         const int* bits = a.skip_bits + ((size_t)h * a.nq + qb) * a.nw;
         const bool want_mass = !FALLBACK && !COMPENSATE && a.mass != nullptr;
         const float2 sc2 = make_float2(a.scale_log2, a.scale_log2);
@@ -594,6 +582,7 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
                         const float2 p = exp2_pair(xv);
                         if (j & 1) acc1 = __fadd2_rn(acc1, p); else acc = __fadd2_rn(acc, p);
                         pk[j] = pack_bf16x2(p.x, p.y);
+                        if (DENSE) rsum = __fadd2_rn(rsum, make_float2(__uint_as_float(pk[j] << 16), __uint_as_float(pk[j] & 0xFFFF0000u)));
                     }
                 } else {
 #pragma unroll
@@ -604,6 +593,7 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
                         p.y = 2 * j + 1 < lim ? p.y : 0.f;
                         acc = __fadd2_rn(acc, p);
                         pk[j] = pack_bf16x2(p.x, p.y);
+                        if (DENSE) rsum = __fadd2_rn(rsum, make_float2(__uint_as_float(pk[j] << 16), __uint_as_float(pk[j] & 0xFFFF0000u)));
                     }
                 }
             } else if (pooled) {
@@ -735,6 +725,7 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
         // (not in m_part: with one or two iterations nothing keeps the other half's warp from still reading its maxima)
         if (DENSE) {
             const float top = ex2_approx(fmaf(best, a.scale_log2, -m));      // the bits of the loop
+            ctl->r_part[ch][trow] = rsum.x + rsum.y;
             ctl->e_part[ch][trow] = best_key < 0 ? 0.f : top - __uint_as_float(pack_bf16x2(top, 0.f) << 16);
             ctl->key_part[ch][trow] = best_key;
         }
@@ -759,8 +750,7 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
         if (nt > 0) ok = mbar_wait_warp(smem_u32(&ctl->ofull), 0, abort_flag, a.status, 303) && ok;
         if (ok) {
             tc_fence_after();
-            float rounded = DENSE ? e_top[0] + e_top[1] : 0.f;
-            for (int x = 0; x < (DENSE ? min(nt, 4) : 0); ++x) rounded += tmem_ld1(lane_base + R_COL + 16 * x);
+            const float rounded = DENSE ? (ctl->r_part[0][trow] + ctl->r_part[1][trow]) + (e_top[0] + e_top[1]) : 0.f;
             const float inv = COMPENSATE ? 1.0f / (1.0f + l) : DENSE ? 1.0f / rounded : 1.0f / l;
             bool finite = true;
             // The outputs are turned in shared memory, 32 rows of a column half per warp, in the ring (every K / V tile has been
