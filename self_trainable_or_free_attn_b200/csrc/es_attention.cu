@@ -46,9 +46,6 @@ constexpr uint32_t O_COL = 256, Q_COL = 384;
 constexpr int NSLOT = 6;      // K / V tiles in flight
 constexpr int Q_SLOT = NSLOT - 1;    // Q passes through this slot before its first K / V tile
 constexpr float kSeedLimit = 60.f;   // largest log2 row sum relative to a seeded offset (see dense_kernel)
-// Dense: a term below 1 / kTopShare of its row, which rounding changes by less than kTopLeast of the row (2^-9 / 256), stays rounded:
-// all terms' rounding together is some two hundred times that.
-constexpr float kTopShare = 256.f, kTopLeast = 1.f / 131072.f;
 constexpr int NBIAS = 8;      // refine iterations whose column biases are staged in shared memory at a time
 
 constexpr uint32_t TILE_BYTES = 128 * HD * 2;    // 32 KB: [d half][128 rows][64 d], 128B-swizzled
@@ -679,27 +676,21 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
                     const float top = fmaxf(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])), fmaxf(fmaxf(mx[4], mx[5]), fmaxf(mx[6], mx[7])));
                     const bool better = top > best;
                     if (__any_sync(0xffffffffu, better)) {
-                        // one that is no large part of what the row has by now needs no key, and the smaller one before it neither
-                        const bool large = better && ex2_approx(fmaf(top, a.scale_log2, -m)) * kTopShare >= lsum.x + lsum.y;
-                        int key = -1;
-                        if (__any_sync(0xffffffffu, large)) {
-                            // its column by halving: each level keeps the half of the candidates that holds the maximum
-                            const bool h5 = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) < top;
-                            const bool h4 = fmaxf(h5 ? mx[4] : mx[0], h5 ? mx[5] : mx[1]) < top;
-                            const float m0 = h5 ? mx[4] : mx[0], m2 = h5 ? mx[6] : mx[2];
-                            const bool h3 = (h4 ? m2 : m0) < top;
-                            uint32_t t[32];
+                        // its column by halving: each level keeps the half of the candidates that holds the maximum
+                        const bool h5 = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) < top;
+                        const bool h4 = fmaxf(h5 ? mx[4] : mx[0], h5 ? mx[5] : mx[1]) < top;
+                        const float m0 = h5 ? mx[4] : mx[0], m2 = h5 ? mx[6] : mx[2];
+                        const bool h3 = (h4 ? m2 : m0) < top;
+                        uint32_t t[32];
 #pragma unroll
-                            for (int c = 0; c < 32; ++c) t[c] = h5 ? s[32 + c] : s[c];
+                        for (int c = 0; c < 32; ++c) t[c] = h5 ? s[32 + c] : s[c];
 #pragma unroll
-                            for (int c = 0; c < 16; ++c) t[c] = h4 ? t[16 + c] : t[c];
-                            int at = 0;
+                        for (int c = 0; c < 16; ++c) t[c] = h4 ? t[16 + c] : t[c];
+                        int at = 0;
 #pragma unroll
-                            for (int c = 0; c < 8; ++c) at = __uint_as_float(h3 ? t[8 + c] : t[c]) == top ? c : at;
-                            if (large) key = cur_blk * BK + 32 * h5 + 16 * h4 + 8 * h3 + at;
-                        }
+                        for (int c = 0; c < 8; ++c) at = __uint_as_float(h3 ? t[8 + c] : t[c]) == top ? c : at;
                         best = better ? top : best;
-                        best_key = better ? key : best_key;
+                        best_key = better ? cur_blk * BK + 32 * h5 + 16 * h4 + 8 * h3 + at : best_key;
                         p_best = better ? __uint_as_float(pack_bf16x2(ex2_approx(fmaf(top, a.scale_log2, -m)), 0.f) << 16) : p_best;
                     }
                 }
@@ -741,8 +732,7 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
 #pragma unroll
         for (int x = 0; x < (DENSE ? 2 : 0); ++x) {
             e_top[x] = ctl->e_part[x][trow];
-            top_key[x] = fabsf(e_top[x]) > l * kTopLeast ? ctl->key_part[x][trow] : -1;
-            if (top_key[x] < 0) e_top[x] = 0.f;
+            top_key[x] = ctl->key_part[x][trow];
             const uint4* src = reinterpret_cast<const uint4*>(a.v + ((size_t)max(top_key[x], 0) * a.H + h) * HD + 64 * ch);
 #pragma unroll
             for (int c = 0; c < 8; ++c) vtop[x][c] = top_key[x] >= 0 ? __ldg(src + c) : make_uint4(0, 0, 0, 0);
@@ -960,15 +950,17 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 // rarely is the row's, and where few keys hold most of a row that is most of P's error. So the outputs are divided by the sum of the
 // rounded P, which cancels the rounding of a dominant term, and every half of a row remembers its largest logit above the sample's
 // and the key: the epilogue adds (P - rounded P) V[key]. Relative error against fp64, two sweeps / as here / without the remembered
-// terms: 32,760 tokens x 12 heads 1.716e-3 / 1.681e-3 / 1.726e-3; 9,360 tokens of random q, k with logits of deviation 3.2
+// terms: 32,760 tokens x 12 heads 1.716e-3 / 1.682e-3 / 1.726e-3; 9,360 tokens of random q, k with logits of deviation 3.2
 // 1.821e-3 / 1.763e-3 / 2.017e-3. Time of the first shape, when this was chosen, 9.7 / 6.2 / 5.6 ms, of 1,560 tokens 95 / 56 / 46 us (one iteration in four
 // searched: 6.1 ms, but 1.95e-3 on the random rows).
+// Every half keeps its term however small its share: leaving those below 1 / 256 of the row rounded was no faster (6.89 ms, 6.84 so).
 // (Flagged tiles, MODE 1, are those whose offset was far off, where a sample's maximum often is too: 0.81 ms of a Wan-14B step with
 // a sample first, 0.47 ms in two sweeps.)
 //
 // Few tiles, or a few more than the SMs, leave most SMs idle: 1,560 tokens of 12 heads are 156 tiles on 148 SMs, two waves of which
 // the second is nearly empty. So the last tiles are cut by iterations (plan_dense): each piece takes its own offset from its own
-// columns and leaves m, the row sums and O in fp32, and a second kernel adds the pieces of a tile in their order. One launch after
+// columns and leaves m, the row sums and O in fp32, and a second kernel adds the pieces of a tile in their order. The error against fp64 is never larger than
+// that of whole tiles (897 to 9,360 tokens, 1 to 24 heads: 0.96 to 1.00 of it; every piece remembers its own largest terms). One launch after
 // the other, us, whole tiles / cut: 1,560 tokens x 12 heads 44.5 / 36.1, x 1 head 23.0 / 14.1, 4,096 x 1 44.2 / 20.9, 6,000 x 4
 // 120 / 91, 8,000 x 12 485 / 422; 4,096 tokens x 8 heads (1.73 waves of 32 iterations) stay whole: 87.7 / 93.0.
 __global__ void __launch_bounds__(NTHREADS, 1)

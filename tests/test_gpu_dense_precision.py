@@ -34,3 +34,19 @@ def test_row_sums_have_no_bias_that_grows_with_the_row(L):
         ref = torch.exp(s[:, :128] - s.logsumexp(1, keepdim=True)) @ vd
         bias += float((out[r:r + 1024] / ref - 1.0).sum()) / (n * 128)
     assert abs(bias) <= 6e-6
+
+
+@pytest.mark.parametrize("L,key", [(4096, 647), (9360, 5000)])
+def test_the_largest_term_above_the_sample_is_exact_however_small_its_share(L, key):
+    """V is zero but at one key, whose logit is every row's largest and in no sampled column: its share is 1 / 1000 or less. The outputs are
+    that term alone, rounded once to bf16: 1.66e-3 rms of the value; with a P rounded to bf16 as well 2.3e-3."""
+    g = torch.Generator(device=DEV).manual_seed(L)
+    k, v = (torch.zeros(L, 1, 128, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    k[key, 0, 0] = 1.0
+    v[key, 0] = 1.0 + torch.rand(128, device=DEV, generator=g)
+    q = torch.zeros(L, 1, 128, device=DEV, dtype=torch.bfloat16)
+    q[:, 0, 0] = (0.2 + 1.1 * torch.rand(L, device=DEV, generator=g)) * 128 ** 0.5
+    out = _dense(q, k, v)[:, 0].double()
+    p = torch.exp(q[:, 0, :1].double() / 128 ** 0.5)
+    ref = p * v[key].double() / (p + (L - 1))
+    assert float((out / ref - 1.0).square().mean().sqrt()) <= 1.9e-3
