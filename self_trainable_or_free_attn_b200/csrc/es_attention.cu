@@ -74,6 +74,7 @@ struct Ctl {
     float e_part[2][BM];               // dense: what rounding took from a half's largest P above the sample's; its key, or -1
     int key_part[2][BM];
     int redo;                          // some row left the range of the offset from a sample
+    int stop;                          // the status word was set before the tile began
 };
 static_assert(sizeof(Ctl) <= 5632, "control block");
 
@@ -157,14 +158,18 @@ struct SchedIter {
     }
 };
 
+// How a tile ended, the same for every thread of the CTA: done; dense mode, to be done again since `sample` did not do (dense_kernel);
+// or stopped by a wait that gave up, in this CTA or another, after which the CTA does no other tile.
+enum TileEnd { TILE_DONE, TILE_AGAIN, TILE_STOP };
+
 // One (query tile, head): `tile` = head * nq + query tile. `again`: the CTA has run a tile before (its barriers exist).
-// Dense mode: `sample` takes the offset from a sample of the columns; true is returned when that did not do (dense_kernel).
+// Dense mode: `sample` takes the offset from a sample of the columns.
 // The CTA runs iterations first .. last - 1 of the tile and leaves a partial result in `part`, or with null the outputs.
 template <int MODE>
-__device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmKm,
-                                               const CUtensorMap& tmVm, const CUtensorMap& tmKr, const CUtensorMap& tmVr,
-                                               const AttnArgs& a, const int tile, const bool again, const bool sample,
-                                               const int first = 0, const int last = 0, float* const part = nullptr) {
+__device__ __forceinline__ TileEnd attention_tile(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmKm,
+                                                  const CUtensorMap& tmVm, const CUtensorMap& tmKr, const CUtensorMap& tmVr,
+                                                  const AttnArgs& a, const int tile, const bool again, const bool sample,
+                                                  const int first = 0, const int last = 0, float* const part = nullptr) {
     constexpr bool COMPENSATE = MODE == 2;     // block-mean compensation of flagged tiles, added to out / lse in place
     constexpr bool DENSE = MODE == 3;          // online softmax over every block: no list, no flags
     constexpr bool FALLBACK = MODE == 1 || DENSE;    // the offset comes from a sweep; MODE 1: of flagged tiles, over their lists
@@ -172,13 +177,13 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
     // adjacent tile numbers are adjacent query tiles of one head: their kv lists overlap in L2
     const int qb = tile % a.nq, h = tile / a.nq;
     const int th_idx = qb * a.H + h;
-    if (MODE == 1 || COMPENSATE) {
-        if (a.flags[th_idx] == 0) return false;    // uniform over the CTA, before anything is allocated
+    if ((MODE == 1 || COMPENSATE) && !a.walk) {
+        if (a.flags[th_idx] == 0) return TILE_DONE;    // uniform over the CTA, before anything is allocated
     }
     // The tile's first global loads do not depend on one another: the list length, the first window of block ids (load
     // warps) and this row's offset (softmax warps) are requested here (in the fallback modes: once the tile is known to be
-    // flagged), before the status check, the barrier set-up and the tensor-memory allocation, whose latencies they then
-    // share instead of following them.
+    // flagged), before the barrier set-up and the tensor-memory allocation, whose latencies they then share instead of
+    // following them.
     const int n64_early = COMPENSATE ? 0 : DENSE ? a.nb : __ldg(a.counts + th_idx);
     int win_early = 0;
     float m_early = 0.f;
@@ -193,8 +198,6 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
     } else if (warp < NSOFT / 32) {
         if (!FALLBACK) m_early = a.offset[((size_t)qb * BM + 32 * (warp & 3) + lane) * a.H + h];
     }
-    // a wait has given up earlier (the status word is set until the host reads it): do not start more work
-    if (*reinterpret_cast<volatile int*>(a.status) != 0) return false;
 
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t base = smem_u32(smem_raw);
@@ -205,6 +208,7 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
     float* mass_rows = reinterpret_cast<float*>(smem_raw + SMEM_MASS);
 
     if (tid == 0) {
+        const int earlier = *reinterpret_cast<volatile int*>(a.status);      // (on its way during the set-up)
         if (base & 1023u) atomicCAS(a.status, 0, 901);   // the swizzled tiles need a 1024-byte aligned base
         if (again) {
             // a CTA that walks a list of tiles makes its barriers anew for every tile
@@ -229,8 +233,9 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
         mbar_init(smem_u32(&ctl->flagbar), 4);
         mbar_init(smem_u32(&ctl->lbar), NSOFT);
         mbar_init(smem_u32(&ctl->sweepbar), 1);
-        ctl->abort = (base & 1023u) ? 1 : 0;
+        ctl->abort = (base & 1023u) || earlier ? 1 : 0;
         ctl->redo = 0;
+        ctl->stop = ctl->abort;
         mbar_fence_init();
         fence_proxy_async_smem();
     }
@@ -243,6 +248,12 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = ctl->tmem_base;
+    if (ctl->stop) {
+        // A wait has given up earlier (the status word is set until the host reads it): no more work is started. One thread reads
+        // the word, which may change at any time: threads that read it each for themselves could part here.
+        if (warp == MMA_WARP) tmem_dealloc(tmem, TMEM_COLS);
+        return TILE_STOP;
+    }
 
     const int n64 = n64_early;
     const int n = DENSE ? last - first : (n64 + 1) >> 1;      // exact iterations: pairs of 64-token blocks
@@ -868,7 +879,8 @@ __device__ __forceinline__ bool attention_tile(const CUtensorMap& tmQ, const CUt
         tc_fence_after();
         tmem_dealloc(tmem, TMEM_COLS);
     }
-    return DENSE && sample && ctl->redo != 0;
+    // (past the barrier nothing of this tile writes them, and the next tile's set-up comes after another one)
+    return *abort_flag ? TILE_STOP : DENSE && sample && ctl->redo != 0 ? TILE_AGAIN : TILE_DONE;
 }
 
 template <int MODE>
@@ -933,7 +945,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             }
         __syncthreads();
         for (int t = 0; lead + t * grid < count; ++t) {
-            attention_tile<MODE>(tmQ, tmK, tmV, tmKm, tmVm, tmKr, tmVr, a, mine[t], again, false);
+            if (attention_tile<MODE>(tmQ, tmK, tmV, tmKm, tmVm, tmKr, tmVr, a, mine[t], again, false) == TILE_STOP) return;
             again = true;
             __syncthreads();
         }
@@ -990,7 +1002,9 @@ dense_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
             }
         }
         if (again) __syncthreads();
-        redo = attention_tile<3>(tmQ, tmK, tmV, tmK, tmV, tmK, tmV, a, tile, again, !redo, first, last, part);
+        const TileEnd end_of_tile = attention_tile<3>(tmQ, tmK, tmV, tmK, tmV, tmK, tmV, a, tile, again, !redo, first, last, part);
+        if (end_of_tile == TILE_STOP) break;
+        redo = end_of_tile == TILE_AGAIN;
     }
     launch_dependents();
 }

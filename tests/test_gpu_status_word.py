@@ -53,3 +53,50 @@ def test_self_test_rejects_limits_out_of_range():
     assert lib.es_selftest_wait_timeout(0, None) < 0 and "limit" in N.last_error()
     assert lib.es_selftest_wait_timeout(10 ** 6, None) < 0
     assert N.device_status() == 0
+
+
+def _calls(L, H, cut):
+    """{name: call on fresh outputs -> outputs} for the attention kernels, with every tile flagged."""
+    from self_trainable_or_free_attn_b200 import _native as N, backends
+    K, lib = backends.kernels(backends.resolve("auto", DEV)), N.load()
+    g = torch.Generator(device=DEV).manual_seed(L)
+    q, k, v = (torch.randn(L, H, 128, device=DEV, generator=g).to(torch.bfloat16) for _ in range(3))
+    nq, nb = -(-L // 128), -(-L // 64)
+    km, vm = (torch.randn(nb, H, 128, device=DEV, generator=g).to(torch.bfloat16) for _ in range(2))
+    counts = torch.full((nq, H), nb, device=DEV, dtype=torch.int32)
+    blocks = torch.arange(nb, device=DEV, dtype=torch.int32).expand(nq, H, nb).contiguous()
+    ones = torch.ones(nq, H, device=DEV, dtype=torch.int32)
+    keep = (torch.rand(H, nq, nb, device=DEV, generator=g) < 0.5).to(torch.uint8)
+
+    def fresh(fn):
+        def call():
+            out, lse = torch.full_like(q, 7.0), torch.full((nq * 128, H), 5.0, device=DEV)
+            fn(out, lse)
+            return out, lse
+        return call
+
+    if cut:
+        assert lib.es_dense_scratch_bytes(L, H) > 0
+        return {"dense": fresh(lambda out, lse: K.dense_attention(q, k, v, out, lse))}
+    return {"whole": fresh(lambda out, lse: N.check(lib.es_dense_attention(
+                q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), L, H, N.stream_ptr()), "dense")),
+            "exact": fresh(lambda out, lse: K.exact_fallback(q, k, v, out, counts, blocks, lse, ones)),
+            "compensate": fresh(lambda out, lse: K.compensate_fallback(q, km, vm, keep, lse, out, ones))}
+
+
+# 100 heads: a CTA of the fallback kernels has several tiles to leave out
+@pytest.mark.parametrize("L,H,cut", [(1560, 12, False), (300, 100, False)])
+def test_no_tile_is_started_while_the_word_is_set(L, H, cut):
+    """The word is set before the launch: a CTA that would do several tiles leaves before its first, as one, and the next call after the
+    word has been read gives the same bits as one before."""
+    from self_trainable_or_free_attn_b200 import _native as N
+    calls = _calls(L, H, cut)
+    good = {name: call() for name, call in calls.items()}
+    assert N.device_status() == 0
+    N.check(N.load().es_selftest_wait_timeout(2000, N.stream_ptr()), "selftest")
+    for name, call in calls.items():
+        out, lse = call()
+        assert bool((out == 7.0).all()) and bool((lse == 5.0).all()), name
+    assert N.device_status() != 0 and N.device_status() == 0
+    for name, call in calls.items():
+        assert all(torch.equal(x, y) for x, y in zip(call(), good[name])), name
