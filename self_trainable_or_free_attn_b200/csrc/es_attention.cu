@@ -1016,6 +1016,8 @@ dense_merge_kernel(const AttnArgs a, const DenseSplit d) {
     constexpr int N4 = MERGE_COLS / 4, AT_ONCE = 4;
     const int t = blockIdx.x, x0 = t * d.n, x1 = x0 + d.n, trow = threadIdx.x;
     wait_prerequisites();
+    // a wait has given up: pieces may be missing, and what the scratch holds in their place is nothing (needed before the stores only)
+    const int stopped = *reinterpret_cast<volatile int*>(a.status);
     const int tile = d.whole + t, qb = tile % a.nq, h = tile / a.nq, row = qb * BM + trow;
     int c = (int)((unsigned)x0 * (unsigned)d.ctas / (unsigned)d.line);        // the first CTA with a piece of the tile
     while (c > 0 && d.edge(c) > x0) --c;
@@ -1067,6 +1069,7 @@ dense_merge_kernel(const AttnArgs a, const DenseSplit d) {
         }
         M = Mn;
     }
+    if (stopped != 0) return;
     if (M == -INFINITY) M = 0.f;
     const bool valid = row < a.L;
     if (blockIdx.y == 0) a.lse[(size_t)row * a.H + h] = valid ? M + log2f(l) : 1e30f;

@@ -84,8 +84,8 @@ def _calls(L, H, cut):
             "compensate": fresh(lambda out, lse: K.compensate_fallback(q, km, vm, keep, lse, out, ones))}
 
 
-# 100 heads: a CTA of the fallback kernels has several tiles to leave out
-@pytest.mark.parametrize("L,H,cut", [(1560, 12, False), (300, 100, False)])
+# 100 heads: a CTA of the fallback kernels has several tiles to leave out; cut tiles have no pieces to be merged then
+@pytest.mark.parametrize("L,H,cut", [(1560, 12, False), (300, 100, False), (1560, 12, True), (4096, 1, True)])
 def test_no_tile_is_started_while_the_word_is_set(L, H, cut):
     """The word is set before the launch: a CTA that would do several tiles leaves before its first, as one, and the next call after the
     word has been read gives the same bits as one before."""
