@@ -79,10 +79,10 @@ int es_dense_attention_split(const void* q, const void* k, const void* v, void* 
 
 /* Online-softmax attention over the block list for the tiles whose flag is set; writes out and lse of those tiles.
  * Replaces echosparse/kernels/triton_ops.py:237 `exact_fallback(q, k, v, out, counts, blocks, lse, flags)`.
- * tile_scratch: device scratch of ceil(L / 128) * H + 1 int32, or NULL. With it there is one CTA per SM and they share the
- * flagged tiles out among themselves (this version finds them without writing to the scratch); without it one CTA per tile is
- * launched and tests its own flag, which costs more than the work when a fraction of a percent of the tiles is flagged. The
- * results are the same. */
+ * tile_scratch: any pointer that is not null (it is neither read nor written: callers of earlier versions pass scratch there,
+ * others may pass `flags` again), or NULL. Not null: there is one CTA per SM and they share the flagged tiles out among
+ * themselves; NULL: one CTA per tile is launched and tests its own flag, which costs more than the work when a fraction of a
+ * percent of the tiles is flagged. The results are the same. */
 int es_exact_fallback(const void* q, const void* k, const void* v, void* out, const int32_t* counts,
                       const int32_t* blocks, int32_t nk, float* lse, const int32_t* flags, int32_t L, int32_t H,
                       int32_t* tile_scratch, void* stream);

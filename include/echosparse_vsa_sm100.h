@@ -159,7 +159,8 @@ int es_vsa_tier_unpool(const float* tok, const float* mid, const float* tail, co
  * rows stays <= max_slots. tasks [(BH * NB + max_slots), 4] = {row, first edge, end edge, slot} (split chunks first, slot =
  * task index, then one direct task with slot -1 per other row); merges [max(1, min(BH * NB, max_slots / 2)), 4] = {row, first
  * slot, chunks, 0}; info [8] = tasks, split rows, split slots, rows, eligible rows, eligible <= budget, threshold without the
- * per-head term, W. All counts stay on the device. Replaces `split_plan` (csrc/vsa/vsa2_api.cpp:464-520, csrc/vsa/split.cu:33-110). */
+ * per-head term, W. All counts stay on the device. workspace: es_vsa_split_plan_workspace_bytes(BH, NB) bytes, NULL where that is
+ * 0. Replaces `split_plan` (csrc/vsa/vsa2_api.cpp:464-520, csrc/vsa/split.cu:33-110). */
 long long es_vsa_split_plan_workspace_bytes(int32_t BH, int32_t NB);
 int es_vsa_split_plan(const int32_t* ptr, int32_t BH, int32_t NB, int32_t chunk, int32_t max_slots, int32_t min_len,
                       double rel_mean, double tail_frac, int32_t resident, int32_t budget, int32_t* tasks, int32_t* merges,

@@ -6,7 +6,6 @@ Every function launches hand-written CUDA through the C ABI on torch's current s
 caller passes. Shapes and dtypes are checked with `assert`, as in the reference; there is no Triton and no CPU path.
 """
 import math
-import threading
 
 import torch
 
@@ -132,28 +131,6 @@ def sparse_attention(q, k, v, k_mean, v_mean, skip_bits, out, counts, blocks, of
     return out
 
 
-_scratch = threading.local()
-_SCRATCH_SIZES = 8
-
-
-def _tile_list_scratch(flags, stream):
-    """Device scratch that the C ABI asks for where flagged tiles are walked (one int32 per tile and one more; the kernels find the
-    tiles by themselves now and leave it alone). A call on another stream or from another thread has scratch of its own. A thread keeps the last few
-    (0.6 us of the host a call, a tensor per call 1.5 and its release: a step of 4,152 tokens 162 -> 170 us with the latter); what it
-    drops, the allocator gives out again in the order of the stream it was used on. A graph outlives that order: a captured call
-    takes its scratch from the graph's pool, and the graph keeps it."""
-    if torch.cuda.is_current_stream_capturing():
-        return torch.empty(flags.numel() + 1, device=flags.device, dtype=torch.int32)
-    pool = _scratch.__dict__
-    key = (flags.device, flags.numel(), stream)
-    buf = pool.get(key)
-    if buf is None:
-        if len(pool) >= _SCRATCH_SIZES:
-            pool.clear()
-        buf = pool[key] = torch.empty(flags.numel() + 1, device=flags.device, dtype=torch.int32)
-    return buf
-
-
 @_timed
 def dense_attention(q, k, v, out, lse):
     """Online-softmax attention over every block. q, k, v, out: (L, H, 128) bf16; lse: (nq * 128, H) float32, log2."""
@@ -176,11 +153,10 @@ def exact_fallback(q, k, v, out, counts, blocks, lse, flags):
     assert hd == D
     _cuda_bf16(q, k, v, out)
     _lists(L, H, counts, blocks)
-    stream = N.stream_ptr()
-    scratch = _tile_list_scratch(flags, stream)
+    # (the flags again for the ABI's `tile_scratch`, which is a switch: CTAs share the flagged tiles out)
     N.check(N.load().es_exact_fallback(N.ptr(q), N.ptr(k), N.ptr(v), N.ptr(out), N.ptr(counts), N.ptr(blocks),
                                        blocks.shape[-1], N.ptr(lse), N.ptr(flags), L, H,
-                                       N.ptr(scratch), stream), "exact_fallback")
+                                       N.ptr(flags), N.stream_ptr()), "exact_fallback")
 
 
 @_timed
@@ -190,10 +166,8 @@ def compensate_fallback(q, k_mean, v_mean, keep, lse, out, flags):
     _cuda_bf16(q, k_mean, v_mean, out)
     nq, nb = _cdiv(L, BM), _cdiv(L, BK)
     assert keep.shape == (H, nq, nb) and keep.dtype == torch.uint8 and keep.is_contiguous()
-    stream = N.stream_ptr()
-    scratch = _tile_list_scratch(flags, stream)
     N.check(N.load().es_compensate_fallback(N.ptr(q), N.ptr(k_mean), N.ptr(v_mean), N.ptr(keep), N.ptr(lse), N.ptr(out),
-                                            N.ptr(flags), L, H, N.ptr(scratch), stream),
+                                            N.ptr(flags), L, H, N.ptr(flags), N.stream_ptr()),
             "compensate_fallback")
 
 
