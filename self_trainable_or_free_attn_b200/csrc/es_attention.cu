@@ -1024,9 +1024,8 @@ dense_merge_kernel(const AttnArgs a, const DenseSplit d) {
     while (d.edge(c + 1) <= x0) ++c;
     const int next = d.edge(c + 1);
     if (next >= x1) return;                               // one CTA did the whole tile
-    // pieces c, c + 1, ..: the first is in its CTA's second slot if the CTA's stretch starts at or before the tile's first
-    // iteration, the others, which start inside the tile, are in the first
-    const float* p = d.part + (size_t)(2 * c + (d.edge(c) <= x0)) * PART_FLOATS;
+    // pieces c, c + 1, ..: the first, which starts the tile, is in its CTA's second slot, the others are in the first
+    const float* p = d.part + (size_t)(2 * c + 1) * PART_FLOATS;
     float M = -INFINITY, l = 0.f, r = 0.f;
     float4 o[N4];
 #pragma unroll
@@ -1121,18 +1120,18 @@ static DenseSplit plan_dense(int tiles, int nb, int sms) {
     DenseSplit d{};
     d.n = (nb + 1) / 2;
     const int waves = tiles / sms, rest = tiles % sms;
-    int best = (waves + (rest > 0)) * (d.n + PIECE_COST) * 19 / 20;       // cut only where that saves a twentieth
+    long long best = 19ll * (waves + (rest > 0)) * (d.n + PIECE_COST) / 20;       // cut only where that saves a twentieth
     if (rest == 0 || 2ll * sms * sms * d.n >= 1ll << 32) return d;
     const int pieces = std::min(sms / rest, d.n);
     if (pieces > 1) {
-        const int t = waves * (d.n + PIECE_COST) + (d.n + pieces - 1) / pieces + PIECE_COST + MERGE_FEW;
+        const long long t = (long long)waves * (d.n + PIECE_COST) + (d.n + pieces - 1) / pieces + PIECE_COST + MERGE_FEW;
         if (t < best) {
             best = t;
             d.whole = waves * sms; d.line = rest * d.n; d.ctas = rest * pieces;
         }
     }
     const int lead = std::max(waves - 1, 0), cut = tiles - lead * sms, ctas = std::min(sms, cut * d.n);
-    const int t = lead * (d.n + PIECE_COST) + (cut * d.n + ctas - 1) / ctas + 2 * PIECE_COST + MERGE_MANY;
+    const long long t = (long long)lead * (d.n + PIECE_COST) + (cut * d.n + ctas - 1) / ctas + 2 * PIECE_COST + MERGE_MANY;
     if (t < best) { d.whole = lead * sms; d.line = cut * d.n; d.ctas = ctas; }
     return d;
 }

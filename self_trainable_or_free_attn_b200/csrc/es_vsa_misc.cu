@@ -1160,7 +1160,7 @@ extern "C" int es_vsa_row_topk(const void* scores, int32_t NB, int32_t bh0, int3
     t.NB = NB; t.W = (NB + 31) / 32; t.bh0 = bh0; t.budget = (long long)NB * K;
     t.q2k_ptr = q2k_ptr; t.q2k_idx = q2k_idx; t.k2q_ptr = k2q_ptr; t.k2q_idx = k2q_idx;
     int* w = static_cast<int*>(workspace);
-    w += (size_t)bh_count * 4;                         // (unused)
+    w += (size_t)bh_count * 4;                         // its thresholds, which rows here have none of
     t.gtcnt = w; w += (size_t)bh_count * NB;
     t.eqcnt = w; w += (size_t)bh_count * NB;
     t.eqbase = w; w += (size_t)bh_count * NB;

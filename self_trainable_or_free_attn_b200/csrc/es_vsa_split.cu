@@ -28,7 +28,7 @@ struct PlanArgs {
     int BH, NB, chunk, max_slots, min_len, resident, budget;
     double rel_mean, tail_frac;
     int *tasks, *merges, *info;
-    int* work;            // [3 * NR] chunk counts, (unused), split flags
+    int* work;            // [2 * NR] chunk counts, split flags (not used where rows are in registers)
 };
 
 // PER: rows of a thread where they fit its registers (8 for up to 8,192 rows; all their loads are on their way together and nothing
@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(1024) split_plan_kernel(const PlanArgs a) {
     const int tid = threadIdx.x, NR = a.BH * a.NB;
     const int per = (NR + 1023) / 1024, lo = min(tid * per, NR), hi = min(lo + per, NR);
     int* cnt = a.work;
-    int* flag = a.work + 2 * NR;
+    int* flag = a.work + NR;
     // exclusive prefix over the threads, the total in s_total: shuffles and two barriers (20 barriers a scan in shared memory, five
     // scans: 20.5 us a plan of 6,144 rows, 16.2 with these, 12.8 with the rows in registers as well)
     auto scan = [&](int v) -> int {
@@ -235,15 +235,18 @@ static int launch_merge(const MergeArgs& a, int n_merge_cap, int D, int dtype, c
 using namespace es;
 using namespace es::vsa;
 
+static bool plan_in_registers(int BH, int NB) { return (long long)BH * NB <= 8 * 1024; }
+
 extern "C" long long es_vsa_split_plan_workspace_bytes(int32_t BH, int32_t NB) {
-    return BH > 0 && NB > 0 ? 3LL * BH * NB * 4 : 0;
+    return BH > 0 && NB > 0 && !plan_in_registers(BH, NB) ? 2LL * BH * NB * 4 : 0;
 }
 
 extern "C" int es_vsa_split_plan(const int32_t* ptr, int32_t BH, int32_t NB, int32_t chunk, int32_t max_slots,
                                  int32_t min_len, double rel_mean, double tail_frac, int32_t resident, int32_t budget,
                                  int32_t* tasks, int32_t* merges, int32_t* info, void* workspace, void* stream) {
-    if (!ptr || !tasks || !merges || !info || !workspace) return set_error(-1, "es_vsa_split_plan: null pointer");
+    if (!ptr || !tasks || !merges || !info) return set_error(-1, "es_vsa_split_plan: null pointer");
     if (BH <= 0 || NB <= 0) return set_error(-1, "es_vsa_split_plan: BH and NB must be positive");
+    if (!workspace && es_vsa_split_plan_workspace_bytes(BH, NB) > 0) return set_error(-1, "es_vsa_split_plan: null workspace");
     if (chunk < 1 || max_slots < 0) return set_error(-1, "es_vsa_split_plan: chunk >= 1 and max_slots >= 0");
     if (min_len < chunk + 1) return set_error(-1, "es_vsa_split_plan: min_len must be at least chunk + 1");
     if (resident < 1 || budget < 0 || rel_mean < 0.0 || tail_frac < 0.0)
@@ -251,7 +254,7 @@ extern "C" int es_vsa_split_plan(const int32_t* ptr, int32_t BH, int32_t NB, int
     if (((uintptr_t)tasks | (uintptr_t)merges) & 15) return set_error(-1, "es_vsa_split_plan: tasks and merges must be 16-byte aligned");
     PlanArgs a{ptr, BH, NB, chunk, max_slots, min_len, resident, budget, rel_mean, tail_frac, tasks, merges, info,
                static_cast<int*>(workspace)};
-    if ((long long)BH * NB <= 8 * 1024) split_plan_kernel<8><<<1, 1024, 0, (cudaStream_t)stream>>>(a);
+    if (plan_in_registers(BH, NB)) split_plan_kernel<8><<<1, 1024, 0, (cudaStream_t)stream>>>(a);
     else split_plan_kernel<0><<<1, 1024, 0, (cudaStream_t)stream>>>(a);
     ES_CHECK_LAUNCH("split_plan_kernel");
     return 0;
