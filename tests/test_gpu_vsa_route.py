@@ -38,3 +38,20 @@ def test_router_scores(pool, nb):
         got = ops.router_scores(qr, kr, cnt.cuda(), pool, ops.ROW_NORMS[norm]).cpu()
         want = R.psp_scores(q, k, cnt, pool, norm)
         assert (got - want).abs().max() <= 1e-3 * want.abs().max()
+
+
+@pytest.mark.parametrize("pool", [1, 2, 4, 8, 16, 32, 64])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_router_scores_of_128_columns(pool, dtype):
+    """At 128 columns the probabilities take the place of the Q tile. Both types, every group size; several key tiles."""
+    from self_trainable_or_free_attn_b200.vsa import ops
+    g = torch.Generator().manual_seed(pool)
+    nb = 17 if pool < 4 else 33
+    cnt = torch.randint(1, 65, (nb,), generator=g, dtype=torch.int32)
+    valid = R.token_valid(cnt, nb * 64)[None, None, :, None]
+    q, k = [(torch.randn(1, 2, nb * 64, 128, generator=g) * valid).to(dtype) for _ in range(2)]
+    for norm in ("paper", "valid_groups"):
+        qr, kr = ops.pool_fwd(q.cuda(), k.cuda(), k.cuda(), cnt.cuda(), pool)[:2]
+        got = ops.router_scores(qr, kr, cnt.cuda(), pool, ops.ROW_NORMS[norm]).cpu()
+        want = R.psp_scores(q, k, cnt, pool, norm, round_to=dtype)
+        assert (got - want).abs().max() <= 1e-3 * want.abs().max()
