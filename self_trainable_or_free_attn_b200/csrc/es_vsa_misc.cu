@@ -5,6 +5,7 @@
 // passes, mma.sync tiles; integer stages (top-k, CSR) are exact and deterministic.
 #include <cooperative_groups.h>
 
+#include <atomic>
 #include <string>
 
 #include "es_api_internal.h"
@@ -1009,6 +1010,27 @@ extern "C" int es_vsa_router_scores(const void* qr, const void* kr, const float*
     return launch_router<1>(a, D, dtype, bh_count, (cudaStream_t)stream);
 }
 
+// Clusters of topk_kernel that the current device runs at once (a cluster's CTAs share a GPC, so it is fewer than SMs / CTAs), asked
+// for once per device; 0 where that fails.
+static int topk_clusters_at_once() {
+    static std::atomic<int> known[64];                   // 1 + the count
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    int n = known[dev].load(std::memory_order_relaxed) - 1;
+    if (n >= 0) return n;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = SEL_CTAS; attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(SEL_CTAS); cfg.blockDim = dim3(1024); cfg.attrs = &attr; cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, topk_kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();                              // the other path needs no clusters at once
+        n = 0;
+    }
+    known[dev].store(n + 1, std::memory_order_relaxed);
+    return n;
+}
+
 extern "C" long long es_vsa_topk_workspace_bytes(int32_t bh_count, int32_t NB) {
     if (bh_count <= 0 || NB <= 0) return 0;
     const long long W = (NB + 31) / 32;
@@ -1040,11 +1062,11 @@ extern "C" int es_vsa_global_topk(const float* scores, int32_t NB, int32_t bh0, 
     a.colcnt = w; w += (size_t)bh_count * NB;
     a.selbits = reinterpret_cast<uint32_t*>(w);
     cudaStream_t st = (cudaStream_t)stream;
-    // One launch where it is gaps and launches that count and every cluster has its place at once (eight SMs each, 18 on 148); beyond,
-    // the stages are launches of their own, whose rows and columns go to all SMs. One call after the other, us, one launch / seven:
-    // 64 blocks x 12 heads 21.0 / 26.7, 256 x 12 26.3 / 32.4, 400 x 8 43.5 / 42.9 (and six launches of the host), 624 x 12 74.5 /
-    // 66.4, 1,600 x 1 324 / 171, 64 x 24 37.5 / 28.5.
-    if (NB <= 384 && bh_count <= 18) {
+    // One launch where all clusters run at once (15 on a B200) and a warp has one row; beyond, the stages are launches of their own,
+    // whose rows and columns go to all SMs. Device time of one call after the other in a graph, us, one launch / seven: 64 blocks x 15
+    // heads 20.8 / 24.8, x 16 35.6 / 26.3 (a second round of clusters); 256 x 12 26.0 / 30.2, x 15 26.0 / 30.6, x 16 49.6 / 33.2;
+    // 272 x 12 34.6 / 35.4, 288 x 12 36.1 / 35.8, 304 x 12 38.3 / 37.4, 384 x 12 42.0 / 40.6, 624 x 12 74.5 / 66.4, 1,600 x 1 324 / 171.
+    if (NB <= 256 && bh_count <= topk_clusters_at_once()) {
         topk_kernel<<<dim3(SEL_CTAS, bh_count), 1024, 0, st>>>(a);
         ES_CHECK_LAUNCH("topk_kernel");
         return 0;

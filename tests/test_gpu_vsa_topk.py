@@ -6,9 +6,9 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
-# one launch: one block; a word and one column; rows of 256 warps and one more; the largest. Seven: one block more, more rows than
-# threads, more heads than clusters at once
-@pytest.mark.parametrize("nb,H", [(1, 3), (33, 18), (257, 3), (384, 2), (385, 2), (1100, 3), (33, 19)])
+# one launch: one block; a word and one column; a row for each of 256 warps. Seven: one block more and a word and one more, more rows
+# than threads, more heads than clusters at once (15 on a B200; 19 on no device of 148 SMs)
+@pytest.mark.parametrize("nb,H", [(1, 3), (33, 15), (33, 16), (33, 18), (256, 15), (257, 3), (384, 2), (385, 2), (1100, 3), (33, 19)])
 @pytest.mark.parametrize("kind", ["random", "ties", "zeros"])
 def test_lists_match_a_stable_sort(nb, H, kind):
     """Score descending, ties to the smaller flat index: the lists are whole numbers and have to be equal."""
@@ -29,3 +29,37 @@ def test_lists_match_a_stable_sort(nb, H, kind):
             want = torch.cat([cnt.cumsum(1) - cnt, cnt.sum(1, keepdim=True)], 1) + budget * torch.arange(B * H, device=DEV)[:, None]
             assert torch.equal(ptr.reshape(B * H, nb + 1).long(), want)
             assert torch.equal(idx[: B * H * budget].long(), m.nonzero()[:, 2])
+
+
+@pytest.mark.parametrize("nb,H,launches", [(256, 2, 1), (257, 2, 7), (33, 19, 7)])
+def test_one_launch_only_where_all_clusters_run_at_once(nb, H, launches):
+    """A head is a cluster of eight CTAs: those past what the device holds would wait for a second round, 50 us instead of 33."""
+    from self_trainable_or_free_attn_b200 import _native as N
+    from self_trainable_or_free_attn_b200.vsa import ops
+    s = torch.rand(1, H, nb, nb, device=DEV)
+    n = N.launch_count()
+    ops.global_topk(s, nb)
+    assert N.launch_count() - n == launches
+
+
+def test_sixteen_heads_are_no_slower_in_one_call_than_in_two():
+    """16 heads do not fit a B200 as clusters at once. In one launch they took 50 us against twice 26 for eight heads each; a launch per
+    stage takes 33. Times are noisy: only a call as slow as two rounds is a fault."""
+    from self_trainable_or_free_attn_b200.vsa import ops
+    s = torch.rand(1, 16, 256, 256, device=DEV)
+
+    def us(x):
+        ops.global_topk(x, 4096)
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            for _ in range(20):
+                ops.global_topk(x, 4096)
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        best = float("inf")
+        for _ in range(5):
+            a.record(); g.replay(); b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b) * 50)
+        return best
+
+    assert us(s) < 1.7 * us(s[:, :8].contiguous())
