@@ -98,23 +98,30 @@ struct RouterArgs {
 // taken from a shared-memory copy of the probabilities in a fixed order (reproducible). GT: G as a compile-time constant for
 // R = 32, 16 and 8 (0: any power of two), so that the sums read 8 or 16 bytes at a time in the same order; the validity of a
 // tile's 64 keys is found once by 64 threads and handed round as two words (with every thread testing its 16 columns, integer
-// divisions were two thirds of the kernel). NB = 512, R = 16, 12 heads: LSE 57 us (137 before), scores
-// 91 us (225); NB = 624: 84 us (191) and 128 us (537; 202 with three CTAs per SM).
-template <int D> constexpr bool ROUTER_P_OVER_Q = TB * D * 2 >= 64 * 64 * 4;
-template <typename T, int D, int MODE, int GT>
-__global__ void __launch_bounds__(128, 4) router_kernel(const RouterArgs a) {
+// divisions were two thirds of the kernel). NB = 512, R = 16, 12 heads: LSE 55 us (137 before), scores
+// 95 us (225); NB = 624: 86 us (191) and 130 us (537; 222 with three CTAs per SM). Rows of the probabilities are 68 floats apart; 64
+// with chunks exchanged by the row was up to 23 % slower (R = 4, 24 blocks: 33 / 41 us), one to three percent faster at R = 16.
+template <int D, int MODE> struct RouterSmem {
+    static constexpr int SP = 68;                                        // MODE 1: row stride of the [64][SP] probabilities
+    static constexpr uint32_t TILE = TB * D * 2, P_BYTES = 64 * SP * 4;
+    static constexpr bool OVER_Q = MODE == 1 && D == 128;
+    static constexpr uint32_t Q_ROOM = OVER_Q ? P_BYTES : TILE;
+    static constexpr uint32_t VALID = Q_ROOM + 2 * TILE, P = OVER_Q ? 0 : VALID + 16;
+    static constexpr uint32_t BYTES = VALID + 16 + (MODE == 1 && !OVER_Q ? P_BYTES : 0);
+};
+template <typename T, int D, int MODE, int GT, int CTAS>
+__global__ void __launch_bounds__(128, CTAS) router_kernel(const RouterArgs a) {
     extern __shared__ __align__(128) uint8_t smem[];
-    constexpr uint32_t TILE = TB * D * 2;
+    using S = RouterSmem<D, MODE>;
+    constexpr uint32_t TILE = S::TILE;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int qt = blockIdx.x, bh = a.bh0 + blockIdx.y;
-    const uint32_t sQ = smem_addr(smem), sK = sQ + TILE;                 // K: two stages
-    uint32_t* sValid = reinterpret_cast<uint32_t*>(smem + 3 * TILE);     // [2 stages][2]: bit r = key r of the tile is valid
-    // MODE 1: [64][64] probabilities, in the place of the Q tile (its fragments are in registers) where that is as large, so that
-    // four CTAs fit an SM. At 39 tiles x 12 heads three leave 24 of 468 CTAs to a second round.
-    float* sP = reinterpret_cast<float*>(smem + (ROUTER_P_OVER_Q<D> ? 0 : 3 * TILE + 16));
-    // element (r, c): a row's chunks of 4 are exchanged by the row, so that neither the fragments' pairs (four rows to a half warp)
-    // nor the chunks read back meet in a bank
-    auto at_p = [&](int r, int c) { return sP + r * 64 + (((c >> 2) ^ ((r & 3) << 1)) << 2) + (c & 3); };
+    const uint32_t sQ = smem_addr(smem), sK = sQ + S::Q_ROOM;            // K: two stages
+    uint32_t* sValid = reinterpret_cast<uint32_t*>(smem + S::VALID);     // [2 stages][2]: bit r = key r of the tile is valid
+    // MODE 1: probabilities, at D = 128 in the place of the Q tile (its fragments are in registers), so that four CTAs fit an SM. At
+    // 39 tiles x 12 heads three leave 24 of 468 CTAs to a second round.
+    float* sP = reinterpret_cast<float*>(smem + S::P);
+    constexpr int SP = S::SP;
     const int G = GT ? GT : a.G, lg = 31 - __clz(G);                     // R divides 64: G is a power of two
     auto valid_row = [&](int r) { return r < a.Lr && (r & (G - 1)) * a.R < a.blk_cnt[r >> lg]; };
     const T* q = static_cast<const T*>(a.qr) + ((size_t)bh * a.Lr_pad + (size_t)qt * TB) * D;
@@ -129,7 +136,9 @@ __global__ void __launch_bounds__(128, 4) router_kernel(const RouterArgs a) {
         const float* lse = a.lse2 + (size_t)bh * a.Lr_pad + (size_t)qt * TB;
         ls0 = lse[r0]; ls1 = lse[r1];
     }
-    const bool qv0 = MODE == 1 && valid_row(qt * TB + r0), qv1 = MODE == 1 && valid_row(qt * TB + r1);
+    // validity of the thread's two query rows, found once, or in every tile where keeping it was slower (one to four percent)
+    constexpr bool ONCE = D == 128 || GT == 2 || GT == 4;
+    bool qv0 = MODE == 1 && ONCE && valid_row(qt * TB + r0), qv1 = MODE == 1 && ONCE && valid_row(qt * TB + r1);
     uint32_t qa[D / 16][4];
     for (int kt = 0; kt < nkt; ++kt) {
         const uint32_t sKt = sK + (uint32_t)(kt & 1) * TILE;
@@ -144,7 +153,7 @@ __global__ void __launch_bounds__(128, 4) router_kernel(const RouterArgs a) {
         if (kt == 0) {
 #pragma unroll
             for (int ks = 0; ks < D / 16; ++ks) load_a<D>(sQ, warp * 16, ks, lane, qa[ks]);
-            if (MODE == 1 && ROUTER_P_OVER_Q<D>) __syncthreads();        // the tile's room is the probabilities' from here on
+            if (S::OVER_Q) __syncthreads();                               // the tile's room is the probabilities' from here on
         }
         float s[8][4];
 #pragma unroll
@@ -188,13 +197,14 @@ __global__ void __launch_bounds__(128, 4) router_kernel(const RouterArgs a) {
             m0 = mn0; m1 = mn1;
         } else {
             // probabilities of this key tile -> shared memory, then fixed-order G x G sums
+            if (!ONCE) { qv0 = valid_row(qt * TB + r0); qv1 = valid_row(qt * TB + r1); }
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const int c = i * 8 + 2 * (lane & 3);
-                *reinterpret_cast<float2*>(at_p(r0, c)) =
+                *reinterpret_cast<float2*>(sP + r0 * SP + c) =
                     make_float2((qv0 && kv[i][0]) ? exp2f(s[i][0] * a.scale_log2 - ls0) : 0.f,
                                 (qv0 && kv[i][1]) ? exp2f(s[i][1] * a.scale_log2 - ls0) : 0.f);
-                *reinterpret_cast<float2*>(at_p(r1, c)) =
+                *reinterpret_cast<float2*>(sP + r1 * SP + c) =
                     make_float2((qv1 && kv[i][0]) ? exp2f(s[i][2] * a.scale_log2 - ls1) : 0.f,
                                 (qv1 && kv[i][1]) ? exp2f(s[i][3] * a.scale_log2 - ls1) : 0.f);
             }
@@ -204,24 +214,25 @@ __global__ void __launch_bounds__(128, 4) router_kernel(const RouterArgs a) {
                 const int bi = e >> (6 - lg), bj = e & (per - 1);
                 const int qblk = qt * per + bi, kblk = kt * per + bj;
                 if (qblk < a.NB && kblk < a.NB) {
+                    const float* p0 = sP + bi * G * SP + bj * G;
                     float acc = 0.f;
                     if (GT >= 4) {
 #pragma unroll
                         for (int x = 0; x < GT; ++x)
 #pragma unroll
                             for (int y = 0; y < GT; y += 4) {
-                                const float4 v = *reinterpret_cast<const float4*>(at_p(bi * GT + x, bj * GT + y));
+                                const float4 v = *reinterpret_cast<const float4*>(p0 + x * SP + y);
                                 acc += v.x; acc += v.y; acc += v.z; acc += v.w;
                             }
                     } else if (GT == 2) {
 #pragma unroll
                         for (int x = 0; x < 2; ++x) {
-                            const float2 v = *reinterpret_cast<const float2*>(at_p(bi * 2 + x, bj * 2));
+                            const float2 v = *reinterpret_cast<const float2*>(p0 + x * SP);
                             acc += v.x; acc += v.y;
                         }
                     } else {
                         for (int x = 0; x < G; ++x)
-                            for (int y = 0; y < G; ++y) acc += *at_p(bi * G + x, bj * G + y);
+                            for (int y = 0; y < G; ++y) acc += p0[x * SP + y];
                     }
                     float norm;
                     if (a.row_norm == 1) norm = 1.f / (float)(G * G);
@@ -958,30 +969,43 @@ extern "C" int es_vsa_pool(const void* q, const void* k, const void* v, void* qr
     return 0;
 }
 
+static int sm_count() {
+    int dev = 0, sms = 0;
+    return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? sms : 148;
+}
+
+// A kernel built for one CTA per SM fewer is a few percent faster (more registers), and so are fewer that run at once, but a round more
+// costs far more: the larger number is taken where it saves a round. 12 heads, us, 3 / 4 CTAs per SM at D = 128: scores, 468 CTAs (NB =
+// 624, R = 16) 222 / 130, 456 208 / 125, 768 (two rounds either way) 364 / 408, 600 (4 heads) 859 / 873; LSE, 468 113 / 86, 192 24.8 /
+// 25.9. 4 / 5 at D = 64: scores, 600 761 / 446, 384 80 / 82; LSE, 600 327 / 279, 768 147 / 167.
+template <typename T, int D, int MODE>
+static int launch_router_as(const RouterArgs& a, int bh_count, cudaStream_t st) {
+    constexpr int FEW = D == 128 ? 3 : 4, MANY = FEW + 1;
+    constexpr bool BY_SMEM = D == 128 && MODE == 1;       // one kernel, and three of them where it asks for more shared memory
+    const dim3 grid(a.Lr_pad / TB, bh_count);
+    const long long n = (long long)grid.x * grid.y, sms = sm_count();
+    const bool many = (n + MANY * sms - 1) / (MANY * sms) < (n + FEW * sms - 1) / (FEW * sms);
+    const int smem = (int)RouterSmem<D, MODE>::BYTES + (BY_SMEM && !many ? 12 * 1024 : 0);
+    auto launch = [&](auto few, auto more) -> int {
+        auto kernel = many ? more : few;
+        if (int rc = opt_in_shared_memory((const void*)kernel, smem)) return rc;
+        kernel<<<grid, 128, smem, st>>>(a);
+        ES_CHECK_LAUNCH("router_kernel");
+        return 0;
+    };
+    constexpr int C0 = BY_SMEM ? MANY : FEW;
+    if (a.G == 2) return launch(router_kernel<T, D, MODE, 2, C0>, router_kernel<T, D, MODE, 2, MANY>);
+    if (a.G == 4) return launch(router_kernel<T, D, MODE, 4, C0>, router_kernel<T, D, MODE, 4, MANY>);
+    if (a.G == 8) return launch(router_kernel<T, D, MODE, 8, C0>, router_kernel<T, D, MODE, 8, MANY>);
+    return launch(router_kernel<T, D, MODE, 0, C0>, router_kernel<T, D, MODE, 0, MANY>);
+}
+
 template <int MODE>
 static int launch_router(const RouterArgs& a, int D, int dtype, int bh_count, cudaStream_t st) {
-    const size_t smem = (size_t)3 * TB * D * 2 + 16 + (MODE == 1 && D == 64 ? 64 * 64 * sizeof(float) : 0);
-    const dim3 grid(a.Lr_pad / TB, bh_count);
-#define ROUTER_LAUNCH(TT, DD, GG)                                                                                       \
-    {                                                                                                                   \
-        if (int rc = opt_in_shared_memory((const void*)router_kernel<TT, DD, MODE, GG>, (int)smem)) return rc;          \
-        router_kernel<TT, DD, MODE, GG><<<grid, 128, smem, st>>>(a);                                                    \
-    }
-#define ROUTER_CASE(TT, DD)                          \
-    {                                                \
-        if (a.G == 2) ROUTER_LAUNCH(TT, DD, 2)       \
-        else if (a.G == 4) ROUTER_LAUNCH(TT, DD, 4)  \
-        else if (a.G == 8) ROUTER_LAUNCH(TT, DD, 8)  \
-        else ROUTER_LAUNCH(TT, DD, 0)                \
-    }
-    if (dtype == 0 && D == 128) ROUTER_CASE(__nv_bfloat16, 128)
-    else if (dtype == 0) ROUTER_CASE(__nv_bfloat16, 64)
-    else if (D == 128) ROUTER_CASE(__half, 128)
-    else ROUTER_CASE(__half, 64)
-#undef ROUTER_CASE
-#undef ROUTER_LAUNCH
-    ES_CHECK_LAUNCH("router_kernel");
-    return 0;
+    if (dtype == 0 && D == 128) return launch_router_as<__nv_bfloat16, 128, MODE>(a, bh_count, st);
+    if (dtype == 0) return launch_router_as<__nv_bfloat16, 64, MODE>(a, bh_count, st);
+    if (D == 128) return launch_router_as<__half, 128, MODE>(a, bh_count, st);
+    return launch_router_as<__half, 64, MODE>(a, bh_count, st);
 }
 
 extern "C" int es_vsa_router_lse(const void* qr, const void* kr, float* lse2, const int32_t* blk_cnt, int32_t BH,

@@ -55,3 +55,20 @@ def test_router_scores_of_128_columns(pool, dtype):
         got = ops.router_scores(qr, kr, cnt.cuda(), pool, ops.ROW_NORMS[norm]).cpu()
         want = R.psp_scores(q, k, cnt, pool, norm, round_to=dtype)
         assert (got - want).abs().max() <= 1e-3 * want.abs().max()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("pool", [1, 8, 16, 32])
+def test_router_scores_do_not_depend_on_the_number_of_heads(D, pool):
+    """By the number of CTAs another kernel, or another number of them per SM, is launched: the same sums, so the same bits. On 148 SMs
+    12 tiles x 52 heads = 624 CTAs are one round of five a SM (D = 64) and two of four; 12 x 40 = 480 one of four (D = 128), two of three."""
+    from self_trainable_or_free_attn_b200.vsa import ops
+    g = torch.Generator(device="cuda").manual_seed(pool)
+    nb, H = 12 * pool, 52 if D == 64 else 40
+    cnt = torch.randint(1, 65, (nb,), device="cuda", generator=g, dtype=torch.int32)
+    q, k = (torch.randn(1, H, nb * 64, D, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    qr, kr = ops.pool_fwd(q, k, k, cnt, pool)[:2]
+    assert qr.shape[2] == 12 * 64
+    all_heads = ops.router_scores(qr, kr, cnt, pool)
+    few = ops.router_scores(qr[:, -2:].contiguous(), kr[:, -2:].contiguous(), cnt, pool)
+    assert torch.equal(all_heads[:, -2:], few) and bool(torch.isfinite(all_heads).all())
