@@ -27,20 +27,28 @@ struct UnpoolArgs {
     int L, RM, mid_stride, tail_stride, add_nb;
     int wide;                      // the fp32 tensors are 16-byte, out 8-byte aligned
 };
-// Four columns a lane, D / 4 lanes a row, every row of a block requested before the first is needed. Bound by HBM: 512 blocks x 12
-// heads, D = 128, all four sources: 84 us (two columns a thread and a row at a time: 106).
-template <typename T, int D>
-__global__ void __launch_bounds__(256) tier_unpool_kernel(const UnpoolArgs a) {
-    constexpr int LR = D / 4, GROUPS = 256 / LR, ITER = TB / GROUPS;       // lanes per row, rows per pass, passes
-    const int blk = blockIdx.x, bh = blockIdx.y, c = 4 * (threadIdx.x % LR), grp = threadIdx.x / LR;
+// Four columns a lane, D / 4 lanes a row. A thread's rows follow one another, so that it loads and divides a group's gradient once or
+// twice instead of once a row. TOK: with the tokens' own gradients, all rows of a thread requested before the first is needed;
+// without them there is less to hold, and smaller CTAs write faster (256 threads: 27 instead of 25 us below, 62 instead of 48 where
+// there is only `tail`, D = 64). Bound by HBM. D = 128, bf16, four groups a block, us, before (a row's division each) / here: 512 blocks
+// x 12 heads, tok + mid + tail 59 / 45, mid + tail 55 / 25; 1,500 x 12 160 / 121 and 150 / 61.
+template <bool TOK> constexpr int UNPOOL_THREADS = TOK ? 256 : 128;
+template <typename T, int D, bool TOK>
+__global__ void __launch_bounds__((UNPOOL_THREADS<TOK>), TOK ? (D == 128 ? 4 : 6) : 16) tier_unpool_kernel(const UnpoolArgs a) {
+    constexpr int LR = D / 4, ROWS = TB / (UNPOOL_THREADS<TOK> / LR), QUADS = ROWS / 4;   // lanes per row, rows of a thread; groups have 4 rows or more
+    const int blk = blockIdx.x, bh = blockIdx.y, c = 4 * (threadIdx.x % LR), r0 = threadIdx.x / LR * ROWS;
     const int cnt = a.blk_cnt[blk], R = TB / a.RM;
     auto load4 = [&](const float* p) { return a.wide ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]); };
-    const size_t first = (size_t)bh * a.L + (size_t)blk * TB;
-    float4 tok[ITER];
+    const size_t first = (size_t)bh * a.L + (size_t)blk * TB + r0;
+    float4 tok[ROWS], m[QUADS];
+    if (TOK) {
 #pragma unroll
-    for (int it = 0; it < ITER; ++it) {
-        const int r = it * GROUPS + grp;
-        if (a.tok && r < cnt) tok[it] = load4(a.tok + (first + r) * D + c);
+        for (int i = 0; i < ROWS; ++i)
+            if (r0 + i < cnt) tok[i] = load4(a.tok + (first + i) * D + c);
+    }
+    if (a.mid) {
+#pragma unroll
+        for (int x = 0; x < QUADS; ++x) m[x] = load4(a.mid + ((size_t)bh * a.mid_stride + (size_t)blk * a.RM + (r0 + 4 * x) / R) * D + c);
     }
     float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
     if (a.tail) t = load4(a.tail + ((size_t)bh * a.tail_stride + blk) * D + c);
@@ -50,24 +58,25 @@ __global__ void __launch_bounds__(256) tier_unpool_kernel(const UnpoolArgs a) {
     }
     t.x /= (float)cnt; t.y /= (float)cnt; t.z /= (float)cnt; t.w /= (float)cnt;
 #pragma unroll
-    for (int it = 0; it < ITER; ++it) {
-        const int r = it * GROUPS + grp;
-        uint32_t out[2] = {0u, 0u};
-        if (r < cnt) {
-            float4 x = t;
-            if (a.mid) {
-                const int g = r / R;
-                const float cg = (float)min(cnt - g * R, R);
-                const float4 m = load4(a.mid + ((size_t)bh * a.mid_stride + (size_t)blk * a.RM + g) * D + c);
-                x.x += m.x / cg; x.y += m.y / cg; x.z += m.z / cg; x.w += m.w / cg;
-            }
-            if (a.tok) { x.x += tok[it].x; x.y += tok[it].y; x.z += tok[it].z; x.w += tok[it].w; }
-            out[0] = Elt<T>::pack(x.x, x.y);
-            out[1] = Elt<T>::pack(x.z, x.w);
+    for (int x = 0; x < QUADS; ++x) {
+        float4 base = t;
+        if (a.mid) {
+            const float cg = (float)min(cnt - (r0 + 4 * x) / R * R, R);    // (not positive: no row of the group is below cnt)
+            base.x += m[x].x / cg; base.y += m[x].y / cg; base.z += m[x].z / cg; base.w += m[x].w / cg;
         }
-        uint32_t* dst = reinterpret_cast<uint32_t*>(static_cast<T*>(a.out) + (first + r) * D + c);
-        if (a.wide) *reinterpret_cast<uint2*>(dst) = make_uint2(out[0], out[1]);
-        else { dst[0] = out[0]; dst[1] = out[1]; }
+#pragma unroll
+        for (int i = 4 * x; i < 4 * x + 4; ++i) {
+            uint32_t out[2] = {0u, 0u};
+            if (r0 + i < cnt) {
+                float4 y = base;
+                if (TOK) { y.x += tok[i].x; y.y += tok[i].y; y.z += tok[i].z; y.w += tok[i].w; }
+                out[0] = Elt<T>::pack(y.x, y.y);
+                out[1] = Elt<T>::pack(y.z, y.w);
+            }
+            uint32_t* dst = reinterpret_cast<uint32_t*>(static_cast<T*>(a.out) + (first + i) * D + c);
+            if (a.wide) *reinterpret_cast<uint2*>(dst) = make_uint2(out[0], out[1]);
+            else { dst[0] = out[0]; dst[1] = out[1]; }
+        }
     }
 }
 
@@ -176,10 +185,11 @@ extern "C" int es_vsa_tier_unpool(const float* tok, const float* mid, const floa
     const UnpoolArgs a{tok, mid, tail, add, out, blk_cnt, L, mid_reps, mid_stride, tail_stride, add_nb, aligned(16, tok, mid, tail, add) && aligned(8, out)};
     cudaStream_t st = (cudaStream_t)stream;
     const dim3 grid(L / TB, BH);
-    if (dtype == 0 && D == 128) tier_unpool_kernel<__nv_bfloat16, 128><<<grid, 256, 0, st>>>(a);
-    else if (dtype == 0) tier_unpool_kernel<__nv_bfloat16, 64><<<grid, 256, 0, st>>>(a);
-    else if (D == 128) tier_unpool_kernel<__half, 128><<<grid, 256, 0, st>>>(a);
-    else tier_unpool_kernel<__half, 64><<<grid, 256, 0, st>>>(a);
+    auto launch = [&](auto with, auto without) { (tok ? with : without)<<<grid, tok ? UNPOOL_THREADS<true> : UNPOOL_THREADS<false>, 0, st>>>(a); };
+    if (dtype == 0 && D == 128) launch(tier_unpool_kernel<__nv_bfloat16, 128, true>, tier_unpool_kernel<__nv_bfloat16, 128, false>);
+    else if (dtype == 0) launch(tier_unpool_kernel<__nv_bfloat16, 64, true>, tier_unpool_kernel<__nv_bfloat16, 64, false>);
+    else if (D == 128) launch(tier_unpool_kernel<__half, 128, true>, tier_unpool_kernel<__half, 128, false>);
+    else launch(tier_unpool_kernel<__half, 64, true>, tier_unpool_kernel<__half, 64, false>);
     ES_CHECK_LAUNCH("tier_unpool_kernel");
     return 0;
 }
