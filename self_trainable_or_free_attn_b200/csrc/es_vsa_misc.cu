@@ -729,10 +729,12 @@ __device__ __forceinline__ void store_piece(void* p, const uint32_t (&w)[4], int
     }
 }
 
-// One CTA per (block, bh), 16 bytes a thread and row, four rows of a thread in flight. Bound by HBM: 32,768 tokens x 12 heads,
-// D = 128, a gate per token: 38 us, twelve CTAs per SM (43 with nine).
-template <typename T, int D>
-__global__ void __launch_bounds__(128, 12) fuse_fwd_kernel(const FuseArgs a) {
+// One CTA per (block, bh), 16 bytes a thread and row, four rows of a thread in flight. Bound by HBM. A kernel per gate mode: none and
+// per token need 32 registers, sixteen CTAs per SM; elementwise at D = 128 ten (48 registers: with twelve, 300 blocks x 5 heads 10.3 ->
+// 12.5 us), at D = 64 twelve (ten: 27 -> 29). 32,768 tokens x 12 heads, D = 128, us, one kernel of twelve CTAs / here: per token 40.3 /
+// 35.1, none 37.5 / 34.7, elementwise 55.4 / 54.7.
+template <typename T, int D, int GATE>
+__global__ void __launch_bounds__(128, GATE == 2 && D == 128 ? 10 : 12) fuse_fwd_kernel(const FuseArgs a) {
     constexpr int CH = D / 8, ROWS = 128 / CH;                 // 16-byte pieces per row, rows per pass
     const int blk = blockIdx.x, bh = blockIdx.y, c = 8 * (threadIdx.x % CH), r0 = threadIdx.x / CH;
     const int cnt = a.blk_cnt[blk];
@@ -752,17 +754,17 @@ __global__ void __launch_bounds__(128, 12) fuse_fwd_kernel(const FuseArgs a) {
             uint32_t f[4], gw[4];
             load_piece(static_cast<const T*>(a.of) + row * D + c, f, a.wide);
             float gt = 1.f;
-            if (a.gate_mode == 1) {
+            if (GATE == 1) {
                 gt = Elt<T>::to_float(static_cast<const T*>(a.gate)[row]);
                 if (a.gate_act == 0) gt = tanhf(gt);
-            } else if (a.gate_mode == 2) {
+            } else if (GATE == 2) {
                 load_piece(static_cast<const T*>(a.gate) + row * D + c, gw, a.wide);
             }
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const float2 x = Elt<T>::unpack(f[i]);
                 float gx = gt, gy = gt;
-                if (a.gate_mode == 2) {
+                if (GATE == 2) {
                     const float2 g = Elt<T>::unpack(gw[i]);
                     gx = g.x; gy = g.y;
                     if (a.gate_act == 0) { gx = tanhf(gx); gy = tanhf(gy); }
@@ -1127,7 +1129,17 @@ extern "C" int es_vsa_fuse_fwd(const void* of, const void* oc, const void* gate,
     a.wide = (((uintptr_t)of | (uintptr_t)oc | (uintptr_t)o | (gate_mode == 2 ? (uintptr_t)gate : 0)) & 15) == 0;
     cudaStream_t st = (cudaStream_t)stream;
     const dim3 grid(L / TB, BH);
-    VSA_LAUNCH(fuse_fwd_kernel, grid, 128, 0, a);
+#define FUSE_FWD_CASE(TT, DD)                                                              \
+    {                                                                                      \
+        if (gate_mode == 0) fuse_fwd_kernel<TT, DD, 0><<<grid, 128, 0, st>>>(a);           \
+        else if (gate_mode == 1) fuse_fwd_kernel<TT, DD, 1><<<grid, 128, 0, st>>>(a);      \
+        else fuse_fwd_kernel<TT, DD, 2><<<grid, 128, 0, st>>>(a);                          \
+    }
+    if (dtype == 0 && D == 128) FUSE_FWD_CASE(__nv_bfloat16, 128)
+    else if (dtype == 0) FUSE_FWD_CASE(__nv_bfloat16, 64)
+    else if (D == 128) FUSE_FWD_CASE(__half, 128)
+    else FUSE_FWD_CASE(__half, 64)
+#undef FUSE_FWD_CASE
     ES_CHECK_LAUNCH("fuse_fwd_kernel");
     return 0;
 }
