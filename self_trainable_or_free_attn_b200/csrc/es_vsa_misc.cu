@@ -23,6 +23,7 @@ struct PoolArgs {
     void *qr, *kr, *vr, *qc, *kc, *vc;
     const int* blk_cnt;
     int L, NB, R, G, Lr_pad, NBc_pad;
+    int first;            // tensor of blockIdx.z = 0
 };
 
 //
@@ -31,7 +32,7 @@ struct PoolArgs {
 // tensors one after the other and a few rows at a time 72.3; 100 blocks x 8 heads, D = 64: 3.2, 10.4.
 template <typename T, int D, int RT>
 __global__ void __launch_bounds__(D / 2) pool_kernel(const PoolArgs a) {
-    const int blk = blockIdx.x, bh = blockIdx.y, t = blockIdx.z, c = 2 * threadIdx.x;
+    const int blk = blockIdx.x, bh = blockIdx.y, t = a.first + blockIdx.z, c = 2 * threadIdx.x;
     const int tiles_c = a.NBc_pad, rows_r = a.Lr_pad, R = RT ? RT : a.R, G = TB / R;
     const void* src = t == 0 ? a.q : t == 1 ? a.k : a.v;
     T* dst_r = static_cast<T*>(t == 0 ? a.qr : t == 1 ? a.kr : a.vr);
@@ -950,10 +951,14 @@ extern "C" int es_vsa_pool(const void* q, const void* k, const void* v, void* qr
     if (Lr_pad < NB * G || NBc_pad < NB) return set_error(-1, "es_vsa_pool: padded sizes smaller than the real ones");
     if ((vr || vc) && !v) return set_error(-1, "es_vsa_pool: v outputs without v");
     if (!aligned(4, q, k, v, qr, kr, vr, qc, kc, vc)) return set_error(-1, "es_vsa_pool: tensors must be 4-byte aligned");
-    PoolArgs a{q, k, v, qr, kr, vr, qc, kc, vc, blk_cnt, L, NB, R, G, Lr_pad, NBc_pad};
+    // tensors without outputs at either end have no CTAs (60,000 empty ones: 10 us)
+    const bool out[3] = {qr || qc, kr || kc, vr || vc};
+    const int first = out[0] ? 0 : out[1] ? 1 : 2, last = out[2] ? 2 : out[1] ? 1 : 0;
+    if (first > last) return 0;
+    PoolArgs a{q, k, v, qr, kr, vr, qc, kc, vc, blk_cnt, L, NB, R, G, Lr_pad, NBc_pad, first};
     cudaStream_t st = (cudaStream_t)stream;
     const int rows = max(max(NB, NBc_pad), (Lr_pad + G - 1) / G);
-    const dim3 grid(rows, BH, 3);
+    const dim3 grid(rows, BH, last - first + 1);
 #define POOL_CASE(TT, DD)                                                          \
     {                                                                              \
         if (R == 16) pool_kernel<TT, DD, 16><<<grid, DD / 2, 0, st>>>(a);          \
