@@ -895,7 +895,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     }
     // Fallback modes, one CTA per SM: every CTA finds the flagged tiles (a fraction of a percent of all, as a rule) and takes every
     // gridDim-th, counted in the order of the tile numbers so that the CTAs at work share a head's K and V in L2. All read all
-    // flags, 94 KB at 591 tiles x 40 heads, in coalesced loads, into a bit per tile in tile order: 2 us. A kernel of its own that made
+    // flags (of a range's heads), 94 KB at 591 tiles x 40 heads, in coalesced loads, into a bit per tile in tile order: 2 us. A kernel of its own that made
     // the list took 25 us there, 0.10 ms of a Wan-14B step, and 2.3 us and a launch at 4,152 tokens x 2 heads.
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint32_t* bits = reinterpret_cast<uint32_t*>(smem_raw + SMEM_MASS);       // the block masses' room: these modes have none
@@ -909,10 +909,11 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     for (int e0 = 0; e0 < total; e0 += step) {
         for (int w = tid; w < WALK_TILES / 32; w += NTHREADS) bits[w] = 0;
         __syncthreads();
+        const int h0 = e0 / a.nq, heads = (min(e0 + step, total) - 1) / a.nq - h0 + 1;     // the range's heads: one range, all of them
 #pragma unroll 8
-        for (int f = tid; f < total; f += NTHREADS) {
-            const int e = (f % a.H) * a.nq + f / a.H - e0;                   // flags are (tile, head), tile numbers head * nq + tile
-            if (__ldg(a.flags + f) != 0 && e >= 0 && e < step) atomicOr(bits + (e >> 5), 1u << (e & 31));
+        for (int f = tid; f < heads * a.nq; f += NTHREADS) {
+            const int qb = f / heads, h = h0 + f % heads, e = h * a.nq + qb - e0;          // flags are (tile, head), tile numbers head * nq + tile
+            if (__ldg(a.flags + (heads == a.H ? f : qb * a.H + h)) != 0 && e >= 0 && e < step) atomicOr(bits + (e >> 5), 1u << (e & 31));
         }
         __syncthreads();
         uint32_t w[PER];
@@ -937,12 +938,22 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         }
         // ranks blockIdx, blockIdx + grid, .. are this CTA's; the first of the range goes to mine[0]
         const int grid = gridDim.x, lead = ((int)blockIdx.x - found % grid + grid) % grid;
+        // (found by their rank: a division for every flagged tile was 3 us where all tiles of a short sequence are flagged)
+        if (n > 0) {
+            int skip = lead - (rank - found);                               // flagged tiles of this thread before the first of this CTA's
+            if (skip < 0) skip = (skip % grid + grid) % grid;
+            int slot = skip < n ? (rank - found + skip - lead) / grid : 0;
 #pragma unroll
-        for (int i = 0; i < PER; ++i)
-            for (uint32_t m = w[i]; m != 0; m &= m - 1, ++rank) {
-                const int at = rank - found - lead;
-                if (at >= 0 && at % grid == 0) mine[at / grid] = e0 + 32 * (tid * PER + i) + __ffs(m) - 1;
+            for (int i = 0; i < PER; ++i) {
+                uint32_t m = w[i];
+                for (int left = __popc(m); left > skip; skip = grid - 1) {
+                    for (left -= skip + 1; skip > 0; --skip) m &= m - 1;
+                    mine[slot++] = e0 + 32 * (tid * PER + i) + __ffs(m) - 1;
+                    m &= m - 1;
+                }
+                skip -= __popc(m);
             }
+        }
         __syncthreads();
         for (int t = 0; lead + t * grid < count; ++t) {
             if (attention_tile<MODE>(tmQ, tmK, tmV, tmKm, tmVm, tmKr, tmVr, a, mine[t], again, false) == TILE_STOP) return;
@@ -965,7 +976,8 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 // terms: 32,760 tokens x 12 heads 1.716e-3 / 1.682e-3 / 1.726e-3; 9,360 tokens of random q, k with logits of deviation 3.2
 // 1.821e-3 / 1.763e-3 / 2.017e-3. Time of the first shape, when this was chosen, 9.7 / 6.2 / 5.6 ms, of 1,560 tokens 95 / 56 / 46 us (one iteration in four
 // searched: 6.1 ms, but 1.95e-3 on the random rows).
-// Every half keeps its term however small its share: leaving those below 1 / 256 of the row rounded was no faster (6.89 ms, 6.84 so).
+// Every half keeps its term however small its share. Leaving those below 1 / 256 of the row rounded was no faster on the first shape
+// (6.89 ms, 6.84 so), on rows of logits with deviation 1, whose largest grows often, by 5 % (12,000 x 24 1.72 ms, 1.82 so).
 // (Flagged tiles, MODE 1, are those whose offset was far off, where a sample's maximum often is too: 0.81 ms of a Wan-14B step with
 // a sample first, 0.47 ms in two sweeps.)
 //
