@@ -780,7 +780,7 @@ __global__ void __launch_bounds__(128, GATE == 2 && D == 128 ? 10 : 12) fuse_fwd
 // delta_f = rowsum(dO O_f); dO_c = sum over the block's valid rows of w dO; delta_c = rowsum(dO_c O_c); dgate = act'(g) * (dO .
 // O_c) per token or per element; dout_f = dO on valid rows, else 0. One CTA per (block, bh), D / 8 lanes with 16 bytes each per
 // row, all of a lane's rows loaded before the first is used; the row groups' shares of dO_c are added in their order. Blocks
-// NB .. NBc_pad - 1 are the padding of dO_c and delta_c: zero. 32,768 tokens x 12 heads, D = 128, a gate per token: 96 us
+// NB .. NBc_pad - 1 are the padding of dO_c and delta_c: zero. 32,768 tokens x 12 heads, D = 128, a gate per token: 63 us
 // (149 us with a CTA-wide sum per row, 143 us with a warp per row and 8 bytes a lane: both bound by their instructions).
 template <typename T, int D, int GATE>
 __device__ __forceinline__ void fuse_bwd_rows(const FuseArgs& a, const int blk, const int bh, const int cnt, const uint32_t (&ow)[4],
@@ -849,7 +849,8 @@ __device__ __forceinline__ void fuse_bwd_rows(const FuseArgs& a, const int blk, 
 
 // Four CTAs per SM (64 registers), three with an elementwise gate at D = 128. 512 blocks x 12 heads, bf16, us, against one kernel for
 // all modes (99 registers at D = 128, two CTAs per SM): token gate 96 -> 63, none 62 -> 42, elementwise 94 -> 85 (four CTAs: 99);
-// at D = 64 39 -> 32 and, elementwise, 45 -> 43 (three: 48).
+// at D = 64 39 -> 32 and, elementwise, 45 -> 43 (three: 48). bf16 at D = 128 spills 50 (token) and 68 bytes (elementwise) a thread for
+// it.
 template <typename T, int D, int GATE>
 __global__ void __launch_bounds__(256, GATE == 2 && D == 128 ? 3 : 4) fuse_bwd_kernel(const FuseArgs a) {
     constexpr int LR = D / 8, GROUPS = 256 / LR;

@@ -21,9 +21,9 @@
 //
 // What bounds it: the hand-overs. The MMAs take 1,024 (768) clocks per two blocks at D = 128 and their operands 1,500 (1,150) of
 // shared memory's, of 3,300 (2,400) measured: a tile's load, its products, P / dS and the second products follow one another
-// with too few slots to have more than one and a half iterations on their way. 32,768 tokens x 12 heads, 32 blocks per list:
-// dK / dV 1.14 ms, dQ 0.85 ms (mma.sync: 2.27 and 1.68 ms); at D = 64 0.86 and 0.71 ms (1.29 and 0.91 ms), where M = D = 64
-// gradient products take half of the tensor pipe.
+// with too few slots to have more than one and a half iterations on their way. 32,768 tokens x 12 heads, 32 random blocks
+// per list, one launch after the other: dK / dV 1.12 ms, dQ 0.89 ms (mma.sync: 2.27 and 1.68 ms); at D = 64 0.84 and 0.71 ms (1.29 and
+// 0.91 ms), where M = D = 64 gradient products take half of the tensor pipe. In a training step, with routed lists: 1.19 and 0.91 ms.
 //
 // BWD_TIER_Q, BWD_REP: the three tiers of resolution, see the modes below. 512 blocks x 12 heads, 32 + 102 blocks in tiers A and B:
 // dQ 1.83 ms, tables 1.08 ms (mma.sync: 2.66 and 2.94 ms).
@@ -230,7 +230,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
 
     if (warp == 9 || warp == 10) {
         // ------------------------------------------------------------ loads: Y1, X1(i) by warp 9, Y2, X2(i) by warp 10 or, into one
-        // ring, all by warp 9. A tile's load is 600 clocks of a warp: with one warp for both dQ took 0.94 ms instead of 0.91; two
+        // ring, all by warp 9. A tile's load is 600 clocks of a warp: with one warp for both dQ took 0.94 ms of a training step instead of 0.91; two
         // warps into the one ring made dK / dV slower, 1.24 -> 1.285 ms.
         const int x_first = warp - 9, x_last = C::SHARED ? 1 : x_first;
         bool ok = *abort_flag == 0;
@@ -514,7 +514,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_consta
             fence_proxy_async_smem();
             mbar_arrive(smem_u32(&ctl->pfull));
         }
-        // the per-block gradients to add, on their way during the last products (fetched where they are added they cost a tile 1,500 clocks: dK / dV 1.24 -> 1.19 ms)
+        // the per-block gradients to add, on their way during the last products (fetched where they are added they cost a tile 1,500 clocks: dK / dV of a training step 1.24 -> 1.19 ms)
         float4 adds[KV ? 2 : 1];
         const float inv = 1.f / (float)cnt_o;
 #pragma unroll
